@@ -12,7 +12,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libsbp.so")
 SOURCES = ["driver.cu", "engine.cu", "blockmodel.cu", "nodal.cu", "merge.cu", "mergeapply.cu",
            "noalloc.cu", "server.cu", "ingest.cu", "host.cpp"]
-HEADERS = ["common.cuh", "kernels.h", "multi.cuh", "job.h", "engine.h"]
+HEADERS = ["common.cuh", "kernels.h", "multi.cuh", "dense.cuh", "job.h", "engine.h"]
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-lineinfo",
     "-gencode", "arch=compute_100a,code=sm_100a",

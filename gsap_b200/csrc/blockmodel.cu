@@ -585,7 +585,6 @@ struct BtArgs {
   const double *ld_out, *ld_in;
   double *dSout, *ambout, *ambin, *sinfull;
   int32_t* nbr_s;
-  uint8_t* use_rand;
   const int32_t* ctl;  // sweep control: gate, and seq += ctl[0] * seq_mul
   int32_t B;
   int draws;
@@ -672,10 +671,7 @@ struct BlockTermsBody {
         int c = warp_pick_row(a, b, scale_draw(x.v[1], deg), lane);
         nb = c >= 0 ? c : 0;
       }
-      if (lane == 0) {
-        a.use_rand[b] = accept_random(x.v[0], deg, (uint64_t)a.B) ? 1 : 0;
-        a.nbr_s[b] = nb;
-      }
+      if (lane == 0) a.nbr_s[b] = accept_random(x.v[0], deg, (uint64_t)a.B) ? -1 : nb;
     }
   }
   }
@@ -971,7 +967,6 @@ struct BtDenseArgs {
   const double *ld_out, *ld_in;
   double *dSout, *ambout, *ambin, *sinfull;
   int32_t* nbr_s;
-  uint8_t* use_rand;
   const int32_t* ctl;  // sweep control: gate, and seq += ctl[0] * seq_mul
   int32_t B;
   int draws;
@@ -1006,8 +1001,7 @@ struct BlockTermsDenseBody {
     }
     }
     if (a.draws)
-      dense_block_draw(a.Md, a.MTd, a.Sd, a.d_out, a.d_in, B, a.seed, seq, b, lane, a.nbr_s,
-                       a.use_rand);
+      dense_block_draw(a.Md, a.MTd, a.Sd, a.d_out, a.d_in, B, a.seed, seq, b, lane, a.nbr_s);
   }
   }
 };
@@ -1186,7 +1180,7 @@ BtArgs bt_args(DevBM& m, int32_t B, int draws, uint64_t seed, uint32_t seq) {
   a.ocnt = m.ocnt; a.icnt = m.icnt; a.d_out = m.d_out; a.d_in = m.d_in;
   a.ld_out = m.ld_out; a.ld_in = m.ld_in;
   a.dSout = m.dSout; a.ambout = m.ambout; a.ambin = m.ambin; a.sinfull = m.sinfull;
-  a.nbr_s = m.nbr_s; a.use_rand = m.use_rand;
+  a.nbr_s = m.nbr_s;
   a.B = B; a.draws = draws; a.seed = seed; a.seq = seq;
   return a;
 }
@@ -1197,7 +1191,7 @@ BtDenseArgs bt_dense_args(DevBM& m, int32_t B, int draws, uint64_t seed, uint32_
   a.Md = m.Md; a.MTd = m.MTd; a.Sd = m.Sd; a.d_out = m.d_out; a.d_in = m.d_in;
   a.ld_out = m.ld_out; a.ld_in = m.ld_in;
   a.dSout = m.dSout; a.ambout = m.ambout; a.ambin = m.ambin; a.sinfull = m.sinfull;
-  a.nbr_s = m.nbr_s; a.use_rand = m.use_rand;
+  a.nbr_s = m.nbr_s;
   a.B = B; a.draws = draws; a.seed = seed; a.seq = seq;
   return a;
 }

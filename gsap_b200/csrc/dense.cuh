@@ -48,15 +48,15 @@ __device__ __forceinline__ int warp_pick_chunked(const uint32_t* orow, const uin
 }
 
 // Block b's draws for the batch with RNG sequence seq (choose_neighbored_block
-// and the per-block uniform, kernels.hpp:942-997, 1024): whether a proposal
-// from b takes a uniform random block (use_rand), else the block of a
-// neighbour drawn by weight from b's out-row ++ in-row (nbr_s).  The whole
-// warp calls it; lane 0 writes.
+// and the per-block uniform, kernels.hpp:942-997, 1024) into nbr_s[b]: -1
+// when a proposal from b takes a uniform random block, else the block of a
+// neighbour drawn by weight from b's out-row ++ in-row.  The whole warp calls
+// it; lane 0 writes.
 __device__ __forceinline__ void dense_block_draw(const uint32_t* Md, const uint32_t* MTd,
                                                  const uint32_t* Sd, const uint32_t* d_out,
                                                  const uint32_t* d_in, int32_t B, uint64_t seed,
-                                                 uint32_t seq, int b, int lane, int32_t* nbr_s,
-                                                 uint8_t* use_rand) {
+                                                 uint32_t seq, int b, int lane,
+                                                 int32_t* nbr_s) {
   const P4 x = draw(seed, kRngNodalBlock, seq, (uint32_t)b);
   const uint64_t deg = (uint64_t)d_out[b] + d_in[b];
   int nb = 0;
@@ -66,10 +66,7 @@ __device__ __forceinline__ void dense_block_draw(const uint32_t* Md, const uint3
                                     Sd + (size_t)b * 2 * K, B, K, scale_draw(x.v[1], deg), lane);
     nb = c >= 0 ? c : 0;
   }
-  if (lane == 0) {
-    use_rand[b] = accept_random(x.v[0], deg, (uint64_t)B) ? 1 : 0;
-    nbr_s[b] = nb;
-  }
+  if (lane == 0) nbr_s[b] = accept_random(x.v[0], deg, (uint64_t)B) ? -1 : nb;
 }
 
 }  // namespace sbp

@@ -164,7 +164,7 @@ size_t job_bytes(int32_t N, int32_t E, int32_t np, int32_t max_itr, int32_t dens
   // blockmodel
   add(n1, 4); add(n1, 4); add(e, 4); add(e, 4); add(e, 4); add(e, 4); add(N, 4); add(N, 4);
   for (int i = 0; i < 6; ++i) add(N, 8);
-  add(N, 4); add(N, 1);
+  add(N, 4);
   // rebuild scratch
   for (int d = 0; d < 2; ++d) {
     add(n1, 4); add(n1, 4); add(N, 4); add(e, 4); add(e, 4); add(e, 4); add(e, 4); add(n1, 4);
@@ -306,7 +306,7 @@ sbp_status job_create(Job& J, int device, int32_t N, int32_t E, int32_t np, int3
   m.ld_out = A.take<double>(N); m.ld_in = A.take<double>(N);
   m.dSout = A.take<double>(N); m.ambout = A.take<double>(N);
   m.ambin = A.take<double>(N); m.sinfull = A.take<double>(N);
-  m.nbr_s = A.take<int32_t>(N); m.use_rand = A.take<uint8_t>(N);
+  m.nbr_s = A.take<int32_t>(N);
   for (int d = 0; d < 2; ++d) {
     RebuildDir& r = J.rs.d[d];
     r.cnt = A.take<int32_t>(n1); r.seg = A.take<int32_t>(n1); r.vofs = A.take<int32_t>(N);
@@ -590,15 +590,15 @@ bool heavy_vertex(const Job& J, int32_t v) {
 }
 
 void classify_batch(const Job& J, const int32_t* verts, int32_t lo, int32_t count,
-                    std::vector<int32_t>& out, int32_t n[3]) {
+                    std::vector<int32_t>& out, int32_t n[kListCounts]) {
   const size_t at = out.size();
   out.resize(at + (size_t)std::max(count, 0));
   int32_t* o = out.data() + at;
-  n[0] = n[1] = n[2] = 0;
+  std::fill(n, n + kListCounts, 0);
   if (count <= 0) return;
   // The kernels run their items in list order, the larger vertices first: a
   // longest-first schedule, so that a launch does not end on a tail of its
-  // slowest items (10% of a 200k partition), and small vertices paired with
+  // slowest items (10% of a 200k partition), and vertices share a warp with
   // ones of about their size.  Each class is ordered by entry count, largest
   // first, ties by batch index (a counting sort: the small and mid classes
   // have at most 2 * kWarpList entries); a vertex's result does not depend on
@@ -612,6 +612,7 @@ void classify_batch(const Job& J, const int32_t* verts, int32_t lo, int32_t coun
     ent[i] = e;
     cls[i] = heavy_vertex(J, v) ? 2 : e <= kSmallEntries ? 0 : 1;
     ++n[cls[i]];
+    if (cls[i] == 1 && e > kGroupEntries / 2) ++n[e > kGroupEntries ? 3 : 4];
     if (cls[i] < 2) emax = std::max(emax, e);
   }
   std::vector<int32_t> start((size_t)emax + 2, 0);
@@ -633,12 +634,14 @@ void classify_batch(const Job& J, const int32_t* verts, int32_t lo, int32_t coun
   std::stable_sort(h, h + nh, [&](int32_t x, int32_t y) { return ent[x] > ent[y]; });
 }
 
-NodalAux nodal_lists(Job& J, const int32_t* dev, const int32_t n[3]) {
+NodalAux nodal_lists(Job& J, const int32_t* dev, const int32_t n[kListCounts]) {
   NodalAux a;
   a.small = dev;
   a.nsmall = n[0];
   a.mid = dev + n[0];
   a.nmid = n[1];
+  a.nlarge = n[3];
+  a.nmid64 = n[4];
   a.heavy = dev + n[0] + n[1];
   a.nheavy = n[2];
   a.err = J.err;
@@ -1107,7 +1110,7 @@ sbp_status sbp_delta_mdl_nodal_mode(const sbp_graph_csr* g, const int32_t* part,
   cudaMemcpyAsync(dv, verts, 4 * (size_t)nv, cudaMemcpyHostToDevice, J.st);
   cudaMemcpyAsync(dp, props, 4 * (size_t)nv, cudaMemcpyHostToDevice, J.st);
   std::vector<int32_t> lists;
-  int32_t ln[3];
+  int32_t ln[kListCounts];
   classify_batch(J, verts, 0, nv, lists, ln);
   if (!lists.empty())
     cudaMemcpyAsync(J.lists, lists.data(), 4 * lists.size(), cudaMemcpyHostToDevice, J.st);
@@ -1191,7 +1194,7 @@ sbp_status sbp_nodal_batch_mode(const sbp_graph_csr* g, int32_t* part, int32_t B
   if (s != SBP_OK) return s;
   int32_t cnt = hi - lo;
   std::vector<int32_t> lists;
-  int32_t ln[3];
+  int32_t ln[kListCounts];
   classify_batch(J, nullptr, lo, cnt, lists, ln);
   if (!lists.empty())
     SBP_CUDA(cudaMemcpyAsync(J.lists, lists.data(), 4 * lists.size(), cudaMemcpyHostToDevice,

@@ -44,12 +44,12 @@ void Run::setup_batches() {
   batch_entries.assign(nb, 0.0);
   lists_all.clear();
   list_off.assign(nb + 1, 0);
-  list_n.assign(3 * (size_t)nb, 0);
+  list_n.assign(kListCounts * (size_t)nb, 0);
   for (int32_t b = 0; b < nb; ++b) {
     int32_t lo = b * BS, hi = (b + 1) * BS;
     batch_entries[b] = (double)(J->h_optr[hi] - J->h_optr[lo]) +
                        (double)(J->h_iptr[hi] - J->h_iptr[lo]);
-    classify_batch(*J, nullptr, lo, BS, lists_all, &list_n[3 * (size_t)b]);
+    classify_batch(*J, nullptr, lo, BS, lists_all, &list_n[kListCounts * (size_t)b]);
     list_off[b + 1] = (int32_t)lists_all.size();
   }
 }
@@ -368,7 +368,7 @@ void Engine::add_run_work(Run& r) {
         const int ms = md.slot(dense);
         add_nodal(s.nodal[ms], s.heavy[ms], dense, md, J.g, J.part, J.m, r.B, r.o.seed, seq, lo,
                   r.BS, J.newlab, J.rec, nullptr,
-                  nodal_lists(J, J.lists + r.list_off[b], &r.list_n[3 * (size_t)b]), ctl, nb);
+                  nodal_lists(J, J.lists + r.list_off[b], &r.list_n[kListCounts * (size_t)b]), ctl, nb);
         if (dense) {
           // the moved vertices' edges, applied to the dense form before the
           // labels change (it reads old and new labels)

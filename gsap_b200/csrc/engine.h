@@ -53,7 +53,7 @@ struct Run {
   double S = 0.0;
   std::vector<double> itr_dS;
   // per batch b, vertices by nodal kernel path (classify_batch): groups of
-  // sizes list_n[3b .. 3b+2] starting at list_off[b] in lists_all
+  // sizes list_n[kListCounts * b ..] starting at list_off[b] in lists_all
   std::vector<int32_t> lists_all, list_off, list_n;
   std::vector<double> batch_entries;
   double nnz_now = 0.0;

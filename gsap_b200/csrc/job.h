@@ -132,11 +132,13 @@ inline ScoreMode score_mode(const sbp_options& o) {
 bool heavy_vertex(const Job& J, int32_t v);
 // Appends the batch indices i in [0, count) of vertices lo + i (verts[i]
 // when verts is given) to `out`, grouped by nodal kernel path: small, mid,
-// heavy (NodalAux); n[k] receives the group sizes.
+// heavy (NodalAux); n receives the three group sizes and the mid list's
+// counts of large vertices and of those of up to kGroupEntries entries.
+constexpr int kListCounts = 5;
 void classify_batch(const Job& J, const int32_t* verts, int32_t lo, int32_t count,
-                    std::vector<int32_t>& out, int32_t n[3]);
-// The NodalAux of groups of sizes n[3] stored back to back at `dev`.
-NodalAux nodal_lists(Job& J, const int32_t* dev, const int32_t n[3]);
+                    std::vector<int32_t>& out, int32_t n[kListCounts]);
+// The NodalAux of groups of such sizes stored back to back at `dev`.
+NodalAux nodal_lists(Job& J, const int32_t* dev, const int32_t n[kListCounts]);
 sbp_status check_options(const sbp_options* o);
 
 struct Timer {

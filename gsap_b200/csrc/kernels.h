@@ -33,8 +33,8 @@ struct DevBM {
   double *ambout = nullptr;   // sum over out-row b of M log2 M - M log2 d_in[c]
   double *ambin = nullptr;    // sum over in-row b of M log2 M - M log2 d_out[c]
   double *sinfull = nullptr;  // ambin[b] - d_in[b] log2 d_in[b]
-  int32_t* nbr_s = nullptr;   // per-block second-hop sample of a nodal batch
-  uint8_t* use_rand = nullptr;
+  int32_t* nbr_s = nullptr;   // per-block draw of a nodal batch: second-hop block, or -1 for a
+                              // uniform proposal
   // dense form for small B: Md[r*B + c] = M[r][c], MTd[c*B + r] = M[r][c]
   uint32_t* Md = nullptr;
   uint32_t* MTd = nullptr;
@@ -330,17 +330,18 @@ cudaError_t init_nodal_attributes();
 // CTA-per-vertex kernel.
 int nodal_heavy_threshold();
 
-// A batch's vertices (indices into the batch) by kernel path: small ones
-// (at most kSmallEntries neighbour entries) go two to a warp, mid ones one to
-// a warp, heavy ones (more than nodal_heavy_threshold() entries in a
-// direction) one to a CTA on the side stream.  err counts hash-table
-// overflows (should stay 0).
-constexpr int32_t kSmallEntries = 16;
+// A batch's vertices (indices into the batch) by kernel path: small ones (at
+// most kSmallEntries neighbour entries), mid ones, and heavy ones (more than
+// nodal_heavy_threshold() entries in a direction), one to a CTA on the side
+// stream.  The mid list runs from the most entries down: the first nlarge
+// have more than kGroupEntries, the next nmid64 more than kGroupEntries / 2.
+// err counts hash-table overflows (should stay 0).
+constexpr int32_t kSmallEntries = 16, kGroupEntries = 64;
 struct NodalAux {
   const int32_t* small = nullptr;
   int32_t nsmall = 0;
   const int32_t* mid = nullptr;
-  int32_t nmid = 0;
+  int32_t nmid = 0, nlarge = 0, nmid64 = 0;
   const int32_t* heavy = nullptr;
   int32_t nheavy = 0;
   int32_t* err = nullptr;

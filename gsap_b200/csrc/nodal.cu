@@ -5,21 +5,18 @@
 // thread walk a whole blockmodel row in a serial sorted merge with the
 // vertex's sorted neighbour-block list (kernels.hpp:494-597, 1153-1726).
 //
-// Here a group of threads owns one vertex: half a warp for vertices of at
-// most kSmallEntries neighbour entries (two per warp), a warp for the other
-// ordinary vertices, a whole CTA for the few with more than kWarpList
-// neighbours in a direction (run on a second stream next to the warp
-// kernel).  The host sorts each batch's vertices into these three lists
-// once per job.
+// Here a group of threads owns one vertex: 8, 16 or 32 lanes for vertices of
+// up to 16, 32 or 64 neighbour entries (two entries a lane), a CTA of four
+// warps for up to kWarpList entries a direction, a larger CTA for the few
+// heavier ones (run on a second stream next to the warp kernel).  The host
+// sorts each batch's vertices into these lists once per job.
 //   * proposal: Philox draws, an exact integer inverse-CDF pick of a
-//     neighbour (a prefix scan over the group's lanes, out- then
-//     in-entries), then the per-block draws of the batch
-//     (kernels.hpp:877-1032);
-//   * neighbour blocks grouped per distinct block: in registers with
-//     __match_any_sync / __reduce_add_sync when a list fits the lane group,
-//     else in a per-warp shared-memory hash table (up to kWarpHashEntries),
-//     else sorted in shared memory (bitonic), else hashed in shared memory in
-//     passes; GSAP sorts all E entries every batch;
+//     neighbour (out- then in-entries; with unit weights the drawn number is
+//     the entry's index, else a prefix scan), then the per-block draws of the
+//     batch (kernels.hpp:877-1032);
+//   * neighbour blocks grouped per distinct block by comparing keys in shared
+//     memory, or (heavy vertices) in a shared-memory hash table; GSAP sorts
+//     all E entries every batch;
 //   * dS: GSAP's seven terms rewritten as "changed cells + row degrees".
 //     A row term  sum_c f(x_c)  with  f(x) = x (log2 x - log2 dcol[c] - L)
 //     splits into  sum_c (x log2 x - x log2 dcol[c])  -  L * sum_c x ;
@@ -41,6 +38,8 @@
 #include "multi.cuh"
 #include "dense.cuh"
 
+#include <type_traits>
+
 namespace sbp {
 
 namespace {
@@ -48,9 +47,7 @@ namespace {
 constexpr int kNodalWarps = 4;
 constexpr int kWarpList = 128;     // entries per direction a warp sorts in shared memory
 constexpr int kHeavyThreads = 256;
-constexpr int kHashSlotsCfg = 8192;
-// the heavy path's hash table: key, sum, first
-constexpr size_t kHeavySmem = 3 * kHashSlotsCfg * sizeof(int32_t);
+constexpr int kHashSlots = 8192;  // of the heavy path's table
 
 struct NodalArgs {
   const double* xlx;        // x log2 x table
@@ -62,7 +59,6 @@ struct NodalArgs {
   const uint32_t *Md, *MTd;
   const double *ld_out, *ld_in;
   const int32_t* nbr_s;
-  const uint8_t* use_rand;
   int32_t B;
   uint64_t seed;
   uint32_t seq;
@@ -75,8 +71,9 @@ struct NodalArgs {
   double* dS_raw;
   const int32_t* heavy;     // batch indices handled by the CTA kernel
   int32_t nheavy;
-  const int32_t *small, *mid;  // batch indices of the warp kernel: two small ones per warp,
-  int32_t nsmall, nmid;        // one mid one per warp
+  const int32_t *small, *mid;  // batch indices of the warp kernel (NodalItems)
+  int32_t nsmall, nmid;
+  int32_t nlarge, nmid64;      // mid vertices by size: large, up to kGroupEntries, the others
   int32_t* err;             // error counter (hash table overflow)
   const int32_t* ctl;       // sweep control: gate, and seq += ctl[0] * seq_mul
   uint32_t seq_mul;
@@ -88,7 +85,7 @@ struct NodalArgs {
 
 // g(x, a) = x log2 x - x a, zero for x == 0
 __device__ __forceinline__ double gterm(const double* tab, uint32_t x, double a) {
-  return x == 0u ? 0.0 : xlx(tab, x) - (double)x * a;
+  return x == 0u ? 0.0 : __fma_rn(-(double)x, a, xlx(tab, x));
 }
 
 // The four rows a move from r to s reads: out-rows r and s, in-rows r and s.
@@ -181,63 +178,100 @@ __device__ __forceinline__ void entry(const NodalArgs& a, const Rows<DENSE>& R, 
   }
 }
 
-// Adds the corner cells (r,r), (r,s), (s,r), (s,s) of M and the row-degree
-// terms to lanes 0..12 of the calling lane group (lane `lane` of the group
-// starting at warp lane hb; a warp, or a half-warp with its own vertex; call
-// it from one warp of a CTA group, after m4..m7 hold the group totals).
-// kernels.hpp:1506-1510, 1573-1578, 1663-1669, 1718-1723 give the new
-// corner counts.
+// Group sums of the four direction weights v has to/from blocks r and s.
+struct RsWeights {
+  uint32_t koR, koS, niR, niS;
+};
+
+// What the corner cells (r,r), (r,s), (s,r), (s,s) of M and the row-degree
+// terms of a move are made from.
+struct Corner {
+  uint32_t Mrr, Mrs, Msr, Mss;
+  uint32_t dor, dos, dir, dis;  // old block degrees
+  double ldo_r, ldo_s, ldi_r, ldi_s;
+  uint32_t kO, kI;              // v's degrees
+};
+
+__device__ __forceinline__ void load_degrees(const NodalArgs& a, int v, int r, int s, Corner& q) {
+  q.kO = a.kdo[v];
+  q.kI = a.kdi[v];
+  q.dor = a.d_out[r];
+  q.dos = a.d_out[s];
+  q.dir = a.d_in[r];
+  q.dis = a.d_in[s];
+  q.ldi_r = a.ld_in[r];
+  q.ldi_s = a.ld_in[s];
+  q.ldo_r = a.ld_out[r];
+  q.ldo_s = a.ld_out[s];
+}
+
+// Term `k` (0..12) of a move's corner and degree terms, 0 for other k; m4..m7
+// are the count changes of the new out-row r, out-row s, in-row r and in-row
+// s away from the corners.  Terms 0-3: the old corner cells, + M log2 M; 4-7:
+// the new corner cells, - g(x); 8-11: + L mass of the four new rows; 12: the
+// old row degrees.  kernels.hpp:1506-1510, 1573-1578, 1663-1669, 1718-1723
+// give the new corner counts.  Straight-line, no lane branches: every lane
+// evaluates the cell form and the row form of its operands and keeps the one
+// its k owns (CELLS / ROWS leave a form out where no lane of a call owns it).
+template <bool CELLS, bool ROWS>
+__device__ __forceinline__ double corner_term(const double* tab, const Corner& q,
+                                              const RsWeights& w, int m4, int m5, int m6, int m7,
+                                              int k) {
+  const uint32_t xrr = q.Mrr - w.koR - w.niR;
+  const uint32_t xrs = q.Mrs != 0u ? q.Mrs - w.koS + w.niR : w.niR;
+  const uint32_t xsr = q.Msr + w.koR - w.niS;
+  const uint32_t xss = q.Mss != 0u ? q.Mss + w.koS + w.niS : w.niS;
+  const bool use_rs = q.Mrs != 0u || w.niR > 0u;                       // cell or extra term
+  const bool use_ss = q.Mss != 0u || (w.koS == 0u && w.niS > 0u);
+  const int j = k & 3;
+  double t = 0.0;
+  if (CELLS) {
+    const uint32_t Mold = j == 0 ? q.Mrr : j == 1 ? q.Mrs : j == 2 ? q.Msr : q.Mss;
+    const uint32_t xnew = j == 0 ? xrr : j == 1 ? xrs : j == 2 ? xsr : xss;
+    const bool on = j == 0 ? q.Mrr != 0u : j == 1 ? use_rs : j == 2 ? q.Msr != 0u : use_ss;
+    const double ld = (j & 1) ? q.ldi_s : q.ldi_r;
+    const bool old_cell = k < 4;
+    const uint32_t X = old_cell ? Mold : xnew;
+    const bool cell_on = old_cell ? Mold != 0u : on;
+    const double cell = old_cell ? xlx(tab, X) : -gterm(tab, X, ld);
+    if (k < 8) t = cell_on ? cell : 0.0;
+  }
+  if (ROWS) {
+    const long long l4 = m4 + (q.Mrr ? (long long)xrr - q.Mrr : 0) +
+                         (use_rs ? (long long)xrs - (long long)q.Mrs : 0);
+    const long long l5 = m5 + (q.Msr ? (long long)xsr - q.Msr : 0) +
+                         (use_ss ? (long long)xss - (long long)q.Mss : 0);
+    const long long mass4 = (long long)q.dor + l4;
+    const long long mass5 = (long long)q.dos + l5;
+    const long long mass6 = (long long)q.dir - (long long)q.Mrr - (long long)q.Msr + m6;
+    const long long mass7 = (long long)q.dis - (long long)q.Mrs - (long long)q.Mss + m7;
+    const long long mass = j == 0 ? mass4 : j == 1 ? mass5 : j == 2 ? mass6 : mass7;
+    const uint32_t d =
+        j == 0 ? q.dor - q.kO : j == 1 ? q.dos + q.kO : j == 2 ? q.dir - q.kI : q.dis + q.kI;
+    const double row = mass != 0 ? l2x(tab, d) * (double)mass : 0.0;
+    const double deg =
+        -((q.dor ? (double)q.dor * q.ldo_r : 0.0) + (q.dos ? (double)q.dos * q.ldo_s : 0.0) +
+          (q.dir ? (double)q.dir * q.ldi_r : 0.0) + (q.dis ? (double)q.dis * q.ldi_s : 0.0));
+    if (k >= 8 && k < 12) t = row;
+    else if (k == 12) t = deg;
+  }
+  return t;
+}
+
+// Adds the corner and degree terms to lanes 0..12 of the calling warp (after
+// m4..m7 hold the group totals; call it from one warp of a CTA group).
 template <bool DENSE>
 __device__ __forceinline__ void corner_terms(const NodalArgs& a, const Rows<DENSE>& R, int v,
-                                             int r, int s, uint32_t koR, uint32_t koS,
-                                             uint32_t niR, uint32_t niS, Acc& q, int lane,
-                                             int hb) {
+                                             int r, int s, const RsWeights& w, Acc& q, int lane) {
   // lane 0: M[r][r], 1: M[r][s], 2: M[s][r], 3: M[s][s]
   const uint32_t mm = lane < 4 ? R.out_at((lane & 2) != 0, (lane & 1) ? s : r) : 0u;
-  const uint32_t Mrr = __shfl_sync(kFull, mm, hb), Mrs = __shfl_sync(kFull, mm, hb + 1);
-  const uint32_t Msr = __shfl_sync(kFull, mm, hb + 2), Mss = __shfl_sync(kFull, mm, hb + 3);
-  const uint32_t xrr = Mrr - koR - niR;
-  const uint32_t xrs = Mrs != 0u ? Mrs - koS + niR : niR;
-  const uint32_t xsr = Msr + koR - niS;
-  const uint32_t xss = Mss != 0u ? Mss + koS + niS : niS;
-  const bool use_rs = Mrs != 0u || niR > 0u;                       // cell or extra term
-  const bool use_ss = Mss != 0u || (koS == 0u && niS > 0u);
-  const long long m4 = q.m4 + (Mrr ? (long long)xrr - Mrr : 0) +
-                       (use_rs ? (long long)xrs - (long long)Mrs : 0);
-  const long long m5 = q.m5 + (Msr ? (long long)xsr - Msr : 0) +
-                       (use_ss ? (long long)xss - (long long)Mss : 0);
-  const uint32_t kO = a.kdo[v], kI = a.kdi[v];
-  const uint32_t dor = a.d_out[r], dos = a.d_out[s], dir = a.d_in[r], dis = a.d_in[s];
-  const long long mass4 = (long long)dor + m4;
-  const long long mass5 = (long long)dos + m5;
-  const long long mass6 = (long long)dir - (long long)Mrr - (long long)Msr + q.m6;
-  const long long mass7 = (long long)dis - (long long)Mrs - (long long)Mss + q.m7;
-  const double ldi_r = a.ld_in[r], ldi_s = a.ld_in[s];
-  const double ldo_r = a.ld_out[r], ldo_s = a.ld_out[s];
-  // Straight-line, no lane branches: every lane evaluates the cell form and
-  // the row form of its operands and keeps the one its lane range owns.
-  // lanes 0-3: old corner cells, + M log2 M; lanes 4-7: new corner cells,
-  // - g(x); lanes 8-11: + L mass of the four new rows; lane 12: the old row
-  // degrees.
-  const int j = lane & 3;
-  const uint32_t Mold = j == 0 ? Mrr : j == 1 ? Mrs : j == 2 ? Msr : Mss;
-  const uint32_t xnew = j == 0 ? xrr : j == 1 ? xrs : j == 2 ? xsr : xss;
-  const bool on = j == 0 ? Mrr != 0u : j == 1 ? use_rs : j == 2 ? Msr != 0u : use_ss;
-  const double ld = (j & 1) ? ldi_s : ldi_r;
-  const bool old_cell = lane < 4;
-  const uint32_t X = old_cell ? Mold : xnew;
-  const bool cell_on = old_cell ? Mold != 0u : on;
-  const double cell = old_cell ? xlx(a.xlx, X) : -gterm(a.xlx, X, ld);
-  const long long mass = j == 0 ? mass4 : j == 1 ? mass5 : j == 2 ? mass6 : mass7;
-  const uint32_t d = j == 0 ? dor - kO : j == 1 ? dos + kO : j == 2 ? dir - kI : dis + kI;
-  const double row = mass != 0 ? l2x(a.xlx, d) * (double)mass : 0.0;
-  const double deg = -((dor ? (double)dor * ldo_r : 0.0) + (dos ? (double)dos * ldo_s : 0.0) +
-                       (dir ? (double)dir * ldi_r : 0.0) + (dis ? (double)dis * ldi_s : 0.0));
-  double t = 0.0;
-  if (lane < 8) t = cell_on ? cell : 0.0;
-  else if (lane < 12) t = row;
-  else if (lane == 12) t = deg;
-  q.acc += t;
+  Corner c;
+  c.Mrr = __shfl_sync(kFull, mm, 0);
+  c.Mrs = __shfl_sync(kFull, mm, 1);
+  c.Msr = __shfl_sync(kFull, mm, 2);
+  c.Mss = __shfl_sync(kFull, mm, 3);
+  load_degrees(a, v, r, s, c);
+  q.acc += corner_term<true, true>(a.xlx, c, w, q.m4, q.m5, q.m6, q.m7, lane);
 }
 
 // A thread group cooperating on one vertex: a warp (G = 32) or a CTA.
@@ -305,153 +339,10 @@ __device__ void stage_sorted(const int32_t* __restrict__ idx, const uint32_t* __
   group_sort<G>(key, P, grp);
 }
 
-// Group sums of the four direction weights v has to/from blocks r and s.
-struct RsWeights {
-  uint32_t koR, koS, niR, niS;
-};
-
-// Finishes a move's dS after every thread of the group has added its
-// entries to q: group totals of the count changes, then the corner and
-// degree terms on warp 0, then the group sum.
-template <bool DENSE, int G>
-__device__ double finish(const NodalArgs& a, const Rows<DENSE>& R, int v, int r, int s,
-                         const RsWeights& w, Acc q, const Group<G>& grp) {
-  q.m4 = (int)grp.sum_ll(q.m4);
-  q.m5 = (int)grp.sum_ll(q.m5);
-  q.m6 = (int)grp.sum_ll(q.m6);
-  q.m7 = (int)grp.sum_ll(q.m7);
-  if (G == 32 || threadIdx.x < 32)
-    corner_terms<DENSE>(a, R, v, r, s, w.koR, w.koS, w.niR, w.niS, q, threadIdx.x & 31, 0);
-  return grp.sum(q.acc);
-}
-
-// dS from v's sorted neighbour-block lists ko[0..no) (out), ki[0..ni) (in).
-template <bool DENSE, int G>
-__device__ double delta_sorted(const NodalArgs& a, int v, int r, int s,
-                               const unsigned long long* ko, int no,
-                               const unsigned long long* ki, int ni, const Group<G>& grp) {
-  const int t = grp.rank();
-  const Rows<DENSE> R(a, r, s);
-  uint32_t koR = 0, koS = 0, niR = 0, niS = 0;
-  for (int k = t; k < no; k += G) {
-    int32_t c = kblk(ko[k]);
-    koR += c == r ? kwt(ko[k]) : 0u;
-    koS += c == s ? kwt(ko[k]) : 0u;
-  }
-  for (int k = t; k < ni; k += G) {
-    int32_t c = kblk(ki[k]);
-    niR += c == r ? kwt(ki[k]) : 0u;
-    niS += c == s ? kwt(ki[k]) : 0u;
-  }
-  RsWeights w{(uint32_t)grp.sum_ll(koR), (uint32_t)grp.sum_ll(koS), (uint32_t)grp.sum_ll(niR),
-              (uint32_t)grp.sum_ll(niS)};
-  Acc q;
-  for (int k = t; k < no; k += G) {
-    const int32_t c = kblk(ko[k]);
-    const bool leader = k == 0 || kblk(ko[k - 1]) != c;
-    uint32_t kc = 0;
-    if (leader)
-      for (int j = k; j < no && kblk(ko[j]) == c; ++j) kc += kwt(ko[j]);
-    entry<DENSE>(a, R, r, s, w.niS, false, c, kwt(ko[k]), leader, kc, q);
-  }
-  for (int k = t; k < ni; k += G) {
-    const int32_t c = kblk(ki[k]);
-    const bool leader = k == 0 || kblk(ki[k - 1]) != c;
-    uint32_t kc = 0;
-    if (leader)
-      for (int j = k; j < ni && kblk(ki[j]) == c; ++j) kc += kwt(ki[j]);
-    entry<DENSE>(a, R, r, s, w.niS, true, c, kwt(ki[k]), leader, kc, q);
-  }
-  return finish<DENSE, G>(a, R, v, r, s, w, q, grp);
-}
-
-// dS from the warp's entries, one per lane and pass (see delta_registers).
-template <bool DENSE>
-__device__ __forceinline__ double delta_from_entries(const NodalArgs& a, const Rows<DENSE>& R,
-                                                     int v, int r, int s, int passes,
-                                                     const int32_t* cs, const uint32_t* ws,
-                                                     const bool* ins, const bool* valid,
-                                                     int lane) {
-  Acc q;
-  RsWeights w{0u, 0u, 0u, 0u};
-#pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    if (passes == 1 && p == 1) break;
-    const bool o = valid[p] && !ins[p], i = valid[p] && ins[p];
-    w.koR += __reduce_add_sync(kFull, o && cs[p] == r ? ws[p] : 0u);
-    w.koS += __reduce_add_sync(kFull, o && cs[p] == s ? ws[p] : 0u);
-    w.niR += __reduce_add_sync(kFull, i && cs[p] == r ? ws[p] : 0u);
-    w.niS += __reduce_add_sync(kFull, i && cs[p] == s ? ws[p] : 0u);
-  }
-#pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    if (passes == 1 && p == 1) break;
-    // direction in the top bit, unique keys for idle lanes
-    const unsigned key = valid[p] ? ((unsigned)cs[p] | (ins[p] ? 0x80000000u : 0u))
-                                  : (0x7fffffe0u + (unsigned)lane);
-    const unsigned peers = __match_any_sync(kFull, key);
-    const uint32_t kc = __reduce_add_sync(peers, ws[p]);
-    if (valid[p])
-      entry<DENSE>(a, R, r, s, w.niS, ins[p], cs[p], ws[p], lane == __ffs(peers) - 1, kc, q);
-  }
-  q.m4 = __reduce_add_sync(kFull, q.m4);
-  q.m5 = __reduce_add_sync(kFull, q.m5);
-  q.m6 = __reduce_add_sync(kFull, q.m6);
-  q.m7 = __reduce_add_sync(kFull, q.m7);
-  corner_terms<DENSE>(a, R, v, r, s, w.koR, w.koS, w.niR, w.niS, q, lane, 0);
-  return warp_sum(q.acc);
-}
-
-// dS when each direction's list fits in one warp: entries of the same block
-// are grouped with __match_any_sync on a direction-tagged key and their
-// weights summed with __reduce_add_sync.  When both lists fit together,
-// one pass covers both directions.
-template <bool DENSE>
-__device__ double delta_registers(const NodalArgs& a, int v, int r, int s, int32_t o0, int no,
-                                  int32_t i0, int ni, int lane) {
-  const Rows<DENSE> R(a, r, s);
-  const int passes = no + ni <= 32 ? 1 : 2;
-  // pass p, lane l: entry index e; combined pass: out-entries then in-entries
-  int32_t cs[2];
-  uint32_t ws[2];
-  bool ins[2], valid[2];
-#pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    int k;
-    bool in;
-    if (passes == 1 && p == 1) {
-      valid[1] = false;
-      ins[1] = false;
-      cs[1] = -1;
-      ws[1] = 0u;
-      break;
-    }
-    if (passes == 1) {
-      in = lane >= no;
-      k = in ? lane - no : lane;
-      valid[p] = p == 0 && lane < no + ni;
-    } else {
-      in = p == 1;
-      k = lane;
-      valid[p] = lane < (in ? ni : no);
-    }
-    ins[p] = in;
-    cs[p] = -1;
-    ws[p] = 0u;
-    if (valid[p]) {
-      cs[p] = in ? __ldg(a.part + __ldg(a.iidx + i0 + k)) : __ldg(a.part + __ldg(a.oidx + o0 + k));
-      ws[p] = in ? __ldg(a.iw + i0 + k) : __ldg(a.ow + o0 + k);
-    }
-  }
-  return delta_from_entries<DENSE>(a, R, v, r, s, passes, cs, ws, ins, valid, lane);
-}
-
-
 // Lists of more than kWarpList entries: per-block totals from a shared-memory
 // hash table, built in passes that each take the blocks of one hash class,
 // so the table never holds more than a few thousand blocks.  Costs
 // O(n * passes) with passes ~ n / 2048.
-constexpr int kHashSlots = kHashSlotsCfg;
 struct HashTab {
   int32_t* key;    // -1 = empty
   uint32_t* sum;
@@ -482,65 +373,6 @@ __device__ int hash_find(const HashTab& h, int32_t c) {
   for (int probe = 0; probe < kHashSlots; ++probe, i = (i + 1) & (kHashSlots - 1))
     if (h.key[i] == c) return (int)i;
   return -1;
-}
-
-template <bool DENSE, int G>
-__device__ double delta_hashed(const NodalArgs& a, int v, int r, int s, HashTab h, int* flag,
-                               const Group<G>& grp) {
-  const int t = grp.rank();
-  const Rows<DENSE> R(a, r, s);
-  const int32_t o0 = a.optr[v], no = a.optr[v + 1] - o0;
-  const int32_t i0 = a.iptr[v], ni = a.iptr[v + 1] - i0;
-  uint32_t koR = 0, koS = 0, niR = 0, niS = 0;
-  for (int k = t; k < no; k += G) {
-    int32_t c = __ldg(a.part + __ldg(a.oidx + o0 + k));
-    uint32_t w = __ldg(a.ow + o0 + k);
-    koR += c == r ? w : 0u;
-    koS += c == s ? w : 0u;
-  }
-  for (int k = t; k < ni; k += G) {
-    int32_t c = __ldg(a.part + __ldg(a.iidx + i0 + k));
-    uint32_t w = __ldg(a.iw + i0 + k);
-    niR += c == r ? w : 0u;
-    niS += c == s ? w : 0u;
-  }
-  koR = (uint32_t)grp.sum_ll(koR);
-  koS = (uint32_t)grp.sum_ll(koS);
-  niR = (uint32_t)grp.sum_ll(niR);
-  niS = (uint32_t)grp.sum_ll(niS);
-  Acc q;
-  for (int dir = 0; dir < 2; ++dir) {
-    const int32_t base = dir == 0 ? o0 : i0, n = dir == 0 ? no : ni;
-    const int32_t* idx = dir == 0 ? a.oidx : a.iidx;
-    const uint32_t* wt = dir == 0 ? a.ow : a.iw;
-    uint32_t P = (uint32_t)((n + kHashSlots / 4 - 1) / (kHashSlots / 4));
-    for (uint32_t pass = 0; pass < P; ++pass) {
-      for (int i = t; i < kHashSlots; i += G) {
-        h.key[i] = -1;
-        h.sum[i] = 0u;
-        h.first[i] = 0x7fffffff;
-      }
-      if (t == 0) *flag = 0;
-      grp.sync();
-      for (int k = t; k < n; k += G) {
-        int32_t c = __ldg(a.part + __ldg(idx + base + k));
-        if (hclass(c, P) == pass && !hash_add(h, c, __ldg(wt + base + k), k)) *flag = 1;
-      }
-      grp.sync();
-      if (*flag) return __longlong_as_double(0x7ff8000000000000ll);  // table overflow
-      for (int k = t; k < n; k += G) {
-        int32_t c = __ldg(a.part + __ldg(idx + base + k));
-        if (hclass(c, P) != pass) continue;
-        int slot = hash_find(h, c);
-        bool leader = h.first[slot] == k;
-        uint32_t kc = h.sum[slot];
-        uint32_t w = __ldg(wt + base + k);
-        entry<DENSE>(a, R, r, s, niS, dir == 1, c, w, leader, kc, q);
-      }
-      grp.sync();
-    }
-  }
-  return finish<DENSE, G>(a, R, v, r, s, RsWeights{koR, koS, niR, niS}, q, grp);
 }
 
 // Neighbour of v whose running weight (out-entries, then in-entries) first
@@ -592,7 +424,7 @@ __device__ __forceinline__ void item(const NodalArgs& a, int i, int lane, int& v
   } else {
     int32_t un = pick_neighbour(a, v, scale_draw(x.v[1], deg), lane);
     int32_t u = a.part[un];
-    s = a.use_rand[u] ? rnd : a.nbr_s[u];
+    s = a.nbr_s[u] < 0 ? rnd : a.nbr_s[u];
   }
 }
 
@@ -616,85 +448,458 @@ __device__ __forceinline__ double group_sum(double x) {
   return x;
 }
 
-// dS of a vertex whose entries fit one lane group of W lanes (entry c, wt,
-// direction `in` on lane hl of the group; delta_from_entries for one pass).
-// The group's masks keep the two half-warps' vertices apart.
-template <bool DENSE, int W>
-__device__ __forceinline__ double delta_group(const NodalArgs& a, const Rows<DENSE>& R, int v,
-                                              int r, int s, int32_t c, uint32_t wt, bool in,
-                                              bool valid, int lane) {
-  const int hl = lane & (W - 1), hb = lane & (32 - W);
-  const unsigned gm = W == 32 ? kFull : (0xFFFFu << hb);
-  const bool o = valid && !in, i = valid && in;
-  RsWeights w;
-  w.koR = __reduce_add_sync(gm, o && c == r ? wt : 0u);
-  w.koS = __reduce_add_sync(gm, o && c == s ? wt : 0u);
-  w.niR = __reduce_add_sync(gm, i && c == r ? wt : 0u);
-  w.niS = __reduce_add_sync(gm, i && c == s ? wt : 0u);
-  // direction in the top bit, unique keys for idle lanes
-  const unsigned key = valid ? ((unsigned)c | (in ? 0x80000000u : 0u)) : (0x7fffffe0u + (unsigned)lane);
-  const unsigned peers = __match_any_sync(gm, key);
-  const uint32_t kc = __reduce_add_sync(peers, wt);
-  Acc q;
-  if (valid) entry<DENSE>(a, R, r, s, w.niS, in, c, wt, lane == __ffs(peers) - 1, kc, q);
-  q.m4 = __reduce_add_sync(gm, q.m4);
-  q.m5 = __reduce_add_sync(gm, q.m5);
-  q.m6 = __reduce_add_sync(gm, q.m6);
-  q.m7 = __reduce_add_sync(gm, q.m7);
-  corner_terms<DENSE>(a, R, v, r, s, w.koR, w.koS, w.niR, w.niS, q, hl, hb);
-  return group_sum<W>(q.acc);
+// ----------------------------------------------------------- GSAP scoring --
+// A move's dS is a sum of per-entry terms and 13 corner and degree terms.
+// The entries are dealt to lanes in a fixed order and each lane subtracts its
+// entries' terms one after the other (the rounding of the sum is part of the
+// result, since a move is accepted iff dS < 0), so what may be arranged
+// freely is everything before the subtraction: the loads, the grouping of
+// equal blocks and the terms themselves.
+//
+// What bounds these kernels is the chain of dependent loads of a vertex (its
+// rows, its entries, their blocks, the proposal's block draw, the counts of
+// the proposed block's rows, the x log2 x table) and, on large batches, the
+// instructions issued per vertex.  So a group holds two entries a lane (the
+// same sums: a butterfly over 2L lanes starts by adding lanes l and l + L),
+// equal blocks are found by comparing against the group's keys in shared
+// memory (__reduce_add_sync over __match_any_sync's groups runs once per
+// distinct mask), the count changes of the four rows come in closed form
+// from v's degrees instead of four more group sums, and everything that does
+// not depend on the proposal is loaded before it is known.
+
+// Counts M[row][c] (out-entries) or M[c][row] (in-entries) of E entries; 0
+// where not wanted.  In the CSR form the binary searches advance together.
+template <bool DENSE, int E>
+__device__ __forceinline__ void row_counts(const NodalArgs& a, int row, const bool* in,
+                                           const int32_t* c, const bool* want, uint32_t* m) {
+  if constexpr (DENSE) {
+#pragma unroll
+    for (int j = 0; j < E; ++j)
+      m[j] = want[j] ? __ldg((in[j] ? a.MTd : a.Md) + (size_t)row * a.B + c[j]) : 0u;
+  } else {
+    int32_t lo[E], hi[E], end[E];
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+      const int32_t* p = (in[j] ? a.bip : a.bop) + row;
+      lo[j] = want[j] ? __ldg(p) : 0;
+      hi[j] = end[j] = want[j] ? __ldg(p + 1) : 0;
+    }
+    bool go = true;
+    while (go) {
+      go = false;
+      int32_t x[E];
+#pragma unroll
+      for (int j = 0; j < E; ++j)
+        x[j] = lo[j] < hi[j] ? __ldg((in[j] ? a.bic : a.boc) + ((lo[j] + hi[j]) >> 1)) : 0;
+#pragma unroll
+      for (int j = 0; j < E; ++j) {
+        if (lo[j] >= hi[j]) continue;
+        const int32_t mid = (lo[j] + hi[j]) >> 1;
+        if (x[j] < c[j]) lo[j] = mid + 1;
+        else hi[j] = mid;
+        go = go || lo[j] < hi[j];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < E; ++j)
+      m[j] = lo[j] < end[j] && __ldg((in[j] ? a.bic : a.boc) + lo[j]) == c[j]
+                 ? __ldg((in[j] ? a.bin : a.bon) + lo[j])
+                 : 0u;
+  }
 }
 
-// Proposal, dS and accept of batch vertex i when its entries fit one lane
-// group of W lanes: one entry per lane, loaded once for the neighbour pick
-// (out- then in-entries, pick_neighbour's order) and for the dS.  With
-// W = 16 each half-warp takes a vertex of at most 16 entries; both halves
-// run every warp-wide step, and a half without a vertex of its own
-// (active = false) repeats its partner's and writes nothing.
-template <bool DENSE, int W>
-__device__ __forceinline__ void fused_group(const NodalArgs& a, int i, bool active, int lane) {
-  const int hl = lane & (W - 1), hb = lane & (32 - W);
-  const unsigned gm = W == 32 ? kFull : (0xFFFFu << hb);
-  const int v = a.lo + i;
+// What a neighbour entry (block c, weight w) subtracts from its lane's sum:
+// t1 for the changed cell of row r, then t2 for the one of row s
+// (kernels.hpp:1444-1726 for out, 1153-1362 for in).  lead marks one entry
+// per distinct block of the direction, kc is v's total weight to/from c, Mo
+// and Mt the counts in rows r and s, ld the log2 of c's degree.  A block
+// absent from the target row gives one term per list entry
+// (kernels.hpp:1648-1652, 1696-1713; 1314-1318, 1348-1358); in-rows leave out
+// blocks r and s.
+__device__ __forceinline__ void entry_terms(const double* tab, bool ok, bool in, int32_t c,
+                                            uint32_t w, bool lead, uint32_t kc, uint32_t Mo,
+                                            uint32_t Mt, double ld, int r, int s, uint32_t niS,
+                                            double& t1, double& t2) {
+  const bool rs = c == r || c == s;
+  const bool cell = ok && lead && !rs;
+  const uint32_t y = Mt != 0u ? Mt + kc : in ? w : w - (c == r ? niS : 0u) + (c == s ? niS : 0u);
+  t1 = cell ? gterm(tab, Mo - kc, ld) - gterm(tab, Mo, ld) : 0.0;
+  t2 = cell || (ok && Mt == 0u && !(in && rs)) ? gterm(tab, y, ld) - gterm(tab, Mt, ld) : 0.0;
+}
+
+// Count changes of the new out-row r, out-row s, in-row r and in-row s away
+// from the corners.  Every block c other than r and s loses v's weight kc
+// from row r's cell and gains it in row s's, so the changes are v's degrees
+// less its weights to r and s; where M[s][r] or M[s][s] is 0, the entries in
+// that block add their own terms' counts (entry_terms): nR and nS of them.
+// All modulo 2^32, as the entry-wise sums are.
+struct RowChange {
+  int m4, m5, m6, m7;
+};
+__device__ __forceinline__ RowChange row_change(const Corner& q, const RsWeights& w, uint32_t nR,
+                                                uint32_t nS) {
+  const uint32_t o = q.kO - w.koR - w.koS, i = q.kI - w.niR - w.niS;
+  return RowChange{(int)(0u - o),
+                   (int)(o + (q.Msr == 0u ? w.koR - nR * w.niS : 0u) +
+                         (q.Mss == 0u ? w.koS + nS * w.niS : 0u)),
+                   (int)(0u - i), (int)i};
+}
+
+// Block proposed by a vertex whose drawn neighbour lies in block cu
+// (kernels.hpp:1000-1032): nbr_s holds the block's second-hop draw, or -1
+// where its proposals are uniform.
+__device__ __forceinline__ int proposed(const NodalArgs& a, int cu, int rnd) {
+  const int nb = a.nbr_s[cu];
+  return nb < 0 ? rnd : nb;
+}
+
+// Sum of the weights ws[b] over the set bits b of m.
+template <class Mask>
+__device__ __forceinline__ uint32_t mask_weight(const uint32_t* ws, Mask m) {
+  uint32_t t = 0u;
+  for (; m; m &= m - 1) t += ws[sizeof(Mask) == 8 ? __ffsll(m) - 1 : __ffs((unsigned)m) - 1];
+  return t;
+}
+
+// One vertex (batch index i) on a group of L lanes with two entries a lane:
+// L = 8 for at most 16 entries (four vertices a warp), L = 16 for at most 32
+// (two), L = 32 for at most 64.  Entry k (out-entries, then in-entries) sits
+// in slot k / L of lane k % L; a full warp whose directions both fit a lane
+// each holds out-entry l and in-entry l in lane l.  buf: 128 words of the
+// warp's shared memory.  Groups without a vertex of their own (active =
+// false) repeat another's and write nothing.
+template <bool GIVEN, bool DENSE, int L>
+__device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool active, int lane,
+                                             uint32_t* buf) {
+  using Mask = typename std::conditional<L == 32, unsigned long long, uint32_t>::type;
+  const int hl = lane & (L - 1), hb = lane & (32 - L);
+  const int v = GIVEN ? a.verts[i] : a.lo + i;
   const int32_t o0 = a.optr[v], no = a.optr[v + 1] - o0;
   const int32_t i0 = a.iptr[v], ni = a.iptr[v + 1] - i0;
-  const P4 x = draw(a.seed, kRngNodalVertex, a.seq + ctl_itr(a.ctl) * a.seq_mul, (uint32_t)v);
-  const int rnd = (int)(x.v[0] % (uint32_t)a.B);
-  const bool in = hl >= no;
-  const bool valid = hl < no + ni;
-  const int k = in ? hl - no : hl;
-  int32_t c = -1;
-  uint32_t w = 0u;
-  if (valid) {
-    const int32_t u = in ? __ldg(a.iidx + i0 + k) : __ldg(a.oidx + o0 + k);
-    w = in ? __ldg(a.iw + i0 + k) : __ldg(a.ow + o0 + k);
-    c = __ldg(a.part + u);
+  const bool split = L == 32 && no <= 32 && ni <= 32;  // a direction per slot
+  int32_t c[2];
+  uint32_t w[2], key[2];
+  bool in[2], ok[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int k = hl + L * j;
+    in[j] = split ? j == 1 : k >= no;
+    const int e = split ? hl : in[j] ? k - no : k;
+    ok[j] = e < (in[j] ? ni : no);
+    c[j] = -1;
+    w[j] = 0u;
+    if (ok[j]) {
+      const int32_t u = __ldg((in[j] ? a.iidx + i0 : a.oidx + o0) + e);
+      w[j] = __ldg((in[j] ? a.iw + i0 : a.ow + o0) + e);
+      c[j] = __ldg(a.part + u);
+    }
   }
   const int r = a.part[v];
-  const uint64_t deg = (uint64_t)a.kdo[v] + a.kdi[v];
-  const uint64_t t = scale_draw(x.v[1], deg);
-  uint64_t incl = w;
+  P4 x{};
+  if (!GIVEN) x = draw(a.seed, kRngNodalVertex, a.seq + ctl_itr(a.ctl) * a.seq_mul, (uint32_t)v);
+  uint32_t* skey = buf + 2 * hb;
+  uint32_t* sw = skey + 64;
 #pragma unroll
-  for (int o = 1; o < W; o <<= 1) {
-    const uint64_t y = __shfl_up_sync(kFull, incl, o);
-    if (hl >= o) incl += y;
+  for (int j = 0; j < 2; ++j) {
+    // direction in the top bit; idle slots match no entry
+    key[j] = ok[j] ? (uint32_t)c[j] | (in[j] ? 0x80000000u : 0u) : 0xffffffffu;
+    skey[hl + L * j] = key[j];
+    sw[hl + L * j] = w[j];
   }
-  const unsigned hit = __ballot_sync(kFull, valid && incl > t) & gm;
-  const int ch = __shfl_sync(kFull, c, hit ? __ffs(hit) - 1 : lane);
-  int s = rnd;
-  if (deg != 0) {
-    const int cu = hit ? ch : a.part[0];
-    s = a.use_rand[cu] ? rnd : a.nbr_s[cu];
+  const bool unit = __all_sync(kFull, w[0] <= 1u && w[1] <= 1u);
+  __syncwarp();
+  // the neighbour whose running weight first exceeds t
+  // (choose_neighbored_node_block, kernels.hpp:877-939): with unit weights
+  // it is entry t
+  int s;
+  if (GIVEN) {
+    s = a.props_in[i];
+  } else {
+    const int rnd = (int)(x.v[0] % (uint32_t)a.B);
+    const uint64_t deg = (uint64_t)a.kdo[v] + a.kdi[v];
+    const uint64_t t = scale_draw(x.v[1], deg);
+    int at = -1;
+    if (unit) {
+      if (deg != 0) at = split && (int)t >= no ? 32 + (int)t - no : (int)t;
+    } else {
+      uint64_t incl[2] = {w[0], w[1]};
+#pragma unroll
+      for (int o = 1; o < L; o <<= 1) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const uint64_t y = __shfl_up_sync(kFull, incl[j], o);
+          if (hl >= o) incl[j] += y;
+        }
+      }
+      incl[1] += __shfl_sync(kFull, incl[0], hb + L - 1);
+      const unsigned gm = L == 32 ? kFull : ((1u << (L & 31)) - 1u) << hb;
+      const unsigned h0 = __ballot_sync(kFull, ok[0] && incl[0] > t) & gm;
+      const unsigned h1 = __ballot_sync(kFull, ok[1] && incl[1] > t) & gm;
+      at = h0 ? __ffs(h0) - 1 - hb : h1 ? L + __ffs(h1) - 1 - hb : -1;
+    }
+    s = rnd;
+    if (deg != 0)
+      s = proposed(a, at >= 0 ? (int)(skey[at] & 0x7fffffffu) : a.part[0], rnd);
   }
   double d = 0.0;
   if (__any_sync(kFull, r != s)) {
-    const Rows<DENSE> R(a, r, s);
-    d = delta_group<DENSE, W>(a, R, v, r, s, c, w, in, valid, lane);
+    // row r's counts and the column degrees need no proposal
+    uint32_t Mo[2], Mt[2];
+    double ld[2];
+    bool want[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      want[j] = ok[j] && c[j] != r;
+      ld[j] = ok[j] ? __ldg((in[j] ? a.ld_out : a.ld_in) + c[j]) : 0.0;
+    }
+    row_counts<DENSE, 2>(a, r, in, c, want, Mo);
+    row_counts<DENSE, 2>(a, s, in, c, ok, Mt);
+    const uint32_t mm =
+        hl < 4 ? Rows<DENSE>(a, r, s).out_at((hl & 2) != 0, (hl & 1) ? s : r) : 0u;
+    Corner q;
+    load_degrees(a, v, r, s, q);
+    // the entries of each block: bit k of eq[j] for entry k
+    Mask eq[2] = {0, 0};
+    const int bound = split ? 32 + ni : no + ni;
+    const int nm = L == 32 ? bound : __reduce_max_sync(kFull, bound);
+#pragma unroll
+    for (int b = 0; b < 2 * L; b += 4) {
+      if (b >= nm) break;
+      const uint4 g = *reinterpret_cast<const uint4*>(skey + b);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (g.x == key[j]) eq[j] |= (Mask)1 << b;
+        if (g.y == key[j]) eq[j] |= (Mask)1 << (b + 1);
+        if (g.z == key[j]) eq[j] |= (Mask)1 << (b + 2);
+        if (g.w == key[j]) eq[j] |= (Mask)1 << (b + 3);
+      }
+    }
+    // the entries in blocks r and s, per direction
+    Mask inR = 0, inS = 0;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const unsigned bR = __ballot_sync(kFull, c[j] == r), bS = __ballot_sync(kFull, c[j] == s);
+      const unsigned lm = L == 32 ? kFull : (1u << (L & 31)) - 1u;
+      inR |= (Mask)((bR >> hb) & lm) << (L * j);
+      inS |= (Mask)((bS >> hb) & lm) << (L * j);
+    }
+    const int nout = split ? 32 : no;
+    const Mask out = nout >= 2 * L ? ~(Mask)0 : ((Mask)1 << nout) - 1;
+    auto count = [](Mask m) {
+      return (uint32_t)(sizeof(Mask) == 8 ? __popcll(m) : __popc((unsigned)m));
+    };
+    const uint32_t nR = count(inR & out), nS = count(inS & out);
+    RsWeights rw{nR, nS, count(inR & ~out), count(inS & ~out)};
+    uint32_t kc[2] = {count(eq[0]), count(eq[1])};
+    if (!unit) {
+      rw = RsWeights{mask_weight(sw, inR & out), mask_weight(sw, inS & out),
+                     mask_weight(sw, inR & ~out), mask_weight(sw, inS & ~out)};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) kc[j] = ok[j] ? mask_weight(sw, eq[j]) : 0u;
+    }
+    q.Mrr = __shfl_sync(kFull, mm, hb);
+    q.Mrs = __shfl_sync(kFull, mm, hb + 1);
+    q.Msr = __shfl_sync(kFull, mm, hb + 2);
+    q.Mss = __shfl_sync(kFull, mm, hb + 3);
+    const RowChange m = row_change(q, rw, nR, nS);
+    double t1[2], t2[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const bool lead = (eq[j] & (((Mask)1 << (hl + L * j)) - 1)) == 0;
+      entry_terms(a.xlx, ok[j], in[j], c[j], w[j], lead, kc[j], Mo[j], Mt[j], ld[j], r, s,
+                  rw.niS, t1[j], t2[j]);
+    }
+    double acc = 0.0 - t1[0];
+    acc -= t2[0];
+    if constexpr (L == 32) {
+      acc -= t1[1];
+      acc -= t2[1];
+      acc += corner_term<true, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, hl);
+    } else {
+      double acc1 = 0.0 - t1[1];
+      acc1 -= t2[1];
+      if constexpr (L == 16) {
+        acc += corner_term<true, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, hl);
+      } else {
+        acc += corner_term<true, false>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, hl);
+        acc1 += corner_term<false, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, hl + 8);
+      }
+      acc += acc1;
+    }
+    d = group_sum<L>(acc);
   }
-  if (hl == 0 && active) write_result(a, false, i, r, s, r != s ? d : 0.0);
+  if (hl == 0 && active) write_result(a, GIVEN, i, r, s, r != s ? d : 0.0);
   __syncwarp();
 }
 
+// A vertex of more than kGroupEntries entries (at most kWarpList a
+// direction) on the CTA, an entry (of up to 256) a thread and slot: on one
+// warp such a vertex, the longest chain of a batch, set the launch time of
+// graphs whose batches fit the GPU at once (20k HH: 34 us a launch, 19 with
+// this path and group_vertex).  The terms are computed by entry and subtracted by warp 0 in the order the warp's lanes would: by
+// entry index up to kWarpList entries, else by rank in the direction's
+// (block, weight) order.
+struct LargeBuf {
+  uint32_t key[2 * kWarpList], w[2 * kWarpList];
+  double t1[2 * kWarpList], t2[2 * kWarpList];
+  uint32_t cnt[6];  // koR, koS, niR, niS, out-entries in r, in s
+};
+
+template <bool GIVEN, bool DENSE>
+__device__ void large_vertex(const NodalArgs& a, int i, LargeBuf& sm) {
+  constexpr int T = kNodalWarps * 32;
+  static_assert(2 * T == 2 * kWarpList, "two slots a thread hold a large vertex's entries");
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int v = GIVEN ? a.verts[i] : a.lo + i;
+  const int32_t o0 = a.optr[v], no = a.optr[v + 1] - o0;
+  const int32_t i0 = a.iptr[v], ni = a.iptr[v + 1] - i0;
+  const int n = no + ni;
+  int32_t c[2];
+  uint32_t w[2], key[2];
+  bool in[2], ok[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int k = tid + T * j;
+    ok[j] = k < n;
+    in[j] = k >= no;
+    const int e = in[j] ? k - no : k;
+    c[j] = -1;
+    w[j] = 0u;
+    if (ok[j]) {
+      const int32_t u = __ldg((in[j] ? a.iidx + i0 : a.oidx + o0) + e);
+      w[j] = __ldg((in[j] ? a.iw + i0 : a.ow + o0) + e);
+      c[j] = __ldg(a.part + u);
+    }
+    key[j] = ok[j] ? (uint32_t)c[j] | (in[j] ? 0x80000000u : 0u) : 0xffffffffu;
+    sm.key[k] = key[j];
+    sm.w[k] = w[j];
+  }
+  const int r = a.part[v];
+  if (tid < 6) sm.cnt[tid] = 0u;
+  const bool unit = __syncthreads_and(w[0] <= 1u && w[1] <= 1u);
+  int s;
+  if (GIVEN) {
+    s = a.props_in[i];
+  } else {
+    const P4 x = draw(a.seed, kRngNodalVertex, a.seq + ctl_itr(a.ctl) * a.seq_mul, (uint32_t)v);
+    const int rnd = (int)(x.v[0] % (uint32_t)a.B);
+    const uint64_t t = scale_draw(x.v[1], (uint64_t)a.kdo[v] + a.kdi[v]);
+    int at = (int)t;
+    if (!unit) {  // the first entry whose running weight exceeds t
+      at = -1;
+      uint64_t acc = 0;
+      for (int k0 = 0; k0 < n && at < 0; k0 += 32) {
+        uint64_t incl = sm.w[k0 + lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint64_t y = __shfl_up_sync(kFull, incl, o);
+          if (lane >= o) incl += y;
+        }
+        const unsigned hit = __ballot_sync(kFull, k0 + lane < n && acc + incl > t);
+        if (hit) at = k0 + __ffs(hit) - 1;
+        acc += __shfl_sync(kFull, incl, 31);
+      }
+    }
+    s = proposed(a, at >= 0 ? (int)(sm.key[at] & 0x7fffffffu) : a.part[0], rnd);
+  }
+  if (r == s) {  // the same in every thread
+    if (tid == 0) write_result(a, GIVEN, i, r, s, 0.0);
+    __syncthreads();
+    return;
+  }
+  uint32_t Mo[2], Mt[2];
+  double ld[2];
+  bool want[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    want[j] = ok[j] && c[j] != r;
+    ld[j] = ok[j] ? __ldg((in[j] ? a.ld_out : a.ld_in) + c[j]) : 0.0;
+    if (c[j] == r) {
+      atomicAdd(sm.cnt + (in[j] ? 2 : 0), w[j]);
+      if (!in[j]) atomicAdd(sm.cnt + 4, 1u);
+    }
+    if (c[j] == s) {
+      atomicAdd(sm.cnt + (in[j] ? 3 : 1), w[j]);
+      if (!in[j]) atomicAdd(sm.cnt + 5, 1u);
+    }
+  }
+  row_counts<DENSE, 2>(a, r, in, c, want, Mo);
+  row_counts<DENSE, 2>(a, s, in, c, ok, Mt);
+  Corner q{};
+  if (tid < 32) {
+    const uint32_t mm =
+        lane < 4 ? Rows<DENSE>(a, r, s).out_at((lane & 2) != 0, (lane & 1) ? s : r) : 0u;
+    load_degrees(a, v, r, s, q);
+    q.Mrr = __shfl_sync(kFull, mm, 0);
+    q.Mrs = __shfl_sync(kFull, mm, 1);
+    q.Msr = __shfl_sync(kFull, mm, 2);
+    q.Mss = __shfl_sync(kFull, mm, 3);
+  }
+  // each entry's block total, whether an entry of its block comes before it
+  // in the summing order, and its place in that order
+  uint32_t kc[2] = {0u, 0u};
+  int pos[2];
+  bool lead[2];
+  if (n <= kWarpList) {
+    bool before = false;
+    for (int b = 0; b < n; b += 4) {  // idle slots match no entry
+      const uint4 g = *reinterpret_cast<const uint4*>(sm.key + b);
+      const uint4 u = *reinterpret_cast<const uint4*>(sm.w + b);
+      kc[0] += (g.x == key[0] ? u.x : 0u) + (g.y == key[0] ? u.y : 0u) +
+               (g.z == key[0] ? u.z : 0u) + (g.w == key[0] ? u.w : 0u);
+      before = before || (b < tid && g.x == key[0]) || (b + 1 < tid && g.y == key[0]) ||
+               (b + 2 < tid && g.z == key[0]) || (b + 3 < tid && g.w == key[0]);
+    }
+    lead[0] = !before;
+    lead[1] = false;
+    pos[0] = tid;
+    pos[1] = tid + T;
+  } else {
+    int rank[2] = {0, 0}, same[2] = {0, 0};
+    for (int b = 0; b < n; ++b) {
+      const uint32_t g = sm.key[b], u = sm.w[b];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const bool e = g == key[j];
+        kc[j] += e ? u : 0u;
+        const bool first = e && (u < w[j] || (u == w[j] && b < tid + T * j));
+        same[j] += first ? 1 : 0;
+        rank[j] += first || g < key[j] ? 1 : 0;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      lead[j] = same[j] == 0;
+      // out-entries' keys rank before every in-entry's
+      pos[j] = in[j] ? kWarpList + rank[j] - no : rank[j];
+    }
+  }
+  __syncthreads();
+  const RsWeights rw{sm.cnt[0], sm.cnt[1], sm.cnt[2], sm.cnt[3]};
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    if (ok[j])
+      entry_terms(a.xlx, true, in[j], c[j], w[j], lead[j], kc[j], Mo[j], Mt[j], ld[j], r, s,
+                  rw.niS, sm.t1[pos[j]], sm.t2[pos[j]]);
+  __syncthreads();
+  if (tid < 32) {
+    double acc = 0.0;
+    const int n0 = n <= kWarpList ? n : no, n1 = n <= kWarpList ? 0 : ni;
+    for (int p = lane; p < n0; p += 32) {
+      acc -= sm.t1[p];
+      acc -= sm.t2[p];
+    }
+    for (int p = kWarpList + lane; p < kWarpList + n1; p += 32) {
+      acc -= sm.t1[p];
+      acc -= sm.t2[p];
+    }
+    const RowChange m = row_change(q, rw, sm.cnt[4], sm.cnt[5]);
+    acc += corner_term<true, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, lane);
+    const double d = warp_sum(acc);
+    if (lane == 0) write_result(a, GIVEN, i, r, s, d);
+  }
+  __syncthreads();  // the CTA's next vertex reuses the buffer
+}
 
 // ------------------------------------------------------------ general mode --
 // Kernels instantiated with GEN = true score a move by the exact change of
@@ -823,7 +1028,7 @@ __device__ double finish_gen(const NodalArgs& a, const Rows<DENSE>& R, int v, in
     q.m6 = (int)grp.sum_ll(q.m6);
     q.m7 = (int)grp.sum_ll(q.m7);
     if (G == 32 || threadIdx.x < 32)
-      corner_terms<DENSE>(a, R, v, r, s, w.koR, w.koS, w.niR, w.niS, q, threadIdx.x & 31, 0);
+      corner_terms<DENSE>(a, R, v, r, s, w, q, threadIdx.x & 31);
   }
   logH = 0.0;
   if (a.mh) {
@@ -1058,246 +1263,395 @@ __device__ __forceinline__ void write_result_gen(const NodalArgs& a, bool given,
   if (a.props_out) a.props_out[i] = s;
 }
 
-// Mid vertices (more entries than the warp's registers hold, at most
-// kWarpHashEntries in both directions): the entries' (direction, block) keys
-// are grouped in a per-warp shared-memory hash table (open addressing, at
-// most half full), which gives each group its total weight and its first
-// entry, the one that adds the group's terms.  One pass, no sort.
-constexpr int kWarpHashEntries = 128;
-constexpr int kWarpHashSlots = 256;
-constexpr uint32_t kEmptyKey = 0xffffffffu;
-
-struct WarpHash {
-  uint32_t* key;  // kWarpHashSlots each
-  uint32_t* sum;
-  int32_t* first;
+// Work items of the warp kernel, larger vertices first (as the host lists
+// them: a longest-first schedule): a CTA per large vertex, then a warp per
+// vertex of up to 64 entries, per two of up to 32 and per four small ones.
+struct NodalItems {
+  int large, mid64, mid32, small;  // large in CTAs, the others in warps
+  __host__ __device__ NodalItems(int nlarge, int nmid64, int nmid32, int nsmall)
+      : large(nlarge), mid64(nmid64), mid32((nmid32 + 1) / 2), small((nsmall + 3) / 4) {}
+  __host__ __device__ int ctas() const {
+    return large + (mid64 + mid32 + small + kNodalWarps - 1) / kNodalWarps;
+  }
 };
 
-__device__ __forceinline__ uint32_t wh_slot(uint32_t key) {
-  return (key * 2654435761u) >> 24;  // 8 bits: kWarpHashSlots = 256
-}
-
-template <bool DENSE>
-__device__ double delta_whash(const NodalArgs& a, int v, int r, int s, int32_t o0, int no,
-                              int32_t i0, int ni, int lane, const WarpHash& h) {
-  constexpr int kPer = kWarpHashEntries / 32;  // entries per lane
-  constexpr uint32_t kMask = kWarpHashSlots - 1;
-  const Rows<DENSE> R(a, r, s);
-  const int n = no + ni;
-  for (int i = lane; i < kWarpHashSlots; i += 32) {
-    h.key[i] = kEmptyKey;
-    h.sum[i] = 0u;
-    h.first[i] = 0x7fffffff;
-  }
-  __syncwarp();
-  int32_t cs[kPer];
-  uint32_t ws[kPer];
-  bool ins[kPer];
-  uint32_t koR = 0, koS = 0, niR = 0, niS = 0;
-#pragma unroll
-  for (int p = 0; p < kPer; ++p) {
-    const int k = lane + 32 * p;
-    cs[p] = -1;
-    ws[p] = 0u;
-    ins[p] = false;
-    if (k < n) {
-      const bool in = k >= no;
-      const int j = in ? i0 + k - no : o0 + k;
-      const int32_t c = __ldg(a.part + __ldg((in ? a.iidx : a.oidx) + j));
-      const uint32_t w = __ldg((in ? a.iw : a.ow) + j);
-      cs[p] = c;
-      ws[p] = w;
-      ins[p] = in;
-      koR += !in && c == r ? w : 0u;
-      koS += !in && c == s ? w : 0u;
-      niR += in && c == r ? w : 0u;
-      niS += in && c == s ? w : 0u;
-      const uint32_t key = (uint32_t)c | (in ? 0x80000000u : 0u);
-      uint32_t sl = wh_slot(key);
-      // at most n <= kWarpHashSlots / 2 keys: a free or matching slot is
-      // found within the table
-      for (int probe = 0; probe < kWarpHashSlots; ++probe, sl = (sl + 1) & kMask) {
-        const uint32_t prev = atomicCAS(h.key + sl, kEmptyKey, key);
-        if (prev == kEmptyKey || prev == key) {
-          atomicAdd(h.sum + sl, w);
-          atomicMin(h.first + sl, k);
-          break;
-        }
+template <bool GIVEN, bool DENSE, bool GEN>
+struct NodalBody {
+  using Args = NodalArgs;
+  static constexpr int kThreads = kNodalWarps * 32, kMinBlocks = DENSE ? 8 : 6;
+  static constexpr size_t kSmem = 0;
+  static __device__ void run(const Args& a, int vb, int vg) {
+    if (ctl_stopped(a.ctl)) return;
+    __shared__ __align__(16) unsigned char raw[sizeof(LargeBuf)];
+    static_assert(kNodalWarps * 128 * sizeof(uint32_t) <= sizeof(LargeBuf), "warp buffers");
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t* buf = reinterpret_cast<uint32_t*>(raw) + 128 * wid;
+    const int nmid32 = a.nmid - a.nlarge - a.nmid64;
+    const NodalItems n(a.nlarge, a.nmid64, nmid32, a.nsmall);
+    const int32_t *mid64 = a.mid + a.nlarge, *mid32 = mid64 + a.nmid64;
+    for (int blk = vb; blk < n.ctas(); blk += vg) {
+      if (blk < n.large) {
+        large_vertex<GIVEN, DENSE>(a, a.mid[blk], *reinterpret_cast<LargeBuf*>(raw));
+        continue;
+      }
+      int it = (blk - n.large) * kNodalWarps + wid;
+      if (it < n.mid64) {
+        group_vertex<GIVEN, DENSE, 32>(a, mid64[it], true, lane, buf);
+        continue;
+      }
+      it -= n.mid64;
+      if (it < n.mid32) {
+        const int q = 2 * it + (lane >> 4);
+        group_vertex<GIVEN, DENSE, 16>(a, mid32[min(q, nmid32 - 1)], q < nmid32, lane, buf);
+        continue;
+      }
+      it -= n.mid32;
+      if (it < n.small) {
+        const int q = 4 * it + (lane >> 3);
+        group_vertex<GIVEN, DENSE, 8>(a, a.small[min(q, a.nsmall - 1)], q < a.nsmall, lane, buf);
       }
     }
   }
-  __syncwarp();
-  const RsWeights w{__reduce_add_sync(kFull, koR), __reduce_add_sync(kFull, koS),
-                    __reduce_add_sync(kFull, niR), __reduce_add_sync(kFull, niS)};
-  Acc q;
-#pragma unroll
-  for (int p = 0; p < kPer; ++p) {
-    const int k = lane + 32 * p;
-    if (k < n) {
-      const uint32_t key = (uint32_t)cs[p] | (ins[p] ? 0x80000000u : 0u);
-      uint32_t sl = wh_slot(key);
-      for (int probe = 0; probe < kWarpHashSlots && h.key[sl] != key; ++probe)
-        sl = (sl + 1) & kMask;
-      entry<DENSE>(a, R, r, s, w.niS, ins[p], cs[p], ws[p], h.first[sl] == k, h.sum[sl], q);
-    }
-  }
-  const double d = finish<DENSE, 32>(a, R, v, r, s, w, q, Group<32>{nullptr});
-  __syncwarp();  // the warp's next vertex reuses the table
-  return d;
-}
+};
 
-// One vertex (batch index i) on the whole warp: the fused path when its
-// entries fit the warp (sampled proposals, GSAP scoring), else the proposal
-// by pick_neighbour and the dS from registers (both lists within a warp),
-// from the warp's hash table (GSAP scoring, up to kWarpHashEntries) or from
-// sorted shared-memory lists.  buf: the warp's kWarpBufWords words of
-// shared memory.
-constexpr int kWarpBufWords = 384;  // 3 KB: the hash table, or the two sorted lists
-template <bool GIVEN, bool DENSE, bool GEN>
-__device__ __forceinline__ void warp_vertex(const NodalArgs& a, int i, int lane,
-                                            unsigned long long* buf) {
+// General mode (exact scoring, Metropolis-Hastings): one vertex on the whole
+// warp, the dS from registers (at most 32 entries) or from sorted
+// shared-memory lists.  buf: the warp's 2 * kWarpList words of shared memory.
+template <bool GIVEN, bool DENSE>
+__device__ __forceinline__ void warp_vertex_gen(const NodalArgs& a, int i, int lane,
+                                                unsigned long long* buf) {
   const Group<32> grp{nullptr};
   unsigned long long* sko = buf;
   unsigned long long* ski = buf + kWarpList;
   const int vv = GIVEN ? a.verts[i] : a.lo + i;
   const int32_t o0 = a.optr[vv], no = a.optr[vv + 1] - o0;
   const int32_t i0 = a.iptr[vv], ni = a.iptr[vv + 1] - i0;
-  if constexpr (GEN) {
-    int v, s;
-    uint32_t u2;
-    item<GIVEN>(a, i, lane, v, s, u2);
-    const int r = a.part[v];
-    double d = 0.0, lh = 0.0;
-    if (r != s) {
-      if (no + ni <= 32) {
-        d = delta_registers_gen<DENSE>(a, v, r, s, o0, no, i0, ni, lane, lh);
-      } else {
-        stage_sorted<32>(a.oidx, a.ow, a.part, o0, no, sko, grp);
-        stage_sorted<32>(a.iidx, a.iw, a.part, i0, ni, ski, grp);
-        d = delta_sorted_gen<DENSE, 32>(a, v, r, s, sko, no, ski, ni, grp, lh);
-      }
-    }
-    if (lane == 0) write_result_gen(a, GIVEN, i, r, s, d, lh, u2);
-    __syncwarp();
-    return;
-  }
-  if (!GIVEN && no + ni <= 32) {
-    fused_group<DENSE, 32>(a, i, true, lane);
-    return;
-  }
   int v, s;
   uint32_t u2;
   item<GIVEN>(a, i, lane, v, s, u2);
   const int r = a.part[v];
-  double d = 0.0;
+  double d = 0.0, lh = 0.0;
   if (r != s) {
-    if (no <= 32 && ni <= 32) {
-      d = delta_registers<DENSE>(a, v, r, s, o0, no, i0, ni, lane);
-    } else if (no + ni <= kWarpHashEntries) {
-      uint32_t* t = reinterpret_cast<uint32_t*>(buf);
-      const WarpHash h{t, t + kWarpHashSlots, reinterpret_cast<int32_t*>(t + 2 * kWarpHashSlots)};
-      d = delta_whash<DENSE>(a, v, r, s, o0, no, i0, ni, lane, h);
+    if (no + ni <= 32) {
+      d = delta_registers_gen<DENSE>(a, v, r, s, o0, no, i0, ni, lane, lh);
     } else {
       stage_sorted<32>(a.oidx, a.ow, a.part, o0, no, sko, grp);
       stage_sorted<32>(a.iidx, a.iw, a.part, i0, ni, ski, grp);
-      d = delta_sorted<DENSE, 32>(a, v, r, s, sko, no, ski, ni, grp);
+      d = delta_sorted_gen<DENSE, 32>(a, v, r, s, sko, no, ski, ni, grp, lh);
     }
   }
-  if (lane == 0) write_result(a, GIVEN, i, r, s, d);
+  if (lane == 0) write_result_gen(a, GIVEN, i, r, s, d, lh, u2);
   __syncwarp();
 }
 
-// Warp work items of a batch: the mid vertices (largest first, as the host
-// lists them), then pairs of small vertices.
-__host__ __device__ __forceinline__ int nodal_items(int nsmall, int nmid) {
+// Items of the general-mode kernel: the mid vertices, then pairs of small
+// ones.
+__host__ __device__ __forceinline__ int nodal_gen_items(int nsmall, int nmid) {
   return (nsmall + 1) / 2 + nmid;
 }
 
-template <bool GIVEN, bool DENSE, bool GEN>
-struct NodalBody {
+template <bool GIVEN, bool DENSE>
+struct NodalBody<GIVEN, DENSE, true> {
   using Args = NodalArgs;
-  static constexpr int kThreads = kNodalWarps * 32, kMinBlocks = GEN ? 4 : DENSE ? 10 : 6;
+  static constexpr int kThreads = kNodalWarps * 32, kMinBlocks = 4;
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
-  if (ctl_stopped(a.ctl)) return;
-  __shared__ unsigned long long s_buf[kNodalWarps][kWarpBufWords];
-  static_assert(2 * kWarpList <= kWarpBufWords && 3 * kWarpHashSlots <= 2 * kWarpBufWords,
-                "per-warp shared buffer");
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nw = vg * kNodalWarps;
-  const int npairs = (a.nsmall + 1) / 2;
-  const int items = npairs + a.nmid;
-  for (int it0 = vb * kNodalWarps + wid; it0 < items; it0 += nw) {
-    int ia, ib = -1;
-    if (it0 < a.nmid) {
-      ia = a.mid[it0];
-    } else {
-      const int it = it0 - a.nmid;
-      ia = a.small[2 * it];
-      const bool two = 2 * it + 1 < a.nsmall;
-      ib = two ? a.small[2 * it + 1] : -1;
-      if constexpr (!GIVEN && !GEN) {
-        // two vertices of at most 16 entries, one per half-warp
-        fused_group<DENSE, 16>(a, lane < 16 || !two ? ia : ib, lane < 16 || two, lane);
-        continue;
+    if (ctl_stopped(a.ctl)) return;
+    __shared__ unsigned long long s_buf[kNodalWarps][2 * kWarpList];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int nw = vg * kNodalWarps;
+    const int items = nodal_gen_items(a.nsmall, a.nmid);
+    for (int it0 = vb * kNodalWarps + wid; it0 < items; it0 += nw) {
+      int ia, ib = -1;
+      if (it0 < a.nmid) {
+        ia = a.mid[it0];
+      } else {
+        const int it = it0 - a.nmid;
+        ia = a.small[2 * it];
+        ib = 2 * it + 1 < a.nsmall ? a.small[2 * it + 1] : -1;
       }
+      // one call site, so that the body stays inline
+      for (int q = 0; q < (ib >= 0 ? 2 : 1); ++q)
+        warp_vertex_gen<GIVEN, DENSE>(a, q ? ib : ia, lane, s_buf[wid]);
     }
-    // one call site, so that the body stays inline
-    for (int q = 0; q < (ib >= 0 ? 2 : 1); ++q)
-      warp_vertex<GIVEN, DENSE, GEN>(a, q ? ib : ia, lane, s_buf[wid]);
-  }
   }
 };
 
-// Vertices with more than kWarpList entries in a direction: one CTA each,
-// per-block totals from the shared-memory hash table (one pass up to a few
-// thousand distinct blocks, more passes beyond).  Sorting both lists in
-// shared memory instead (the warp path's method) made the nodal kernels of a
-// 200k-vertex partition about 6 ms slower, for the same dS.
+// A vertex of more than kWarpList entries in a direction on a CTA.  Its
+// threads take the entries of each direction strided by kHeavyThreads, and
+// each subtracts its entries' terms in the order of P hash classes of blocks
+// (P = entries / 2048), then of the index: the order of a table that holds
+// one class at a time, kept because the sum's rounding is part of the
+// result.  What is free is the table: one of both directions' blocks, filled
+// once and sized to the vertex, whenever its blocks are sure to fit (n
+// entries, or 2 B blocks, at most half the slots), else one per class.  Four
+// entries a thread are in flight at a time and the keys of the first
+// kHeavyStage entries stay in shared memory.  What bounds it is the latency
+// of the chain of steps, a launch of few CTAs (20k HH graph, 12-30 such
+// vertices a graph: 13 us a launch in the median, 27 with a warp walking the
+// vertex's entries for the proposal and the table cleared, filled and read
+// per direction).
+constexpr int kHeavyStage = 4096;
+constexpr size_t kHeavySmem = (3 * kHashSlots + kHeavyStage) * sizeof(int32_t);
+
+template <bool GIVEN, bool DENSE>
+__device__ void heavy_vertex(const NodalArgs& a, int i, const Group<kHeavyThreads>& grp) {
+  constexpr int T = kHeavyThreads, U = 4;
+  extern __shared__ unsigned long long hsm[];
+  __shared__ unsigned long long wsum[T / 32];
+  __shared__ uint32_t cnt[6];  // koR, koS, niR, niS, out-entries in r, in s
+  __shared__ int s_at, overflow;
+  int32_t* const tkey = (int32_t*)hsm;
+  uint32_t* const tsum = (uint32_t*)hsm + kHashSlots;
+  int32_t* const tfirst = (int32_t*)hsm + 2 * kHashSlots;
+  uint32_t* const stage = (uint32_t*)hsm + 3 * kHashSlots;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const int v = GIVEN ? a.verts[i] : a.lo + i;
+  const int32_t o0 = a.optr[v], no = a.optr[v + 1] - o0;
+  const int32_t i0 = a.iptr[v], ni = a.iptr[v + 1] - i0;
+  const int n = no + ni;
+  const int r = a.part[v];
+  const uint64_t deg = (uint64_t)a.kdo[v] + a.kdi[v];
+  const bool unit = deg == (uint64_t)n;  // weights are at least 1
+  // entry k: out-entries, then in-entries; the direction in the top bit
+  auto load_key = [&](int k) {
+    return k < no ? (uint32_t)__ldg(a.part + __ldg(a.oidx + o0 + k))
+                  : (uint32_t)__ldg(a.part + __ldg(a.iidx + i0 + k - no)) | 0x80000000u;
+  };
+  auto entry_key = [&](int k) { return k < kHeavyStage ? stage[k] : load_key(k); };
+  auto entry_w = [&](int k) {
+    return unit ? 1u : k < no ? __ldg(a.ow + o0 + k) : __ldg(a.iw + i0 + k - no);
+  };
+  const int nst = min(n, kHeavyStage);
+#pragma unroll 4
+  for (int k = t; k < nst; k += T) stage[k] = load_key(k);
+  const bool fits = n <= kHashSlots / 2 || 2LL * a.B <= kHashSlots / 2;
+  int slots = 512;
+  while (slots < kHashSlots && (!fits || slots < 2 * min(n, 2 * a.B))) slots <<= 1;
+  const uint32_t smask = (uint32_t)slots - 1u;
+  auto clear = [&] {
+    for (int k = t; k < slots; k += T) {
+      tkey[k] = -1;
+      tsum[k] = 0u;
+      tfirst[k] = 0x7fffffff;
+    }
+  };
+  // a tagged key is never -1: blocks lie below 2^31 - 1
+  auto slot0 = [&](uint32_t key) { return (key * 2654435761u) >> 16 & smask; };
+  auto add = [&](uint32_t key, uint32_t w, int k) {
+    uint32_t q = slot0(key);
+    for (int probe = 0; probe < slots; ++probe, q = (q + 1) & smask) {
+      const int32_t cur = atomicCAS(tkey + q, -1, (int32_t)key);
+      if (cur == -1 || cur == (int32_t)key) {
+        atomicAdd(tsum + q, w);
+        atomicMin(tfirst + q, k);
+        return;
+      }
+    }
+    overflow = 1;
+  };
+  clear();
+  if (t < 6) cnt[t] = 0u;
+  if (t == 0) {
+    overflow = 0;
+    s_at = -1;
+  }
+  __syncthreads();
+  int s;
+  if (GIVEN) {
+    s = a.props_in[i];
+  } else {
+    const P4 x = draw(a.seed, kRngNodalVertex, a.seq + ctl_itr(a.ctl) * a.seq_mul, (uint32_t)v);
+    const int rnd = (int)(x.v[0] % (uint32_t)a.B);
+    const uint64_t target = scale_draw(x.v[1], deg);
+    int at = (int)target;
+    if (!unit) {
+      // the first entry whose running weight exceeds the target: the thread
+      // whose run of consecutive entries holds it
+      const int per = (n + T - 1) / T, k0 = min(n, t * per), k1 = min(n, k0 + per);
+      uint64_t own = 0;
+      for (int k = k0; k < k1; ++k) own += entry_w(k);
+      uint64_t incl = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) wsum[wid] = incl;
+      __syncthreads();
+      for (int q = 0; q < wid; ++q) incl += wsum[q];
+      uint64_t run = incl - own;
+      if (run <= target && target < incl)
+        for (int k = k0; k < k1; ++k) {
+          run += entry_w(k);
+          if (run > target) {
+            s_at = k;
+            break;
+          }
+        }
+      __syncthreads();
+      at = s_at;
+    }
+    s = proposed(a, at >= 0 ? (int)(entry_key(at) & 0x7fffffffu) : a.part[0], rnd);
+  }
+  if (r == s) {  // the same in every thread
+    if (t == 0) write_result(a, GIVEN, i, r, s, 0.0);
+    __syncthreads();
+    return;
+  }
+  Corner q{};
+  const Rows<DENSE> R(a, r, s);
+  if (t < 32) {
+    const uint32_t mm = lane < 4 ? R.out_at((lane & 2) != 0, (lane & 1) ? s : r) : 0u;
+    load_degrees(a, v, r, s, q);
+    q.Mrr = __shfl_sync(kFull, mm, 0);
+    q.Mrs = __shfl_sync(kFull, mm, 1);
+    q.Msr = __shfl_sync(kFull, mm, 2);
+    q.Mss = __shfl_sync(kFull, mm, 3);
+  }
+#pragma unroll 4
+  for (int k = t; k < n; k += T) {
+    const uint32_t key = entry_key(k), w = entry_w(k);
+    const int c = (int)(key & 0x7fffffffu);
+    const bool in = k >= no;
+    if (c == r) {
+      atomicAdd(cnt + (in ? 2 : 0), w);
+      if (!in) atomicAdd(cnt + 4, 1u);
+    }
+    if (c == s) {
+      atomicAdd(cnt + (in ? 3 : 1), w);
+      if (!in) atomicAdd(cnt + 5, 1u);
+    }
+    if (fits) add(key, w, k);
+  }
+  __syncthreads();
+  const RsWeights rw{cnt[0], cnt[1], cnt[2], cnt[3]};
+  double acc = 0.0;
+  for (int dir = 0; dir < 2; ++dir) {
+    const int lo = dir ? no : 0, hi = dir ? n : no;
+    const uint32_t P = (uint32_t)((hi - lo + kHashSlots / 4 - 1) / (kHashSlots / 4));
+    for (uint32_t pass = 0; pass < P; ++pass) {
+      auto mine = [&](uint32_t key) {
+        return P == 1 || hclass((int32_t)(key & 0x7fffffffu), P) == pass;
+      };
+      if (!fits) {
+        __syncthreads();
+        clear();
+        __syncthreads();
+        for (int k = lo + t; k < hi; k += T) {
+          const uint32_t key = entry_key(k);
+          if (mine(key)) add(key, entry_w(k), k);
+        }
+        __syncthreads();
+      }
+      for (int k = lo + t; k < hi;) {
+        bool in[U], ok[U], want[U], lead[U];
+        int32_t c[U];
+        uint32_t w[U], kc[U], Mo[U], Mt[U];
+        double ld[U], t1[U], t2[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          ok[u] = false;
+          in[u] = dir == 1;
+          c[u] = 0;
+          w[u] = kc[u] = 0u;
+          lead[u] = false;
+          uint32_t key = 0u;
+          int at = 0;
+          while (k < hi && !ok[u]) {
+            key = entry_key(k);
+            at = k;
+            k += T;
+            ok[u] = mine(key);
+          }
+          if (ok[u]) {
+            c[u] = (int32_t)(key & 0x7fffffffu);
+            w[u] = entry_w(at);
+            uint32_t sl = slot0(key);
+            for (int probe = 0; probe < slots && tkey[sl] != (int32_t)key; ++probe)
+              sl = (sl + 1) & smask;
+            lead[u] = tfirst[sl] == at;
+            kc[u] = tsum[sl];
+          }
+          want[u] = ok[u] && c[u] != r;
+          ld[u] = ok[u] ? __ldg((dir ? a.ld_out : a.ld_in) + c[u]) : 0.0;
+        }
+        row_counts<DENSE, U>(a, r, in, c, want, Mo);
+        row_counts<DENSE, U>(a, s, in, c, ok, Mt);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          entry_terms(a.xlx, ok[u], in[u], c[u], w[u], lead[u], kc[u], Mo[u], Mt[u], ld[u], r, s,
+                      rw.niS, t1[u], t2[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          acc -= t1[u];
+          acc -= t2[u];
+        }
+      }
+    }
+  }
+  if (t < 32) {
+    const RowChange m = row_change(q, rw, cnt[4], cnt[5]);
+    acc += corner_term<true, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, lane);
+  }
+  const double d = grp.sum(acc);
+  if (t == 0) {
+    if (overflow) atomicAdd(a.err, 1);
+    write_result(a, GIVEN, i, r, s, d);
+  }
+  __syncthreads();  // the CTA's next vertex reuses the shared memory
+}
+
+// Heavy vertices: one CTA each.
 template <bool GIVEN, bool DENSE, bool GEN>
 struct NodalHeavyBody {
   using Args = NodalArgs;
   static constexpr int kThreads = kHeavyThreads, kMinBlocks = 2;
   static constexpr size_t kSmem = kHeavySmem;
   static __device__ void run(const Args& a, int vb, int vg) {
-  if (ctl_stopped(a.ctl)) return;
-  extern __shared__ unsigned long long hsm[];
-  __shared__ double red[kHeavyThreads / 32];
-  __shared__ int flag, sh_v, sh_s;
-  __shared__ uint32_t sh_u2;
-  Group<kHeavyThreads> grp{red};
-  HashTab ht{(int32_t*)hsm, (uint32_t*)hsm + kHashSlots, (int32_t*)hsm + 2 * kHashSlots};
-  for (int h = vb; h < a.nheavy; h += vg) {
-    const int i = a.heavy[h];
-    if (threadIdx.x < 32) {
-      int v, s;
-      uint32_t u2;
-      item<GIVEN>(a, i, threadIdx.x, v, s, u2);
-      if (threadIdx.x == 0) {
-        sh_v = v;
-        sh_s = s;
-        sh_u2 = u2;
-      }
-    }
-    __syncthreads();
-    const int v = sh_v, s = sh_s;
-    const int r = a.part[v];
-    const int32_t o0 = a.optr[v], no = a.optr[v + 1] - o0;
-    const int32_t i0 = a.iptr[v], ni = a.iptr[v + 1] - i0;
-    double d = 0.0, lh = 0.0;
-    if (r != s) {
-      if constexpr (GEN)
-        d = delta_hashed_gen<DENSE, kHeavyThreads>(a, v, r, s, ht, &flag, grp, lh);
-      else
-        d = delta_hashed<DENSE, kHeavyThreads>(a, v, r, s, ht, &flag, grp);
-      if (threadIdx.x == 0 && d != d) atomicAdd(a.err, 1);
-    }
-    if (threadIdx.x == 0) {
-      if constexpr (GEN) write_result_gen(a, GIVEN, i, r, s, d, lh, sh_u2);
-      else write_result(a, GIVEN, i, r, s, d);
-    }
-    __syncthreads();
+    if (ctl_stopped(a.ctl)) return;
+    __shared__ double red[kHeavyThreads / 32];
+    const Group<kHeavyThreads> grp{red};
+    for (int h = vb; h < a.nheavy; h += vg) heavy_vertex<GIVEN, DENSE>(a, a.heavy[h], grp);
   }
+};
+
+template <bool GIVEN, bool DENSE>
+struct NodalHeavyBody<GIVEN, DENSE, true> {
+  using Args = NodalArgs;
+  static constexpr int kThreads = kHeavyThreads, kMinBlocks = 2;
+  static constexpr size_t kSmem = kHeavySmem;
+  static __device__ void run(const Args& a, int vb, int vg) {
+    if (ctl_stopped(a.ctl)) return;
+    extern __shared__ unsigned long long hsm[];
+    __shared__ double red[kHeavyThreads / 32];
+    __shared__ int flag, sh_v, sh_s;
+    __shared__ uint32_t sh_u2;
+    Group<kHeavyThreads> grp{red};
+    HashTab ht{(int32_t*)hsm, (uint32_t*)hsm + kHashSlots, (int32_t*)hsm + 2 * kHashSlots};
+    for (int h = vb; h < a.nheavy; h += vg) {
+      const int i = a.heavy[h];
+      if (threadIdx.x < 32) {
+        int v, s;
+        uint32_t u2;
+        item<GIVEN>(a, i, threadIdx.x, v, s, u2);
+        if (threadIdx.x == 0) {
+          sh_v = v;
+          sh_s = s;
+          sh_u2 = u2;
+        }
+      }
+      __syncthreads();
+      const int v = sh_v, s = sh_s;
+      const int r = a.part[v];
+      double d = 0.0, lh = 0.0;
+      if (r != s) {
+        d = delta_hashed_gen<DENSE, kHeavyThreads>(a, v, r, s, ht, &flag, grp, lh);
+        if (threadIdx.x == 0 && d != d) atomicAdd(a.err, 1);
+      }
+      if (threadIdx.x == 0) write_result_gen(a, GIVEN, i, r, s, d, lh, sh_u2);
+      __syncthreads();
+    }
   }
 };
 
@@ -1328,7 +1682,6 @@ struct CommitArgs {
   // draw_seq_mul) by the virtual blocks past ncommit
   const uint32_t *Md, *MTd, *Sd;
   int32_t* nbr_s;
-  uint8_t* use_rand;
   uint64_t seed;
   uint32_t draw_seq, draw_seq_mul;
   int32_t lo, count, B, slot_mul;
@@ -1347,7 +1700,7 @@ struct CommitBody {
       const int nw = ((vg - a.ncommit) * kCommitThreads) >> 5;
       for (int b = ((vb - a.ncommit) * kCommitThreads + tid) >> 5; b < a.B; b += nw)
         dense_block_draw(a.Md, a.MTd, a.Sd, a.d_out, a.d_in, a.B, a.seed, seq, b, lane,
-                         a.nbr_s, a.use_rand);
+                         a.nbr_s);
       return;
     }
     const int nc = a.ncommit;
@@ -1452,7 +1805,7 @@ NodalArgs make_args(const DevGraph& g, const int32_t* part, const DevBM& m, int3
   a.bon = m.ocnt; a.bin = m.icnt; a.d_out = m.d_out; a.d_in = m.d_in;
   a.Md = m.Md; a.MTd = m.MTd;
   a.ld_out = m.ld_out; a.ld_in = m.ld_in;
-  a.nbr_s = m.nbr_s; a.use_rand = m.use_rand;
+  a.nbr_s = m.nbr_s;
   a.B = B;
   a.heavy = aux.heavy;
   a.nheavy = aux.nheavy;
@@ -1460,14 +1813,16 @@ NodalArgs make_args(const DevGraph& g, const int32_t* part, const DevBM& m, int3
   a.nsmall = aux.nsmall;
   a.mid = aux.mid;
   a.nmid = aux.nmid;
+  a.nlarge = aux.nlarge;
+  a.nmid64 = aux.nmid64;
   a.err = aux.err;
   return a;
 }
 
-// CTAs of the warp kernel: one warp per work item.
-int nodal_grid(const NodalArgs& a) {
-  int g = (nodal_items(a.nsmall, a.nmid) + kNodalWarps - 1) / kNodalWarps;
-  return g < 1 ? 1 : (g > 148 * 64 ? 148 * 64 : g);
+// CTAs of the warp kernel.
+int32_t nodal_ctas(const NodalArgs& a, bool gen) {
+  if (gen) return ceil_div(nodal_gen_items(a.nsmall, a.nmid), kNodalWarps);
+  return NodalItems(a.nlarge, a.nmid64, a.nmid - a.nlarge - a.nmid64, a.nsmall).ctas();
 }
 
 template <bool GIVEN, bool DENSE, bool GEN>
@@ -1479,7 +1834,7 @@ void launch_pair(const NodalArgs& a, const NodalAux& aux, cudaStream_t st) {
     launch_single<NodalHeavyBody<GIVEN, DENSE, GEN>>(a, std::min(a.nheavy, 2 * 148), aux.side);
     cudaEventRecord(aux.join, aux.side);
   }
-  launch_single<NodalBody<GIVEN, DENSE, GEN>>(a, nodal_grid(a), st);
+  launch_single<NodalBody<GIVEN, DENSE, GEN>>(a, nodal_ctas(a, GEN), st);
   if (a.nheavy > 0) cudaStreamWaitEvent(st, aux.join, 0);
 }
 
@@ -1593,8 +1948,7 @@ void add_nodal(Slot& warp, Slot& heavy, bool dense, const ScoreMode& md, const D
   a.ctl = ctl;
   a.seq_mul = seq_mul;
   set_mode(a, md);
-  slot_push(slot_bind(warp, kmNodal[md.slot(dense)]), a,
-            ceil_div(nodal_items(aux.nsmall, aux.nmid), kNodalWarps));
+  slot_push(slot_bind(warp, kmNodal[md.slot(dense)]), a, nodal_ctas(a, md.general()));
   slot_push(slot_bind(heavy, kmNodalHeavy[md.slot(dense)]), a, aux.nheavy);
 }
 
@@ -1611,7 +1965,6 @@ void add_commit(Slot& s, int32_t* part, int32_t lo, int32_t count, const int32_t
     a.MTd = dense_m->MTd;
     a.Sd = dense_m->Sd;
     a.nbr_s = dense_m->nbr_s;
-    a.use_rand = dense_m->use_rand;
     a.seed = seed;
     a.draw_seq = draw_seq;
     a.draw_seq_mul = draw_seq_mul;

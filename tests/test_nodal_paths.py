@@ -1,0 +1,69 @@
+"""Nodal dS, proposals and accepted moves at the edges of the kernel paths: a
+vertex goes to 8, 16 or 32 lanes, to a CTA or to the heavy-vertex CTA by its
+entry counts; each edge of each path, unit and mixed weights, both forms of
+the blockmodel, against the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+REL = 1e-9  # the FP64 tolerance of the entropy terms, floor of 1 bit
+N = 12000
+# (out-entries, in-entries) of vertices 0, 1, ...
+SHAPES = [(0, 0), (1, 0), (0, 1), (7, 1), (8, 8), (16, 0), (0, 16), (9, 8), (17, 0), (16, 16),
+          (32, 0), (0, 32), (32, 1), (1, 32), (32, 32), (33, 0), (0, 33), (33, 31), (31, 33),
+          (64, 0), (0, 64), (33, 32), (65, 0), (0, 65), (64, 64), (128, 0), (0, 128), (65, 64),
+          (128, 1), (1, 128), (127, 127), (128, 128), (129, 0), (0, 129), (129, 129),
+          (0, 2048), (2048, 2048), (1, 2049), (2047, 2050), (5, 4091), (5, 4092), (3, 5000),
+          (4100, 4100)]
+
+
+def shaped_graph(sbp, weighted):
+    rng = np.random.default_rng(8)
+    K = len(SHAPES)
+    src, dst = [], []
+    for v, (no, ni) in enumerate(SHAPES):
+        src += [np.full(no, v), rng.integers(K, N, ni)]
+        dst += [rng.integers(K, N, no), np.full(ni, v)]
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    w = rng.integers(1, 6, src.size).astype(np.uint32) if weighted else None
+    return sbp.Graph.from_edges(N, src, dst, w)
+
+
+def close(a, b):
+    with np.errstate(invalid="ignore"):
+        return (a == b) | (np.abs(a - b) <= REL * np.maximum(np.abs(b), 1.0))
+
+
+@pytest.mark.parametrize("weighted", [False, True], ids=["unit", "weighted"])
+@pytest.mark.parametrize("dmax", ["0", "4096"], ids=["csr", "dense"])
+@pytest.mark.parametrize("B", [2, 300, 3000, N])
+def test_path_edges(sbp, orc, monkeypatch, weighted, dmax, B):
+    monkeypatch.setenv("SBP_DENSE_MAX", dmax)
+    g = shaped_graph(sbp, weighted)
+    rng = np.random.default_rng(B)
+    p = rng.integers(0, B, N).astype(np.int32)
+    p[-B:] = np.arange(B, dtype=np.int32)
+    # every shape, to random blocks, to its own and to neighbours' blocks
+    K = len(SHAPES)
+    verts = np.tile(np.arange(K, dtype=np.int32), 12)
+    props = rng.integers(0, B, verts.size).astype(np.int32)
+    src, dst, _ = g.edges()
+    for i, v in enumerate(verts):
+        near = dst[src == v] if i % 3 == 0 else src[dst == v]
+        if i % 3 < 2 and near.size:
+            props[i] = p[near[rng.integers(near.size)]]
+    got = sbp.delta_mdl_nodal(g, p, B, verts, props)
+    want, _ = orc.nodal_delta(g, p, B, verts, props)
+    ok = close(got, want)
+    assert ok.all(), (verts[~ok], props[~ok], got[~ok], want[~ok])
+    for seq in range(3):
+        pa, da, xa, _ = sbp.nodal_batch(g, p, B, 21, seq, 0, K)
+        pb, db, xb, _ = orc.nodal_batch(g, p, B, 21, seq, 0, K)
+        assert np.array_equal(xa, xb), "proposals differ"
+        assert close(da, db).all()
+        # a dS within its tolerance of 0 (0 before rounding, as of the vertex
+        # without edges) may round to either sign: all other moves agree
+        moves = (np.abs(da) > REL) | (np.abs(db) > REL)
+        assert np.array_equal(pa[:K][moves], pb[:K][moves]), "accepted moves differ"
+        assert np.array_equal(pa[:K] != p[:K], da < 0.0)
