@@ -5,25 +5,23 @@
 // neighbour blocks, bb_segsort over block segments, six memsets, two
 // remove_if compactions with a host read-back and mgpu::segreduce
 // (calculate_new_csr, partition.hpp:707-849; about 30 launches and ten hidden
-// allocations or synchronisations per call).  Here it is seven launches
-// with no host round trip, both directions (out rows / in rows) in each:
+// allocations or synchronisations per call).  Here it is six launches with no
+// host round trip, both directions (out rows / in rows) in each:
 //
 //   count    per vertex: entries of its row segment, slot inside the segment
-//   scan     segment offsets
+//   scan     segment offsets, where the rows stay
 //   scatter  per graph entry: (neighbour block, weight) into its segment
-//   rows     per segment: sort by column and sum runs; a warp per short
-//            segment (bitonic sort in shared memory), a CTA per long one
-//            (shared-memory histogram when B fits, else bitonic sort, else a
-//            windowed histogram)
-//   scan     compacted row pointers
-//   compact  per row: copy the unique (column, count) pairs into place, the
-//            row sum (weighted block degree) and its log2
+//   tile     short segments: a thread per entry, ranked by comparison
+//   rank     longer ones: a warp each, ranked through a bitmap of columns
+//   big      the longest: a CTA or a cluster of eight CTAs each
 //
 // The result is exact integer work and identical to the oracle's builder.
 #include "common.cuh"
 #include "kernels.h"
 #include "multi.cuh"
 #include "dense.cuh"
+
+#include <cooperative_groups.h>
 
 #include <algorithm>
 #include <map>
@@ -160,24 +158,28 @@ struct ScanApplyBody {
 constexpr int kScanSingleMax = 8 * kScanTile;
 
 // ------------------------------------------------------------ rebuild ------
+// M's rows are left at their segments' offsets: row b occupies
+// [ptr[b], end[b]) of the segment [ptr[b], ptr[b+1]) of the entries its
+// edges made, with unused entries after it.  A compact CSR needs the rows'
+// unique counts before their offsets, so it costs another scan and a copy of
+// every entry (200k HH, E = 2M: 80 us of a 430 us rebuild); nothing that
+// reads M needs its rows back to back.
 struct RbSide {
   const int32_t* gptr;
   const int32_t* gidx;
   const uint32_t* gw;
   const int32_t* gsrc;
   int32_t* cnt;
-  int32_t* seg;
   int32_t* vofs;
   int32_t* tcol;
   uint32_t* tw;
-  int32_t* ucol;  // unique (column, count) pairs of each segment, at its offset
-  uint32_t* uw;
-  int32_t* uniq;
-  int32_t* big;
-  int32_t* big_count;
+  int32_t *mid, *big, *giant;  // longer segments by kernel path
+  int32_t* nlist;              // their counts
   int32_t* bptr;
+  int32_t* bend;
   int32_t* bcol;
   uint32_t* bcnt;
+  uint32_t* bcum;
   uint32_t* bdeg;
   double* bld;
 };
@@ -186,8 +188,12 @@ struct RbArgs {
   RbSide s[2];
   const int32_t* part;
   const int32_t* ctl;
+  const double* xlx;
+  int32_t* nnz;
   int32_t N, E, B;
-  int32_t warp_cap;  // longest segment a warp reduces; longer ones go to a CTA
+  int32_t tile_cap;   // longest segment ranked by comparison (RbTileBody)
+  int32_t warp_max;   // longest segment ranked by a warp (RbRankBody)
+  int32_t tile_rows;  // rows of a tile
 };
 
 // The rebuild bodies work on both directions: virtual block vb serves
@@ -237,357 +243,446 @@ struct RbScatterBody {
     if (j >= a.E) return;
     int v = __ldg(d.gsrc + j);
     int b = __ldg(a.part + v);
-    int pos = __ldg(d.seg + b) + __ldg(d.vofs + v) + (j - __ldg(d.gptr + v));
+    int pos = __ldg(d.bptr + b) + __ldg(d.vofs + v) + (j - __ldg(d.gptr + v));
     d.tcol[pos] = __ldg(a.part + __ldg(d.gidx + j));
     d.tw[pos] = __ldg(d.gw + j);
   }
 };
 
-constexpr int kWarpCap = 256;  // longest segment sorted by one warp
-constexpr int kRowsWarps = 8;
-
-__device__ __forceinline__ void warp_bitonic(unsigned long long* key, int P, int lane) {
-  for (int k = 2; k <= P; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = lane; i < P; i += 32) {
-        int ixj = i ^ j;
-        if (ixj > i) {
-          unsigned long long x = key[i], y = key[ixj];
-          bool asc = (i & k) == 0;
-          if ((x > y) == asc) {
-            key[i] = y;
-            key[ixj] = x;
-          }
-        }
-      }
-      __syncwarp();
-    }
-  }
+// End, degree and its log2 of row b with u unique entries and weight sum deg.
+__device__ __forceinline__ void row_done(const RbArgs& a, const RbSide& d, int b, int base, int u,
+                                         uint32_t deg) {
+  d.bend[b] = base + u;
+  d.bdeg[b] = deg;
+  d.bld[b] = l2x(a.xlx, deg);
 }
 
-// Short segments: one warp each.  Long ones are listed for rb_rows_big.
-struct RbRowsSmallBody {
-  using Args = RbArgs;
-  static constexpr int kThreads = kRowsWarps * 32, kMinBlocks = 1;
-  static constexpr size_t kSmem = 0;
-  static __device__ void run(const Args& a, int vb, int vg) {
-  if (ctl_stopped(a.ctl)) return;
-  __shared__ unsigned long long sk[kRowsWarps][kWarpCap];
-  const RbSide& d = a.s[vb & 1];
-  vb >>= 1;
-  vg >>= 1;
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned long long* key = sk[wid];
-  for (int b = vb * kRowsWarps + wid; b < a.B; b += vg * kRowsWarps) {
-    int base = d.seg[b];
-    int n = d.seg[b + 1] - base;
-    if (n > a.warp_cap) {
-      if (lane == 0) d.big[atomicAdd(d.big_count, 1)] = b;
-      continue;
-    }
-    if (n == 0) {
-      if (lane == 0) d.uniq[b] = 0;
-      continue;
-    }
-    if (n <= 32) {
-      // one entry per lane: lanes with equal columns group and sum in
-      // registers; each group's leader writes at its column's rank among
-      // the distinct columns (ascending order, as a sort would give)
-      const bool valid = lane < n;
-      const uint32_t c = valid ? (uint32_t)d.tcol[base + lane] : 0xffffffffu;
-      const uint32_t w = valid ? d.tw[base + lane] : 0u;
-      const unsigned peers = __match_any_sync(kFull, c);
-      const uint32_t sum = __reduce_add_sync(peers, w);
-      const bool leader = valid && __ffs(peers) - 1 == lane;
-      const unsigned leaders = __ballot_sync(kFull, leader);
-      int rank = 0;
-      for (unsigned m = leaders; m; m &= m - 1) {
-        const uint32_t cj = __shfl_sync(kFull, c, __ffs(m) - 1);
-        rank += cj < c ? 1 : 0;
-      }
-      if (leader) {
-        d.ucol[base + rank] = (int32_t)c;
-        d.uw[base + rank] = sum;
-      }
-      if (lane == 0) d.uniq[b] = __popc(leaders);
-      continue;
-    }
-    int P = 32;
-    while (P < n) P <<= 1;
-    for (int i = lane; i < P; i += 32)
-      key[i] = i < n ? ((unsigned long long)(uint32_t)d.tcol[base + i] << 32) | d.tw[base + i]
-                     : ~0ull;
-    __syncwarp();
-    warp_bitonic(key, P, lane);
-    int running = 0;
-    for (int i0 = 0; i0 < n; i0 += 32) {
-      int i = i0 + lane;
-      bool valid = i < n;
-      uint32_t c = valid ? (uint32_t)(key[i] >> 32) : 0u;
-      bool head = valid && (i == 0 || (uint32_t)(key[i - 1] >> 32) != c);
-      unsigned mask = __ballot_sync(kFull, head);
-      if (head) {
-        int pos = running + __popc(mask & ((1u << lane) - 1));
-        uint32_t s = 0;
-        for (int j = i; j < n && (uint32_t)(key[j] >> 32) == c; ++j) s += (uint32_t)key[j];
-        d.ucol[base + pos] = (int32_t)c;
-        d.uw[base + pos] = s;
-      }
-      running += __popc(mask);
-    }
-    if (lane == 0) d.uniq[b] = running;
-    __syncwarp();
-  }
-  }
-};
+constexpr int kBigCap = 12288;  // longest segment a CTA takes; longer ones go to a cluster
 
-constexpr int kBigThreads = 512;
-constexpr int kHistCap = 16384;  // columns counted in shared memory at once
-constexpr int kSortCap = 8192;   // longest segment sorted in shared memory
-constexpr int kMaxWindows = 256; // column windows a long segment is bucketed into
-constexpr size_t kBigSmem = 65536;
-
-struct RbRowsBigBody {
-  using Args = RbArgs;
-  static constexpr int kThreads = kBigThreads, kMinBlocks = 2;
-  static constexpr size_t kSmem = kBigSmem;
-  static __device__ void run(const Args& a, int vb, int vg) {
-  if (ctl_stopped(a.ctl)) return;
-  extern __shared__ unsigned long long big_sm[];
-  __shared__ int sh[33];
-  __shared__ uint32_t touched[kHistCap / 32];  // bitmap of the histogram's nonzero columns
-  __shared__ int wstart[kMaxWindows + 1];      // a long segment's entries by column window
-  const RbSide& d = a.s[vb & 1];
-  vb >>= 1;
-  vg >>= 1;
-  uint32_t* hist = (uint32_t*)big_sm;
-  int nbig = *d.big_count;
-  int T = blockDim.x, tid = threadIdx.x;
-  const int nwords = (a.B + 31) >> 5;
-  if (a.B <= kHistCap && vb < nbig) {
-    // every row fits one histogram: it and the bitmap start zero and each
-    // row's extraction clears what the row touched
-    for (int i = tid; i < a.B; i += T) hist[i] = 0u;
-    for (int i = tid; i < nwords; i += T) touched[i] = 0u;
-    __syncthreads();
-  }
-  for (int idx = vb; idx < nbig; idx += vg) {
-    int b = d.big[idx];
-    int base = d.seg[b];
-    int n = d.seg[b + 1] - base;
-    int running = 0;
-    if (a.B <= kHistCap) {
-      // histogram of the row plus a bitmap of its columns; the extraction
-      // walks B/32 bitmap words, not B bins, so a row costs O(n + B/32)
-      for (int i = tid; i < n; i += T) {
-        const int c = d.tcol[base + i];
-        atomicAdd(hist + c, d.tw[base + i]);
-        atomicOr(touched + (c >> 5), 1u << (c & 31));
-      }
-      __syncthreads();
-      const int per = (nwords + T - 1) / T;
-      const int x0 = min(nwords, tid * per), x1 = min(nwords, x0 + per);
-      int nz = 0;
-      for (int x = x0; x < x1; ++x) nz += __popc(touched[x]);
-      int tot;
-      int pos = cta_excl_scan(nz, sh, &tot);
-      for (int x = x0; x < x1; ++x) {
-        uint32_t m = touched[x];
-        touched[x] = 0u;
-        while (m) {
-          const int c = (x << 5) + __ffs(m) - 1;
-          m &= m - 1;
-          d.ucol[base + pos] = c;
-          d.uw[base + pos] = hist[c];
-          hist[c] = 0u;
-          ++pos;
-        }
-      }
-      running = tot;
-      __syncthreads();
-    } else if (n > kSortCap && (a.B + kHistCap - 1) / kHistCap <= kMaxWindows) {
-      // Long segment, many columns: bucket the entries by column window of
-      // kHistCap (a counting sort into the segment's own output range), then
-      // one histogram pass per window over that window's entries only, with
-      // the touched-column bitmap.  Window w's results start at or before
-      // its bucket (every result consumes an entry of an earlier or the
-      // same window) and end at or before the next bucket, and are written
-      // after the window's entries are read: the range serves as both.
-      const int W = (a.B + kHistCap - 1) / kHistCap;
-      uint32_t* cursor = hist;  // W counters, before the histogram use
-      for (int i = tid; i < W; i += T) cursor[i] = 0u;
-      __syncthreads();
-      for (int i = tid; i < n; i += T) atomicAdd(cursor + d.tcol[base + i] / kHistCap, 1u);
-      __syncthreads();
-      if (tid == 0) {
-        int acc = 0;
-        for (int w = 0; w < W; ++w) {
-          wstart[w] = acc;
-          acc += (int)cursor[w];
-          cursor[w] = (uint32_t)wstart[w];
-        }
-        wstart[W] = acc;
-      }
-      __syncthreads();
-      for (int i = tid; i < n; i += T) {
-        const int c = d.tcol[base + i];
-        const int at = (int)atomicAdd(cursor + c / kHistCap, 1u);
-        d.ucol[base + at] = c;
-        d.uw[base + at] = d.tw[base + i];
-      }
-      __syncthreads();
-      for (int i = tid; i < kHistCap; i += T) hist[i] = 0u;
-      for (int i = tid; i < kHistCap / 32; i += T) touched[i] = 0u;
-      __syncthreads();
-      for (int w = 0; w < W; ++w) {
-        const int w0 = w * kHistCap, e0 = wstart[w], e1 = wstart[w + 1];
-        const int nwords_w = (min(kHistCap, a.B - w0) + 31) >> 5;
-        for (int i = e0 + tid; i < e1; i += T) {
-          const int c = d.ucol[base + i] - w0;
-          atomicAdd(hist + c, d.uw[base + i]);
-          atomicOr(touched + (c >> 5), 1u << (c & 31));
-        }
-        __syncthreads();
-        const int per = (nwords_w + T - 1) / T;
-        const int x0 = min(nwords_w, tid * per), x1 = min(nwords_w, x0 + per);
-        int nz = 0;
-        for (int x = x0; x < x1; ++x) nz += __popc(touched[x]);
-        int tot;
-        int pos = cta_excl_scan(nz, sh, &tot) + running;
-        for (int x = x0; x < x1; ++x) {
-          uint32_t m = touched[x];
-          touched[x] = 0u;
-          while (m) {
-            const int c = (x << 5) + __ffs(m) - 1;
-            m &= m - 1;
-            d.ucol[base + pos] = w0 + c;
-            d.uw[base + pos] = hist[c];
-            hist[c] = 0u;
-            ++pos;
-          }
-        }
-        running += tot;
-        __syncthreads();
-      }
-    } else if (n > kSortCap) {
-      // histogram over column windows of kHistCap
-      for (int w0 = 0; w0 < a.B; w0 += kHistCap) {
-        int W = min(kHistCap, a.B - w0);
-        for (int i = tid; i < W; i += T) hist[i] = 0u;
-        __syncthreads();
-        for (int i = tid; i < n; i += T) {
-          int c = d.tcol[base + i] - w0;
-          if (c >= 0 && c < W) atomicAdd(hist + c, d.tw[base + i]);
-        }
-        __syncthreads();
-        int per = (W + T - 1) / T;
-        int c0 = min(W, tid * per), c1 = min(W, c0 + per);
-        int nz = 0;
-        for (int c = c0; c < c1; ++c) nz += hist[c] != 0u;
-        int tot;
-        int pos = cta_excl_scan(nz, sh, &tot) + running;
-        for (int c = c0; c < c1; ++c) {
-          uint32_t h = hist[c];
-          if (h) {
-            d.ucol[base + pos] = w0 + c;
-            d.uw[base + pos] = h;
-            ++pos;
-          }
-        }
-        running += tot;
-        __syncthreads();
-      }
-    } else {
-      // bitonic sort of (column, weight) keys
-      unsigned long long* key = big_sm;
-      int P = 32;
-      while (P < n) P <<= 1;
-      for (int i = tid; i < P; i += T)
-        key[i] = i < n ? ((unsigned long long)(uint32_t)d.tcol[base + i] << 32) | d.tw[base + i]
-                       : ~0ull;
-      __syncthreads();
-      for (int k = 2; k <= P; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-          for (int i = tid; i < P; i += T) {
-            int ixj = i ^ j;
-            if (ixj > i) {
-              unsigned long long x = key[i], y = key[ixj];
-              bool asc = (i & k) == 0;
-              if ((x > y) == asc) {
-                key[i] = y;
-                key[ixj] = x;
-              }
-            }
-          }
-          __syncthreads();
-        }
-      }
-      for (int i0 = 0; i0 < n; i0 += T) {
-        int i = i0 + tid;
-        bool valid = i < n;
-        uint32_t c = valid ? (uint32_t)(key[i] >> 32) : 0u;
-        bool head = valid && (i == 0 || (uint32_t)(key[i - 1] >> 32) != c);
-        int tot;
-        int pos = cta_excl_scan(head ? 1 : 0, sh, &tot) + running;
-        if (head) {
-          uint32_t s = 0;
-          for (int j = i; j < n && (uint32_t)(key[j] >> 32) == c; ++j) s += (uint32_t)key[j];
-          d.ucol[base + pos] = (int32_t)c;
-          d.uw[base + pos] = s;
-        }
-        running += tot;
-      }
-      __syncthreads();
-    }
-    if (tid == 0) d.uniq[b] = running;
-    __syncthreads();
-  }
-  }
-};
-
-// Per row: unique entries into place, weighted degree and its log2.
-struct RbCompactBody {
+// Short segments: a CTA takes tile_rows consecutive rows and gives every
+// entry a thread, which compares it with its segment's entries in shared
+// memory: the number before it in (column, index) order is its place in the
+// sorted segment, the equal ones give the column's total, and the first of
+// them the entry that carries it.  Eight lanes a row then close up the
+// carried entries.  Longer segments are listed for the kernels below.  A
+// warp per segment (a match over its lanes, or a bitonic sort) took 141 us a
+// rebuild of the 200k HH graph at B = 55k-85k, issuing for idle lanes.
+constexpr int kTileEntries = 2048, kTileMaxCap = 128;
+struct RbTileBody {
   using Args = RbArgs;
   static constexpr int kThreads = 256, kMinBlocks = 1;
   static constexpr size_t kSmem = 0;
-  static __device__ void run(const Args& a, int vb, int vg) {
-  if (ctl_stopped(a.ctl)) return;
-  const RbSide& d = a.s[vb & 1];
-  vb >>= 1;
-  vg >>= 1;
-  int lane = threadIdx.x & 31;
-  int w = (vb * blockDim.x + threadIdx.x) >> 5;
-  int nw = (vg * blockDim.x) >> 5;
-  for (int b = w; b < a.B; b += nw) {
-    int src = d.seg[b], dst = d.bptr[b], u = d.uniq[b];
-    unsigned long long s = 0;
-    for (int i = lane; i < u; i += 32) {
-      uint32_t c = d.uw[src + i];
-      d.bcol[dst + i] = d.ucol[src + i];
-      d.bcnt[dst + i] = c;
-      s += c;
+  static __device__ void run(const Args& a, int vb, int) {
+    if (ctl_stopped(a.ctl)) return;
+    __shared__ uint32_t key[kTileEntries], w[kTileEntries], skey[kTileEntries], sw[kTileEntries];
+    __shared__ uint8_t owner[kTileEntries];
+    __shared__ int off[kThreads + 1], src[kThreads];
+    __shared__ int sh[33];
+    __shared__ int s_nnz;
+    const RbSide& d = a.s[vb & 1];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int b0 = (vb >> 1) * a.tile_rows, nr = min(a.tile_rows, a.B - b0);
+    int len = 0;
+    if (tid < nr) {
+      const int b = b0 + tid, base = d.bptr[b];
+      len = d.bptr[b + 1] - base;
+      src[tid] = base;
+      if (len > a.tile_cap) {
+        const int k = len <= a.warp_max ? 0 : len <= kBigCap ? 1 : 2;
+        (k == 0 ? d.mid : k == 1 ? d.big : d.giant)[atomicAdd(d.nlist + k, 1)] = b;
+        len = 0;
+      } else if (len == 0) {
+        row_done(a, d, b, base, 0, 0u);
+      }
     }
-    s = warp_sum_ull(s);
-    if (lane == 0) {
-      uint32_t deg = (uint32_t)s;
-      d.bdeg[b] = deg;
-      d.bld[b] = log2((double)deg);
+    if (tid == 0) s_nnz = 0;
+    int total;
+    const int at = cta_excl_scan(len, sh, &total);
+    off[tid] = at;
+    if (tid == 0) off[kThreads] = total;
+    __syncthreads();
+    // rounds of rows whose offsets lie in a window, so that their entries fit
+    const int win = kTileEntries - a.tile_cap;
+    const int g = tid >> 3, gl = tid & 7;
+    int nnz = 0;
+    for (int q0 = 0; q0 < total; q0 += win) {
+      for (int r = g; r < nr; r += kThreads / 8) {
+        const int o = off[r] - q0, n = off[r + 1] - off[r];
+        if (n == 0 || o < 0 || o >= win) continue;
+        for (int i = gl; i < n; i += 8) {
+          key[o + i] = (uint32_t)d.tcol[src[r] + i];
+          w[o + i] = d.tw[src[r] + i];
+          owner[o + i] = (uint8_t)r;
+        }
+      }
+      __syncthreads();
+      // the round's entries end where the next round's first row starts
+      int end = 0;
+      {
+        const bool mine = tid < nr && len > 0 && at - q0 >= 0 && at - q0 < win;
+        end = mine ? at - q0 + len : 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) end = max(end, __shfl_xor_sync(kFull, end, o));
+        if (lane == 0) sh[tid >> 5] = end;
+        __syncthreads();
+        end = 0;
+        for (int i = 0; i < kThreads / 32; ++i) end = max(end, sh[i]);
+      }
+      for (int e = tid; e < end; e += kThreads) {
+        const int r = owner[e], s0 = off[r] - q0, s1 = s0 + off[r + 1] - off[r];
+        const uint32_t k = key[e];
+        int lt = 0, before = 0;
+        uint32_t sum = 0u;
+        for (int j = s0; j < s1; ++j) {
+          const uint32_t x = key[j];
+          lt += x < k ? 1 : 0;
+          if (x == k) {
+            sum += w[j];
+            before += j < e ? 1 : 0;
+          }
+        }
+        skey[s0 + lt + before] = k;
+        sw[s0 + lt + before] = before ? 0u : sum;  // weights are >= 1: 0 marks a repeat
+      }
+      __syncthreads();
+      for (int r0 = 0; r0 < nr; r0 += kThreads / 8) {
+        const int r = r0 + g;
+        const int o = r < nr ? off[r] - q0 : -1, n = r < nr ? off[r + 1] - off[r] : 0;
+        const bool live = n > 0 && o >= 0 && o < win;
+        const int steps = live ? (n + 7) >> 3 : 0;
+        int u = 0;
+        uint32_t deg = 0u;
+        const int most = __reduce_max_sync(kFull, steps);
+        for (int i = 0; i < most; ++i) {
+          const int p = 8 * i + gl;
+          const uint32_t c = live && p < n ? sw[o + p] : 0u;
+          const unsigned m = __ballot_sync(kFull, c != 0u) >> (lane & 24) & 0xffu;
+          if (c) {
+            const int z = src[r] + u + __popc(m & ((1u << gl) - 1u));
+            d.bcol[z] = (int32_t)skey[o + p];
+            d.bcnt[z] = c;
+            deg += c;
+          }
+          u += __popc(m);
+        }
+#pragma unroll
+        for (int x = 4; x > 0; x >>= 1) deg += __shfl_xor_sync(kFull, deg, x);
+        if (live && gl == 0) {
+          row_done(a, d, b0 + r, src[r], u, deg);
+          nnz += u;
+        }
+      }
+      __syncthreads();
+    }
+    if (vb & 1) return;  // the two directions have the same entries
+    if (nnz) atomicAdd(&s_nnz, nnz);
+    __syncthreads();
+    if (tid == 0 && s_nnz) atomicAdd(a.nnz, s_nnz);
+  }
+};
+
+// Longer segments by a bitmap of their columns: a column's place among the
+// distinct ones is the number of bits below it (the words before it, then
+// its own word), so no sort is needed; its total is added at that place.
+// Columns are taken in windows of the bitmap's size.  A warp's shared memory:
+// a window's bitmap and running counts, and the totals.
+constexpr int kRankMax = 1024;       // longest segment a warp takes
+constexpr int kRankWords = 512;      // bitmap words of a window
+constexpr int kRankWarps = 8;
+constexpr size_t kRankWarpBytes = kRankWords * 6 + kRankMax * 4;
+struct RbRankBody {
+  using Args = RbArgs;
+  static constexpr int kThreads = kRankWarps * 32, kMinBlocks = 1;
+  static constexpr size_t kSmem = kRankWarps * kRankWarpBytes;
+  static __device__ void run(const Args& a, int vb, int vg) {
+    if (ctl_stopped(a.ctl)) return;
+    extern __shared__ unsigned char rank_sm[];
+    const RbSide& d = a.s[vb & 1];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint32_t* cnt = (uint32_t*)(rank_sm + wid * kRankWarpBytes);
+    uint32_t* bm = cnt + kRankMax;
+    uint16_t* pre = (uint16_t*)(bm + kRankWords);
+    const int nmid = d.nlist[0];
+    int nnz = 0;
+    for (int idx = (vb >> 1) * kRankWarps + wid; idx < nmid; idx += (vg >> 1) * kRankWarps) {
+      const int b = d.mid[idx], base = d.bptr[b], n = d.bptr[b + 1] - base;
+      for (int i = lane; i < n; i += 32) cnt[i] = 0u;
+      int u = 0;
+      for (int w0 = 0; w0 < a.B; w0 += 32 * kRankWords) {
+        const int cols = min(32 * kRankWords, a.B - w0), nw = (cols + 31) >> 5;
+        for (int x = lane; x < nw; x += 32) bm[x] = 0u;
+        __syncwarp();
+#pragma unroll 4
+        for (int i = lane; i < n; i += 32) {
+          const int c = d.tcol[base + i] - w0;
+          if ((unsigned)c < (unsigned)cols) atomicOr(bm + (c >> 5), 1u << (c & 31));
+        }
+        __syncwarp();
+        int run = 0;
+        for (int x0 = 0; x0 < nw; x0 += 32) {
+          const int x = x0 + lane;
+          const int p = x < nw ? __popc(bm[x]) : 0;
+          const int incl = (int)warp_incl_scan_u((unsigned)p, lane);
+          if (x < nw) pre[x] = (uint16_t)(run + incl - p);
+          run += __shfl_sync(kFull, incl, 31);
+        }
+        __syncwarp();
+#pragma unroll 4
+        for (int i = lane; i < n; i += 32) {
+          const int c = d.tcol[base + i] - w0;
+          if ((unsigned)c >= (unsigned)cols) continue;
+          const int at = u + pre[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u));
+          atomicAdd(cnt + at, d.tw[base + i]);
+          d.bcol[base + at] = c + w0;
+        }
+        u += run;
+        __syncwarp();
+      }
+      uint32_t deg = 0u;
+      for (int i0 = 0; i0 < u; i0 += 32) {
+        const int i = i0 + lane;
+        const uint32_t c = i < u ? cnt[i] : 0u;
+        const uint32_t incl = warp_incl_scan_u(c, lane);
+        if (i < u) {
+          d.bcnt[base + i] = c;
+          d.bcum[base + i] = deg + incl;
+        }
+        deg += __shfl_sync(kFull, incl, 31);
+      }
+      if (lane == 0) row_done(a, d, b, base, u, deg);
+      nnz += u;
+      __syncwarp();
+    }
+    if (!(vb & 1) && lane == 0 && nnz) atomicAdd(a.nnz, nnz);
+  }
+};
+
+// The longest segments, the same way: up to kBigCap entries by a CTA, longer
+// ones (a block that many merged into: 50k-500k entries of the 200k HH graph)
+// by a cluster of eight CTAs, each with an eighth of the entries.  Each CTA
+// marks its entries' columns, merges an eighth of the eight bitmaps through
+// distributed shared memory and hands the merged words and their running
+// counts to all; the totals are then added in place.  One CTA for such a
+// segment took 157 us of every rebuild of the 200k HH graph, and up to 1.1 ms;
+// the cluster 17 us (at most 48).
+constexpr int kBigThreads = 512, kBigCluster = 8;
+constexpr int kBigWords = 4096;  // bitmap words of a window (131072 columns)
+constexpr size_t kBigSmem = (size_t)(2 * kBigWords + kBigCap) * 4;
+static_assert(kBigCap >= kBigWords, "the giant path's third array of words");
+struct RbBigBody {
+  using Args = RbArgs;
+  static constexpr int kThreads = kBigThreads, kMinBlocks = 2, kCluster = kBigCluster;
+  static constexpr size_t kSmem = kBigSmem;
+
+  static __device__ void big_row(const RbArgs& a, const RbSide& d, int b, uint32_t* bm,
+                                 uint32_t* pre, uint32_t* cnt, int* sh, int& nnz) {
+    constexpr int T = kBigThreads, kPer = kBigWords / T;
+    const int tid = threadIdx.x;
+    const int base = d.bptr[b], n = d.bptr[b + 1] - base;
+    for (int i = tid; i < n; i += T) cnt[i] = 0u;
+    int u = 0;
+    for (int w0 = 0; w0 < a.B; w0 += 32 * kBigWords) {
+      const int cols = min(32 * kBigWords, a.B - w0), nw = (cols + 31) >> 5;
+      for (int x = tid; x < nw; x += T) bm[x] = 0u;
+      __syncthreads();
+#pragma unroll 4
+      for (int i = tid; i < n; i += T) {
+        const int c = d.tcol[base + i] - w0;
+        if ((unsigned)c < (unsigned)cols) atomicOr(bm + (c >> 5), 1u << (c & 31));
+      }
+      __syncthreads();
+      int nz = 0;
+      const int per = (nw + T - 1) / T;
+      for (int j = 0; j < per && j < kPer; ++j) {
+        const int x = tid * per + j;
+        nz += x < nw ? __popc(bm[x]) : 0;
+      }
+      int tot;
+      int run = cta_excl_scan(nz, sh, &tot);
+      for (int j = 0; j < per && j < kPer; ++j) {
+        const int x = tid * per + j;
+        if (x >= nw) break;
+        pre[x] = (uint32_t)run;
+        run += __popc(bm[x]);
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int i = tid; i < n; i += T) {
+        const int c = d.tcol[base + i] - w0;
+        if ((unsigned)c >= (unsigned)cols) continue;
+        const int at = u + (int)pre[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u));
+        atomicAdd(cnt + at, d.tw[base + i]);
+        d.bcol[base + at] = c + w0;
+      }
+      u += tot;
+      __syncthreads();
+    }
+    uint32_t deg = 0u;
+    for (int i0 = 0; i0 < u; i0 += T) {
+      const int i = i0 + tid;
+      const uint32_t c = i < u ? cnt[i] : 0u;
+      int tot;
+      const uint32_t ex = (uint32_t)cta_excl_scan((int)c, sh, &tot);
+      if (i < u) {
+        d.bcnt[base + i] = c;
+        d.bcum[base + i] = deg + ex + c;
+      }
+      deg += (uint32_t)tot;
+    }
+    if (tid == 0) row_done(a, d, b, base, u, deg);
+    nnz += u;
+    __syncthreads();
+  }
+
+  static __device__ void giant_row(const RbArgs& a, const RbSide& d, int b, uint32_t* part,
+                                   uint32_t* merged, uint32_t* pre, uint32_t* tots, int* sh,
+                                   int& nnz) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    constexpr int T = kBigThreads, C = kBigCluster;
+    const int tid = threadIdx.x, q = (int)cl.block_rank();
+    const int base = d.bptr[b], n = d.bptr[b + 1] - base;
+    const int e0 = (int)((long long)n * q / C), e1 = (int)((long long)n * (q + 1) / C);
+    for (int i = e0 + tid; i < e1; i += T) d.bcnt[base + i] = 0u;
+    int u = 0;
+    for (int w0 = 0; w0 < a.B; w0 += 32 * kBigWords) {
+      const int cols = min(32 * kBigWords, a.B - w0), nw = (cols + 31) >> 5;
+      const int seg = (nw + C - 1) / C;  // words a CTA merges: at most T
+      for (int x = tid; x < nw; x += T) part[x] = 0u;
+      __syncthreads();
+#pragma unroll 4
+      for (int i = e0 + tid; i < e1; i += T) {
+        const int c = d.tcol[base + i] - w0;
+        if ((unsigned)c < (unsigned)cols) atomicOr(part + (c >> 5), 1u << (c & 31));
+      }
+      cl.sync();
+      const int x = q * seg + tid;
+      uint32_t m = 0u;
+      const bool mine = tid < seg && x < nw;
+      if (mine)
+        for (int p = 0; p < C; ++p) m |= cl.map_shared_rank(part, p)[x];
+      int tot;
+      const int ex = cta_excl_scan(__popc(m), sh, &tot);
+      if (mine)
+        for (int p = 0; p < C; ++p) {
+          cl.map_shared_rank(merged, p)[x] = m;
+          cl.map_shared_rank(pre, p)[x] = (uint32_t)ex;
+        }
+      if (tid < C) cl.map_shared_rank(tots, tid)[q] = (uint32_t)tot;
+      cl.sync();
+      uint32_t first[C];  // distinct columns before each segment of words
+      uint32_t run = (uint32_t)u;
+#pragma unroll
+      for (int p = 0; p < C; ++p) {
+        first[p] = run;
+        run += tots[p];
+      }
+      for (int i = e0 + tid; i < e1; i += T) {
+        const int c = d.tcol[base + i] - w0;
+        if ((unsigned)c >= (unsigned)cols) continue;
+        const int word = c >> 5, sg = word / seg;
+        uint32_t f = first[0];
+#pragma unroll
+        for (int p = 1; p < C; ++p) f = sg == p ? first[p] : f;
+        const int at = (int)(f + pre[word]) + __popc(merged[word] & ((1u << (c & 31)) - 1u));
+        atomicAdd(d.bcnt + base + at, d.tw[base + i]);
+        d.bcol[base + at] = c + w0;
+      }
+      u = (int)run;
+    }
+    __threadfence();
+    cl.sync();
+    // running counts: each CTA an eighth of the distinct columns
+    const int u0 = (int)((long long)u * q / C), u1 = (int)((long long)u * (q + 1) / C);
+    uint32_t own = 0u;
+    for (int i = u0 + tid; i < u1; i += T) own += __ldcg(d.bcnt + base + i);
+    int tot;
+    cta_excl_scan((int)own, sh, &tot);
+    if (tid < C) cl.map_shared_rank(tots, tid)[C + q] = (uint32_t)tot;
+    cl.sync();
+    uint32_t run = 0u, deg = 0u;
+#pragma unroll
+    for (int p = 0; p < C; ++p) {
+      if (p == q) run = deg;
+      deg += tots[C + p];
+    }
+    for (int i0 = u0; i0 < u1; i0 += T) {
+      const int i = i0 + tid;
+      const uint32_t c = i < u1 ? __ldcg(d.bcnt + base + i) : 0u;
+      const uint32_t ex = (uint32_t)cta_excl_scan((int)c, sh, &tot);
+      if (i < u1) d.bcum[base + i] = run + ex + c;
+      run += (uint32_t)tot;
+    }
+    if (q == 0) {
+      if (tid == 0) row_done(a, d, b, base, u, deg);
+      nnz += u;
     }
   }
+
+  static __device__ void run(const Args& a, int vb, int vg) {
+    if (ctl_stopped(a.ctl)) return;
+    extern __shared__ __align__(16) unsigned char big_raw[];
+    __shared__ int sh[33];
+    __shared__ uint32_t tots[2 * kBigCluster];
+    uint32_t* const w1 = (uint32_t*)big_raw;
+    uint32_t* const w2 = w1 + kBigWords;
+    uint32_t* const w3 = w2 + kBigWords;
+    // clusters take directions in turn; a cluster's CTAs are consecutive
+    const int cluster = vb / kBigCluster, rank = vb % kBigCluster, nc = vg / kBigCluster / 2;
+    const int dir = cluster & 1, ci = cluster >> 1;
+    const RbSide& d = a.s[dir];
+    const int nbig = d.nlist[1], ngiant = d.nlist[2];
+    int nnz = 0;
+    for (int k = ci; k < ngiant; k += nc) giant_row(a, d, d.giant[k], w1, w2, w3, tots, sh, nnz);
+    for (int k = ci * kBigCluster + rank; k < nbig; k += nc * kBigCluster)
+      big_row(a, d, d.big[k], w1, w2, w3, sh, nnz);
+    if (dir == 0 && threadIdx.x == 0 && nnz) atomicAdd(a.nnz, nnz);
+  }
+};
+
+// A compact copy of one direction's rows (sbp_build_blockmodel hands the
+// rows out back to back): lengths, and after their scan the entries.
+struct RbCompactArgs {
+  const int32_t *bptr, *bend, *bcol;
+  const uint32_t* bcnt;
+  int32_t* len;
+  const int32_t* ptr;
+  int32_t* col;
+  uint32_t* cnt;
+  int32_t B, fill;  // fill 0: lengths, 1: entries
+};
+
+struct RbCompactBody {
+  using Args = RbCompactArgs;
+  static constexpr int kThreads = 256, kMinBlocks = 1;
+  static constexpr size_t kSmem = 0;
+  static __device__ void run(const Args& a, int vb, int vg) {
+    const int lane = threadIdx.x & 31;
+    for (int b = (vb * kThreads + threadIdx.x) >> 5; b < a.B; b += (vg * kThreads) >> 5) {
+      const int src = a.bptr[b], u = a.bend[b] - src;
+      if (!a.fill) {
+        if (lane == 0) a.len[b] = u;
+        continue;
+      }
+      const int dst = a.ptr[b];
+      for (int i = lane; i < u; i += 32) {
+        a.col[dst + i] = a.bcol[src + i];
+        a.cnt[dst + i] = a.bcnt[src + i];
+      }
+    }
   }
 };
 
 // ------------------------------------------------------------ block terms --
 struct BtArgs {
   const double* xlx;
-  const int32_t *optr, *ocol, *iptr, *icol;
-  const uint32_t *ocnt, *icnt, *d_out, *d_in;
+  const int32_t *optr, *oend, *ocol, *iptr, *iend, *icol;
+  const uint32_t *ocnt, *icnt, *ocum, *icum, *d_out, *d_in;
   const double *ld_out, *ld_in;
   double *dSout, *ambout, *ambin, *sinfull;
   int32_t* nbr_s;
   const int32_t* ctl;  // sweep control: gate, and seq += ctl[0] * seq_mul
-  int32_t B;
-  int draws;
+  int32_t B, pad;
   uint64_t seed;
   uint32_t seq, seq_mul;
 };
@@ -604,33 +699,76 @@ __device__ __forceinline__ double row_total(double s, uint32_t d, double ld) {
   return d ? __dsub_rn(s, __dmul_rn((double)d, ld)) : s;
 }
 
-// First entry k of out-row ++ in-row of block b whose running count exceeds
-// t; the whole warp returns the column (or -1).
-__device__ int warp_pick_row(const BtArgs& a, int b, uint64_t t, int lane) {
-  int o0 = a.optr[b], no = a.optr[b + 1] - o0;
-  int i0 = a.iptr[b], ni = a.iptr[b + 1] - i0;
-  int n = no + ni;
-  uint64_t acc = 0;
-  for (int k0 = 0; k0 < n; k0 += 32) {
-    int k = k0 + lane;
-    uint64_t w = 0;
-    int col = -1;
-    if (k < n) {
-      if (k < no) { w = a.ocnt[o0 + k]; col = a.ocol[o0 + k]; }
-      else { w = a.icnt[i0 + k - no]; col = a.icol[i0 + k - no]; }
-    }
-    uint64_t incl = w;
+// The draws of a nodal batch from the CSR rows (as dense_block_draw): eight
+// lanes a block find the first entry of out-row ++ in-row whose running
+// count exceeds the drawn number.  The block's out-degree tells the row; a
+// row of up to kTileMaxCap entries is summed along, a longer one has running
+// counts (the rebuild writes them) and is searched eight ways a step.  A
+// warp summing along every row took 91 us a batch of the 200k HH graph, up to
+// 700 where a block had 50k entries; this takes 24 us.
+struct BlockDrawBody {
+  using Args = BtArgs;
+  static constexpr int kThreads = 256, kMinBlocks = 1;
+  static constexpr size_t kSmem = 0;
+  static __device__ void run(const Args& a, int vb, int vg) {
+    if (ctl_stopped(a.ctl)) return;
+    const uint32_t seq = a.seq + ctl_itr(a.ctl) * a.seq_mul;
+    const int lane = threadIdx.x & 31, gl = lane & 7, hb = lane & 24;
+    const int ng = (vg * kThreads) >> 3;
+    for (int b0 = (vb * kThreads + threadIdx.x) >> 3; b0 - (hb >> 3) < a.B; b0 += ng) {
+      const int b = min(b0, a.B - 1);  // idle groups repeat the last block
+      const P4 x = draw(a.seed, kRngNodalBlock, seq, (uint32_t)b);
+      const uint32_t dout = a.d_out[b];
+      const uint64_t deg = (uint64_t)dout + a.d_in[b];
+      const uint64_t t64 = scale_draw(x.v[1], deg);
+      const bool in = t64 >= dout;
+      const uint32_t t = (uint32_t)(in ? t64 - dout : t64);  // below the row's sum
+      const int lo = (in ? a.iptr : a.optr)[b];
+      const int n = deg ? (in ? a.iend : a.oend)[b] - lo : 0;
+      const uint32_t* cnt = (in ? a.icnt : a.ocnt) + lo;
+      const uint32_t* cum = (in ? a.icum : a.ocum) + lo;
+      // [first, first + len): where the entry is; base: the count before it
+      int first = 0, len = n;
+      const bool longrow = n > kTileMaxCap;
+      while (__any_sync(kFull, longrow && len > 8)) {
+        const bool go = longrow && len > 8;
+        const int step = (len + 7) >> 3;
+        const int at = first + min((gl + 1) * step, len) - 1;
+        const unsigned m =
+            __ballot_sync(kFull, go && __ldg(cum + at) > t) >> hb & 0xffu;
+        if (go) {
+          const int j = __ffs(m) - 1;
+          first += j * step;
+          len = min(step, len - j * step);
+        }
+      }
+      int found = -1;
+      uint32_t run = 0u;
+      for (int i = 0; __any_sync(kFull, found < 0 && i < len); i += 8) {
+        const int k = first + i + gl;
+        const bool ok = i + gl < len;
+        uint32_t incl = 0u;
+        if (ok) incl = longrow ? __ldg(cum + k) : __ldg(cnt + k);
+        if (!longrow) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint64_t y = __shfl_up_sync(kFull, incl, o);
-      if (lane >= o) incl += y;
+          for (int o = 1; o < 8; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffu << hb, incl, o, 8);
+            if (gl >= o) incl += y;
+          }
+          incl += run;
+          run = __shfl_sync(0xffu << hb, incl, 7, 8);
+        }
+        __syncwarp();
+        const unsigned m = __ballot_sync(kFull, ok && incl > t) >> hb & 0xffu;
+        if (found < 0 && m) found = first + i + __ffs(m) - 1;
+      }
+      if (gl == 0 && b0 < a.B) {
+        const int nb = found >= 0 ? (in ? a.icol : a.ocol)[lo + found] : 0;
+        a.nbr_s[b] = accept_random(x.v[0], deg, (uint64_t)a.B) ? -1 : nb;
+      }
     }
-    unsigned hit = __ballot_sync(kFull, k < n && acc + incl > t);
-    if (hit) return __shfl_sync(kFull, col, __ffs(hit) - 1);
-    acc += __shfl_sync(kFull, incl, 31);
   }
-  return -1;
-}
+};
 
 struct BlockTermsBody {
   using Args = BtArgs;
@@ -638,22 +776,20 @@ struct BlockTermsBody {
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
   if (ctl_stopped(a.ctl)) return;
-  const uint32_t seq = a.seq + ctl_itr(a.ctl) * a.seq_mul;
   int lane = threadIdx.x & 31;
   int w = (vb * blockDim.x + threadIdx.x) >> 5;
   int nw = (vg * blockDim.x) >> 5;
   for (int b = w; b < a.B; b += nw) {
-    if (a.draws != 1) {
     double acc = 0.0;
     // the row's k-th nonzero is added by lane k % 32, in order of k
     // (unrolled so that several entries' loads are in flight at once)
 #pragma unroll 4
-    for (int i = a.optr[b] + lane; i < a.optr[b + 1]; i += 32)
+    for (int i = a.optr[b] + lane; i < a.oend[b]; i += 32)
       acc += cell_term(a.xlx, a.ocnt[i], a.ld_in[a.ocol[i]]);
     double ao = warp_sum(acc);
     acc = 0.0;
 #pragma unroll 4
-    for (int i = a.iptr[b] + lane; i < a.iptr[b + 1]; i += 32)
+    for (int i = a.iptr[b] + lane; i < a.iend[b]; i += 32)
       acc += cell_term(a.xlx, a.icnt[i], a.ld_out[a.icol[i]]);
     double ai = warp_sum(acc);
     if (lane == 0) {
@@ -661,17 +797,6 @@ struct BlockTermsBody {
       a.dSout[b] = row_total(ao, a.d_out[b], a.ld_out[b]);
       a.ambin[b] = ai;
       a.sinfull[b] = row_total(ai, a.d_in[b], a.ld_in[b]);
-    }
-    }
-    if (a.draws) {
-      P4 x = draw(a.seed, kRngNodalBlock, seq, (uint32_t)b);
-      uint64_t deg = (uint64_t)a.d_out[b] + a.d_in[b];
-      int nb = 0;
-      if (deg > 0) {
-        int c = warp_pick_row(a, b, scale_draw(x.v[1], deg), lane);
-        nb = c >= 0 ? c : 0;
-      }
-      if (lane == 0) a.nbr_s[b] = accept_random(x.v[0], deg, (uint64_t)a.B) ? -1 : nb;
     }
   }
   }
@@ -742,7 +867,7 @@ struct DenseDegreesBody {
 // integer sums as adding every edge (the counts are the edges' weight sums),
 // from nnz entries instead of E edges; a warp per old block row.
 struct DenseMapArgs {
-  const int32_t *bop, *boc;
+  const int32_t *bop, *boe, *boc;
   const uint32_t* bon;
   const int32_t* map;
   uint32_t *Md, *MTd, *Sd;
@@ -758,7 +883,7 @@ struct DenseFromCsrBody {
     const int K = (a.B + 31) >> 5;
     for (int r = (vb * kThreads + threadIdx.x) >> 5; r < a.B_old; r += (vg * kThreads) >> 5) {
       const int R = a.map[r];
-      for (int i = a.bop[r] + lane; i < a.bop[r + 1]; i += 32) {
+      for (int i = a.bop[r] + lane; i < a.boe[r]; i += 32) {
         const int C = a.map[a.boc[i]];
         const uint32_t w = a.bon[i];
         atomicAdd(a.Md + (size_t)R * a.B + C, w);
@@ -780,8 +905,10 @@ struct DenseCsrArgs {
   const uint32_t *Md, *MTd;
   int32_t *cnt_o, *cnt_i;  // per row: nonzero cells (the scan's input)
   const int32_t *optr, *iptr;
+  int32_t *oend, *iend;
   int32_t *ocol, *icol;
   uint32_t *ocnt, *icnt;
+  int32_t* nnz;
   int32_t B, fill;  // fill 0: count, 1: write the rows
 };
 
@@ -817,7 +944,13 @@ struct DenseCsrBody {
         }
         n += __popc(nz);
       }
-      if (!a.fill && lane == 0) (in ? a.cnt_i : a.cnt_o)[b] = n;
+      if (lane != 0) continue;
+      if (!a.fill) {
+        (in ? a.cnt_i : a.cnt_o)[b] = n;
+      } else {
+        (in ? a.iend : a.oend)[b] = k + n;
+        if (t == B - 1) *a.nnz = k + n;
+      }
     }
   }
 };
@@ -1129,8 +1262,15 @@ int grid_for(long long items, int per_block, int cap) {
 RbArgs rb_args(const DevGraph& g, const int32_t* part, int32_t B, DevBM& m, RebuildScratch& rs,
                const RebuildTune& t) {
   RbArgs a{};
-  a.warp_cap = std::max(32, std::min(kWarpCap, t.warp_cap));
+  a.tile_cap = std::max(32, std::min(kTileMaxCap, t.warp_cap));
+  a.warp_max = std::max(256, std::min(kRankMax, t.big_entries));
+  // about half a tile's entries, so that most tiles take one round
+  a.tile_rows = (int32_t)std::max<long long>(
+      8, std::min<long long>(RbTileBody::kThreads,
+                             (long long)kTileEntries / 2 * B / std::max(g.E, 1)));
   a.part = part;
+  a.xlx = m.xlx;
+  a.nnz = m.nnz;
   a.N = g.N;
   a.E = g.E;
   a.B = B;
@@ -1142,18 +1282,18 @@ RbArgs rb_args(const DevGraph& g, const int32_t* part, int32_t B, DevBM& m, Rebu
     s.gw = dir == 0 ? g.ow : g.iw;
     s.gsrc = dir == 0 ? g.osrc : g.isrc;
     s.cnt = r.cnt;
-    s.seg = r.seg;
     s.vofs = r.vofs;
     s.tcol = r.tcol;
     s.tw = r.tw;
-    s.ucol = r.ucol;
-    s.uw = r.uw;
-    s.uniq = r.uniq;
+    s.mid = r.mid;
     s.big = r.big;
-    s.big_count = rs.big_count + dir;
+    s.giant = r.giant;
+    s.nlist = rs.nlist + 3 * dir;
     s.bptr = dir == 0 ? m.optr : m.iptr;
+    s.bend = dir == 0 ? m.oend : m.iend;
     s.bcol = dir == 0 ? m.ocol : m.icol;
     s.bcnt = dir == 0 ? m.ocnt : m.icnt;
+    s.bcum = dir == 0 ? m.ocum : m.icum;
     s.bdeg = dir == 0 ? m.d_out : m.d_in;
     s.bld = dir == 0 ? m.ld_out : m.ld_in;
   }
@@ -1163,25 +1303,29 @@ RbArgs rb_args(const DevGraph& g, const int32_t* part, int32_t B, DevBM& m, Rebu
 // Virtual grids: functions of one job's sizes only.
 int32_t vg_count(const RbArgs& a) { return 2 * ceil_div(a.N, 256); }
 int32_t vg_scatter(const RbArgs& a) { return a.E > 0 ? 2 * ceil_div(a.E, 256) : 0; }
-int32_t vg_rows_small(const RbArgs& a) { return 2 * grid_for(a.B, kRowsWarps, 4096); }
-int32_t vg_rows_big(const RbArgs& a, const RebuildTune& t) {
-  const int32_t per = ceil_div(std::max(a.E, 1), std::max(256, t.big_entries));
-  return 2 * std::max(1, std::min(t.big_ctas > 0 ? t.big_ctas : 2 * 148, per));
+int32_t vg_tile(const RbArgs& a) { return 2 * ceil_div(a.B, a.tile_rows); }
+// segments longer than tile_cap entries number at most E / tile_cap
+int32_t vg_rank(const RbArgs& a) {
+  return 2 * grid_for(a.E / (a.tile_cap + 1), kRankWarps, 148 * 2);
 }
-int32_t vg_compact(const RbArgs& a) { return 2 * grid_for((long long)a.B * 32, 256, 4096); }
+int32_t vg_big(const RbArgs& a) {
+  return 2 * kBigCluster * grid_for(a.E / (a.warp_max + 1), kBigCluster, 16);
+}
 int32_t vg_words(long long n) {
   return n <= 0 ? 0 : (int32_t)std::min<long long>(4096, (n + 2047) / 2048);
 }
 
-BtArgs bt_args(DevBM& m, int32_t B, int draws, uint64_t seed, uint32_t seq) {
+BtArgs bt_args(DevBM& m, int32_t B, uint64_t seed, uint32_t seq) {
   BtArgs a{};
   a.xlx = m.xlx;
-  a.optr = m.optr; a.ocol = m.ocol; a.iptr = m.iptr; a.icol = m.icol;
-  a.ocnt = m.ocnt; a.icnt = m.icnt; a.d_out = m.d_out; a.d_in = m.d_in;
+  a.optr = m.optr; a.oend = m.oend; a.ocol = m.ocol;
+  a.iptr = m.iptr; a.iend = m.iend; a.icol = m.icol;
+  a.ocnt = m.ocnt; a.icnt = m.icnt; a.ocum = m.ocum; a.icum = m.icum;
+  a.d_out = m.d_out; a.d_in = m.d_in;
   a.ld_out = m.ld_out; a.ld_in = m.ld_in;
   a.dSout = m.dSout; a.ambout = m.ambout; a.ambin = m.ambin; a.sinfull = m.sinfull;
   a.nbr_s = m.nbr_s;
-  a.B = B; a.draws = draws; a.seed = seed; a.seq = seq;
+  a.B = B; a.seed = seed; a.seq = seq;
   return a;
 }
 
@@ -1208,6 +1352,7 @@ DenseArgs dense_args(const DevGraph& g, const int32_t* part, int32_t B, DevBM& m
 }
 
 int32_t vg_block_terms(int32_t B) { return grid_for((long long)B * 32, 256, 8192); }
+int32_t vg_block_draw(int32_t B) { return grid_for((long long)B * 8, 256, 8192); }
 int32_t vg_dense_update(int32_t count) {
   return grid_for((long long)count, 256 / 32 * kDuVerts, 148 * 16);
 }
@@ -1217,9 +1362,10 @@ const MultiKernel kmScanSingle = multi_kernel_desc<ScanSingleBody>("scan_single"
 const MultiKernel kmScanApply = multi_kernel_desc<ScanApplyBody>("scan_apply");
 const MultiKernel kmRbCount = multi_kernel_desc<RbCountBody>("rb_count");
 const MultiKernel kmRbScatter = multi_kernel_desc<RbScatterBody>("rb_scatter");
-const MultiKernel kmRbRowsSmall = multi_kernel_desc<RbRowsSmallBody>("rb_rows_small");
-const MultiKernel kmRbRowsBig = multi_kernel_desc<RbRowsBigBody>("rb_rows_big");
-const MultiKernel kmRbCompact = multi_kernel_desc<RbCompactBody>("rb_compact");
+const MultiKernel kmRbTile = multi_kernel_desc<RbTileBody>("rb_tile");
+const MultiKernel kmRbRank = multi_kernel_desc<RbRankBody>("rb_rank");
+const MultiKernel kmRbBig = multi_kernel_desc<RbBigBody>("rb_big");
+const MultiKernel kmBlockDraw = multi_kernel_desc<BlockDrawBody>("block_draw");
 const MultiKernel kmBlockTerms = multi_kernel_desc<BlockTermsBody>("block_terms");
 const MultiKernel kmBlockTermsDense = multi_kernel_desc<BlockTermsDenseBody>("block_terms_dense");
 const MultiKernel kmDenseEdges = multi_kernel_desc<DenseEdgesBody>("dense_edges");
@@ -1269,12 +1415,8 @@ void add_exclusive_scan(Slot* sl, const int32_t* in, int32_t* out, int32_t n, in
 }
 
 cudaError_t init_kernel_attributes() {
-  cudaError_t e = cudaFuncSetAttribute(single_kernel<RbRowsBigBody>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kBigSmem);
-  cudaError_t e2 = cudaFuncSetAttribute(multi_kernel<RbRowsBigBody>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)kBigSmem);
+  cudaError_t e = allow_smem<RbRankBody>();
+  cudaError_t e2 = allow_smem<RbBigBody>();
   return e != cudaSuccess ? e : e2;
 }
 
@@ -1299,26 +1441,43 @@ void scan_exclusive(const int32_t* in, int32_t* out, int32_t n, int32_t* tile, c
   launch_single<ScanApplyBody>(a, tiles, st);
 }
 
+RebuildListCaps rebuild_list_caps(int32_t N, int32_t E) {
+  return RebuildListCaps{(size_t)std::min(N, E / 32) + 1, (size_t)E / 256 + 1,
+                         (size_t)E / kBigCap + 1};
+}
+
 void rebuild_blockmodel(const DevGraph& g, const int32_t* part, int32_t B, DevBM& m,
                         RebuildScratch& rs, cudaStream_t st, const RebuildTune& t) {
   RbArgs a = rb_args(g, part, B, m, rs, t);
   for (int dir = 0; dir < 2; ++dir)
     cudaMemsetAsync(rs.d[dir].cnt, 0, sizeof(int32_t) * (size_t)B, st);
-  cudaMemsetAsync(rs.big_count, 0, sizeof(int32_t) * 2, st);
+  cudaMemsetAsync(rs.nlist, 0, sizeof(int32_t) * kRebuildCounters, st);
   launch_single<RbCountBody>(a, vg_count(a), st);
   for (int dir = 0; dir < 2; ++dir)
-    scan_exclusive(rs.d[dir].cnt, rs.d[dir].seg, B, rs.tile + dir * (rs.tile_cap / 2), st);
-  launch_single<RbScatterBody>(a, vg_scatter(a), st);
-  launch_single<RbRowsSmallBody>(a, vg_rows_small(a), st);
-  launch_single<RbRowsBigBody>(a, vg_rows_big(a, t), st);
-  for (int dir = 0; dir < 2; ++dir)
-    scan_exclusive(rs.d[dir].uniq, dir == 0 ? m.optr : m.iptr, B,
+    scan_exclusive(rs.d[dir].cnt, dir == 0 ? m.optr : m.iptr, B,
                    rs.tile + dir * (rs.tile_cap / 2), st);
-  launch_single<RbCompactBody>(a, vg_compact(a), st);
+  launch_single<RbScatterBody>(a, vg_scatter(a), st);
+  launch_single<RbTileBody>(a, vg_tile(a), st);
+  launch_single<RbRankBody>(a, vg_rank(a), st);
+  launch_single<RbBigBody>(a, vg_big(a), st);
+}
+
+void compact_rows(const DevBM& m, int32_t B, bool in, RebuildScratch& rs, int32_t* ptr,
+                  int32_t* col, uint32_t* cnt, cudaStream_t st) {
+  const RebuildDir& r = rs.d[in ? 1 : 0];
+  RbCompactArgs a{in ? m.iptr : m.optr, in ? m.iend : m.oend, in ? m.icol : m.ocol,
+                  in ? m.icnt : m.ocnt, r.cnt, ptr, col, cnt, B, 0};
+  const int32_t vg = grid_for((long long)B * 32, RbCompactBody::kThreads, 4096);
+  launch_single<RbCompactBody>(a, vg, st);
+  scan_exclusive(r.cnt, ptr, B, rs.tile, st);
+  a.fill = 1;
+  launch_single<RbCompactBody>(a, vg, st);
 }
 
 void block_terms(DevBM& m, int32_t B, int draws, uint64_t seed, uint32_t seq, cudaStream_t st) {
-  launch_single<BlockTermsBody>(bt_args(m, B, draws, seed, seq), vg_block_terms(B), st);
+  const BtArgs a = bt_args(m, B, seed, seq);
+  if (draws) launch_single<BlockDrawBody>(a, vg_block_draw(B), st);
+  else launch_single<BlockTermsBody>(a, vg_block_terms(B), st);
 }
 
 void fill_xlx_table(double* tab, cudaStream_t st) {
@@ -1361,8 +1520,8 @@ void mdl_data_sum(const DevBM& m, int32_t B, double* out, cudaStream_t st) {
 }
 
 // -------------------------------------------------------------- autotuner --
-// The rebuild's segment width (the longest segment one warp reduces; longer
-// ones go to a CTA) and the CTA grid for the long segments are picked by
+// The rebuild's segment widths (the longest segment ranked by comparison, and
+// the longest one a warp ranks through a bitmap) are picked by
 // timing rebuilds of a job's own blockmodel, once per device and size class
 // (log2 of B and of the mean segment length E/B).  Every candidate builds
 // the same matrix, so the choice changes only the time.
@@ -1401,8 +1560,8 @@ bool rebuild_tuned(int device, int32_t E, int32_t B, RebuildTune* out) {
 cudaError_t tune_rebuild(int device, const DevGraph& g, const int32_t* part, int32_t B, DevBM& m,
                          RebuildScratch& rs, cudaStream_t st, RebuildTune* out) {
   std::vector<RebuildTune> cands;
-  for (int wc : {32, 64, 128, 256})
-    for (int be : {2048, 512}) cands.push_back(RebuildTune{wc, 0, be});
+  for (int wc : {32, 64, 128})
+    for (int be : {1024, 512}) cands.push_back(RebuildTune{wc, be});
   cudaEvent_t e0, e1;
   cudaError_t err = cudaEventCreate(&e0);
   if (err != cudaSuccess) return err;
@@ -1442,18 +1601,17 @@ void RebuildSlots::clear() {
 }
 
 std::vector<Slot*> RebuildSlots::all() {
-  return {&zero,     &count,     &scan1[0],   &scan1[1], &scan1[2], &scatter,
-          &rows_small, &rows_big, &dense_count, &scan2[0], &scan2[1], &scan2[2], &compact,
-          &dense_fill};
+  return {&zero, &count, &scan1[0], &scan1[1], &scan1[2], &scatter, &tile, &rank, &big,
+          &dense_count, &scan2[0], &scan2[1], &scan2[2], &dense_fill};
 }
 
 void add_csr_from_dense(RebuildSlots& s, int32_t B, DevBM& m, RebuildScratch& rs) {
-  DenseCsrArgs a{m.Md, m.MTd, rs.d[0].uniq, rs.d[1].uniq, m.optr, m.iptr,
-                 m.ocol, m.icol, m.ocnt, m.icnt, B, 0};
+  DenseCsrArgs a{m.Md, m.MTd, rs.d[0].cnt, rs.d[1].cnt, m.optr, m.iptr, m.oend, m.iend,
+                 m.ocol, m.icol, m.ocnt, m.icnt, m.nnz, B, 0};
   const int32_t vg = grid_for((long long)2 * B * 32, 256, 148 * 16);
   slot_push(slot_bind(s.dense_count, kmDenseCsr), a, vg);
   for (int dir = 0; dir < 2; ++dir)
-    add_scan(s.scan2, rs.d[dir].uniq, dir == 0 ? m.optr : m.iptr, B,
+    add_scan(s.scan2, rs.d[dir].cnt, dir == 0 ? m.optr : m.iptr, B,
              rs.tile + dir * (rs.tile_cap / 2), nullptr);
   a.fill = 1;
   slot_push(slot_bind(s.dense_fill, kmDenseCsr), a, vg);
@@ -1464,17 +1622,15 @@ void add_rebuild(RebuildSlots& s, const DevGraph& g, const int32_t* part, int32_
   RbArgs a = rb_args(g, part, B, m, rs, t);
   a.ctl = ctl;
   for (int dir = 0; dir < 2; ++dir) add_zero(s.zero, rs.d[dir].cnt, (size_t)B, ctl);
-  add_zero(s.zero, rs.big_count, 2, ctl);
+  add_zero(s.zero, rs.nlist, kRebuildCounters, ctl);
   slot_push(slot_bind(s.count, kmRbCount), a, vg_count(a));
   for (int dir = 0; dir < 2; ++dir)
-    add_scan(s.scan1, rs.d[dir].cnt, rs.d[dir].seg, B, rs.tile + dir * (rs.tile_cap / 2), ctl);
-  slot_push(slot_bind(s.scatter, kmRbScatter), a, vg_scatter(a));
-  slot_push(slot_bind(s.rows_small, kmRbRowsSmall), a, vg_rows_small(a));
-  slot_push(slot_bind(s.rows_big, kmRbRowsBig), a, vg_rows_big(a, t));
-  for (int dir = 0; dir < 2; ++dir)
-    add_scan(s.scan2, rs.d[dir].uniq, dir == 0 ? m.optr : m.iptr, B,
+    add_scan(s.scan1, rs.d[dir].cnt, dir == 0 ? m.optr : m.iptr, B,
              rs.tile + dir * (rs.tile_cap / 2), ctl);
-  slot_push(slot_bind(s.compact, kmRbCompact), a, vg_compact(a));
+  slot_push(slot_bind(s.scatter, kmRbScatter), a, vg_scatter(a));
+  slot_push(slot_bind(s.tile, kmRbTile), a, vg_tile(a));
+  slot_push(slot_bind(s.rank, kmRbRank), a, vg_rank(a));
+  slot_push(slot_bind(s.big, kmRbBig), a, vg_big(a));
 }
 
 void DenseBuildSlots::clear() {
@@ -1505,7 +1661,7 @@ void add_dense_build_mapped(DenseBuildSlots& s, const DevGraph& g, const int32_t
   add_zero(s.zero, m.Sd, (size_t)2 * B * ((B + 31) / 32));
   add_zero(s.zero, m.d_out, (size_t)B);
   add_zero(s.zero, m.d_in, (size_t)B);
-  DenseMapArgs b{m.optr, m.ocol, m.ocnt, map, m.Md, m.MTd, m.Sd, B_old, B};
+  DenseMapArgs b{m.optr, m.oend, m.ocol, m.ocnt, map, m.Md, m.MTd, m.Sd, B_old, B};
   slot_push(slot_bind(s.mapped, kmDenseFromCsr), b, grid_for((long long)B_old * 32, 256, 148 * 16));
   DenseArgs a = dense_args(g, part, B, m);
   slot_push(slot_bind(s.degrees, kmDenseDegrees), a, ceil_div(g.N, 256));
@@ -1523,12 +1679,18 @@ void add_dense_update(Slot& s, const DevGraph& g, const int32_t* part, int32_t l
   slot_push(slot_bind(s, kmDenseUpdate), a, vg_dense_update(count));
 }
 
-void add_block_terms(Slot& s, DevBM& m, int32_t B, int draws, uint64_t seed, uint32_t seq,
-                     const int32_t* ctl, uint32_t seq_mul) {
-  BtArgs a = bt_args(m, B, draws, seed, seq);
+void add_block_terms(Slot& s, DevBM& m, int32_t B, const int32_t* ctl) {
+  BtArgs a = bt_args(m, B, 0, 0);
+  a.ctl = ctl;
+  slot_push(slot_bind(s, kmBlockTerms), a, vg_block_terms(B));
+}
+
+void add_block_draw(Slot& s, DevBM& m, int32_t B, uint64_t seed, uint32_t seq,
+                    const int32_t* ctl, uint32_t seq_mul) {
+  BtArgs a = bt_args(m, B, seed, seq);
   a.ctl = ctl;
   a.seq_mul = seq_mul;
-  slot_push(slot_bind(s, kmBlockTerms), a, vg_block_terms(B));
+  slot_push(slot_bind(s, kmBlockDraw), a, vg_block_draw(B));
 }
 
 void add_block_terms_dense(Slot& s, DevBM& m, int32_t B, int draws, uint64_t seed,

@@ -153,6 +153,7 @@ static int32_t scan_tiles_cap(int32_t N) { return 2 * (2 * ((N + 1) / 2048 + 2) 
 
 size_t job_bytes(int32_t N, int32_t E, int32_t np, int32_t max_itr, int32_t dense_cap) {
   const int32_t tiles = scan_tiles_cap(N);
+  const RebuildListCaps caps = rebuild_list_caps(N, E);
   size_t n1 = (size_t)N + 1, e = (size_t)E > 0 ? (size_t)E : 1;
   size_t b = 0;
   auto add = [&](size_t elems, size_t sz) { b += ((elems * sz) + 255) & ~size_t(255); };
@@ -162,15 +163,16 @@ size_t job_bytes(int32_t N, int32_t E, int32_t np, int32_t max_itr, int32_t dens
   // labels, snapshots, map
   for (int i = 0; i < 6; ++i) add(n1, 4);
   // blockmodel
-  add(n1, 4); add(n1, 4); add(e, 4); add(e, 4); add(e, 4); add(e, 4); add(N, 4); add(N, 4);
+  add(n1, 4); add(n1, 4); add(N, 4); add(N, 4); add(N, 4); add(N, 4);
+  for (int i = 0; i < 6; ++i) add(e, 4);
   for (int i = 0; i < 6; ++i) add(N, 8);
   add(N, 4);
   // rebuild scratch
   for (int d = 0; d < 2; ++d) {
-    add(n1, 4); add(n1, 4); add(N, 4); add(e, 4); add(e, 4); add(e, 4); add(e, 4); add(n1, 4);
-    add(N, 4);
+    add(n1, 4); add(N, 4); add(e, 4); add(e, 4);
+    add(caps.mid, 4); add(caps.big, 4); add(caps.giant, 4);
   }
-  add(2, 4);
+  add(kRebuildCounters, 4);
   add((size_t)tiles, 4);
   // nodal / merge
   add(N, 8);
@@ -302,19 +304,23 @@ sbp_status job_create(Job& J, int device, int32_t N, int32_t E, int32_t np, int3
   m.optr = A.take<int32_t>(n1); m.iptr = A.take<int32_t>(n1);
   m.ocol = A.take<int32_t>(e); m.icol = A.take<int32_t>(e);
   m.ocnt = A.take<uint32_t>(e); m.icnt = A.take<uint32_t>(e);
+  m.ocum = A.take<uint32_t>(e); m.icum = A.take<uint32_t>(e);
+  m.oend = A.take<int32_t>(N); m.iend = A.take<int32_t>(N);
   m.d_out = A.take<uint32_t>(N); m.d_in = A.take<uint32_t>(N);
   m.ld_out = A.take<double>(N); m.ld_in = A.take<double>(N);
   m.dSout = A.take<double>(N); m.ambout = A.take<double>(N);
   m.ambin = A.take<double>(N); m.sinfull = A.take<double>(N);
   m.nbr_s = A.take<int32_t>(N);
+  const RebuildListCaps caps = rebuild_list_caps(N, E);
   for (int d = 0; d < 2; ++d) {
     RebuildDir& r = J.rs.d[d];
-    r.cnt = A.take<int32_t>(n1); r.seg = A.take<int32_t>(n1); r.vofs = A.take<int32_t>(N);
+    r.cnt = A.take<int32_t>(n1); r.vofs = A.take<int32_t>(N);
     r.tcol = A.take<int32_t>(e); r.tw = A.take<uint32_t>(e);
-    r.ucol = A.take<int32_t>(e); r.uw = A.take<uint32_t>(e);
-    r.uniq = A.take<int32_t>(n1); r.big = A.take<int32_t>(N);
+    r.mid = A.take<int32_t>(caps.mid); r.big = A.take<int32_t>(caps.big);
+    r.giant = A.take<int32_t>(caps.giant);
   }
-  J.rs.big_count = A.take<int32_t>(2);
+  J.rs.nlist = A.take<int32_t>(kRebuildCounters);
+  m.nnz = J.rs.nlist + kRebuildCounters - 1;
   J.rs.tile = A.take<int32_t>(tiles);
   J.rs.tile_cap = tiles;
   J.rec = A.take<double>(N);
@@ -1060,17 +1066,22 @@ sbp_status sbp_build_blockmodel(const sbp_graph_csr* g, const int32_t* part, int
   sbp_status s = prepare(J, g, part, B, 1, 1);
   if (s != SBP_OK) return s;
   int32_t n = 0;
-  SBP_CUDA(cudaMemcpyAsync(&n, J.m.optr + B, 4, cudaMemcpyDeviceToHost, J.st));
-  SBP_CUDA(cudaStreamSynchronize(J.st));
-  SBP_CUDA(cudaGetLastError());
-  size_t b1 = (size_t)B + 1;
-  if (out_ptr) SBP_CUDA(cudaMemcpy(out_ptr, J.m.optr, 4 * b1, cudaMemcpyDeviceToHost));
-  if (in_ptr) SBP_CUDA(cudaMemcpy(in_ptr, J.m.iptr, 4 * b1, cudaMemcpyDeviceToHost));
-  if (n > 0) {
-    if (out_col) SBP_CUDA(cudaMemcpy(out_col, J.m.ocol, 4 * (size_t)n, cudaMemcpyDeviceToHost));
-    if (out_cnt) SBP_CUDA(cudaMemcpy(out_cnt, J.m.ocnt, 4 * (size_t)n, cudaMemcpyDeviceToHost));
-    if (in_col) SBP_CUDA(cudaMemcpy(in_col, J.m.icol, 4 * (size_t)n, cudaMemcpyDeviceToHost));
-    if (in_cnt) SBP_CUDA(cudaMemcpy(in_cnt, J.m.icnt, 4 * (size_t)n, cudaMemcpyDeviceToHost));
+  SBP_CUDA(cudaMemcpyAsync(&n, J.m.nnz, 4, cudaMemcpyDeviceToHost, J.st));
+  const size_t b1 = (size_t)B + 1;
+  int32_t* const ptrs[2] = {out_ptr, in_ptr};
+  int32_t* const cols[2] = {out_col, in_col};
+  uint32_t* const cnts[2] = {out_cnt, in_cnt};
+  for (int dir = 0; dir < 2; ++dir) {
+    // the rows back to back, in scratch that the rebuild no longer needs
+    int32_t *ptr = J.map, *col = J.rs.d[dir].tcol;
+    uint32_t* cnt = J.rs.d[dir].tw;
+    compact_rows(J.m, B, dir == 1, J.rs, ptr, col, cnt, J.st);
+    SBP_CUDA(cudaStreamSynchronize(J.st));
+    SBP_CUDA(cudaGetLastError());
+    if (ptrs[dir]) SBP_CUDA(cudaMemcpy(ptrs[dir], ptr, 4 * b1, cudaMemcpyDeviceToHost));
+    if (n <= 0) continue;
+    if (cols[dir]) SBP_CUDA(cudaMemcpy(cols[dir], col, 4 * (size_t)n, cudaMemcpyDeviceToHost));
+    if (cnts[dir]) SBP_CUDA(cudaMemcpy(cnts[dir], cnt, 4 * (size_t)n, cudaMemcpyDeviceToHost));
   }
   if (d_out) SBP_CUDA(cudaMemcpy(d_out, J.m.d_out, 4 * (size_t)B, cudaMemcpyDeviceToHost));
   if (d_in) SBP_CUDA(cudaMemcpy(d_in, J.m.d_in, 4 * (size_t)B, cudaMemcpyDeviceToHost));

@@ -314,7 +314,7 @@ void Engine::add_run_work(Run& r) {
       add_rebuild(pre_rebuild, J.g, J.part, r.B, J.m, J.rs, nullptr, tune_for(J, r.B));
       r.pre_bytes += 4.0 * N + 24.0 * J.E + 16.0 * r.nnz_now + 8.0 * r.B;
     }
-    add_block_terms(m_bt, J.m, r.B, 0, r.o.seed, 0);
+    add_block_terms(m_bt, J.m, r.B);
     const MergeGrid grid = merge_grid(J, r.o);
     add_merge_props(m_props, J.m, r.B, J.np, r.o.seed, r.seq, J.props, grid);
     add_merge_delta(m_delta, m_delta8, m_best, J.m, r.B, J.E, J.np, J.props, nullptr, J.best,
@@ -363,7 +363,7 @@ void Engine::add_run_work(Run& r) {
           if (k == 0 && b == 0)
             add_block_terms_dense(s.bt_dense, J.m, r.B, 1, r.o.seed, seq, ctl, nb);
         } else {
-          add_block_terms(s.bt_csr, J.m, r.B, 1, r.o.seed, seq, ctl, nb);
+          add_block_draw(s.bt_csr, J.m, r.B, r.o.seed, seq, ctl, nb);
         }
         const int ms = md.slot(dense);
         add_nodal(s.nodal[ms], s.heavy[ms], dense, md, J.g, J.part, J.m, r.B, r.o.seed, seq, lo,
@@ -387,14 +387,14 @@ void Engine::add_run_work(Run& r) {
         add_sweep_ctl(e.ctl, J.ctl, J.dsum, J.dataS, 0.0, 0.0, 0, r.sweeps_total);
       } else {
         if (dense) add_block_terms_dense(e.bt_dense, J.m, r.B, 0, r.o.seed, 0, ctl, 0);
-        else add_block_terms(e.bt_csr, J.m, r.B, 0, r.o.seed, 0, ctl, 0);
+        else add_block_terms(e.bt_csr, J.m, r.B, ctl);
         add_mdl_sum(e.mdl, J.m, r.B, J.dataS, ctl);
         add_sweep_ctl(e.ctl, J.ctl, J.dsum, J.dataS, mS, thr, r.o.window, r.o.max_nodal_itr);
       }
     }
     add_copy(s_gather, rd_dev_ptr(r.rd_off), J.ctl, 2);
     add_copy(s_gather, rd_dev_ptr(r.rd_off + 8), J.err, 1);
-    add_copy(s_gather, rd_dev_ptr(r.rd_off + 12), J.m.optr + r.B, 1);
+    add_copy(s_gather, rd_dev_ptr(r.rd_off + 12), J.m.nnz, 1);
     if (!r.sweeps_only) {
       const size_t K = (size_t)r.sweep_k;
       add_copy(s_gather, rd_dev_ptr(r.rd_off + 16), J.dsum + r.itr, 2 * K);

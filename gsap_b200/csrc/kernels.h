@@ -24,10 +24,16 @@ struct DevGraph {
 
 // Blockmodel M (out CSR rows = source block, in CSR rows = destination
 // block), weighted block degrees and their log2, and the per-block sums the
-// dS kernels start from.  Capacities: rows N+1, entries E.
+// dS kernels start from.  Row b's entries are [ptr[b], end[b]); the rows
+// ascend but need not lie back to back.  Capacities: rows N+1, entries E.
+// ocum / icum: running counts along a row, written by the rebuild for rows
+// of more than 128 entries.  nnz: entries of the out CSR.
 struct DevBM {
-  int32_t *optr = nullptr, *ocol = nullptr, *iptr = nullptr, *icol = nullptr;
-  uint32_t *ocnt = nullptr, *icnt = nullptr, *d_out = nullptr, *d_in = nullptr;
+  int32_t *optr = nullptr, *oend = nullptr, *ocol = nullptr;
+  int32_t *iptr = nullptr, *iend = nullptr, *icol = nullptr;
+  uint32_t *ocnt = nullptr, *icnt = nullptr, *ocum = nullptr, *icum = nullptr;
+  uint32_t *d_out = nullptr, *d_in = nullptr;
+  int32_t* nnz = nullptr;
   double *ld_out = nullptr, *ld_in = nullptr;
   double *dSout = nullptr;    // sum over out-row b of M (log2 M - log2 d_out[b] - log2 d_in[c])
   double *ambout = nullptr;   // sum over out-row b of M log2 M - M log2 d_in[c]
@@ -60,28 +66,34 @@ constexpr int kCommitCtas = 256;
 
 // Scratch of one rebuild direction.
 struct RebuildDir {
-  int32_t *cnt = nullptr, *seg = nullptr, *vofs = nullptr, *tcol = nullptr, *uniq = nullptr;
+  int32_t *cnt = nullptr, *vofs = nullptr, *tcol = nullptr;
   uint32_t* tw = nullptr;
-  int32_t* ucol = nullptr;
-  uint32_t* uw = nullptr;
-  int32_t* big = nullptr;
+  // rows by the kernel that reduces their segment; a list's capacity is what
+  // E entries can make (rebuild_list_caps)
+  int32_t *mid = nullptr, *big = nullptr, *giant = nullptr;
 };
 
+// Counters a rebuild starts from zero: per direction the three lists', then
+// the entries of the out CSR (DevBM::nnz).
+constexpr int kRebuildCounters = 7;
 struct RebuildScratch {
   RebuildDir d[2];
-  int32_t* big_count = nullptr;  // 2 ints
-  int32_t* tile = nullptr;       // scan tile sums (capacity >= 2 * tiles)
+  int32_t* nlist = nullptr;  // kRebuildCounters ints
+  int32_t* tile = nullptr;   // scan tile sums (capacity >= 2 * tiles)
   int32_t tile_cap = 0;
 };
+struct RebuildListCaps {
+  size_t mid, big, giant;
+};
+RebuildListCaps rebuild_list_caps(int32_t N, int32_t E);
 
 // Launch shape of a rebuild (the autotuner's choice; results never depend
-// on it): segments longer than warp_cap entries are reduced by a CTA,
-// big_ctas CTAs per direction (0: 296 at most) take one per big_entries graph
-// entries.
+// on it): segments of up to warp_cap (32 to 128) entries are ranked by
+// comparison, up to big_entries (256 to 1024) by a warp, longer ones by a
+// CTA or a cluster.
 struct RebuildTune {
-  int32_t warp_cap = 256;
-  int32_t big_ctas = 0;
-  int32_t big_entries = 2048;
+  int32_t warp_cap = 64;
+  int32_t big_entries = 1024;
 };
 
 // How a nodal move is scored and accepted.  exact = 0: GSAP's dS terms
@@ -138,8 +150,8 @@ inline Slot& slot_bind(Slot& s, const MultiKernel& k) {
 
 // The launches of a blockmodel rebuild, in order.
 struct RebuildSlots {
-  Slot zero, count, scan1[3], scatter, rows_small, rows_big, scan2[3], compact;
-  Slot dense_count, dense_fill;  // the CSR form from a fresh dense form instead
+  Slot zero, count, scan1[3], scatter, tile, rank, big;
+  Slot dense_count, scan2[3], dense_fill;  // the CSR form from a fresh dense form instead
   void clear();
   std::vector<Slot*> all();
 };
@@ -171,8 +183,10 @@ void add_dense_build(DenseBuildSlots& s, const DevGraph& g, const int32_t* part,
                      DevBM& m);
 void add_dense_update(Slot& s, const DevGraph& g, const int32_t* part, int32_t lo, int32_t count,
                       const int32_t* newlab, int32_t B, DevBM& m, const int32_t* ctl = nullptr);
-void add_block_terms(Slot& s, DevBM& m, int32_t B, int draws, uint64_t seed, uint32_t seq,
-                     const int32_t* ctl = nullptr, uint32_t seq_mul = 0);
+void add_block_terms(Slot& s, DevBM& m, int32_t B, const int32_t* ctl = nullptr);
+// The per-block draws of the nodal batch with RNG sequence seq (CSR form).
+void add_block_draw(Slot& s, DevBM& m, int32_t B, uint64_t seed, uint32_t seq,
+                    const int32_t* ctl = nullptr, uint32_t seq_mul = 0);
 void add_block_terms_dense(Slot& s, DevBM& m, int32_t B, int draws, uint64_t seed,
                            uint32_t seq, const int32_t* ctl = nullptr, uint32_t seq_mul = 0);
 // data_S into out[ctl[0]] (out[0] without ctl).
@@ -304,10 +318,14 @@ void rebuild_blockmodel(const DevGraph& g, const int32_t* part, int32_t B, DevBM
                         RebuildScratch& rs, cudaStream_t st,
                         const RebuildTune& t = RebuildTune{});
 
+// One direction's rows back to back: row pointers (B+1), columns and counts.
+void compact_rows(const DevBM& m, int32_t B, bool in, RebuildScratch& rs, int32_t* ptr,
+                  int32_t* col, uint32_t* cnt, cudaStream_t st);
+
 // Per-block work: draws == 0 computes the per-block sums (dSout, ambout,
-// ambin, sinfull; the MDL and the merge phase read them), draws == 1 only
-// the per-block draws of nodal batch `seq` (choose_neighbored_block and the
-// per-block uniform, kernels.hpp:942-997, 1024), draws == 2 both.
+// ambin, sinfull; the MDL and the merge phase read them), draws == 1 the
+// per-block draws of nodal batch `seq` (choose_neighbored_block and the
+// per-block uniform, kernels.hpp:942-997, 1024).
 void block_terms(DevBM& m, int32_t B, int draws, uint64_t seed, uint32_t seq, cudaStream_t st);
 
 // Dense form (B*B counts and their transpose, degrees and their log2) of the

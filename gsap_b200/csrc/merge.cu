@@ -29,8 +29,9 @@ int32_t vg_merge_delta(int32_t B);
 
 struct MergeArgs {
   const double* xlx;
-  const int32_t *optr, *ocol, *iptr, *icol;
+  const int32_t *optr, *oend, *ocol, *iptr, *iend, *icol;
   const uint32_t *ocnt, *icnt, *d_out, *d_in;
+  const int32_t* nnz;
   const double *ld_out, *ld_in, *dSout, *ambout, *ambin, *sinfull;
   int32_t B, np;
   uint64_t seed;
@@ -56,7 +57,7 @@ struct MergeArgs {
 __device__ __forceinline__ long long merge_grid_end(const MergeArgs& a) {
   const long long n = (long long)a.B * a.np;
   if (!a.ref_grid) return n;
-  const long long T = ((long long)a.optr[a.B] + 255) / 256 * 256;
+  const long long T = ((long long)*a.nnz + 255) / 256 * 256;
   return T < n ? T : n;
 }
 
@@ -66,7 +67,7 @@ __device__ __forceinline__ uint32_t cnt_at(const MergeArgs& a, int b, int k, int
   return k < no ? __ldg(a.ocnt + a.optr[b] + k) : __ldg(a.icnt + a.iptr[b] + k - no);
 }
 __device__ __forceinline__ int col_at(const MergeArgs& a, int b, int k) {
-  int o0 = a.optr[b], no = a.optr[b + 1] - o0;
+  int o0 = a.optr[b], no = a.oend[b] - o0;
   return k < no ? __ldg(a.ocol + o0 + k) : __ldg(a.icol + a.iptr[b] + k - no);
 }
 
@@ -86,8 +87,8 @@ __device__ __forceinline__ unsigned long long warp_incl_scan_ull(unsigned long l
 // own threshold t; returns that entry's index in the lane that asked, -1
 // where none does.  The same picks as a serial running sum.
 __device__ int warp_pick(const MergeArgs& a, int b, uint64_t t, bool want, int lane) {
-  const int no = a.optr[b + 1] - a.optr[b];
-  const int n = no + (a.iptr[b + 1] - a.iptr[b]);
+  const int no = a.oend[b] - a.optr[b];
+  const int n = no + (a.iend[b] - a.iptr[b]);
   int found = -1;
   unsigned open = __ballot_sync(kFull, want);
   unsigned long long base = 0;
@@ -158,7 +159,7 @@ __device__ void MergePropsBody::run(const MergeArgs& a, int vb, int vg) {
       const uint64_t tL = __shfl_sync(kFull, (unsigned long long)scale_draw(x.v[3], deg_u), L);
       const int k2 = warp_pick(a, uL, tL, lane == L, lane);
       if (lane == L && k2 >= 0) {
-        const int n = (a.optr[u + 1] - a.optr[u]) + (a.iptr[u + 1] - a.iptr[u]);
+        const int n = (a.oend[u] - a.optr[u]) + (a.iend[u] - a.iptr[u]);
         for (int q = k2; q < n; ++q) {
           const int c = col_at(a, u, q);
           if (c != r) {
@@ -199,23 +200,23 @@ __device__ double merge_one(const MergeArgs& a, int r, int s, int s2, int gl, bo
   // merged out-rows (calculate_dS_new_out, kernels.hpp:233-320)
   double acc_o = 0.0, acc_i = 0.0;
   const double ldo_r = a.ld_out[r], ldo_s = a.ld_out[s], ldi_r = a.ld_in[r], ldi_s = a.ld_in[s];
-  const uint32_t Mrr = row_lookup(a.ocol, a.ocnt, a.optr[r], a.optr[r + 1], r);
-  const uint32_t Mrs = row_lookup(a.ocol, a.ocnt, a.optr[r], a.optr[r + 1], s);
-  const uint32_t Msr = row_lookup(a.ocol, a.ocnt, a.optr[s], a.optr[s + 1], r);
-  const uint32_t Mss = row_lookup(a.ocol, a.ocnt, a.optr[s], a.optr[s + 1], s);
+  const uint32_t Mrr = row_lookup(a.ocol, a.ocnt, a.optr[r], a.oend[r], r);
+  const uint32_t Mrs = row_lookup(a.ocol, a.ocnt, a.optr[r], a.oend[r], s);
+  const uint32_t Msr = row_lookup(a.ocol, a.ocnt, a.optr[s], a.oend[s], r);
+  const uint32_t Mss = row_lookup(a.ocol, a.ocnt, a.optr[s], a.oend[s], s);
   if (!active) {
   } else if (r == s) {
-    for (int i = a.optr[r] + gl; i < a.optr[r + 1]; i += G)
+    for (int i = a.optr[r] + gl; i < a.oend[r]; i += G)
       acc_o += gterm(a.xlx, 2u * a.ocnt[i], a.ld_in[a.ocol[i]]);
-    for (int i = a.iptr[r] + gl; i < a.iptr[r + 1]; i += G) {
+    for (int i = a.iptr[r] + gl; i < a.iend[r]; i += G) {
       int c = a.icol[i];
       if (c != r) acc_i += gterm(a.xlx, 2u * a.icnt[i], a.ld_out[c]);
     }
   } else {
     int x = r, y = s;
-    if (a.optr[s + 1] - a.optr[s] < a.optr[r + 1] - a.optr[r]) { x = s; y = r; }
-    int y0 = a.optr[y], y1 = a.optr[y + 1];
-    for (int i = a.optr[x] + gl; i < a.optr[x + 1]; i += G) {
+    if (a.oend[s] - a.optr[s] < a.oend[r] - a.optr[r]) { x = s; y = r; }
+    int y0 = a.optr[y], y1 = a.oend[y];
+    for (int i = a.optr[x] + gl; i < a.oend[x]; i += G) {
       int c = a.ocol[i];
       double ld = a.ld_in[c];
       uint32_t my = row_lookup(a.ocol, a.ocnt, y0, y1, c);
@@ -223,9 +224,9 @@ __device__ double merge_one(const MergeArgs& a, int r, int s, int s2, int gl, bo
     }
     if (gl == 0) acc_o += a.ambout[y];
     x = r; y = s;
-    if (a.iptr[s + 1] - a.iptr[s] < a.iptr[r + 1] - a.iptr[r]) { x = s; y = r; }
-    y0 = a.iptr[y]; y1 = a.iptr[y + 1];
-    for (int i = a.iptr[x] + gl; i < a.iptr[x + 1]; i += G) {
+    if (a.iend[s] - a.iptr[s] < a.iend[r] - a.iptr[r]) { x = s; y = r; }
+    y0 = a.iptr[y]; y1 = a.iend[y];
+    for (int i = a.iptr[x] + gl; i < a.iend[x]; i += G) {
       int c = a.icol[i];
       if (c == r || c == s) continue;
       double ld = a.ld_out[c];
@@ -257,7 +258,7 @@ __device__ double merge_one(const MergeArgs& a, int r, int s, int s2, int gl, bo
   if (given_in_s) {
     in_s = in_s_given;
   } else {
-    uint32_t Ms2s = s2 == s ? 0u : row_lookup(a.ocol, a.ocnt, a.optr[s2], a.optr[s2 + 1], s);
+    uint32_t Ms2s = s2 == s ? 0u : row_lookup(a.ocol, a.ocnt, a.optr[s2], a.oend[s2], s);
     in_s = a.sinfull[s] - fterm(a.xlx, Mss, ldo_s, ldi_s) - fterm(a.xlx, Ms2s, a.ld_out[s2], ldi_s);
   }
   *in_r_out = in_r;
@@ -276,28 +277,28 @@ __device__ double merge_one_exact(const MergeArgs& a, int r, int s, int gl, bool
   double acc = 0.0;  // - (change of the off-corner cells)
   if (active) {
     int x = r, y = s;
-    if (a.optr[s + 1] - a.optr[s] < a.optr[r + 1] - a.optr[r]) { x = s; y = r; }
-    int y0 = a.optr[y], y1 = a.optr[y + 1];
-    for (int i = a.optr[x] + gl; i < a.optr[x + 1]; i += G) {
+    if (a.oend[s] - a.optr[s] < a.oend[r] - a.optr[r]) { x = s; y = r; }
+    int y0 = a.optr[y], y1 = a.oend[y];
+    for (int i = a.optr[x] + gl; i < a.oend[x]; i += G) {
       const int c = a.ocol[i];
       if (c == r || c == s) continue;
       const uint32_t b = row_lookup(a.ocol, a.ocnt, y0, y1, c);
       if (b) acc -= xlx(a.xlx, a.ocnt[i] + b) - xlx(a.xlx, a.ocnt[i]) - xlx(a.xlx, b);
     }
     x = r; y = s;
-    if (a.iptr[s + 1] - a.iptr[s] < a.iptr[r + 1] - a.iptr[r]) { x = s; y = r; }
-    y0 = a.iptr[y]; y1 = a.iptr[y + 1];
-    for (int i = a.iptr[x] + gl; i < a.iptr[x + 1]; i += G) {
+    if (a.iend[s] - a.iptr[s] < a.iend[r] - a.iptr[r]) { x = s; y = r; }
+    y0 = a.iptr[y]; y1 = a.iend[y];
+    for (int i = a.iptr[x] + gl; i < a.iend[x]; i += G) {
       const int c = a.icol[i];
       if (c == r || c == s) continue;
       const uint32_t b = row_lookup(a.icol, a.icnt, y0, y1, c);
       if (b) acc -= xlx(a.xlx, a.icnt[i] + b) - xlx(a.xlx, a.icnt[i]) - xlx(a.xlx, b);
     }
     if (gl == 0) {
-      const uint32_t Mrr = row_lookup(a.ocol, a.ocnt, a.optr[r], a.optr[r + 1], r);
-      const uint32_t Mrs = row_lookup(a.ocol, a.ocnt, a.optr[r], a.optr[r + 1], s);
-      const uint32_t Msr = row_lookup(a.ocol, a.ocnt, a.optr[s], a.optr[s + 1], r);
-      const uint32_t Mss = row_lookup(a.ocol, a.ocnt, a.optr[s], a.optr[s + 1], s);
+      const uint32_t Mrr = row_lookup(a.ocol, a.ocnt, a.optr[r], a.oend[r], r);
+      const uint32_t Mrs = row_lookup(a.ocol, a.ocnt, a.optr[r], a.oend[r], s);
+      const uint32_t Msr = row_lookup(a.ocol, a.ocnt, a.optr[s], a.oend[s], r);
+      const uint32_t Mss = row_lookup(a.ocol, a.ocnt, a.optr[s], a.oend[s], s);
       const uint32_t dor = a.d_out[r], dos = a.d_out[s], dir = a.d_in[r], dis = a.d_in[s];
       const double corner = xlx(a.xlx, Mrr + Mrs + Msr + Mss) - xlx(a.xlx, Mrr) -
                             xlx(a.xlx, Mrs) - xlx(a.xlx, Msr) - xlx(a.xlx, Mss);
@@ -470,7 +471,9 @@ const MultiKernel kmRelabel = multi_kernel_desc<RelabelBody>("relabel");
 MergeArgs make_args(const DevBM& m, int32_t B, int32_t np, const MergeGrid& grid) {
   MergeArgs a{};
   a.xlx = m.xlx;
-  a.optr = m.optr; a.ocol = m.ocol; a.iptr = m.iptr; a.icol = m.icol;
+  a.optr = m.optr; a.oend = m.oend; a.ocol = m.ocol;
+  a.iptr = m.iptr; a.iend = m.iend; a.icol = m.icol;
+  a.nnz = m.nnz;
   a.ocnt = m.ocnt; a.icnt = m.icnt; a.d_out = m.d_out; a.d_in = m.d_in;
   a.ld_out = m.ld_out; a.ld_in = m.ld_in; a.dSout = m.dSout; a.ambout = m.ambout;
   a.ambin = m.ambin; a.sinfull = m.sinfull;

@@ -23,8 +23,21 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 namespace sbp {
+
+// A body that sets kCluster runs its blocks in clusters of that size: its
+// virtual grids are multiples of it, so a cluster's blocks belong to one job
+// and are consecutive virtual blocks.
+template <class Body, class = void>
+struct ClusterOf {
+  static constexpr int value = 1;
+};
+template <class Body>
+struct ClusterOf<Body, std::void_t<decltype(Body::kCluster)>> {
+  static constexpr int value = Body::kCluster;
+};
 
 template <class Body>
 __global__ void __launch_bounds__(Body::kThreads, Body::kMinBlocks)
@@ -33,7 +46,13 @@ __global__ void __launch_bounds__(Body::kThreads, Body::kMinBlocks)
 }
 
 template <class Body>
-__global__ void __launch_bounds__(Body::kThreads, Body::kMinBlocks) multi_kernel(MultiSpan sp) {
+__global__ void __launch_bounds__(Body::kThreads, Body::kMinBlocks)
+    __cluster_dims__(ClusterOf<Body>::value, 1, 1) single_cluster_kernel(typename Body::Args a) {
+  Body::run(a, (int)blockIdx.x, (int)gridDim.x);
+}
+
+template <class Body>
+__device__ __forceinline__ void run_multi(const MultiSpan& sp) {
   using Args = typename Body::Args;
   static_assert(sizeof(Args) % 8 == 0, "argument records are copied in 8-byte words");
   constexpr int kWords = (int)(sizeof(Args) / 8);
@@ -71,6 +90,17 @@ __global__ void __launch_bounds__(Body::kThreads, Body::kMinBlocks) multi_kernel
   }
 }
 
+template <class Body>
+__global__ void __launch_bounds__(Body::kThreads, Body::kMinBlocks) multi_kernel(MultiSpan sp) {
+  run_multi<Body>(sp);
+}
+
+template <class Body>
+__global__ void __launch_bounds__(Body::kThreads, Body::kMinBlocks)
+    __cluster_dims__(ClusterOf<Body>::value, 1, 1) multi_cluster_kernel(MultiSpan sp) {
+  run_multi<Body>(sp);
+}
+
 constexpr int kMaxMultiGrid = 1 << 22;
 
 template <class Body>
@@ -78,14 +108,38 @@ void launch_multi(const MultiSpan& sp, cudaStream_t st) {
   if (sp.total <= 0) return;
   const int grid = std::min(sp.total, kMaxMultiGrid);
   ++g_launches;
-  multi_kernel<Body><<<grid, Body::kThreads, Body::kSmem, st>>>(sp);
+  if constexpr (ClusterOf<Body>::value > 1)
+    multi_cluster_kernel<Body><<<grid, Body::kThreads, Body::kSmem, st>>>(sp);
+  else
+    multi_kernel<Body><<<grid, Body::kThreads, Body::kSmem, st>>>(sp);
 }
 
 template <class Body>
 void launch_single(const typename Body::Args& a, int grid, cudaStream_t st) {
   if (grid <= 0) return;
   ++g_launches;
-  single_kernel<Body><<<grid, Body::kThreads, Body::kSmem, st>>>(a);
+  if constexpr (ClusterOf<Body>::value > 1)
+    single_cluster_kernel<Body><<<grid, Body::kThreads, Body::kSmem, st>>>(a);
+  else
+    single_kernel<Body><<<grid, Body::kThreads, Body::kSmem, st>>>(a);
+}
+
+// Opts both kernels of a body in to its dynamic shared memory; once per
+// device, before the first launch.
+template <class Body>
+cudaError_t allow_smem() {
+  auto set = [](const void* f) {
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Body::kSmem);
+  };
+  cudaError_t e, e2;
+  if constexpr (ClusterOf<Body>::value > 1) {
+    e = set((const void*)single_cluster_kernel<Body>);
+    e2 = set((const void*)multi_cluster_kernel<Body>);
+  } else {
+    e = set((const void*)single_kernel<Body>);
+    e2 = set((const void*)multi_kernel<Body>);
+  }
+  return e != cudaSuccess ? e : e2;
 }
 
 // One job's record through the by-value kernel, same virtual grid: a slot

@@ -54,7 +54,7 @@ struct NodalArgs {
   const int32_t *optr, *oidx, *iptr, *iidx;
   const uint32_t *ow, *iw, *kdo, *kdi;
   const int32_t* part;
-  const int32_t *bop, *boc, *bip, *bic;
+  const int32_t *bop, *boe, *boc, *bip, *bie, *bic;
   const uint32_t *bon, *bin, *d_out, *d_in;
   const uint32_t *Md, *MTd;
   const double *ld_out, *ld_in;
@@ -98,9 +98,9 @@ struct Rows<false> {
   const uint32_t *on, *inn;
   int32_t rO0, rO1, sO0, sO1, rI0, rI1, sI0, sI1;
   __device__ Rows(const NodalArgs& a, int r, int s)
-      : oc(a.boc), ic(a.bic), on(a.bon), inn(a.bin), rO0(a.bop[r]), rO1(a.bop[r + 1]),
-        sO0(a.bop[s]), sO1(a.bop[s + 1]), rI0(a.bip[r]), rI1(a.bip[r + 1]), sI0(a.bip[s]),
-        sI1(a.bip[s + 1]) {}
+      : oc(a.boc), ic(a.bic), on(a.bon), inn(a.bin), rO0(a.bop[r]), rO1(a.boe[r]),
+        sO0(a.bop[s]), sO1(a.boe[s]), rI0(a.bip[r]), rI1(a.bie[r]), sI0(a.bip[s]),
+        sI1(a.bie[s]) {}
   __device__ __forceinline__ uint32_t out_r(int c) const { return row_lookup(oc, on, rO0, rO1, c); }
   __device__ __forceinline__ uint32_t out_s(int c) const { return row_lookup(oc, on, sO0, sO1, c); }
   __device__ __forceinline__ uint32_t in_r(int c) const { return row_lookup(ic, inn, rI0, rI1, c); }
@@ -480,9 +480,8 @@ __device__ __forceinline__ void row_counts(const NodalArgs& a, int row, const bo
     int32_t lo[E], hi[E], end[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
-      const int32_t* p = (in[j] ? a.bip : a.bop) + row;
-      lo[j] = want[j] ? __ldg(p) : 0;
-      hi[j] = end[j] = want[j] ? __ldg(p + 1) : 0;
+      lo[j] = want[j] ? __ldg((in[j] ? a.bip : a.bop) + row) : 0;
+      hi[j] = end[j] = want[j] ? __ldg((in[j] ? a.bie : a.boe) + row) : 0;
     }
     bool go = true;
     while (go) {
@@ -1801,7 +1800,8 @@ NodalArgs make_args(const DevGraph& g, const int32_t* part, const DevBM& m, int3
   a.optr = g.optr; a.oidx = g.oidx; a.iptr = g.iptr; a.iidx = g.iidx;
   a.ow = g.ow; a.iw = g.iw; a.kdo = g.kdo; a.kdi = g.kdi;
   a.part = part;
-  a.bop = m.optr; a.boc = m.ocol; a.bip = m.iptr; a.bic = m.icol;
+  a.bop = m.optr; a.boe = m.oend; a.boc = m.ocol;
+  a.bip = m.iptr; a.bie = m.iend; a.bic = m.icol;
   a.bon = m.ocnt; a.bin = m.icnt; a.d_out = m.d_out; a.d_in = m.d_in;
   a.Md = m.Md; a.MTd = m.MTd;
   a.ld_out = m.ld_out; a.ld_in = m.ld_in;
