@@ -144,10 +144,22 @@ class Engine {
   void *up_host = nullptr, *up_dev = nullptr, *desc_host = nullptr, *desc_dev = nullptr;
   void *rd_host = nullptr, *rd_dev = nullptr;
   size_t up_cap = 0, desc_cap = 0, rd_cap = 0;
-  cudaGraphExec_t graph_exec = nullptr;  // the last captured sweep tick
-  std::vector<unsigned char> graph_key;    // what the graph's launches were made from
-  std::vector<unsigned char> key_scratch;
-  long long graph_kernels = 0;            // kernel launches the graph holds
+  // The queued sweeps of a tick as an executable graph.  One per sequence of
+  // kernels (`shape`), at most kMaxGraphs, the least recently used replaced:
+  // a graph of the same shape takes new arguments in place (some 60 us),
+  // one of another shape has to be instantiated (1.7 ms), and a partition
+  // passes through two or three shapes (CSR and dense sweeps).
+  struct SweepGraph {
+    cudaGraphExec_t exec = nullptr;
+    std::vector<unsigned char> shape, key;  // key: what its launches were made from
+    long long kernels = 0;                  // kernel launches it holds
+    long long used = 0;
+  };
+  static constexpr size_t kMaxGraphs = 6;
+  std::vector<SweepGraph> graphs;
+  long long graph_use = 0;
+  std::vector<unsigned char> key_scratch, shape_scratch;
+  std::vector<unsigned char> last_key, last_shape;  // of the tick before
   int nb_slots_ = 0;  // batch positions per queued sweep in this tick's slots
 
   void* up_dev_ptr(size_t off) { return (char*)up_dev + off; }
