@@ -619,6 +619,7 @@ void classify_batch(const Job& J, const int32_t* verts, int32_t lo, int32_t coun
     cls[i] = heavy_vertex(J, v) ? 2 : e <= kSmallEntries ? 0 : 1;
     ++n[cls[i]];
     if (cls[i] == 1 && e > kGroupEntries / 2) ++n[e > kGroupEntries ? 3 : 4];
+    if (cls[i] == 2 && e > kHubEntries) ++n[5];
     if (cls[i] < 2) emax = std::max(emax, e);
   }
   std::vector<int32_t> start((size_t)emax + 2, 0);
@@ -650,6 +651,7 @@ NodalAux nodal_lists(Job& J, const int32_t* dev, const int32_t n[kListCounts]) {
   a.nmid64 = n[4];
   a.heavy = dev + n[0] + n[1];
   a.nheavy = n[2];
+  a.nhub = n[5];
   a.err = J.err;
   a.side = J.side;
   a.fork = J.fork;

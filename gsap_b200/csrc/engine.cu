@@ -191,7 +191,9 @@ Engine::~Engine() {
   if (ev_first) cudaEventDestroy(ev_first);
   if (fork) cudaEventDestroy(fork);
   if (join) cudaEventDestroy(join);
+  if (join2) cudaEventDestroy(join2);
   if (side) cudaStreamDestroy(side);
+  if (side2) cudaStreamDestroy(side2);
   cudaStreamDestroy(st);
 }
 
@@ -200,6 +202,8 @@ sbp_status Engine::init(int dev) {
   SBP_CUDA(cudaSetDevice(device));
   SBP_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   SBP_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+  SBP_CUDA(cudaStreamCreateWithFlags(&side2, cudaStreamNonBlocking));
+  SBP_CUDA(cudaEventCreateWithFlags(&join2, cudaEventDisableTiming));
   SBP_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
   SBP_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
   return SBP_OK;
@@ -239,6 +243,7 @@ void Engine::clear_slots() {
   for (auto& b : sw) {
     for (Slot* s : {&b.bt_csr, &b.bt_dense, &b.dupd, &b.commit}) s->clear();
     for (Slot& s : b.heavy) s.clear();
+    for (Slot& s : b.hub) s.clear();
     for (Slot& s : b.nodal) s.clear();
     b.rebuild.clear();
   }
@@ -367,7 +372,7 @@ void Engine::add_run_work(Run& r) {
           add_block_draw(s.bt_csr, J.m, r.B, r.o.seed, seq, ctl, nb);
         }
         const int ms = md.slot(dense);
-        add_nodal(s.nodal[ms], s.heavy[ms], dense, md, J.g, J.part, J.m, r.B, r.o.seed, seq, lo,
+        add_nodal(s.nodal[ms], s.heavy[ms], s.hub[dense ? 1 : 0], dense, md, J.g, J.part, J.m, r.B, r.o.seed, seq, lo,
                   r.BS, J.newlab, J.rec, nullptr,
                   nodal_lists(J, J.lists + r.list_off[b], &r.list_n[kListCounts * (size_t)b]), ctl, nb);
         if (dense) {
@@ -523,6 +528,7 @@ sbp_status Engine::tick() {
       order.push_back(&w.bt_csr);
       order.push_back(&w.bt_dense);
       for (Slot& x : w.heavy) order.push_back(&x);
+      for (Slot& x : w.hub) order.push_back(&x);
       for (Slot& x : w.nodal) order.push_back(&x);
       order.push_back(&w.dupd);
       order.push_back(&w.commit);
@@ -613,11 +619,23 @@ sbp_status Engine::tick() {
         sbp_status q = emit_until(&w.bt_dense);
         if (q != SBP_OK) return q;
         if (timing) SBP_CUDA(record(be[1]));
-        bool heavy = false;
-        for (const Slot& x : w.heavy) heavy = heavy || !x.empty();
+        // heavy vertices and hubs on the side streams, next to the warp kernels
+        auto any = [](auto& slots) {
+          bool some = false;
+          for (const Slot& x : slots) some = some || !x.empty();
+          return some;
+        };
+        const bool heavy = any(w.heavy), hub = any(w.hub);
+        if (heavy || hub) SBP_CUDA(cudaEventRecord(fork, st));
+        if (hub) {
+          SBP_CUDA(cudaStreamWaitEvent(side2, fork, 0));
+          for (Slot& x : w.hub) {
+            q = launch_slot(x, slot_off(&x), side2);
+            if (q != SBP_OK) return q;
+          }
+          SBP_CUDA(cudaEventRecord(join2, side2));
+        }
         if (heavy) {
-          // heavy vertices on the side stream, next to the warp kernels
-          SBP_CUDA(cudaEventRecord(fork, st));
           SBP_CUDA(cudaStreamWaitEvent(side, fork, 0));
           for (Slot& x : w.heavy) {
             q = launch_slot(x, slot_off(&x), side);
@@ -625,10 +643,11 @@ sbp_status Engine::tick() {
           }
           SBP_CUDA(cudaEventRecord(join, side));
         }
-        i += 4;  // the heavy slots
+        i += 6;  // the heavy and hub slots
         q = emit_until(&w.nodal[3]);
         if (q != SBP_OK) return q;
         if (heavy) SBP_CUDA(cudaStreamWaitEvent(st, join, 0));
+        if (hub) SBP_CUDA(cudaStreamWaitEvent(st, join2, 0));
         if (timing) SBP_CUDA(record(be[2]));
         q = emit_until(&w.commit);
         if (q != SBP_OK) return q;

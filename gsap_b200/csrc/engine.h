@@ -98,7 +98,7 @@ struct Run {
 // The launches of one nodal batch position across runs.
 struct SweepSlots {
   // heavy / nodal indexed by ScoreMode::slot(dense)
-  Slot bt_csr, bt_dense, heavy[4], nodal[4], dupd, commit;
+  Slot bt_csr, bt_dense, heavy[4], hub[2], nodal[4], dupd, commit;
   RebuildSlots rebuild;
 };
 
@@ -110,8 +110,8 @@ struct SweepEndSlots {
 class Engine {
  public:
   int device = 0;
-  cudaStream_t st = nullptr, side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
+  cudaStream_t st = nullptr, side = nullptr, side2 = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr;
   std::vector<Run*> runs;
   long long ticks = 0;
   cudaEvent_t ev_first = nullptr;  // recorded at the first tick

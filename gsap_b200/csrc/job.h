@@ -132,9 +132,9 @@ inline ScoreMode score_mode(const sbp_options& o) {
 bool heavy_vertex(const Job& J, int32_t v);
 // Appends the batch indices i in [0, count) of vertices lo + i (verts[i]
 // when verts is given) to `out`, grouped by nodal kernel path: small, mid,
-// heavy (NodalAux); n receives the three group sizes and the mid list's
-// counts of large vertices and of those of up to kGroupEntries entries.
-constexpr int kListCounts = 5;
+// heavy (NodalAux); n receives the three group sizes, the mid list's counts of
+// large vertices and of those of up to kGroupEntries entries, and the hubs.
+constexpr int kListCounts = 6;
 void classify_batch(const Job& J, const int32_t* verts, int32_t lo, int32_t count,
                     std::vector<int32_t>& out, int32_t n[kListCounts]);
 // The NodalAux of groups of such sizes stored back to back at `dev`.

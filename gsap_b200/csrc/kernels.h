@@ -198,11 +198,11 @@ void add_zero(Slot& s, void* p, size_t words, const int32_t* ctl = nullptr);
 void add_copy(Slot& s, void* dst, const void* src, size_t words);
 void add_iota(Slot& s, int32_t* p, int32_t n);
 // Nodal batch of one job: the warp kernel's record goes to `warp`, the
-// CTA-per-vertex kernel's (heavy vertices) to `heavy`.  Use separate slots
-// per md.slot(dense): dense and CSR jobs, GSAP-mode and general-mode jobs
-// run different kernels.
+// CTA-per-vertex kernel's (heavy vertices) to `heavy`, the hubs' to `hub`.
+// Use separate slots per md.slot(dense): dense and CSR jobs, GSAP-mode and
+// general-mode jobs run different kernels.
 struct NodalAux;
-void add_nodal(Slot& warp, Slot& heavy, bool dense, const ScoreMode& md, const DevGraph& g,
+void add_nodal(Slot& warp, Slot& heavy, Slot& hub, bool dense, const ScoreMode& md, const DevGraph& g,
                const int32_t* part,
                const DevBM& m, int32_t B, uint64_t seed, uint32_t seq, int32_t lo, int32_t count,
                int32_t* newlab, double* rec, int32_t* props, const NodalAux& lists,
@@ -350,18 +350,18 @@ int nodal_heavy_threshold();
 
 // A batch's vertices (indices into the batch) by kernel path: small ones (at
 // most kSmallEntries neighbour entries), mid ones, and heavy ones (more than
-// nodal_heavy_threshold() entries in a direction), one to a CTA on the side
-// stream.  The mid list runs from the most entries down: the first nlarge
+// nodal_heavy_threshold() entries in a direction), on a side stream; the first
+// nhub of these have more than kHubEntries entries in all.  The mid list runs from the most entries down: the first nlarge
 // have more than kGroupEntries, the next nmid64 more than kGroupEntries / 2.
 // err counts hash-table overflows (should stay 0).
-constexpr int32_t kSmallEntries = 16, kGroupEntries = 64;
+constexpr int32_t kSmallEntries = 16, kGroupEntries = 64, kHubEntries = 1024;
 struct NodalAux {
   const int32_t* small = nullptr;
   int32_t nsmall = 0;
   const int32_t* mid = nullptr;
   int32_t nmid = 0, nlarge = 0, nmid64 = 0;
   const int32_t* heavy = nullptr;
-  int32_t nheavy = 0;
+  int32_t nheavy = 0, nhub = 0;
   int32_t* err = nullptr;
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;

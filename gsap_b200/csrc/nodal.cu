@@ -38,6 +38,8 @@
 #include "multi.cuh"
 #include "dense.cuh"
 
+#include <cooperative_groups.h>
+
 #include <type_traits>
 
 namespace sbp {
@@ -69,8 +71,8 @@ struct NodalArgs {
   double* rec;
   int32_t* props_out;
   double* dS_raw;
-  const int32_t* heavy;     // batch indices handled by the CTA kernel
-  int32_t nheavy;
+  const int32_t* heavy;     // batch indices handled by the CTA kernels, hubs first
+  int32_t nheavy, nhub;
   const int32_t *small, *mid;  // batch indices of the warp kernel (NodalItems)
   int32_t nsmall, nmid;
   int32_t nlarge, nmid64;      // mid vertices by size: large, up to kGroupEntries, the others
@@ -1376,216 +1378,216 @@ struct NodalBody<GIVEN, DENSE, true> {
   }
 };
 
-// A vertex of more than kWarpList entries in a direction on a CTA.  Its
-// threads take the entries of each direction strided by kHeavyThreads, and
-// each subtracts its entries' terms in the order of P hash classes of blocks
-// (P = entries / 2048), then of the index: the order of a table that holds
-// one class at a time, kept because the sum's rounding is part of the
-// result.  What is free is the table: one of both directions' blocks, filled
-// once and sized to the vertex, whenever its blocks are sure to fit (n
-// entries, or 2 B blocks, at most half the slots), else one per class.  Four
-// entries a thread are in flight at a time and the keys of the first
-// kHeavyStage entries stay in shared memory.  What bounds it is the latency
-// of the chain of steps, a launch of few CTAs (20k HH graph, 12-30 such
-// vertices a graph: 13 us a launch in the median, 27 with a warp walking the
-// vertex's entries for the proposal and the table cleared, filled and read
-// per direction).
-constexpr int kHeavyStage = 4096;
-constexpr size_t kHeavySmem = (3 * kHashSlots + kHeavyStage) * sizeof(int32_t);
+// What the CTA paths of heavy vertices share: a vertex's entries (out-entries,
+// then in-entries) as direction-tagged keys, and a shared-memory table from
+// key to the key's total weight and first entry (open addressing).
+struct HeavyEntries {
+  const NodalArgs& a;
+  int32_t o0, i0;
+  int no, n;
+  bool unit;  // every weight is 1
+  __device__ HeavyEntries(const NodalArgs& args, int v)
+      : a(args), o0(args.optr[v]), i0(args.iptr[v]), no(args.optr[v + 1] - o0),
+        n(no + args.iptr[v + 1] - i0) {
+    // weights are at least 1
+    unit = (uint64_t)args.kdo[v] + args.kdi[v] == (uint64_t)n;
+  }
+  __device__ __forceinline__ uint32_t key(int k) const {
+    return k < no ? (uint32_t)__ldg(a.part + __ldg(a.oidx + o0 + k))
+                  : (uint32_t)__ldg(a.part + __ldg(a.iidx + i0 + k - no)) | 0x80000000u;
+  }
+  __device__ __forceinline__ uint32_t w(int k) const {
+    return unit ? 1u : k < no ? __ldg(a.ow + o0 + k) : __ldg(a.iw + i0 + k - no);
+  }
+};
+
+struct HeavyTab {
+  int32_t* key;  // -1 = empty (blocks lie below 2^31 - 1, so no key is -1)
+  uint32_t* sum;
+  int32_t* first;
+  int slots;  // a power of two
+  __device__ __forceinline__ void clear() const {
+    for (int k = threadIdx.x; k < slots; k += kHeavyThreads) {
+      key[k] = -1;
+      sum[k] = 0u;
+      first[k] = 0x7fffffff;
+    }
+  }
+  __device__ __forceinline__ uint32_t slot(uint32_t x) const {
+    return (x * 2654435761u) >> 16 & (uint32_t)(slots - 1);
+  }
+  // entry k of key x and weight w; false when the table is full
+  __device__ __forceinline__ bool add(uint32_t x, uint32_t w, int k) const {
+    uint32_t q = slot(x);
+    for (int probe = 0; probe < slots; ++probe, q = (q + 1) & (uint32_t)(slots - 1)) {
+      int32_t cur = *(volatile int32_t*)(key + q);
+      if (cur == -1) cur = atomicCAS(key + q, -1, (int32_t)x);
+      if (cur == -1 || cur == (int32_t)x) {
+        atomicAdd(sum + q, w);
+        atomicMin(first + q, k);
+        return true;
+      }
+    }
+    return false;
+  }
+  __device__ __forceinline__ uint32_t find(uint32_t x) const {
+    uint32_t q = slot(x);
+    for (int probe = 0; probe < slots && key[q] != (int32_t)x; ++probe)
+      q = (q + 1) & (uint32_t)(slots - 1);
+    return q;
+  }
+};
+
+// The block that v proposes (the same in every thread of the CTA); wsum and
+// at are the CTA's shared scratch, get(k) an entry's key.
+template <bool GIVEN, class Get>
+__device__ __forceinline__ int heavy_proposal(const NodalArgs& a, int i, int v,
+                                              const HeavyEntries& e, unsigned long long* wsum,
+                                              int* at, Get get) {
+  if (GIVEN) return a.props_in[i];
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const P4 x = draw(a.seed, kRngNodalVertex, a.seq + ctl_itr(a.ctl) * a.seq_mul, (uint32_t)v);
+  const int rnd = (int)(x.v[0] % (uint32_t)a.B);
+  const uint64_t target = scale_draw(x.v[1], (uint64_t)a.kdo[v] + a.kdi[v]);
+  int k = (int)target;
+  if (!e.unit) {
+    // the first entry whose running weight exceeds the target: the thread
+    // whose run of consecutive entries holds it
+    if (t == 0) *at = -1;
+    const int per = (e.n + kHeavyThreads - 1) / kHeavyThreads;
+    const int k0 = min(e.n, t * per), k1 = min(e.n, k0 + per);
+    uint64_t own = 0;
+    for (int q = k0; q < k1; ++q) own += e.w(q);
+    uint64_t incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[wid] = incl;
+    __syncthreads();
+    for (int q = 0; q < wid; ++q) incl += wsum[q];
+    uint64_t run = incl - own;
+    if (run <= target && target < incl)
+      for (int q = k0; q < k1; ++q) {
+        run += e.w(q);
+        if (run > target) {
+          *at = q;
+          break;
+        }
+      }
+    __syncthreads();
+    k = *at;
+  }
+  return proposed(a, k >= 0 ? (int)(get(k) & 0x7fffffffu) : a.part[0], rnd);
+}
+
+// koR, koS, niR, niS, out-entries in r, in s of one entry into cnt[0..5].
+__device__ __forceinline__ void add_rs(uint32_t* cnt, bool in, int c, int r, int s, uint32_t w) {
+  if (c == r) {
+    atomicAdd(cnt + (in ? 2 : 0), w);
+    if (!in) atomicAdd(cnt + 4, 1u);
+  }
+  if (c == s) {
+    atomicAdd(cnt + (in ? 3 : 1), w);
+    if (!in) atomicAdd(cnt + 5, 1u);
+  }
+}
+
+// Corner counts and degrees for corner_term, on a full warp.
+template <bool DENSE>
+__device__ __forceinline__ Corner load_corner(const NodalArgs& a, int v, int r, int s, int lane) {
+  const uint32_t mm =
+      lane < 4 ? Rows<DENSE>(a, r, s).out_at((lane & 2) != 0, (lane & 1) ? s : r) : 0u;
+  Corner q{};
+  load_degrees(a, v, r, s, q);
+  q.Mrr = __shfl_sync(kFull, mm, 0);
+  q.Mrs = __shfl_sync(kFull, mm, 1);
+  q.Msr = __shfl_sync(kFull, mm, 2);
+  q.Mss = __shfl_sync(kFull, mm, 3);
+  return q;
+}
+
+// A vertex of more than kWarpList entries in a direction, at most
+// kHubEntries in all, on a CTA: its threads take the entries of each
+// direction strided by kHeavyThreads and subtract their terms in that order.
+// Up to four entries a thread are in flight at a time.  The table and the
+// keys take 28 KB of shared memory, so that the SM keeps its L1 for these
+// CTAs and the warp kernel's beside them (with the hubs' 112 KB here, the
+// terms of a 500-entry vertex alone took 5.6 us, all of it L2 latency).  13 us
+// a launch at 200k HH.
+constexpr size_t kHeavySmem = (3 * 2 * kHubEntries + kHubEntries) * sizeof(int32_t);
 
 template <bool GIVEN, bool DENSE>
 __device__ void heavy_vertex(const NodalArgs& a, int i, const Group<kHeavyThreads>& grp) {
   constexpr int T = kHeavyThreads, U = 4;
   extern __shared__ unsigned long long hsm[];
   __shared__ unsigned long long wsum[T / 32];
-  __shared__ uint32_t cnt[6];  // koR, koS, niR, niS, out-entries in r, in s
-  __shared__ int s_at, overflow;
-  int32_t* const tkey = (int32_t*)hsm;
-  uint32_t* const tsum = (uint32_t*)hsm + kHashSlots;
-  int32_t* const tfirst = (int32_t*)hsm + 2 * kHashSlots;
-  uint32_t* const stage = (uint32_t*)hsm + 3 * kHashSlots;
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  __shared__ uint32_t cnt[6];
+  __shared__ int s_at;
+  const int t = threadIdx.x, lane = t & 31;
   const int v = GIVEN ? a.verts[i] : a.lo + i;
-  const int32_t o0 = a.optr[v], no = a.optr[v + 1] - o0;
-  const int32_t i0 = a.iptr[v], ni = a.iptr[v + 1] - i0;
-  const int n = no + ni;
-  const int r = a.part[v];
-  const uint64_t deg = (uint64_t)a.kdo[v] + a.kdi[v];
-  const bool unit = deg == (uint64_t)n;  // weights are at least 1
-  // entry k: out-entries, then in-entries; the direction in the top bit
-  auto load_key = [&](int k) {
-    return k < no ? (uint32_t)__ldg(a.part + __ldg(a.oidx + o0 + k))
-                  : (uint32_t)__ldg(a.part + __ldg(a.iidx + i0 + k - no)) | 0x80000000u;
-  };
-  auto entry_key = [&](int k) { return k < kHeavyStage ? stage[k] : load_key(k); };
-  auto entry_w = [&](int k) {
-    return unit ? 1u : k < no ? __ldg(a.ow + o0 + k) : __ldg(a.iw + i0 + k - no);
-  };
-  const int nst = min(n, kHeavyStage);
-#pragma unroll 4
-  for (int k = t; k < nst; k += T) stage[k] = load_key(k);
-  const bool fits = n <= kHashSlots / 2 || 2LL * a.B <= kHashSlots / 2;
+  const HeavyEntries e(a, v);
+  const int n = e.n, no = e.no;
   int slots = 512;
-  while (slots < kHashSlots && (!fits || slots < 2 * min(n, 2 * a.B))) slots <<= 1;
-  const uint32_t smask = (uint32_t)slots - 1u;
-  auto clear = [&] {
-    for (int k = t; k < slots; k += T) {
-      tkey[k] = -1;
-      tsum[k] = 0u;
-      tfirst[k] = 0x7fffffff;
-    }
-  };
-  // a tagged key is never -1: blocks lie below 2^31 - 1
-  auto slot0 = [&](uint32_t key) { return (key * 2654435761u) >> 16 & smask; };
-  auto add = [&](uint32_t key, uint32_t w, int k) {
-    uint32_t q = slot0(key);
-    for (int probe = 0; probe < slots; ++probe, q = (q + 1) & smask) {
-      const int32_t cur = atomicCAS(tkey + q, -1, (int32_t)key);
-      if (cur == -1 || cur == (int32_t)key) {
-        atomicAdd(tsum + q, w);
-        atomicMin(tfirst + q, k);
-        return;
-      }
-    }
-    overflow = 1;
-  };
-  clear();
+  while (slots < 2 * n) slots <<= 1;
+  const HeavyTab tab{(int32_t*)hsm, (uint32_t*)hsm + 2 * kHubEntries,
+                     (int32_t*)hsm + 4 * kHubEntries, slots};
+  uint32_t* const stage = (uint32_t*)hsm + 6 * kHubEntries;
+#pragma unroll 4
+  for (int k = t; k < n; k += T) stage[k] = e.key(k);
+  const int r = a.part[v];
+  tab.clear();
   if (t < 6) cnt[t] = 0u;
-  if (t == 0) {
-    overflow = 0;
-    s_at = -1;
-  }
   __syncthreads();
-  int s;
-  if (GIVEN) {
-    s = a.props_in[i];
-  } else {
-    const P4 x = draw(a.seed, kRngNodalVertex, a.seq + ctl_itr(a.ctl) * a.seq_mul, (uint32_t)v);
-    const int rnd = (int)(x.v[0] % (uint32_t)a.B);
-    const uint64_t target = scale_draw(x.v[1], deg);
-    int at = (int)target;
-    if (!unit) {
-      // the first entry whose running weight exceeds the target: the thread
-      // whose run of consecutive entries holds it
-      const int per = (n + T - 1) / T, k0 = min(n, t * per), k1 = min(n, k0 + per);
-      uint64_t own = 0;
-      for (int k = k0; k < k1; ++k) own += entry_w(k);
-      uint64_t incl = own;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint64_t y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= o) incl += y;
-      }
-      if (lane == 31) wsum[wid] = incl;
-      __syncthreads();
-      for (int q = 0; q < wid; ++q) incl += wsum[q];
-      uint64_t run = incl - own;
-      if (run <= target && target < incl)
-        for (int k = k0; k < k1; ++k) {
-          run += entry_w(k);
-          if (run > target) {
-            s_at = k;
-            break;
-          }
-        }
-      __syncthreads();
-      at = s_at;
-    }
-    s = proposed(a, at >= 0 ? (int)(entry_key(at) & 0x7fffffffu) : a.part[0], rnd);
-  }
+  const int s =
+      heavy_proposal<GIVEN>(a, i, v, e, wsum, &s_at, [&](int k) { return stage[k]; });
   if (r == s) {  // the same in every thread
     if (t == 0) write_result(a, GIVEN, i, r, s, 0.0);
     __syncthreads();
     return;
   }
   Corner q{};
-  const Rows<DENSE> R(a, r, s);
-  if (t < 32) {
-    const uint32_t mm = lane < 4 ? R.out_at((lane & 2) != 0, (lane & 1) ? s : r) : 0u;
-    load_degrees(a, v, r, s, q);
-    q.Mrr = __shfl_sync(kFull, mm, 0);
-    q.Mrs = __shfl_sync(kFull, mm, 1);
-    q.Msr = __shfl_sync(kFull, mm, 2);
-    q.Mss = __shfl_sync(kFull, mm, 3);
-  }
-#pragma unroll 4
+  if (t < 32) q = load_corner<DENSE>(a, v, r, s, lane);
   for (int k = t; k < n; k += T) {
-    const uint32_t key = entry_key(k), w = entry_w(k);
-    const int c = (int)(key & 0x7fffffffu);
-    const bool in = k >= no;
-    if (c == r) {
-      atomicAdd(cnt + (in ? 2 : 0), w);
-      if (!in) atomicAdd(cnt + 4, 1u);
-    }
-    if (c == s) {
-      atomicAdd(cnt + (in ? 3 : 1), w);
-      if (!in) atomicAdd(cnt + 5, 1u);
-    }
-    if (fits) add(key, w, k);
+    const uint32_t key = stage[k], w = e.w(k);
+    add_rs(cnt, k >= no, (int)(key & 0x7fffffffu), r, s, w);
+    tab.add(key, w, k);  // at most half full
   }
   __syncthreads();
   const RsWeights rw{cnt[0], cnt[1], cnt[2], cnt[3]};
   double acc = 0.0;
   for (int dir = 0; dir < 2; ++dir) {
-    const int lo = dir ? no : 0, hi = dir ? n : no;
-    const uint32_t P = (uint32_t)((hi - lo + kHashSlots / 4 - 1) / (kHashSlots / 4));
-    for (uint32_t pass = 0; pass < P; ++pass) {
-      auto mine = [&](uint32_t key) {
-        return P == 1 || hclass((int32_t)(key & 0x7fffffffu), P) == pass;
-      };
-      if (!fits) {
-        __syncthreads();
-        clear();
-        __syncthreads();
-        for (int k = lo + t; k < hi; k += T) {
-          const uint32_t key = entry_key(k);
-          if (mine(key)) add(key, entry_w(k), k);
-        }
-        __syncthreads();
+    const int hi = dir ? n : no;
+    for (int k = (dir ? no : 0) + t; k < hi; k += U * T) {
+      bool in[U], ok[U], want[U], lead[U];
+      int32_t c[U];
+      uint32_t w[U], kc[U], Mo[U], Mt[U];
+      double ld[U], t1[U], t2[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int at = k + u * T;
+        ok[u] = at < hi;
+        in[u] = dir == 1;
+        const uint32_t key = ok[u] ? stage[at] : 0u;
+        c[u] = (int32_t)(key & 0x7fffffffu);
+        w[u] = ok[u] ? e.w(at) : 0u;
+        const uint32_t sl = ok[u] ? tab.find(key) : 0u;
+        lead[u] = tab.first[sl] == at;
+        kc[u] = tab.sum[sl];
+        want[u] = ok[u] && c[u] != r;
+        ld[u] = ok[u] ? __ldg((dir ? a.ld_out : a.ld_in) + c[u]) : 0.0;
       }
-      for (int k = lo + t; k < hi;) {
-        bool in[U], ok[U], want[U], lead[U];
-        int32_t c[U];
-        uint32_t w[U], kc[U], Mo[U], Mt[U];
-        double ld[U], t1[U], t2[U];
+      row_counts<DENSE, U>(a, r, in, c, want, Mo);
+      row_counts<DENSE, U>(a, s, in, c, ok, Mt);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          ok[u] = false;
-          in[u] = dir == 1;
-          c[u] = 0;
-          w[u] = kc[u] = 0u;
-          lead[u] = false;
-          uint32_t key = 0u;
-          int at = 0;
-          while (k < hi && !ok[u]) {
-            key = entry_key(k);
-            at = k;
-            k += T;
-            ok[u] = mine(key);
-          }
-          if (ok[u]) {
-            c[u] = (int32_t)(key & 0x7fffffffu);
-            w[u] = entry_w(at);
-            uint32_t sl = slot0(key);
-            for (int probe = 0; probe < slots && tkey[sl] != (int32_t)key; ++probe)
-              sl = (sl + 1) & smask;
-            lead[u] = tfirst[sl] == at;
-            kc[u] = tsum[sl];
-          }
-          want[u] = ok[u] && c[u] != r;
-          ld[u] = ok[u] ? __ldg((dir ? a.ld_out : a.ld_in) + c[u]) : 0.0;
-        }
-        row_counts<DENSE, U>(a, r, in, c, want, Mo);
-        row_counts<DENSE, U>(a, s, in, c, ok, Mt);
+      for (int u = 0; u < U; ++u)
+        entry_terms(a.xlx, ok[u], in[u], c[u], w[u], lead[u], kc[u], Mo[u], Mt[u], ld[u], r, s,
+                    rw.niS, t1[u], t2[u]);
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          entry_terms(a.xlx, ok[u], in[u], c[u], w[u], lead[u], kc[u], Mo[u], Mt[u], ld[u], r, s,
-                      rw.niS, t1[u], t2[u]);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          acc -= t1[u];
-          acc -= t2[u];
-        }
+      for (int u = 0; u < U; ++u) {
+        acc -= t1[u];
+        acc -= t2[u];
       }
     }
   }
@@ -1594,14 +1596,162 @@ __device__ void heavy_vertex(const NodalArgs& a, int i, const Group<kHeavyThread
     acc += corner_term<true, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, lane);
   }
   const double d = grp.sum(acc);
-  if (t == 0) {
-    if (overflow) atomicAdd(a.err, 1);
-    write_result(a, GIVEN, i, r, s, d);
-  }
+  if (t == 0) write_result(a, GIVEN, i, r, s, d);
   __syncthreads();  // the CTA's next vertex reuses the shared memory
 }
 
-// Heavy vertices: one CTA each.
+// A hub, more than kHubEntries entries, on a cluster of eight CTAs.  The sum
+// it must give is that of 256 threads that take the entries of a direction
+// strided by 256, each subtracting its entries' terms in the order of P hash
+// classes of blocks (P = entries / 2048; the order of a table that holds one
+// class at a time), then of the index, summed by warps.  CTA q does warp q's
+// part, eight lanes a thread: they compute the terms of its next eight
+// entries together and subtract them in order.  Every CTA fills its own
+// table of all entries, one of both directions' blocks where they are sure to
+// fit (n entries, or 2 B blocks, at most half the slots), else one per class.
+// One CTA took 119 us for a hub of 5,400 entries at B = 600 and 233 at B =
+// 20k, the longest chain of every batch of such a graph; a launch of this
+// kernel over its three hubs a batch takes 26 us in the median.
+constexpr int kHubCluster = 8;
+constexpr int kHubList = 64;  // a thread's entries in order, up to 256 * kHubList entries
+constexpr size_t kHubSmem = (3 * kHashSlots + 32 * kHubList) * sizeof(int32_t);
+static_assert(kHeavyThreads == 32 * kHubCluster, "a virtual warp per CTA");
+
+template <bool GIVEN, bool DENSE>
+__device__ void hub_vertex(const NodalArgs& a, int i, int& parity) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  constexpr int T = kHeavyThreads, G = 8;
+  extern __shared__ unsigned long long hsm[];
+  __shared__ unsigned long long wsum[T / 32];
+  __shared__ double accs[32], red[2][kHubCluster];
+  __shared__ uint32_t cnt[6];
+  __shared__ int s_at, overflow;
+  const int t = threadIdx.x, lane = t & 31, rank = (int)cl.block_rank();
+  const int v = GIVEN ? a.verts[i] : a.lo + i;
+  const HeavyEntries e(a, v);
+  const int n = e.n, no = e.no;
+  const bool fits = n <= kHashSlots / 2 || 2LL * a.B <= kHashSlots / 2;
+  int slots = 512;
+  while (slots < kHashSlots && (!fits || slots < 2 * min(n, 2 * a.B))) slots <<= 1;
+  const HeavyTab tab{(int32_t*)hsm, (uint32_t*)hsm + kHashSlots, (int32_t*)hsm + 2 * kHashSlots,
+                     slots};
+  int32_t* const list = (int32_t*)hsm + 3 * kHashSlots;  // of each virtual thread
+  const int r = a.part[v];
+  tab.clear();
+  if (t < 6) cnt[t] = 0u;
+  if (t == 0) overflow = 0;
+  __syncthreads();
+  const int s = heavy_proposal<GIVEN>(a, i, v, e, wsum, &s_at, [&](int k) { return e.key(k); });
+  if (r == s) {  // the same in every thread of the cluster
+    if (rank == 0 && t == 0) write_result(a, GIVEN, i, r, s, 0.0);
+    __syncthreads();
+    return;
+  }
+#pragma unroll 4
+  for (int k = t; k < n; k += T) {
+    const uint32_t key = e.key(k), w = e.w(k);
+    add_rs(cnt, k >= no, (int)(key & 0x7fffffffu), r, s, w);
+    if (fits && !tab.add(key, w, k)) overflow = 1;
+  }
+  __syncthreads();
+  const RsWeights rw{cnt[0], cnt[1], cnt[2], cnt[3]};
+  const int vt = t >> 3, h = t & (G - 1), hb = lane & 24;  // virtual thread of the warp, helper
+  const int first = 32 * rank + vt;
+  double acc = 0.0;
+  for (int dir = 0; dir < 2; ++dir) {
+    const int lo = dir ? no : 0, hi = dir ? n : no;
+    const uint32_t P = (uint32_t)((hi - lo + kHashSlots / 4 - 1) / (kHashSlots / 4));
+    const int len = hi - lo > first ? (hi - lo - first + T - 1) / T : 0;
+    const bool listed = hi - lo <= T * kHubList;
+    int32_t* const mine = list + vt * kHubList;
+    if (listed && P > 1) {
+      // the thread's entries by class, then index
+      int at = 0;
+      for (uint32_t pass = 0; pass < P; ++pass)
+        for (int j0 = 0; j0 < kHubList; j0 += G) {
+          const int j = j0 + h;
+          const int k = lo + first + j * T;
+          const bool m = j < len && hclass((int32_t)(e.key(k) & 0x7fffffffu), P) == pass;
+          const unsigned mm = __ballot_sync(kFull, m) >> hb & 0xffu;
+          if (m) mine[at + __popc(mm & ((1u << h) - 1u))] = k;
+          at += __popc(mm);
+        }
+    } else if (listed) {
+      for (int j = h; j < len; j += G) mine[j] = lo + first + j * T;
+    }
+    __syncwarp();
+    // one sweep over the list, or (a class's own table, or no list) one per
+    // class that leaves out the other classes' entries
+    const uint32_t sweeps = fits && listed ? (P ? 1 : 0) : P;
+    for (uint32_t pass = 0; pass < sweeps; ++pass) {
+      if (!fits) {
+        __syncthreads();
+        tab.clear();
+        __syncthreads();
+#pragma unroll 4
+        for (int k = lo + t; k < hi; k += T) {
+          const uint32_t key = e.key(k);
+          if (hclass((int32_t)(key & 0x7fffffffu), P) == pass && !tab.add(key, e.w(k), k))
+            overflow = 1;
+        }
+        __syncthreads();
+      }
+      const int most = (hi - lo + T - 1) / T;  // of any virtual thread: uniform
+      for (int j0 = 0; j0 < most; j0 += G) {
+        const int j = j0 + h;
+        const int k = j >= len ? lo : listed ? mine[j] : lo + first + j * T;
+        const uint32_t key = j < len ? e.key(k) : 0u;
+        const int32_t c = (int32_t)(key & 0x7fffffffu);
+        const bool in = dir == 1;
+        const bool ok = j < len && (sweeps == 1 || hclass(c, P) == pass);
+        const uint32_t w = ok ? e.w(k) : 0u;
+        const uint32_t sl = ok ? tab.find(key) : 0u;
+        const bool want = ok && c != r;
+        const double ld = ok ? __ldg((in ? a.ld_out : a.ld_in) + c) : 0.0;
+        uint32_t Mo, Mt;
+        row_counts<DENSE, 1>(a, r, &in, &c, &want, &Mo);
+        row_counts<DENSE, 1>(a, s, &in, &c, &ok, &Mt);
+        double t1, t2;
+        entry_terms(a.xlx, ok, in, c, w, tab.first[sl] == k, tab.sum[sl], Mo, Mt, ld, r, s,
+                    rw.niS, t1, t2);
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+          acc -= __shfl_sync(kFull, t1, hb + u);
+          acc -= __shfl_sync(kFull, t2, hb + u);
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (h == 0) accs[vt] = acc;
+  __syncthreads();
+  if (t < 32) {
+    acc = accs[lane];
+    if (rank == 0) {
+      const Corner q = load_corner<DENSE>(a, v, r, s, lane);
+      const RowChange m = row_change(q, rw, cnt[4], cnt[5]);
+      acc += corner_term<true, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, lane);
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) {
+      cl.map_shared_rank(&red[0][0], 0)[parity * kHubCluster + rank] = acc;
+      if (overflow) atomicAdd(a.err, 1);
+    }
+  }
+  cl.sync();
+  if (rank == 0 && t == 0) {
+    double d = 0.0;
+    for (int q = 0; q < kHubCluster; ++q) d += red[parity][q];
+    write_result(a, GIVEN, i, r, s, d);
+  }
+  // the next hub's sums go to the other half: it ends with a cluster barrier
+  // that this one's reader reaches first
+  parity ^= 1;
+  __syncthreads();
+}
+
+// Heavy vertices but the hubs: one CTA each.
 template <bool GIVEN, bool DENSE, bool GEN>
 struct NodalHeavyBody {
   using Args = NodalArgs;
@@ -1611,15 +1761,31 @@ struct NodalHeavyBody {
     if (ctl_stopped(a.ctl)) return;
     __shared__ double red[kHeavyThreads / 32];
     const Group<kHeavyThreads> grp{red};
-    for (int h = vb; h < a.nheavy; h += vg) heavy_vertex<GIVEN, DENSE>(a, a.heavy[h], grp);
+    for (int h = a.nhub + vb; h < a.nheavy; h += vg)
+      heavy_vertex<GIVEN, DENSE>(a, a.heavy[h], grp);
   }
 };
 
+// Hubs: one cluster each.
+template <bool GIVEN, bool DENSE>
+struct NodalHubBody {
+  using Args = NodalArgs;
+  static constexpr int kThreads = kHeavyThreads, kMinBlocks = 1, kCluster = kHubCluster;
+  static constexpr size_t kSmem = kHubSmem;
+  static __device__ void run(const Args& a, int vb, int vg) {
+    if (ctl_stopped(a.ctl)) return;
+    int parity = 0;
+    for (int h = vb / kHubCluster; h < a.nhub; h += vg / kHubCluster)
+      hub_vertex<GIVEN, DENSE>(a, a.heavy[h], parity);
+  }
+};
+
+// General mode: every heavy vertex on a CTA.
 template <bool GIVEN, bool DENSE>
 struct NodalHeavyBody<GIVEN, DENSE, true> {
   using Args = NodalArgs;
   static constexpr int kThreads = kHeavyThreads, kMinBlocks = 2;
-  static constexpr size_t kSmem = kHeavySmem;
+  static constexpr size_t kSmem = 3 * kHashSlots * sizeof(int32_t);
   static __device__ void run(const Args& a, int vb, int vg) {
     if (ctl_stopped(a.ctl)) return;
     extern __shared__ unsigned long long hsm[];
@@ -1809,6 +1975,7 @@ NodalArgs make_args(const DevGraph& g, const int32_t* part, const DevBM& m, int3
   a.B = B;
   a.heavy = aux.heavy;
   a.nheavy = aux.nheavy;
+  a.nhub = aux.nhub;
   a.small = aux.small;
   a.nsmall = aux.nsmall;
   a.mid = aux.mid;
@@ -1827,11 +1994,15 @@ int32_t nodal_ctas(const NodalArgs& a, bool gen) {
 
 template <bool GIVEN, bool DENSE, bool GEN>
 void launch_pair(const NodalArgs& a, const NodalAux& aux, cudaStream_t st) {
+  const int nhub = GEN ? 0 : a.nhub;
   if (a.nheavy > 0) {
     // heavy vertices on the side stream, next to the warp kernel
     cudaEventRecord(aux.fork, st);
     cudaStreamWaitEvent(aux.side, aux.fork, 0);
-    launch_single<NodalHeavyBody<GIVEN, DENSE, GEN>>(a, std::min(a.nheavy, 2 * 148), aux.side);
+    if (nhub > 0)
+      launch_single<NodalHubBody<GIVEN, DENSE>>(a, kHubCluster * std::min(nhub, 18), aux.side);
+    launch_single<NodalHeavyBody<GIVEN, DENSE, GEN>>(a, std::min(a.nheavy - nhub, 4 * 148),
+                                                     aux.side);
     cudaEventRecord(aux.join, aux.side);
   }
   launch_single<NodalBody<GIVEN, DENSE, GEN>>(a, nodal_ctas(a, GEN), st);
@@ -1856,6 +2027,9 @@ const MultiKernel kmNodalHeavy[4] = {
     multi_kernel_desc<NodalHeavyBody<false, false, true>>("nodal_heavy_gen_csr"),
     multi_kernel_desc<NodalHeavyBody<false, true, true>>("nodal_heavy_gen_dense")};
 
+const MultiKernel kmNodalHub[2] = {multi_kernel_desc<NodalHubBody<false, false>>("nodal_hub_csr"),
+                                   multi_kernel_desc<NodalHubBody<false, true>>("nodal_hub_dense")};
+
 void set_mode(NodalArgs& a, const ScoreMode& md) {
   a.exact = md.exact;
   a.mh = md.mh;
@@ -1865,26 +2039,22 @@ const MultiKernel kmCommit = multi_kernel_desc<CommitBody>("commit");
 
 }  // namespace
 
-cudaError_t init_nodal_attributes() {
+template <class... Bodies>
+cudaError_t allow_smem_all() {
   cudaError_t e = cudaSuccess;
-  auto set = [&](const void* f) {
-    cudaError_t x = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kHeavySmem);
+  for (cudaError_t x : {allow_smem<Bodies>()...})
     if (x != cudaSuccess) e = x;
-  };
-  set((const void*)single_kernel<NodalHeavyBody<false, false, false>>);
-  set((const void*)single_kernel<NodalHeavyBody<false, true, false>>);
-  set((const void*)single_kernel<NodalHeavyBody<true, false, false>>);
-  set((const void*)single_kernel<NodalHeavyBody<true, true, false>>);
-  set((const void*)multi_kernel<NodalHeavyBody<false, false, false>>);
-  set((const void*)multi_kernel<NodalHeavyBody<false, true, false>>);
-  set((const void*)single_kernel<NodalHeavyBody<false, false, true>>);
-  set((const void*)single_kernel<NodalHeavyBody<false, true, true>>);
-  set((const void*)single_kernel<NodalHeavyBody<true, false, true>>);
-  set((const void*)single_kernel<NodalHeavyBody<true, true, true>>);
-  set((const void*)multi_kernel<NodalHeavyBody<false, false, true>>);
-  set((const void*)multi_kernel<NodalHeavyBody<false, true, true>>);
   return e;
+}
+
+cudaError_t init_nodal_attributes() {
+  const cudaError_t e =
+      allow_smem_all<NodalHeavyBody<false, false, true>, NodalHeavyBody<false, true, true>,
+                     NodalHeavyBody<true, false, true>, NodalHeavyBody<true, true, true>>();
+  const cudaError_t e2 =
+      allow_smem_all<NodalHubBody<false, false>, NodalHubBody<false, true>,
+                     NodalHubBody<true, false>, NodalHubBody<true, true>>();
+  return e != cudaSuccess ? e : e2;
 }
 
 int nodal_heavy_threshold() { return kWarpList; }
@@ -1931,7 +2101,7 @@ void nodal_commit(int32_t* part, int32_t lo, int32_t count, const int32_t* newla
       vg_commit(count), st);
 }
 
-void add_nodal(Slot& warp, Slot& heavy, bool dense, const ScoreMode& md, const DevGraph& g,
+void add_nodal(Slot& warp, Slot& heavy, Slot& hub, bool dense, const ScoreMode& md, const DevGraph& g,
                const int32_t* part,
                const DevBM& m, int32_t B, uint64_t seed, uint32_t seq, int32_t lo, int32_t count,
                int32_t* newlab, double* rec, int32_t* props, const NodalAux& aux,
@@ -1949,7 +2119,9 @@ void add_nodal(Slot& warp, Slot& heavy, bool dense, const ScoreMode& md, const D
   a.seq_mul = seq_mul;
   set_mode(a, md);
   slot_push(slot_bind(warp, kmNodal[md.slot(dense)]), a, nodal_ctas(a, md.general()));
-  slot_push(slot_bind(heavy, kmNodalHeavy[md.slot(dense)]), a, aux.nheavy);
+  const int32_t nhub = md.general() ? 0 : aux.nhub;
+  slot_push(slot_bind(heavy, kmNodalHeavy[md.slot(dense)]), a, aux.nheavy - nhub);
+  if (nhub > 0) slot_push(slot_bind(hub, kmNodalHub[dense ? 1 : 0]), a, kHubCluster * nhub);
 }
 
 void add_commit(Slot& s, int32_t* part, int32_t lo, int32_t count, const int32_t* newlab,

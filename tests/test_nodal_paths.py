@@ -67,3 +67,33 @@ def test_path_edges(sbp, orc, monkeypatch, weighted, dmax, B):
         moves = (np.abs(da) > REL) | (np.abs(db) > REL)
         assert np.array_equal(pa[:K][moves], pb[:K][moves]), "accepted moves differ"
         assert np.array_equal(pa[:K] != p[:K], da < 0.0)
+
+
+# hubs: the edge to them (1024 entries in all), more than one hash class of
+# blocks, lists longer than a thread's share
+HUBS = [(1000, 24), (1000, 25), (200, 824), (200, 825), (3, 2100), (4100, 60), (3, 17000),
+        (20000, 9)]
+
+
+# cells of a few thousand counts at most, whose x log2 x rounds by less than
+# 1e-11 each: REL holds with room
+@pytest.mark.parametrize("dmax", ["0", "4096"], ids=["csr", "dense"])
+@pytest.mark.parametrize("B,weighted", [(300, False), (3000, False), (3000, True), (N, True)])
+def test_hub_edges(sbp, orc, monkeypatch, dmax, B, weighted):
+    monkeypatch.setenv("SBP_DENSE_MAX", dmax)
+    monkeypatch.setattr("test_nodal_paths.SHAPES", HUBS)
+    g = shaped_graph(sbp, weighted)
+    rng = np.random.default_rng(B + 1)
+    p = rng.integers(0, B, N).astype(np.int32)
+    p[-B:] = np.arange(B, dtype=np.int32)
+    K = len(HUBS)
+    verts = np.tile(np.arange(K, dtype=np.int32), 8)
+    props = rng.integers(0, B, verts.size).astype(np.int32)
+    got = sbp.delta_mdl_nodal(g, p, B, verts, props)
+    want, _ = orc.nodal_delta(g, p, B, verts, props)
+    assert close(got, want).all()
+    for seq in range(4):
+        _, da, xa, _ = sbp.nodal_batch(g, p, B, 21, seq, 0, K)
+        _, db, xb, _ = orc.nodal_batch(g, p, B, 21, seq, 0, K)
+        assert np.array_equal(xa, xb), "proposals differ"
+        assert close(da, db).all()
