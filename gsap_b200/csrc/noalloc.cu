@@ -5,10 +5,10 @@
 // the objective: hosts that own all device memory through their own pool and
 // do not let a library allocate behind their back, and serving loops that
 // forbid the device-wide synchronisation a cudaMalloc or cudaFree can cost.
-// For them this entry point keeps its scratch (the log2 of the block degrees
-// and the per-CTA partial sums) in one file-scope device array of fixed size,
-// created when the library is loaded and held by every GPU that loads it
-// until the process exits.  The caller passes the inputs and the outputs.
+// For them this entry point keeps its scratch (the per-CTA partial sums) in
+// one file-scope device array of fixed size, created when the library is
+// loaded and held by every GPU that loads it until the process exits.  The
+// caller passes the inputs and the outputs.
 //
 // Limits and rules of use:
 //   * at most kStaticMaxBlocks (65,536) blocks; larger B is rejected;
@@ -19,8 +19,8 @@
 //     the entry point must not be called on that device afterwards;
 //   * every call on a device shares the one array, and the array keeps the
 //     last call's contents: calls that overlap on the GPU (different
-//     streams, or work still running) race on it.  Each call clears what
-//     must start at zero (the CTA ticket of the reduction) itself.
+//     streams, or work still running) race on it.  Each call leaves what must
+//     start at zero (the CTA ticket of the reduction) at zero.
 #include "../../include/sbp.h"
 #include "common.cuh"
 
@@ -38,72 +38,101 @@ constexpr int kStaticCtas = 128;
 constexpr int kStaticThreads = 256;
 
 struct StaticScratch {
-  double ld_out[kStaticMaxBlocks];
-  double ld_in[kStaticMaxBlocks];
-  double part[kStaticCtas];
+  double sum[kStaticCtas], err[kStaticCtas];
   unsigned ticket;
 };
 
-// ~1 MB: the whole scratch of sbp_mdl_device_static.
+// The whole scratch of sbp_mdl_device_static.
 static __device__ __align__(256) unsigned char g_mdl_scratch[sizeof(StaticScratch)];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 StaticScratch* g_addr[kMaxDevices] = {};
 
-// log2 of the block degrees; also clears the ticket of the reduction.
-__global__ void static_logs_kernel(StaticScratch* sc, int32_t B, const uint32_t* __restrict__ d_out,
-                                   const uint32_t* __restrict__ d_in) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b == 0) sc->ticket = 0u;
-  for (; b < B; b += gridDim.x * blockDim.x) {
-    sc->ld_out[b] = log2((double)d_out[b]);
-    sc->ld_in[b] = log2((double)d_in[b]);
+// A sum and the rounding errors left out of it (Knuth's two-sum): whatever
+// the order of the additions, value() is rounded about once.
+struct ExactSum {
+  double s = 0.0, e = 0.0;
+  __device__ __forceinline__ void add(double x) {
+    const double t = __dadd_rn(s, x);
+    const double z = __dsub_rn(t, s);
+    e = __dadd_rn(e, __dadd_rn(__dsub_rn(s, __dsub_rn(t, z)), __dsub_rn(x, z)));
+    s = t;
   }
+  __device__ __forceinline__ void add(const ExactSum& o) {
+    add(o.s);
+    e = __dadd_rn(e, o.e);
+  }
+  // an infinite term (a count in a column of degree 0) leaves no error term
+  __device__ __forceinline__ double value() const { return isfinite(s) ? __dadd_rn(s, e) : s; }
+};
+
+__device__ __forceinline__ ExactSum warp_total(ExactSum x) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    ExactSum y;
+    y.s = __shfl_xor_sync(kFull, x.s, o);
+    y.e = __shfl_xor_sync(kFull, x.e, o);
+    x.add(y);
+  }
+  return x;
 }
 
 // data_S = sum over blocks b of sum over out-row b of
 //   M (log2 M - log2 d_out[b] - log2 d_in[c])
 // (compute_overall_S_transform, kernels.hpp:1066-1093), then
-// S = model - data_S (partition.hpp:696-701).  Rows are dealt to threads in
-// a fixed order, CTA partials land in the scratch and the last CTA (ticket)
-// adds them in CTA order: the result does not depend on scheduling.
+// S = model - data_S (partition.hpp:696-701).  The rows' sums of M are the
+// degrees, so the terms are one per entry, whatever its row, and one per
+// block: threads stride over both, and no launch waits for the other.  A
+// thread per row took 200 us at 350 rows of 350 entries, a chain of dependent
+// loads, behind a launch of its own for the logarithms; a call of this takes 9.  CTA sums land in the scratch and the last
+// CTA (ticket) adds them; the additions carry their errors, so the result
+// does not depend on the split.
 __global__ void __launch_bounds__(kStaticThreads) static_mdl_kernel(
     StaticScratch* sc, int32_t B, const int32_t* __restrict__ optr,
     const int32_t* __restrict__ ocol, const uint32_t* __restrict__ ocnt,
-    const uint32_t* __restrict__ d_out, double model, double* S, double* data_S) {
-  __shared__ double sh[kStaticThreads];
+    const uint32_t* __restrict__ d_out, const uint32_t* __restrict__ d_in, double model,
+    double* S, double* data_S) {
+  constexpr int kWarps = kStaticThreads / 32;
+  __shared__ ExactSum sh[kWarps];
   __shared__ bool last;
-  const int tid = threadIdx.x;
-  double acc = 0.0;
-  for (int b = blockIdx.x * kStaticThreads + tid; b < B; b += gridDim.x * kStaticThreads) {
-    const double ldo = sc->ld_out[b];
-    double row = 0.0;
-    for (int i = optr[b]; i < optr[b + 1]; ++i) {
-      const uint32_t m = ocnt[i];
-      if (m) row += xlog2x(m) - (double)m * sc->ld_in[ocol[i]];
-    }
-    const uint32_t d = d_out[b];
-    acc += row - (d ? (double)d * ldo : 0.0);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int first = blockIdx.x * kStaticThreads + tid, step = gridDim.x * kStaticThreads;
+  ExactSum acc;
+  for (int b = first; b < B; b += step) acc.add(-xlog2x(d_out[b]));
+  const int end = optr[B];
+#pragma unroll 4
+  for (long long i = (long long)optr[0] + first; i < end; i += step) {
+    const uint32_t m = ocnt[i];
+    const double ld = log2((double)d_in[ocol[i]]);
+    if (m) acc.add(xlog2x(m) - (double)m * ld);
   }
-  sh[tid] = acc;
+  acc = warp_total(acc);
+  if (lane == 0) sh[wid] = acc;
   __syncthreads();
-  for (int o = kStaticThreads / 2; o > 0; o >>= 1) {
-    if (tid < o) sh[tid] += sh[tid + o];
-    __syncthreads();
-  }
   if (tid == 0) {
-    sc->part[blockIdx.x] = sh[0];
+    for (int k = 1; k < kWarps; ++k) acc.add(sh[k]);
+    sc->sum[blockIdx.x] = acc.s;
+    sc->err[blockIdx.x] = acc.e;
     __threadfence();
     last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (last && tid == 0) {
+  if (last && wid == 0) {
     __threadfence();
-    double t = 0.0;
-    for (int k = 0; k < (int)gridDim.x; ++k) t += ((volatile double*)sc->part)[k];
-    *data_S = t;
-    *S = model - t;
+    ExactSum t;
+    for (int k = lane; k < (int)gridDim.x; k += 32) {
+      ExactSum x;
+      x.s = ((volatile double*)sc->sum)[k];
+      x.e = ((volatile double*)sc->err)[k];
+      t.add(x);
+    }
+    t = warp_total(t);
+    if (lane == 0) {
+      *data_S = t.value();
+      *S = model - t.value();
+      sc->ticket = 0u;
+    }
   }
 }
 
@@ -147,13 +176,11 @@ extern "C" sbp_status sbp_mdl_device_static(int32_t N, int32_t E, int32_t B,
   const double model =
       (double)E * (1.0 + x) * std::log(1.0 + x) - x * std::log(x) + (double)N * std::log(b);
   // A launch error left pending by earlier, unrelated work is cleared first
-  // so that the status below belongs to these two launches (a sticky error,
-  // which ends the context, is reported again by the check after them).
+  // so that the status below belongs to this launch (a sticky error,
+  // which ends the context, is reported again by the check after it).
   (void)cudaGetLastError();
-  static_logs_kernel<<<(B + kStaticThreads - 1) / kStaticThreads, kStaticThreads, 0, st>>>(
-      sc, B, d_out, d_in);
   static_mdl_kernel<<<kStaticCtas, kStaticThreads, 0, st>>>(sc, B, out_ptr, out_col, out_cnt,
-                                                            d_out, model, S, data_S);
+                                                            d_out, d_in, model, S, data_S);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return host_fail(SBP_ERR_CUDA, cudaGetErrorString(e));
   return SBP_OK;

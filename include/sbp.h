@@ -386,7 +386,7 @@ sbp_status sbp_mdl_mode(const sbp_graph_csr* g, const int32_t* part, int32_t B, 
  * anything: for callers that cannot let a library allocate device memory,
  * such as hosts that own all device memory through their own pool, or
  * serving loops that forbid the synchronisation a cudaMalloc or cudaFree can
- * cost.  The caller passes inputs and outputs; the scratch is a fixed ~1 MB
+ * cost.  The caller passes inputs and outputs; the scratch is a fixed ~2 KB
  * device array of the library, held by every GPU that loads it until the
  * process exits, so B <= 65536 (larger B returns SBP_ERR_INVALID).  The first
  * call on a device looks that array's address up (once per device, with the
