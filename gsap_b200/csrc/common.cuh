@@ -121,7 +121,7 @@ __device__ __forceinline__ double xlog2x(uint32_t w) {
 // with the same functions), larger ones computed.
 constexpr uint32_t kXlxTable = 1u << 16;
 static __device__ __forceinline__ double xlog2x_big(uint32_t w) {
-  return (double)w * log2((double)w);
+  return __dmul_rn((double)w, log2((double)w));  // never contracted into a sum
 }
 __device__ __forceinline__ double xlx(const double* __restrict__ tab, uint32_t w) {
   return w < kXlxTable ? __ldg(tab + w) : xlog2x_big(w);

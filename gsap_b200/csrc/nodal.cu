@@ -301,46 +301,6 @@ struct Group {
   }
 };
 
-// Ascending bitonic sort of P (power of two) keys by the group.
-template <int G>
-__device__ void group_sort(unsigned long long* key, int P, const Group<G>& grp) {
-  const int t = grp.rank();
-  for (int k = 2; k <= P; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = t; i < P; i += G) {
-        int ixj = i ^ j;
-        if (ixj > i) {
-          unsigned long long x = key[i], y = key[ixj];
-          bool asc = (i & k) == 0;
-          if ((x > y) == asc) {
-            key[i] = y;
-            key[ixj] = x;
-          }
-        }
-      }
-      grp.sync();
-    }
-  }
-}
-
-__device__ __forceinline__ int32_t kblk(unsigned long long k) { return (int32_t)(k >> 32); }
-__device__ __forceinline__ uint32_t kwt(unsigned long long k) { return (uint32_t)k; }
-
-// Stage v's neighbour blocks of one direction as sorted (block, weight) keys.
-template <int G>
-__device__ void stage_sorted(const int32_t* __restrict__ idx, const uint32_t* __restrict__ w,
-                             const int32_t* __restrict__ part, int32_t base, int n,
-                             unsigned long long* key, const Group<G>& grp) {
-  int P = 32;
-  while (P < n) P <<= 1;
-  for (int k = grp.rank(); k < P; k += G)
-    key[k] = k < n ? ((unsigned long long)(uint32_t)__ldg(part + __ldg(idx + base + k)) << 32) |
-                         __ldg(w + base + k)
-                   : ~0ull;
-  grp.sync();
-  group_sort<G>(key, P, grp);
-}
-
 // Lists of more than kWarpList entries: per-block totals from a shared-memory
 // hash table, built in passes that each take the blocks of one hash class,
 // so the table never holds more than a few thousand blocks.  Costs
@@ -450,7 +410,149 @@ __device__ __forceinline__ double group_sum(double x) {
   return x;
 }
 
-// ----------------------------------------------------------- GSAP scoring --
+// ------------------------------------------------------------ general mode --
+// Kernels instantiated with GEN = true score a move by the exact change of
+// the MDL (exact = 1) or by GSAP's terms (exact = 0), and accept it by
+// Metropolis-Hastings (mh = 1) or iff dS < 0.
+//
+// Exact dS.  S = model - data_S with
+//   data_S = sum_cells M log2 M - sum_rows d_out log2 d_out - sum_cols d_in log2 d_in
+// and the model term fixed while B is.  Moving v from r to s, with kout[c]
+// and kin[c] v's weight to and from block c (self loops of weight `self`
+// apart), moves kout[c] from cell (r,c) to (s,c) and kin[c] from (c,r) to
+// (c,s) for every c other than r and s, changes the four corner cells as in
+// corner_exact, and moves v's out- and in-degree between the rows and
+// columns r and s; dS = -(change of data_S).  Only those cells and four
+// degrees enter, each as x log2 x.
+//
+// Hastings ratio of GSAP's proposal (kernels.hpp:877-1032): v picks an
+// incident edge with probability proportional to its weight, the edge's
+// other end lies in block t, and s is proposed with probability
+// (M_ts + M_st + 1) / (d_t + B), d_t = d_out[t] + d_in[t], so
+//   p(r -> s) = sum_t k_t (M_ts + M_st + 1) / (d_t + B) / k_v
+// with k_t v's weight to and from t (a self loop counts in both directions)
+// and k_v the sum of the k_t.  The reverse move reads the blockmodel after
+// the move, in which the self loops sit in block s.  A move is accepted when
+//   u < 2^(-beta dS) p(s -> r) / p(r -> s)
+// with u the vertex's third draw scaled to [0, 1).
+
+struct Hast {
+  double f = 0.0, b = 0.0;  // forward and reverse proposal weights (k_v times p)
+};
+
+// acc plus term `k` (0..15) of the corner cells and the four degrees of the
+// exact dS, acc for other k: terms 0-3 the old cells (r,r), (r,s), (s,r), (s,s), 4-7 the
+// same cells after the move, 8-11 the new degrees d_out[r], d_out[s], d_in[r],
+// d_in[s], 12-15 the old ones.  koR..niS include the self loops (their other
+// end is in r).  The rounding is spelled out, so that it does not hang on what
+// the compiler contracts: beyond the table a product w log2 w joins the sum
+// in one rounding, but for the old degrees.
+__device__ __forceinline__ double corner_exact(const double* tab, const Corner& q,
+                                               const RsWeights& w, uint32_t self, int k,
+                                               double acc) {
+  if (k >= 16) return acc;
+  const int j = k & 3;
+  uint32_t X;
+  if (k < 8) {
+    const uint32_t M = j == 0 ? q.Mrr : j == 1 ? q.Mrs : j == 2 ? q.Msr : q.Mss;
+    // unsigned wrap-around in the middle is fine: the results are >= 0
+    const uint32_t x = j == 0   ? M - w.koR - w.niR + self
+                       : j == 1 ? M - w.koS + (w.niR - self)
+                       : j == 2 ? M + (w.koR - self) - w.niS
+                                : M + w.koS + w.niS + self;
+    X = k < 4 ? M : x;
+  } else {
+    const uint32_t d0 = j == 0 ? q.dor : j == 1 ? q.dos : j == 2 ? q.dir : q.dis;
+    const uint32_t d1 =
+        j == 0 ? d0 - q.kO : j == 1 ? d0 + q.kO : j == 2 ? d0 - q.kI : d0 + q.kI;
+    X = k < 12 ? d1 : d0;
+  }
+  const bool plus = k < 4 || (k >= 8 && k < 12);
+  if (X >= kXlxTable && k < 12)
+    return __fma_rn(plus ? (double)X : -(double)X, log2((double)X), acc);
+  const double t = xlx(tab, X);
+  return __dadd_rn(acc, plus ? t : -t);
+}
+
+// Exact change of - data_S in the off-corner cells of a neighbour block, once
+// per block and direction (lead; c other than r and s).
+__device__ __forceinline__ double exact_term(const double* tab, uint32_t Mo, uint32_t Mt,
+                                             uint32_t kc) {
+  return __dsub_rn(__dadd_rn(__dsub_rn(xlx(tab, Mo), xlx(tab, Mo - kc)), xlx(tab, Mt)),
+                   xlx(tab, Mt + kc));
+}
+
+// Proposal weights of a neighbour block t other than r and s, kt = v's
+// weight to and from t.
+template <bool DENSE>
+__device__ __forceinline__ void hast_block(const NodalArgs& a, const Rows<DENSE>& R, int32_t t,
+                                           uint32_t kt, Hast& h) {
+  const double D = (double)a.d_out[t] + (double)a.d_in[t] + (double)a.B;
+  const double k = (double)kt;
+  h.f += k * ((double)R.in_s(t) + (double)R.out_s(t) + 1.0) / D;
+  h.b += k * ((double)R.in_r(t) + (double)R.out_r(t) - k + 1.0) / D;
+}
+
+// Proposal weights of blocks r and s (one thread of the group).
+template <bool DENSE>
+__device__ __forceinline__ void hast_rs(const NodalArgs& a, const Rows<DENSE>& R, int v, int r,
+                                        int s, const RsWeights& w, uint32_t self, Hast& h) {
+  const uint32_t Mrr = R.out_at(false, r), Mrs = R.out_at(false, s);
+  const uint32_t Msr = R.out_at(true, r), Mss = R.out_at(true, s);
+  const uint32_t xrr = Mrr - w.koR - w.niR + self;
+  const uint32_t xrs = Mrs - w.koS + (w.niR - self);
+  const uint32_t xsr = Msr + (w.koR - self) - w.niS;
+  const double kv = (double)a.kdo[v] + (double)a.kdi[v], Bd = (double)a.B;
+  const double Dr = (double)a.d_out[r] + (double)a.d_in[r];
+  const double Ds = (double)a.d_out[s] + (double)a.d_in[s];
+  const double kr = (double)w.koR + (double)w.niR, ks = (double)w.koS + (double)w.niS;
+  const double sl = 2.0 * (double)self;
+  h.f += kr * ((double)Mrs + (double)Msr + 1.0) / (Dr + Bd);
+  h.f += ks * ((double)Mss + (double)Mss + 1.0) / (Ds + Bd);
+  h.b += (kr - sl) * ((double)xrr + (double)xrr + 1.0) / (Dr - kv + Bd);
+  h.b += (ks + sl) * ((double)xsr + (double)xrs + 1.0) / (Ds + kv + Bd);
+}
+
+// Corner counts and degrees for corner_term, on a full warp.
+template <bool DENSE>
+__device__ __forceinline__ Corner load_corner(const NodalArgs& a, int v, int r, int s, int lane) {
+  const uint32_t mm =
+      lane < 4 ? Rows<DENSE>(a, r, s).out_at((lane & 2) != 0, (lane & 1) ? s : r) : 0u;
+  Corner q{};
+  load_degrees(a, v, r, s, q);
+  q.Mrr = __shfl_sync(kFull, mm, 0);
+  q.Mrs = __shfl_sync(kFull, mm, 1);
+  q.Msr = __shfl_sync(kFull, mm, 2);
+  q.Mss = __shfl_sync(kFull, mm, 3);
+  return q;
+}
+
+constexpr double kLn2 = 0.6931471805599453;
+
+// Accept test of a general-mode move (r != s).
+__device__ __forceinline__ bool accept_move(const NodalArgs& a, double d, double logH,
+                                            uint32_t u) {
+  if (!a.mh) return d < 0.0;
+  // -beta * dS * ln 2 + logH, rounded step by step (no contraction)
+  const double x = __dadd_rn(__dmul_rn(__dmul_rn(-a.beta, d), kLn2), logH);
+  if (x >= 0.0) return true;
+  return log((double)u * 2.3283064365386963e-10) < x;
+}
+
+__device__ __forceinline__ void write_result_gen(const NodalArgs& a, bool given, int i, int r,
+                                                 int s, double d, double logH, uint32_t u) {
+  if (given) {
+    a.dS_raw[i] = d;
+    if (a.logH_raw) a.logH_raw[i] = logH;
+    return;
+  }
+  const bool acc = r != s && accept_move(a, d, logH, u);
+  a.newlab[i] = acc ? s : r;
+  a.rec[i] = acc ? d : 0.0;
+  if (a.props_out) a.props_out[i] = s;
+}
+
+// ------------------------------------------------------------- warp paths --
 // A move's dS is a sum of per-entry terms and 13 corner and degree terms.
 // The entries are dealt to lanes in a fixed order and each lane subtracts its
 // entries' terms one after the other (the rounding of the sum is part of the
@@ -568,8 +670,9 @@ __device__ __forceinline__ uint32_t mask_weight(const uint32_t* ws, Mask m) {
 // in slot k / L of lane k % L; a full warp whose directions both fit a lane
 // each holds out-entry l and in-entry l in lane l.  buf: 128 words of the
 // warp's shared memory.  Groups without a vertex of their own (active =
-// false) repeat another's and write nothing.
-template <bool GIVEN, bool DENSE, int L>
+// false) repeat another's and write nothing.  GEN: the general mode (L = 8 or
+// 16).
+template <bool GIVEN, bool DENSE, bool GEN, int L>
 __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool active, int lane,
                                              uint32_t* buf) {
   using Mask = typename std::conditional<L == 32, unsigned long long, uint32_t>::type;
@@ -580,7 +683,7 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
   const bool split = L == 32 && no <= 32 && ni <= 32;  // a direction per slot
   int32_t c[2];
   uint32_t w[2], key[2];
-  bool in[2], ok[2];
+  bool in[2], ok[2], loop[2];  // loop: an out-entry to v itself
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int k = hl + L * j;
@@ -589,10 +692,12 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
     ok[j] = e < (in[j] ? ni : no);
     c[j] = -1;
     w[j] = 0u;
+    loop[j] = false;
     if (ok[j]) {
       const int32_t u = __ldg((in[j] ? a.iidx + i0 : a.oidx + o0) + e);
       w[j] = __ldg((in[j] ? a.iw + i0 : a.ow + o0) + e);
       c[j] = __ldg(a.part + u);
+      loop[j] = GEN && !in[j] && u == v;
     }
   }
   const int r = a.part[v];
@@ -642,7 +747,7 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
     if (deg != 0)
       s = proposed(a, at >= 0 ? (int)(skey[at] & 0x7fffffffu) : a.part[0], rnd);
   }
-  double d = 0.0;
+  double d = 0.0, logH = 0.0;
   if (__any_sync(kFull, r != s)) {
     // row r's counts and the column degrees need no proposal
     uint32_t Mo[2], Mt[2];
@@ -660,7 +765,8 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
     Corner q;
     load_degrees(a, v, r, s, q);
     // the entries of each block: bit k of eq[j] for entry k
-    Mask eq[2] = {0, 0};
+    // (general mode: anyd, over both directions)
+    Mask eq[2] = {0, 0}, anyd[2] = {0, 0};
     const int bound = split ? 32 + ni : no + ni;
     const int nm = L == 32 ? bound : __reduce_max_sync(kFull, bound);
 #pragma unroll
@@ -673,16 +779,23 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
         if (g.y == key[j]) eq[j] |= (Mask)1 << (b + 1);
         if (g.z == key[j]) eq[j] |= (Mask)1 << (b + 2);
         if (g.w == key[j]) eq[j] |= (Mask)1 << (b + 3);
+        if constexpr (GEN) {
+          if (((g.x ^ key[j]) << 1) == 0u) anyd[j] |= (Mask)1 << b;
+          if (((g.y ^ key[j]) << 1) == 0u) anyd[j] |= (Mask)1 << (b + 1);
+          if (((g.z ^ key[j]) << 1) == 0u) anyd[j] |= (Mask)1 << (b + 2);
+          if (((g.w ^ key[j]) << 1) == 0u) anyd[j] |= (Mask)1 << (b + 3);
+        }
       }
     }
-    // the entries in blocks r and s, per direction
-    Mask inR = 0, inS = 0;
+    // the entries in blocks r and s, per direction, and the self loops
+    Mask inR = 0, inS = 0, selfs = 0;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const unsigned bR = __ballot_sync(kFull, c[j] == r), bS = __ballot_sync(kFull, c[j] == s);
       const unsigned lm = L == 32 ? kFull : (1u << (L & 31)) - 1u;
       inR |= (Mask)((bR >> hb) & lm) << (L * j);
       inS |= (Mask)((bS >> hb) & lm) << (L * j);
+      if constexpr (GEN) selfs |= (Mask)((__ballot_sync(kFull, loop[j]) >> hb) & lm) << (L * j);
     }
     const int nout = split ? 32 : no;
     const Mask out = nout >= 2 * L ? ~(Mask)0 : ((Mask)1 << nout) - 1;
@@ -706,9 +819,17 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
     double t1[2], t2[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const bool lead = (eq[j] & (((Mask)1 << (hl + L * j)) - 1)) == 0;
-      entry_terms(a.xlx, ok[j], in[j], c[j], w[j], lead, kc[j], Mo[j], Mt[j], ld[j], r, s,
-                  rw.niS, t1[j], t2[j]);
+      const Mask below = ((Mask)1 << (hl + L * j)) - 1;
+      const bool lead = (eq[j] & below) == 0;
+      if (GEN && a.exact) {
+        t1[j] = ok[j] && lead && c[j] != r && c[j] != s
+                    ? -exact_term(a.xlx, Mo[j], Mt[j], kc[j])
+                    : 0.0;
+        t2[j] = 0.0;
+      } else {
+        entry_terms(a.xlx, ok[j], in[j], c[j], w[j], lead, kc[j], Mo[j], Mt[j], ld[j], r, s,
+                    rw.niS, t1[j], t2[j]);
+      }
     }
     double acc = 0.0 - t1[0];
     acc -= t2[0];
@@ -719,17 +840,40 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
     } else {
       double acc1 = 0.0 - t1[1];
       acc1 -= t2[1];
-      if constexpr (L == 16) {
+      uint32_t self = 0u;
+      if constexpr (GEN) self = unit ? count(selfs) : mask_weight(sw, selfs);
+      if (GEN && a.exact) {
+        acc = corner_exact(a.xlx, q, rw, self, hl, acc);
+        if constexpr (L == 8) acc1 = corner_exact(a.xlx, q, rw, self, hl + 8, acc1);
+      } else if constexpr (L == 16) {
         acc += corner_term<true, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, hl);
       } else {
         acc += corner_term<true, false>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, hl);
         acc1 += corner_term<false, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, hl + 8);
       }
       acc += acc1;
+      if (GEN && a.mh) {
+        // proposal weights once per block over both directions, then r and s
+        Hast h[2];
+        const Rows<DENSE> R(a, r, s);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const bool lead = (anyd[j] & (((Mask)1 << (hl + L * j)) - 1)) == 0;
+          if (ok[j] && lead && c[j] != r && c[j] != s)
+            hast_block<DENSE>(a, R, c[j], unit ? count(anyd[j]) : mask_weight(sw, anyd[j]), h[j]);
+        }
+        if (hl == 0) hast_rs<DENSE>(a, R, v, r, s, rw, self, h[0]);
+        const double f = group_sum<L>(h[0].f + h[1].f), bk = group_sum<L>(h[0].b + h[1].b);
+        if (no + ni != 0) logH = log(bk) - log(f);
+      }
     }
     d = group_sum<L>(acc);
   }
-  if (hl == 0 && active) write_result(a, GIVEN, i, r, s, r != s ? d : 0.0);
+  if (hl == 0 && active) {
+    d = r != s ? d : 0.0;
+    if constexpr (GEN) write_result_gen(a, GIVEN, i, r, s, d, r != s ? logH : 0.0, x.v[2]);
+    else write_result(a, GIVEN, i, r, s, d);
+  }
   __syncwarp();
 }
 
@@ -737,20 +881,27 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
 // direction) on the CTA, an entry (of up to 256) a thread and slot: on one
 // warp such a vertex, the longest chain of a batch, set the launch time of
 // graphs whose batches fit the GPU at once (20k HH: 34 us a launch, 19 with
-// this path and group_vertex).  The terms are computed by entry and subtracted by warp 0 in the order the warp's lanes would: by
-// entry index up to kWarpList entries, else by rank in the direction's
-// (block, weight) order.
+// this path and group_vertex).  The terms are computed by entry and
+// subtracted by warp 0 in the order the warp's lanes would: by entry index up
+// to kWarpList entries, else by rank in the direction's (block, weight)
+// order.  GEN: the general mode, always by rank, and with T = 32 on one warp
+// for vertices of up to 64 entries.
+template <int T, bool GEN>
 struct LargeBuf {
-  uint32_t key[2 * kWarpList], w[2 * kWarpList];
-  double t1[2 * kWarpList], t2[2 * kWarpList];
-  uint32_t cnt[6];  // koR, koS, niR, niS, out-entries in r, in s
+  uint32_t key[2 * T], w[2 * T];
+  double t1[2 * T], t2[2 * T];
+  double f[GEN ? 2 * T : 1], b[GEN ? 2 * T : 1];  // proposal weights
+  uint32_t cnt[7];  // koR, koS, niR, niS, out-entries in r, in s, self loops
 };
 
-template <bool GIVEN, bool DENSE>
-__device__ void large_vertex(const NodalArgs& a, int i, LargeBuf& sm) {
-  constexpr int T = kNodalWarps * 32;
-  static_assert(2 * T == 2 * kWarpList, "two slots a thread hold a large vertex's entries");
-  const int tid = threadIdx.x, lane = tid & 31;
+template <bool GIVEN, bool DENSE, bool GEN, int T>
+__device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
+  static_assert(T == 32 || (T == kNodalWarps * 32 && T == kWarpList), "a warp or the CTA");
+  const int tid = T == 32 ? threadIdx.x & 31 : threadIdx.x, lane = tid & 31;
+  auto sync = [] {
+    if (T == 32) __syncwarp();
+    else __syncthreads();
+  };
   const int v = GIVEN ? a.verts[i] : a.lo + i;
   const int32_t o0 = a.optr[v], no = a.optr[v + 1] - o0;
   const int32_t i0 = a.iptr[v], ni = a.iptr[v + 1] - i0;
@@ -758,6 +909,7 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf& sm) {
   int32_t c[2];
   uint32_t w[2], key[2];
   bool in[2], ok[2];
+  uint32_t selfp = 0u;
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int k = tid + T * j;
@@ -770,19 +922,29 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf& sm) {
       const int32_t u = __ldg((in[j] ? a.iidx + i0 : a.oidx + o0) + e);
       w[j] = __ldg((in[j] ? a.iw + i0 : a.ow + o0) + e);
       c[j] = __ldg(a.part + u);
+      if (GEN && !in[j] && u == v) selfp += w[j];
     }
     key[j] = ok[j] ? (uint32_t)c[j] | (in[j] ? 0x80000000u : 0u) : 0xffffffffu;
     sm.key[k] = key[j];
     sm.w[k] = w[j];
   }
   const int r = a.part[v];
-  if (tid < 6) sm.cnt[tid] = 0u;
-  const bool unit = __syncthreads_and(w[0] <= 1u && w[1] <= 1u);
+  if (tid < 7) sm.cnt[tid] = 0u;
+  const bool light = w[0] <= 1u && w[1] <= 1u;
+  bool unit;
+  if (T == 32) {
+    unit = __all_sync(kFull, light);
+    __syncwarp();
+  } else {
+    unit = __syncthreads_and(light);
+  }
+  uint32_t u2 = 0u;
   int s;
   if (GIVEN) {
     s = a.props_in[i];
   } else {
     const P4 x = draw(a.seed, kRngNodalVertex, a.seq + ctl_itr(a.ctl) * a.seq_mul, (uint32_t)v);
+    u2 = x.v[2];
     const int rnd = (int)(x.v[0] % (uint32_t)a.B);
     const uint64_t t = scale_draw(x.v[1], (uint64_t)a.kdo[v] + a.kdi[v]);
     int at = (int)t;
@@ -804,8 +966,11 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf& sm) {
     s = proposed(a, at >= 0 ? (int)(sm.key[at] & 0x7fffffffu) : a.part[0], rnd);
   }
   if (r == s) {  // the same in every thread
-    if (tid == 0) write_result(a, GIVEN, i, r, s, 0.0);
-    __syncthreads();
+    if (tid == 0) {
+      if constexpr (GEN) write_result_gen(a, GIVEN, i, r, s, 0.0, 0.0, u2);
+      else write_result(a, GIVEN, i, r, s, 0.0);
+    }
+    sync();
     return;
   }
   uint32_t Mo[2], Mt[2];
@@ -824,24 +989,20 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf& sm) {
       if (!in[j]) atomicAdd(sm.cnt + 5, 1u);
     }
   }
+  if (GEN && selfp) atomicAdd(sm.cnt + 6, selfp);
   row_counts<DENSE, 2>(a, r, in, c, want, Mo);
   row_counts<DENSE, 2>(a, s, in, c, ok, Mt);
   Corner q{};
-  if (tid < 32) {
-    const uint32_t mm =
-        lane < 4 ? Rows<DENSE>(a, r, s).out_at((lane & 2) != 0, (lane & 1) ? s : r) : 0u;
-    load_degrees(a, v, r, s, q);
-    q.Mrr = __shfl_sync(kFull, mm, 0);
-    q.Mrs = __shfl_sync(kFull, mm, 1);
-    q.Msr = __shfl_sync(kFull, mm, 2);
-    q.Mss = __shfl_sync(kFull, mm, 3);
-  }
+  if (tid < 32) q = load_corner<DENSE>(a, v, r, s, lane);
   // each entry's block total, whether an entry of its block comes before it
   // in the summing order, and its place in that order
-  uint32_t kc[2] = {0u, 0u};
+  // (general mode: also the block's total over both directions, and whether
+  // it has an out-entry)
+  uint32_t kc[2] = {0u, 0u}, kany[2] = {0u, 0u};
   int pos[2];
-  bool lead[2];
-  if (n <= kWarpList) {
+  bool lead[2], outside[2] = {false, false};
+  const bool by_index = !GEN && n <= kWarpList;
+  if (by_index) {
     bool before = false;
     for (int b = 0; b < n; b += 4) {  // idle slots match no entry
       const uint4 g = *reinterpret_cast<const uint4*>(sm.key + b);
@@ -866,143 +1027,85 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf& sm) {
         const bool first = e && (u < w[j] || (u == w[j] && b < tid + T * j));
         same[j] += first ? 1 : 0;
         rank[j] += first || g < key[j] ? 1 : 0;
+        if constexpr (GEN) {
+          const bool same_block = ((g ^ key[j]) << 1) == 0u;
+          kany[j] += same_block ? u : 0u;
+          outside[j] = outside[j] || (same_block && b < no);
+        }
       }
     }
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       lead[j] = same[j] == 0;
-      // out-entries' keys rank before every in-entry's
-      pos[j] = in[j] ? kWarpList + rank[j] - no : rank[j];
+      pos[j] = rank[j];  // out-entries' keys rank before every in-entry's
     }
   }
-  __syncthreads();
+  sync();
   const RsWeights rw{sm.cnt[0], sm.cnt[1], sm.cnt[2], sm.cnt[3]};
 #pragma unroll
-  for (int j = 0; j < 2; ++j)
-    if (ok[j])
+  for (int j = 0; j < 2; ++j) {
+    if (!ok[j]) continue;
+    if (GEN && a.exact) {
+      sm.t1[pos[j]] = lead[j] && c[j] != r && c[j] != s
+                          ? -exact_term(a.xlx, Mo[j], Mt[j], kc[j])
+                          : 0.0;
+      sm.t2[pos[j]] = 0.0;
+    } else {
       entry_terms(a.xlx, true, in[j], c[j], w[j], lead[j], kc[j], Mo[j], Mt[j], ld[j], r, s,
                   rw.niS, sm.t1[pos[j]], sm.t2[pos[j]]);
-  __syncthreads();
+    }
+    if constexpr (GEN) {
+      // a block on both lists is counted with the out-list
+      Hast h;
+      if (a.mh && lead[j] && c[j] != r && c[j] != s && !(in[j] && outside[j]))
+        hast_block<DENSE>(a, Rows<DENSE>(a, r, s), c[j], kany[j], h);
+      sm.f[pos[j]] = h.f;
+      sm.b[pos[j]] = h.b;
+    }
+  }
+  sync();
   if (tid < 32) {
     double acc = 0.0;
-    const int n0 = n <= kWarpList ? n : no, n1 = n <= kWarpList ? 0 : ni;
-    for (int p = lane; p < n0; p += 32) {
-      acc -= sm.t1[p];
-      acc -= sm.t2[p];
+    Hast h;
+    const int n0 = by_index ? n : no;
+    for (int lo = 0, hi = n0; lo < n; lo = hi, hi = n)
+      for (int p = lo + lane; p < hi; p += 32) {
+        acc -= sm.t1[p];
+        acc -= sm.t2[p];
+        if constexpr (GEN) {
+          h.f += sm.f[p];
+          h.b += sm.b[p];
+        }
+      }
+    if (GEN && a.exact) {
+      acc = corner_exact(a.xlx, q, rw, sm.cnt[6], lane, acc);
+    } else {
+      const RowChange m = row_change(q, rw, sm.cnt[4], sm.cnt[5]);
+      acc += corner_term<true, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, lane);
     }
-    for (int p = kWarpList + lane; p < kWarpList + n1; p += 32) {
-      acc -= sm.t1[p];
-      acc -= sm.t2[p];
-    }
-    const RowChange m = row_change(q, rw, sm.cnt[4], sm.cnt[5]);
-    acc += corner_term<true, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, lane);
     const double d = warp_sum(acc);
-    if (lane == 0) write_result(a, GIVEN, i, r, s, d);
+    if constexpr (GEN) {
+      double logH = 0.0;
+      if (a.mh) {
+        if (lane == 0) hast_rs<DENSE>(a, Rows<DENSE>(a, r, s), v, r, s, rw, sm.cnt[6], h);
+        const double f = warp_sum(h.f), b = warp_sum(h.b);
+        logH = log(b) - log(f);
+      }
+      if (lane == 0) write_result_gen(a, GIVEN, i, r, s, d, logH, u2);
+    } else if (lane == 0) {
+      write_result(a, GIVEN, i, r, s, d);
+    }
   }
-  __syncthreads();  // the CTA's next vertex reuses the buffer
+  sync();  // the next vertex reuses the buffer
 }
 
-// ------------------------------------------------------------ general mode --
-// Kernels instantiated with GEN = true score a move by the exact change of
-// the MDL (exact = 1) or by GSAP's terms (exact = 0), and accept it by
-// Metropolis-Hastings (mh = 1) or iff dS < 0.
-//
-// Exact dS.  S = model - data_S with
-//   data_S = sum_cells M log2 M - sum_rows d_out log2 d_out - sum_cols d_in log2 d_in
-// and the model term fixed while B is.  Moving v from r to s, with kout[c]
-// and kin[c] v's weight to and from block c (self loops of weight `self`
-// apart), moves kout[c] from cell (r,c) to (s,c) and kin[c] from (c,r) to
-// (c,s) for every c other than r and s, changes the four corner cells as in
-// corner_exact, and moves v's out- and in-degree between the rows and
-// columns r and s; dS = -(change of data_S).  Only those cells and four
-// degrees enter, each as x log2 x.
-//
-// Hastings ratio of GSAP's proposal (kernels.hpp:877-1032): v picks an
-// incident edge with probability proportional to its weight, the edge's
-// other end lies in block t, and s is proposed with probability
-// (M_ts + M_st + 1) / (d_t + B), d_t = d_out[t] + d_in[t], so
-//   p(r -> s) = sum_t k_t (M_ts + M_st + 1) / (d_t + B) / k_v
-// with k_t v's weight to and from t (a self loop counts in both directions)
-// and k_v the sum of the k_t.  The reverse move reads the blockmodel after
-// the move, in which the self loops sit in block s.  A move is accepted when
-//   u < 2^(-beta dS) p(s -> r) / p(r -> s)
-// with u the vertex's third draw scaled to [0, 1).
-
-struct Hast {
-  double f = 0.0, b = 0.0;  // forward and reverse proposal weights (k_v times p)
-};
-
-// Exact dS of the off-corner cells of one neighbour block c (direction
-// `in`, v's total weight kc to or from c, counted once per block).
+// exact_term of an entry added to q where it leads its block.
 template <bool DENSE>
 __device__ __forceinline__ void entry_exact(const NodalArgs& a, const Rows<DENSE>& R, int r, int s,
                                             bool in, int32_t c, bool leader, uint32_t kc,
                                             Acc& q) {
   if (!leader || c == r || c == s) return;
-  const uint32_t Mo = in ? R.in_r(c) : R.out_r(c);
-  const uint32_t Mt = in ? R.in_s(c) : R.out_s(c);
-  q.acc += xlx(a.xlx, Mo) - xlx(a.xlx, Mo - kc) + xlx(a.xlx, Mt) - xlx(a.xlx, Mt + kc);
-}
-
-// Corner cells and the four degrees of the exact dS, on lanes 0..15 of the
-// calling warp: lanes 0-3 the old cells (r,r), (r,s), (s,r), (s,s), lanes
-// 4-7 the same cells after the move, lanes 8-11 the new degrees d_out[r],
-// d_out[s], d_in[r], d_in[s], lanes 12-15 the old ones.  koR..niS include
-// the self loops (their other end is in r).
-template <bool DENSE>
-__device__ __forceinline__ void corner_exact(const NodalArgs& a, const Rows<DENSE>& R, int v,
-                                             int r, int s, const RsWeights& w, uint32_t self,
-                                             Acc& q) {
-  const int lane = threadIdx.x & 31;
-  if (lane >= 16) return;
-  const int j = lane & 3;
-  double t;
-  if (lane < 8) {
-    const uint32_t M = R.out_at((j & 2) != 0, (j & 1) ? s : r);
-    // unsigned wrap-around in the middle is fine: the results are >= 0
-    const uint32_t x = j == 0   ? M - w.koR - w.niR + self
-                       : j == 1 ? M - w.koS + (w.niR - self)
-                       : j == 2 ? M + (w.koR - self) - w.niS
-                                : M + w.koS + w.niS + self;
-    t = lane < 4 ? xlx(a.xlx, M) : -xlx(a.xlx, x);
-  } else {
-    const uint32_t kO = a.kdo[v], kI = a.kdi[v];
-    const uint32_t d0 = j == 0 ? a.d_out[r] : j == 1 ? a.d_out[s] : j == 2 ? a.d_in[r] : a.d_in[s];
-    const uint32_t d1 = j == 0 ? d0 - kO : j == 1 ? d0 + kO : j == 2 ? d0 - kI : d0 + kI;
-    t = lane < 12 ? xlx(a.xlx, d1) : -xlx(a.xlx, d0);
-  }
-  q.acc += t;
-}
-
-// Proposal weights of a neighbour block t other than r and s, kt = v's
-// weight to and from t.
-template <bool DENSE>
-__device__ __forceinline__ void hast_block(const NodalArgs& a, const Rows<DENSE>& R, int32_t t,
-                                           uint32_t kt, Hast& h) {
-  const double D = (double)a.d_out[t] + (double)a.d_in[t] + (double)a.B;
-  const double k = (double)kt;
-  h.f += k * ((double)R.in_s(t) + (double)R.out_s(t) + 1.0) / D;
-  h.b += k * ((double)R.in_r(t) + (double)R.out_r(t) - k + 1.0) / D;
-}
-
-// Proposal weights of blocks r and s (one thread of the group).
-template <bool DENSE>
-__device__ __forceinline__ void hast_rs(const NodalArgs& a, const Rows<DENSE>& R, int v, int r,
-                                        int s, const RsWeights& w, uint32_t self, Hast& h) {
-  const uint32_t Mrr = R.out_at(false, r), Mrs = R.out_at(false, s);
-  const uint32_t Msr = R.out_at(true, r), Mss = R.out_at(true, s);
-  const uint32_t xrr = Mrr - w.koR - w.niR + self;
-  const uint32_t xrs = Mrs - w.koS + (w.niR - self);
-  const uint32_t xsr = Msr + (w.koR - self) - w.niS;
-  const double kv = (double)a.kdo[v] + (double)a.kdi[v], Bd = (double)a.B;
-  const double Dr = (double)a.d_out[r] + (double)a.d_in[r];
-  const double Ds = (double)a.d_out[s] + (double)a.d_in[s];
-  const double kr = (double)w.koR + (double)w.niR, ks = (double)w.koS + (double)w.niS;
-  const double sl = 2.0 * (double)self;
-  h.f += kr * ((double)Mrs + (double)Msr + 1.0) / (Dr + Bd);
-  h.f += ks * ((double)Mss + (double)Mss + 1.0) / (Ds + Bd);
-  h.b += (kr - sl) * ((double)xrr + (double)xrr + 1.0) / (Dr - kv + Bd);
-  h.b += (ks + sl) * ((double)xsr + (double)xrs + 1.0) / (Ds + kv + Bd);
+  q.acc += exact_term(a.xlx, in ? R.in_r(c) : R.out_r(c), in ? R.in_s(c) : R.out_s(c), kc);
 }
 
 // v's self-loop weight (group sum over its out-list).
@@ -1022,7 +1125,9 @@ __device__ double finish_gen(const NodalArgs& a, const Rows<DENSE>& R, int v, in
                              const RsWeights& w, uint32_t self, Acc q, Hast h,
                              const Group<G>& grp, double& logH) {
   if (a.exact) {
-    if (G == 32 || threadIdx.x < 32) corner_exact<DENSE>(a, R, v, r, s, w, self, q);
+    if (G == 32 || threadIdx.x < 32)
+      q.acc = corner_exact(a.xlx, load_corner<DENSE>(a, v, r, s, threadIdx.x & 31), w, self,
+                           threadIdx.x & 31, q.acc);
   } else {
     q.m4 = (int)grp.sum_ll(q.m4);
     q.m5 = (int)grp.sum_ll(q.m5);
@@ -1037,118 +1142,6 @@ __device__ double finish_gen(const NodalArgs& a, const Rows<DENSE>& R, int v, in
     if ((uint64_t)a.kdo[v] + a.kdi[v] != 0u) logH = log(b) - log(f);
   }
   return grp.sum(q.acc);
-}
-
-// Both lists fit one warp together: lane l holds entry l (out-entries,
-// then in-entries).
-template <bool DENSE>
-__device__ double delta_registers_gen(const NodalArgs& a, int v, int r, int s, int32_t o0, int no,
-                                      int32_t i0, int ni, int lane, double& logH) {
-  const Rows<DENSE> R(a, r, s);
-  const bool in = lane >= no, valid = lane < no + ni;
-  const int k = in ? lane - no : lane;
-  int32_t c = -1;
-  uint32_t w = 0u, selfp = 0u;
-  if (valid) {
-    const int32_t u = in ? __ldg(a.iidx + i0 + k) : __ldg(a.oidx + o0 + k);
-    w = in ? __ldg(a.iw + i0 + k) : __ldg(a.ow + o0 + k);
-    c = __ldg(a.part + u);
-    if (!in && u == v) selfp = w;
-  }
-  RsWeights rw;
-  rw.koR = __reduce_add_sync(kFull, valid && !in && c == r ? w : 0u);
-  rw.koS = __reduce_add_sync(kFull, valid && !in && c == s ? w : 0u);
-  rw.niR = __reduce_add_sync(kFull, valid && in && c == r ? w : 0u);
-  rw.niS = __reduce_add_sync(kFull, valid && in && c == s ? w : 0u);
-  const uint32_t self = __reduce_add_sync(kFull, selfp);
-  Acc q;
-  const unsigned key = valid ? ((unsigned)c | (in ? 0x80000000u : 0u)) : (0x7fffffe0u + (unsigned)lane);
-  const unsigned peers = __match_any_sync(kFull, key);
-  const uint32_t kc = __reduce_add_sync(peers, w);
-  const bool leader = lane == __ffs(peers) - 1;
-  if (valid) {
-    if (a.exact) entry_exact<DENSE>(a, R, r, s, in, c, leader, kc, q);
-    else entry<DENSE>(a, R, r, s, rw.niS, in, c, w, leader, kc, q);
-  }
-  Hast h;
-  if (a.mh) {
-    // per block over both directions
-    const unsigned pa = __match_any_sync(kFull, valid ? (unsigned)c : 0x7fffffe0u + (unsigned)lane);
-    const uint32_t kt = __reduce_add_sync(pa, w);
-    if (valid && lane == __ffs(pa) - 1 && c != r && c != s) hast_block<DENSE>(a, R, c, kt, h);
-    if (lane == 0) hast_rs<DENSE>(a, R, v, r, s, rw, self, h);
-  }
-  return finish_gen<DENSE, 32>(a, R, v, r, s, rw, self, q, h, Group<32>{nullptr}, logH);
-}
-
-// Weight of block c's run in a sorted list; false when c is absent.
-__device__ __forceinline__ bool run_weight(const unsigned long long* key, int n, int32_t c,
-                                           uint32_t& w) {
-  const unsigned long long k0 = (unsigned long long)(uint32_t)c << 32;
-  int lo = 0, hi = n;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (key[mid] < k0) lo = mid + 1;
-    else hi = mid;
-  }
-  w = 0u;
-  const bool found = lo < n && kblk(key[lo]) == c;
-  for (; lo < n && kblk(key[lo]) == c; ++lo) w += kwt(key[lo]);
-  return found;
-}
-
-template <bool DENSE, int G>
-__device__ double delta_sorted_gen(const NodalArgs& a, int v, int r, int s,
-                                   const unsigned long long* ko, int no,
-                                   const unsigned long long* ki, int ni, const Group<G>& grp,
-                                   double& logH) {
-  const int t = grp.rank();
-  const Rows<DENSE> R(a, r, s);
-  uint32_t koR = 0, koS = 0, niR = 0, niS = 0;
-  for (int k = t; k < no; k += G) {
-    int32_t c = kblk(ko[k]);
-    koR += c == r ? kwt(ko[k]) : 0u;
-    koS += c == s ? kwt(ko[k]) : 0u;
-  }
-  for (int k = t; k < ni; k += G) {
-    int32_t c = kblk(ki[k]);
-    niR += c == r ? kwt(ki[k]) : 0u;
-    niS += c == s ? kwt(ki[k]) : 0u;
-  }
-  const RsWeights w{(uint32_t)grp.sum_ll(koR), (uint32_t)grp.sum_ll(koS),
-                    (uint32_t)grp.sum_ll(niR), (uint32_t)grp.sum_ll(niS)};
-  const uint32_t self = self_weight<G>(a, v, grp);
-  Acc q;
-  Hast h;
-  for (int k = t; k < no; k += G) {
-    const int32_t c = kblk(ko[k]);
-    const bool leader = k == 0 || kblk(ko[k - 1]) != c;
-    uint32_t kc = 0;
-    if (leader)
-      for (int j = k; j < no && kblk(ko[j]) == c; ++j) kc += kwt(ko[j]);
-    if (a.exact) entry_exact<DENSE>(a, R, r, s, false, c, leader, kc, q);
-    else entry<DENSE>(a, R, r, s, w.niS, false, c, kwt(ko[k]), leader, kc, q);
-    if (a.mh && leader && c != r && c != s) {
-      uint32_t kin;
-      run_weight(ki, ni, c, kin);
-      hast_block<DENSE>(a, R, c, kc + kin, h);
-    }
-  }
-  for (int k = t; k < ni; k += G) {
-    const int32_t c = kblk(ki[k]);
-    const bool leader = k == 0 || kblk(ki[k - 1]) != c;
-    uint32_t kc = 0;
-    if (leader)
-      for (int j = k; j < ni && kblk(ki[j]) == c; ++j) kc += kwt(ki[j]);
-    if (a.exact) entry_exact<DENSE>(a, R, r, s, true, c, leader, kc, q);
-    else entry<DENSE>(a, R, r, s, w.niS, true, c, kwt(ki[k]), leader, kc, q);
-    uint32_t kout;
-    // blocks on both lists were counted with the out-list
-    if (a.mh && leader && c != r && c != s && !run_weight(ko, no, c, kout))
-      hast_block<DENSE>(a, R, c, kc, h);
-  }
-  if (a.mh && t == 0) hast_rs<DENSE>(a, R, v, r, s, w, self, h);
-  return finish_gen<DENSE, G>(a, R, v, r, s, w, self, q, h, grp, logH);
 }
 
 template <bool DENSE, int G>
@@ -1239,31 +1232,6 @@ __device__ double delta_hashed_gen(const NodalArgs& a, int v, int r, int s, Hash
   return finish_gen<DENSE, G>(a, R, v, r, s, rw, self, q, hs, grp, logH);
 }
 
-constexpr double kLn2 = 0.6931471805599453;
-
-// Accept test of a general-mode move (r != s).
-__device__ __forceinline__ bool accept_move(const NodalArgs& a, double d, double logH,
-                                            uint32_t u) {
-  if (!a.mh) return d < 0.0;
-  // -beta * dS * ln 2 + logH, rounded step by step (no contraction)
-  const double x = __dadd_rn(__dmul_rn(__dmul_rn(-a.beta, d), kLn2), logH);
-  if (x >= 0.0) return true;
-  return log((double)u * 2.3283064365386963e-10) < x;
-}
-
-__device__ __forceinline__ void write_result_gen(const NodalArgs& a, bool given, int i, int r,
-                                                 int s, double d, double logH, uint32_t u) {
-  if (given) {
-    a.dS_raw[i] = d;
-    if (a.logH_raw) a.logH_raw[i] = logH;
-    return;
-  }
-  const bool acc = r != s && accept_move(a, d, logH, u);
-  a.newlab[i] = acc ? s : r;
-  a.rec[i] = acc ? d : 0.0;
-  if (a.props_out) a.props_out[i] = s;
-}
-
 // Work items of the warp kernel, larger vertices first (as the host lists
 // them: a longest-first schedule): a CTA per large vertex, then a warp per
 // vertex of up to 64 entries, per two of up to 32 and per four small ones.
@@ -1279,101 +1247,50 @@ struct NodalItems {
 template <bool GIVEN, bool DENSE, bool GEN>
 struct NodalBody {
   using Args = NodalArgs;
-  static constexpr int kThreads = kNodalWarps * 32, kMinBlocks = DENSE ? 8 : 6;
+  static constexpr int kThreads = kNodalWarps * 32;
+  static constexpr int kMinBlocks = GEN ? 5 : DENSE ? 8 : 6;
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
     if (ctl_stopped(a.ctl)) return;
-    __shared__ __align__(16) unsigned char raw[sizeof(LargeBuf)];
-    static_assert(kNodalWarps * 128 * sizeof(uint32_t) <= sizeof(LargeBuf), "warp buffers");
+    using Large = LargeBuf<kThreads, GEN>;
+    // per warp: the keys and weights of group_vertex, or (general mode) a
+    // 33-64-entry vertex's LargeBuf
+    using Mid = LargeBuf<32, GEN>;
+    constexpr size_t kWarpBytes = GEN ? (sizeof(Mid) + 15) / 16 * 16 : 128 * sizeof(uint32_t);
+    constexpr size_t kBytes =
+        sizeof(Large) > kNodalWarps * kWarpBytes ? sizeof(Large) : kNodalWarps * kWarpBytes;
+    __shared__ __align__(16) unsigned char raw[kBytes];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t* buf = reinterpret_cast<uint32_t*>(raw) + 128 * wid;
+    unsigned char* const own = raw + kWarpBytes * wid;
+    uint32_t* const buf = reinterpret_cast<uint32_t*>(own);
     const int nmid32 = a.nmid - a.nlarge - a.nmid64;
     const NodalItems n(a.nlarge, a.nmid64, nmid32, a.nsmall);
     const int32_t *mid64 = a.mid + a.nlarge, *mid32 = mid64 + a.nmid64;
     for (int blk = vb; blk < n.ctas(); blk += vg) {
       if (blk < n.large) {
-        large_vertex<GIVEN, DENSE>(a, a.mid[blk], *reinterpret_cast<LargeBuf*>(raw));
+        large_vertex<GIVEN, DENSE, GEN, kThreads>(a, a.mid[blk], *reinterpret_cast<Large*>(raw));
         continue;
       }
       int it = (blk - n.large) * kNodalWarps + wid;
       if (it < n.mid64) {
-        group_vertex<GIVEN, DENSE, 32>(a, mid64[it], true, lane, buf);
+        if constexpr (GEN)
+          large_vertex<GIVEN, DENSE, GEN, 32>(a, mid64[it], *reinterpret_cast<Mid*>(own));
+        else
+          group_vertex<GIVEN, DENSE, GEN, 32>(a, mid64[it], true, lane, buf);
         continue;
       }
       it -= n.mid64;
       if (it < n.mid32) {
         const int q = 2 * it + (lane >> 4);
-        group_vertex<GIVEN, DENSE, 16>(a, mid32[min(q, nmid32 - 1)], q < nmid32, lane, buf);
+        group_vertex<GIVEN, DENSE, GEN, 16>(a, mid32[min(q, nmid32 - 1)], q < nmid32, lane, buf);
         continue;
       }
       it -= n.mid32;
       if (it < n.small) {
         const int q = 4 * it + (lane >> 3);
-        group_vertex<GIVEN, DENSE, 8>(a, a.small[min(q, a.nsmall - 1)], q < a.nsmall, lane, buf);
+        group_vertex<GIVEN, DENSE, GEN, 8>(a, a.small[min(q, a.nsmall - 1)], q < a.nsmall, lane,
+                                           buf);
       }
-    }
-  }
-};
-
-// General mode (exact scoring, Metropolis-Hastings): one vertex on the whole
-// warp, the dS from registers (at most 32 entries) or from sorted
-// shared-memory lists.  buf: the warp's 2 * kWarpList words of shared memory.
-template <bool GIVEN, bool DENSE>
-__device__ __forceinline__ void warp_vertex_gen(const NodalArgs& a, int i, int lane,
-                                                unsigned long long* buf) {
-  const Group<32> grp{nullptr};
-  unsigned long long* sko = buf;
-  unsigned long long* ski = buf + kWarpList;
-  const int vv = GIVEN ? a.verts[i] : a.lo + i;
-  const int32_t o0 = a.optr[vv], no = a.optr[vv + 1] - o0;
-  const int32_t i0 = a.iptr[vv], ni = a.iptr[vv + 1] - i0;
-  int v, s;
-  uint32_t u2;
-  item<GIVEN>(a, i, lane, v, s, u2);
-  const int r = a.part[v];
-  double d = 0.0, lh = 0.0;
-  if (r != s) {
-    if (no + ni <= 32) {
-      d = delta_registers_gen<DENSE>(a, v, r, s, o0, no, i0, ni, lane, lh);
-    } else {
-      stage_sorted<32>(a.oidx, a.ow, a.part, o0, no, sko, grp);
-      stage_sorted<32>(a.iidx, a.iw, a.part, i0, ni, ski, grp);
-      d = delta_sorted_gen<DENSE, 32>(a, v, r, s, sko, no, ski, ni, grp, lh);
-    }
-  }
-  if (lane == 0) write_result_gen(a, GIVEN, i, r, s, d, lh, u2);
-  __syncwarp();
-}
-
-// Items of the general-mode kernel: the mid vertices, then pairs of small
-// ones.
-__host__ __device__ __forceinline__ int nodal_gen_items(int nsmall, int nmid) {
-  return (nsmall + 1) / 2 + nmid;
-}
-
-template <bool GIVEN, bool DENSE>
-struct NodalBody<GIVEN, DENSE, true> {
-  using Args = NodalArgs;
-  static constexpr int kThreads = kNodalWarps * 32, kMinBlocks = 4;
-  static constexpr size_t kSmem = 0;
-  static __device__ void run(const Args& a, int vb, int vg) {
-    if (ctl_stopped(a.ctl)) return;
-    __shared__ unsigned long long s_buf[kNodalWarps][2 * kWarpList];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int nw = vg * kNodalWarps;
-    const int items = nodal_gen_items(a.nsmall, a.nmid);
-    for (int it0 = vb * kNodalWarps + wid; it0 < items; it0 += nw) {
-      int ia, ib = -1;
-      if (it0 < a.nmid) {
-        ia = a.mid[it0];
-      } else {
-        const int it = it0 - a.nmid;
-        ia = a.small[2 * it];
-        ib = 2 * it + 1 < a.nsmall ? a.small[2 * it + 1] : -1;
-      }
-      // one call site, so that the body stays inline
-      for (int q = 0; q < (ib >= 0 ? 2 : 1); ++q)
-        warp_vertex_gen<GIVEN, DENSE>(a, q ? ib : ia, lane, s_buf[wid]);
     }
   }
 };
@@ -1492,20 +1409,6 @@ __device__ __forceinline__ void add_rs(uint32_t* cnt, bool in, int c, int r, int
     atomicAdd(cnt + (in ? 3 : 1), w);
     if (!in) atomicAdd(cnt + 5, 1u);
   }
-}
-
-// Corner counts and degrees for corner_term, on a full warp.
-template <bool DENSE>
-__device__ __forceinline__ Corner load_corner(const NodalArgs& a, int v, int r, int s, int lane) {
-  const uint32_t mm =
-      lane < 4 ? Rows<DENSE>(a, r, s).out_at((lane & 2) != 0, (lane & 1) ? s : r) : 0u;
-  Corner q{};
-  load_degrees(a, v, r, s, q);
-  q.Mrr = __shfl_sync(kFull, mm, 0);
-  q.Mrs = __shfl_sync(kFull, mm, 1);
-  q.Msr = __shfl_sync(kFull, mm, 2);
-  q.Mss = __shfl_sync(kFull, mm, 3);
-  return q;
 }
 
 // A vertex of more than kWarpList entries in a direction, at most
@@ -1987,8 +1890,7 @@ NodalArgs make_args(const DevGraph& g, const int32_t* part, const DevBM& m, int3
 }
 
 // CTAs of the warp kernel.
-int32_t nodal_ctas(const NodalArgs& a, bool gen) {
-  if (gen) return ceil_div(nodal_gen_items(a.nsmall, a.nmid), kNodalWarps);
+int32_t nodal_ctas(const NodalArgs& a) {
   return NodalItems(a.nlarge, a.nmid64, a.nmid - a.nlarge - a.nmid64, a.nsmall).ctas();
 }
 
@@ -2005,7 +1907,7 @@ void launch_pair(const NodalArgs& a, const NodalAux& aux, cudaStream_t st) {
                                                      aux.side);
     cudaEventRecord(aux.join, aux.side);
   }
-  launch_single<NodalBody<GIVEN, DENSE, GEN>>(a, nodal_ctas(a, GEN), st);
+  launch_single<NodalBody<GIVEN, DENSE, GEN>>(a, nodal_ctas(a), st);
   if (a.nheavy > 0) cudaStreamWaitEvent(st, aux.join, 0);
 }
 
@@ -2118,7 +2020,7 @@ void add_nodal(Slot& warp, Slot& heavy, Slot& hub, bool dense, const ScoreMode& 
   a.ctl = ctl;
   a.seq_mul = seq_mul;
   set_mode(a, md);
-  slot_push(slot_bind(warp, kmNodal[md.slot(dense)]), a, nodal_ctas(a, md.general()));
+  slot_push(slot_bind(warp, kmNodal[md.slot(dense)]), a, nodal_ctas(a));
   const int32_t nhub = md.general() ? 0 : aux.nhub;
   slot_push(slot_bind(heavy, kmNodalHeavy[md.slot(dense)]), a, aux.nheavy - nhub);
   if (nhub > 0) slot_push(slot_bind(hub, kmNodalHub[dense ? 1 : 0]), a, kHubCluster * nhub);

@@ -388,7 +388,7 @@ sbp_status sbp_mdl_mode(const sbp_graph_csr* g, const int32_t* part, int32_t B, 
  * serving loops that forbid the synchronisation a cudaMalloc or cudaFree can
  * cost.  The caller passes inputs and outputs; the scratch is a fixed ~2 KB
  * device array of the library, held by every GPU that loads it until the
- * process exits, so B <= 65536 (larger B returns SBP_ERR_INVALID).  The first
+ * process exits.  B <= 65536 (larger B returns SBP_ERR_INVALID).  The first
  * call on a device looks that array's address up (once per device, with the
  * device current), so make it before any stream capture; the address is not
  * valid after a cudaDeviceReset.  All calls share the array, which keeps the
