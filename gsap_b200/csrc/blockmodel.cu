@@ -817,7 +817,10 @@ struct DenseArgs {
   uint32_t *Md, *MTd, *Sd, *d_out, *d_in;
   double *ld_out, *ld_in;
   const int32_t* ctl;
-  int32_t N, E, B, lo, count, pad;
+  // update: the batch's heavy vertices (more than heavy_min entries in a
+  // direction), and the vertices a warp covers
+  const int32_t* heavy;
+  int32_t N, E, B, lo, count, nheavy, heavy_min, per_warp;
 };
 
 // Chunk sums of a dense cell (r, c): out-row r's chunk of column c and
@@ -971,84 +974,113 @@ struct DenseLogsBody {
 // The moved vertices of a batch: its out-edges move from (r, old block of
 // w) to (s, new block of w); its in-edges from unmoved sources move from
 // (b(u), r) to (b(u), s).  Edges between two moved vertices are handled
-// once, from the source's out-edges.  A lane per batch vertex finds the
-// moved ones (about a tenth of a batch once the first sweeps are done);
-// the warp then applies each moved vertex's entries together, lane-strided.
-// A warp covers kDuVerts batch vertices, so that the moved ones (a few per
-// warp at most) are spread over many warps: their dependent loads are the
-// latency of the launch.
+// once, from the source's out-edges.
+//
+// What bounds a launch is the latency of its longest warp.  A warp covers a
+// few batch vertices (one for batches of a few thousand, up to eight, so that
+// every SM has some 16 warps): a lane each finds the moved ones and loads
+// their row bounds, then the warp strides over all their entries together,
+// whatever vertex they belong to.  Heavy vertices, listed, have a CTA each.
+// A warp that took eight vertices' moved ones, and their two directions, one
+// after the other took 7.5 us a launch at 20k HH in the median and up to 86
+// where a heavy vertex moved (13 and 230 at 200k); this 5.3, at most 24.
 constexpr int kDuVerts = 8;
+struct DenseMove {
+  int32_t r, s, o0, no, i0, ni;
+};
+
+// Applies entry e (out-entries, then in-entries) of a moved vertex.
+__device__ __forceinline__ void dense_move_entry(const DenseArgs& a, const DenseMove& v, int e) {
+  const int32_t lo = a.lo, count = a.count, B = a.B;
+  const int K = (B + 31) >> 5;
+  const bool in = e >= v.no;
+  const int j = in ? v.i0 + e - v.no : v.o0 + e;
+  const int x = __ldg((in ? a.iidx : a.oidx) + j);
+  const uint32_t wt = __ldg((in ? a.iw : a.ow) + j);
+  const int bo = __ldg(a.part + x);
+  const int bn = x >= lo && x < lo + count ? __ldg(a.newlab + x - lo) : bo;
+  if (in && bn != bo) return;  // moved source
+  // the cell the edge leaves and the one it joins
+  const int r0 = in ? bo : v.r, c0 = in ? v.r : bo;
+  const int r1 = in ? bo : v.s, c1 = in ? v.s : bn;
+  atomicSub(a.Md + (size_t)r0 * B + c0, wt);
+  atomicSub(a.MTd + (size_t)c0 * B + r0, wt);
+  atomicAdd(a.Md + (size_t)r1 * B + c1, wt);
+  atomicAdd(a.MTd + (size_t)c1 * B + r1, wt);
+  atomicSub(sd_out(a.Sd, K, r0, c0), wt);
+  atomicSub(sd_in(a.Sd, K, r0, c0), wt);
+  atomicAdd(sd_out(a.Sd, K, r1, c1), wt);
+  atomicAdd(sd_in(a.Sd, K, r1, c1), wt);
+}
+
+__device__ __forceinline__ void dense_move_degrees(const DenseArgs& a, int v, int r, int s) {
+  const uint32_t o = a.kdo[v], i = a.kdi[v];
+  atomicSub(a.d_out + r, o);
+  atomicAdd(a.d_out + s, o);
+  atomicSub(a.d_in + r, i);
+  atomicAdd(a.d_in + s, i);
+}
+
 struct DenseUpdateBody {
   using Args = DenseArgs;
   static constexpr int kThreads = 256, kMinBlocks = 1;
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
-  if (ctl_stopped(a.ctl)) return;
-  const int32_t* __restrict__ optr = a.optr;
-  const int32_t* __restrict__ oidx = a.oidx;
-  const uint32_t* __restrict__ ow = a.ow;
-  const int32_t* __restrict__ iptr = a.iptr;
-  const int32_t* __restrict__ iidx = a.iidx;
-  const uint32_t* __restrict__ iw = a.iw;
-  const uint32_t* __restrict__ kdo = a.kdo;
-  const uint32_t* __restrict__ kdi = a.kdi;
-  const int32_t* __restrict__ part = a.part;
-  const int32_t* __restrict__ newlab = a.newlab;
-  const int32_t lo = a.lo, count = a.count, B = a.B;
-  uint32_t *Md = a.Md, *MTd = a.MTd, *Sd = a.Sd, *d_out = a.d_out, *d_in = a.d_in;
-  const int K = (B + 31) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int nw = (vg * kThreads) >> 5;
-  for (int w0 = ((vb * kThreads + threadIdx.x) >> 5) * kDuVerts; w0 < count;
-       w0 += nw * kDuVerts) {
+    if (ctl_stopped(a.ctl)) return;
+    const int lane = threadIdx.x & 31;
+    if (vb < a.nheavy) {
+      const int i = a.heavy[vb], v = a.lo + i;
+      DenseMove m{a.part[v], a.newlab[i], a.optr[v], 0, a.iptr[v], 0};
+      m.no = a.optr[v + 1] - m.o0;
+      m.ni = a.iptr[v + 1] - m.i0;
+      if (m.r == m.s) return;
+      if (threadIdx.x == 0) dense_move_degrees(a, v, m.r, m.s);
+#pragma unroll 4
+      for (int e = threadIdx.x; e < m.no + m.ni; e += kThreads) dense_move_entry(a, m, e);
+      return;
+    }
+    const int per = a.per_warp;
+    const int w0 = (((vb - a.nheavy) * kThreads + threadIdx.x) >> 5) * per;
     const int i = w0 + lane;
-    int32_t r0 = 0, s0 = 0;
-    if (lane < kDuVerts && i < count) {
-      r0 = part[lo + i];
-      s0 = newlab[i];
-    }
-    unsigned moved = __ballot_sync(kFull, lane < kDuVerts && i < count && r0 != s0);
-    while (moved) {
-      const int src = __ffs(moved) - 1;
-      moved &= moved - 1;
-      const int v = lo + w0 + src;
-      const int r = __shfl_sync(kFull, r0, src), s = __shfl_sync(kFull, s0, src);
-      if (lane == 0) {
-        atomicSub(d_out + r, kdo[v]);
-        atomicAdd(d_out + s, kdo[v]);
-        atomicSub(d_in + r, kdi[v]);
-        atomicAdd(d_in + s, kdi[v]);
-      }
-      for (int j = optr[v] + lane; j < optr[v + 1]; j += 32) {
-        const int x = __ldg(oidx + j);
-        const uint32_t wt = __ldg(ow + j);
-        const int bo = __ldg(part + x);
-        const int bn = (x >= lo && x < lo + count) ? newlab[x - lo] : bo;
-        atomicSub(Md + (size_t)r * B + bo, wt);
-        atomicSub(MTd + (size_t)bo * B + r, wt);
-        atomicAdd(Md + (size_t)s * B + bn, wt);
-        atomicAdd(MTd + (size_t)bn * B + s, wt);
-        atomicSub(sd_out(Sd, K, r, bo), wt);
-        atomicSub(sd_in(Sd, K, r, bo), wt);
-        atomicAdd(sd_out(Sd, K, s, bn), wt);
-        atomicAdd(sd_in(Sd, K, s, bn), wt);
-      }
-      for (int j = iptr[v] + lane; j < iptr[v + 1]; j += 32) {
-        const int u = __ldg(iidx + j);
-        const int bu = __ldg(part + u);
-        if (u >= lo && u < lo + count && newlab[u - lo] != bu) continue;  // moved source
-        const uint32_t wt = __ldg(iw + j);
-        atomicSub(Md + (size_t)bu * B + r, wt);
-        atomicSub(MTd + (size_t)r * B + bu, wt);
-        atomicAdd(Md + (size_t)bu * B + s, wt);
-        atomicAdd(MTd + (size_t)s * B + bu, wt);
-        atomicSub(sd_out(Sd, K, bu, r), wt);
-        atomicSub(sd_in(Sd, K, bu, r), wt);
-        atomicAdd(sd_out(Sd, K, bu, s), wt);
-        atomicAdd(sd_in(Sd, K, bu, s), wt);
+    DenseMove m{0, 0, 0, 0, 0, 0};
+    if (lane < per && i < a.count) {
+      const int v = a.lo + i;
+      m.r = a.part[v];
+      m.s = a.newlab[i];
+      if (m.r != m.s) {
+        m.o0 = a.optr[v];
+        m.no = a.optr[v + 1] - m.o0;
+        m.i0 = a.iptr[v];
+        m.ni = a.iptr[v + 1] - m.i0;
+        if (m.no > a.heavy_min || m.ni > a.heavy_min) m.no = m.ni = 0;  // listed
+        else dense_move_degrees(a, v, m.r, m.s);
       }
     }
-  }
+    int incl = m.no + m.ni;
+#pragma unroll
+    for (int o = 1; o < kDuVerts; o <<= 1) {
+      const int y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(kFull, incl, kDuVerts - 1);
+#pragma unroll 2
+    for (int e0 = 0; e0 < total; e0 += 32) {
+      const int e = e0 + lane;
+      // the vertex of entry e: the first whose running count exceeds it
+      int j = 0;
+#pragma unroll
+      for (int q = 0; q < kDuVerts; ++q) j += __shfl_sync(kFull, incl, q) <= e ? 1 : 0;
+      j = min(j, kDuVerts - 1);
+      DenseMove u;
+      u.r = __shfl_sync(kFull, m.r, j);
+      u.s = __shfl_sync(kFull, m.s, j);
+      u.o0 = __shfl_sync(kFull, m.o0, j);
+      u.no = __shfl_sync(kFull, m.no, j);
+      u.i0 = __shfl_sync(kFull, m.i0, j);
+      u.ni = __shfl_sync(kFull, m.ni, j);
+      const int first = __shfl_sync(kFull, incl, j) - u.no - u.ni;
+      if (e < total) dense_move_entry(a, u, e - first);
+    }
   }
 };
 
@@ -1353,8 +1385,20 @@ DenseArgs dense_args(const DevGraph& g, const int32_t* part, int32_t B, DevBM& m
 
 int32_t vg_block_terms(int32_t B) { return grid_for((long long)B * 32, 256, 8192); }
 int32_t vg_block_draw(int32_t B) { return grid_for((long long)B * 8, 256, 8192); }
-int32_t vg_dense_update(int32_t count) {
-  return grid_for((long long)count, 256 / 32 * kDuVerts, 148 * 16);
+// The update's arguments for a batch: some 16 warps an SM where the batch
+// has the vertices for it.
+void set_update(DenseArgs& a, int32_t lo, int32_t count, const int32_t* newlab,
+                const NodalAux& lists) {
+  a.lo = lo;
+  a.count = count;
+  a.newlab = newlab;
+  a.heavy = lists.heavy;
+  a.nheavy = lists.nheavy;
+  a.heavy_min = nodal_heavy_threshold();
+  a.per_warp = std::max(1, std::min(kDuVerts, count / (148 * 16)));
+}
+int32_t vg_dense_update(const DenseArgs& a) {
+  return a.nheavy + ceil_div(a.count, DenseUpdateBody::kThreads / 32 * a.per_warp);
 }
 
 const MultiKernel kmScanTile = multi_kernel_desc<ScanTileBody>("scan_tile");
@@ -1496,16 +1540,6 @@ void dense_build(const DevGraph& g, const int32_t* part, int32_t B, DevBM& m, cu
   if (g.E > 0) launch_single<DenseEdgesBody>(a, ceil_div(g.E, 256), st);
   launch_single<DenseDegreesBody>(a, ceil_div(g.N, 256), st);
   launch_single<DenseLogsBody>(a, ceil_div(B, 256), st);
-}
-
-void dense_update(const DevGraph& g, const int32_t* part, int32_t lo, int32_t count,
-                  const int32_t* newlab, int32_t B, DevBM& m, cudaStream_t st) {
-  if (count <= 0) return;
-  DenseArgs a = dense_args(g, part, B, m);
-  a.lo = lo;
-  a.count = count;
-  a.newlab = newlab;
-  launch_single<DenseUpdateBody>(a, vg_dense_update(count), st);
 }
 
 void block_terms_dense(DevBM& m, int32_t B, int draws, uint64_t seed, uint32_t seq,
@@ -1669,14 +1703,13 @@ void add_dense_build_mapped(DenseBuildSlots& s, const DevGraph& g, const int32_t
 }
 
 void add_dense_update(Slot& s, const DevGraph& g, const int32_t* part, int32_t lo, int32_t count,
-                      const int32_t* newlab, int32_t B, DevBM& m, const int32_t* ctl) {
+                      const int32_t* newlab, int32_t B, DevBM& m, const NodalAux& lists,
+                      const int32_t* ctl) {
   if (count <= 0) return;
   DenseArgs a = dense_args(g, part, B, m);
   a.ctl = ctl;
-  a.lo = lo;
-  a.count = count;
-  a.newlab = newlab;
-  slot_push(slot_bind(s, kmDenseUpdate), a, vg_dense_update(count));
+  set_update(a, lo, count, newlab, lists);
+  slot_push(slot_bind(s, kmDenseUpdate), a, vg_dense_update(a));
 }
 
 void add_block_terms(Slot& s, DevBM& m, int32_t B, const int32_t* ctl) {

@@ -372,13 +372,15 @@ void Engine::add_run_work(Run& r) {
           add_block_draw(s.bt_csr, J.m, r.B, r.o.seed, seq, ctl, nb);
         }
         const int ms = md.slot(dense);
+        const NodalAux lists =
+            nodal_lists(J, J.lists + r.list_off[b], &r.list_n[kListCounts * (size_t)b]);
         add_nodal(s.nodal[ms], s.heavy[ms], s.hub[dense ? 1 : 0], dense, md, J.g, J.part, J.m, r.B, r.o.seed, seq, lo,
                   r.BS, J.newlab, J.rec, nullptr,
-                  nodal_lists(J, J.lists + r.list_off[b], &r.list_n[kListCounts * (size_t)b]), ctl, nb);
+                  lists, ctl, nb);
         if (dense) {
           // the moved vertices' edges, applied to the dense form before the
           // labels change (it reads old and new labels)
-          add_dense_update(s.dupd, J.g, J.part, lo, r.BS, J.newlab, r.B, J.m, ctl);
+          add_dense_update(s.dupd, J.g, J.part, lo, r.BS, J.newlab, r.B, J.m, lists, ctl);
           const bool last = k == r.sweep_k - 1 && b == nb - 1;
           add_commit(s.commit, J.part, lo, r.BS, J.newlab, J.rec, slot_sum, slot_acc, &J.m,
                      r.B, J.cs, ctl, slot_mul, !last, r.o.seed, seq + 1, nb);

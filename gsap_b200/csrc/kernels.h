@@ -163,6 +163,8 @@ struct DenseBuildSlots {
   std::vector<Slot*> all();
 };
 
+struct NodalAux;
+
 // Record builders: each adds one job's launch record(s) to the slot(s), with
 // a virtual grid that depends on that job's sizes only.  `ctl` (optional)
 // is the job's sweep control (int32 pair in device memory: sweeps done in
@@ -182,7 +184,8 @@ void add_dense_build_mapped(DenseBuildSlots& s, const DevGraph& g, const int32_t
 void add_dense_build(DenseBuildSlots& s, const DevGraph& g, const int32_t* part, int32_t B,
                      DevBM& m);
 void add_dense_update(Slot& s, const DevGraph& g, const int32_t* part, int32_t lo, int32_t count,
-                      const int32_t* newlab, int32_t B, DevBM& m, const int32_t* ctl = nullptr);
+                      const int32_t* newlab, int32_t B, DevBM& m, const NodalAux& lists,
+                      const int32_t* ctl = nullptr);
 void add_block_terms(Slot& s, DevBM& m, int32_t B, const int32_t* ctl = nullptr);
 // The per-block draws of the nodal batch with RNG sequence seq (CSR form).
 void add_block_draw(Slot& s, DevBM& m, int32_t B, uint64_t seed, uint32_t seq,
@@ -201,7 +204,6 @@ void add_iota(Slot& s, int32_t* p, int32_t n);
 // CTA-per-vertex kernel's (heavy vertices) to `heavy`, the hubs' to `hub`.
 // Use separate slots per md.slot(dense): dense and CSR jobs, GSAP-mode and
 // general-mode jobs run different kernels.
-struct NodalAux;
 void add_nodal(Slot& warp, Slot& heavy, Slot& hub, bool dense, const ScoreMode& md, const DevGraph& g,
                const int32_t* part,
                const DevBM& m, int32_t B, uint64_t seed, uint32_t seq, int32_t lo, int32_t count,
@@ -331,11 +333,6 @@ void block_terms(DevBM& m, int32_t B, int draws, uint64_t seed, uint32_t seq, cu
 // Dense form (B*B counts and their transpose, degrees and their log2) of the
 // labels' blockmodel, built from scratch.
 void dense_build(const DevGraph& g, const int32_t* part, int32_t B, DevBM& m, cudaStream_t st);
-// Applies a batch's moves to the dense form: `part` still holds the old
-// labels, newlab[i] the new label of vertex lo+i.  Degrees are updated; their
-// log2 are refreshed by nodal_commit (dense mode).
-void dense_update(const DevGraph& g, const int32_t* part, int32_t lo, int32_t count,
-                  const int32_t* newlab, int32_t B, DevBM& m, cudaStream_t st);
 // block_terms for the dense form.
 void block_terms_dense(DevBM& m, int32_t B, int draws, uint64_t seed, uint32_t seq,
                        cudaStream_t st);

@@ -1248,7 +1248,7 @@ template <bool GIVEN, bool DENSE, bool GEN>
 struct NodalBody {
   using Args = NodalArgs;
   static constexpr int kThreads = kNodalWarps * 32;
-  static constexpr int kMinBlocks = GEN ? 5 : DENSE ? 8 : 6;
+  static constexpr int kMinBlocks = GEN ? 5 : 8;
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
     if (ctl_stopped(a.ctl)) return;

@@ -97,3 +97,19 @@ def test_hub_edges(sbp, orc, monkeypatch, dmax, B, weighted):
         _, db, xb, _ = orc.nodal_batch(g, p, B, 21, seq, 0, K)
         assert np.array_equal(xa, xb), "proposals differ"
         assert close(da, db).all()
+
+
+@pytest.mark.parametrize("weighted", [False, True], ids=["unit", "weighted"])
+@pytest.mark.parametrize("B", [2, 33, 300])
+@pytest.mark.parametrize("batches", [1, 7, N // 40])
+def test_dense_update_edges(sbp, weighted, B, batches):
+    # the dense form updated from the moves of vertices of every size, batches
+    # of 40 to 12,000 vertices, against the CSR form rebuilt after each batch
+    g = shaped_graph(sbp, weighted)
+    p = np.random.default_rng(B).integers(0, B, N).astype(np.int32)
+    p[-B:] = np.arange(B, dtype=np.int32)
+    sweeps = 1 if batches > 7 else 3
+    a, b = (sbp.nodal_sweeps(g, p, B, 3, 5, num_batches=batches, sweeps=sweeps, dense_max=d)
+            for d in (0, N))
+    assert (a[0] != p).any()
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
