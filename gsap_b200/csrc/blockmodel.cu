@@ -351,22 +351,27 @@ struct RbTileBody {
         const bool live = n > 0 && o >= 0 && o < win;
         const int steps = live ? (n + 7) >> 3 : 0;
         int u = 0;
-        uint32_t deg = 0u;
+        uint32_t deg = 0u;  // the count so far
         const int most = __reduce_max_sync(kFull, steps);
         for (int i = 0; i < most; ++i) {
           const int p = 8 * i + gl;
           const uint32_t c = live && p < n ? sw[o + p] : 0u;
           const unsigned m = __ballot_sync(kFull, c != 0u) >> (lane & 24) & 0xffu;
+          uint32_t incl = c;
+#pragma unroll
+          for (int x = 1; x < 8; x <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, incl, x, 8);
+            if (gl >= x) incl += y;
+          }
           if (c) {
             const int z = src[r] + u + __popc(m & ((1u << gl) - 1u));
             d.bcol[z] = (int32_t)skey[o + p];
             d.bcnt[z] = c;
-            deg += c;
+            d.bcum[z] = deg + incl;
           }
+          deg += __shfl_sync(kFull, incl, 7, 8);
           u += __popc(m);
         }
-#pragma unroll
-        for (int x = 4; x > 0; x >>= 1) deg += __shfl_xor_sync(kFull, deg, x);
         if (live && gl == 0) {
           row_done(a, d, b0 + r, src[r], u, deg);
           nnz += u;
@@ -700,12 +705,10 @@ __device__ __forceinline__ double row_total(double s, uint32_t d, double ld) {
 }
 
 // The draws of a nodal batch from the CSR rows (as dense_block_draw): eight
-// lanes a block find the first entry of out-row ++ in-row whose running
-// count exceeds the drawn number.  The block's out-degree tells the row; a
-// row of up to kTileMaxCap entries is summed along, a longer one has running
-// counts (the rebuild writes them) and is searched eight ways a step.  A
-// warp summing along every row took 91 us a batch of the 200k HH graph, up to
-// 700 where a block had 50k entries; this takes 24 us.
+// lanes a block search the first entry of out-row ++ in-row whose running
+// count exceeds the drawn number, eight ways a step; the block's out-degree
+// tells the row.  A warp summing along every row took 91 us a batch of the
+// 200k HH graph, up to 700 where a block had 50k entries; this takes 9.
 struct BlockDrawBody {
   using Args = BtArgs;
   static constexpr int kThreads = 256, kMinBlocks = 1;
@@ -724,46 +727,22 @@ struct BlockDrawBody {
       const bool in = t64 >= dout;
       const uint32_t t = (uint32_t)(in ? t64 - dout : t64);  // below the row's sum
       const int lo = (in ? a.iptr : a.optr)[b];
-      const int n = deg ? (in ? a.iend : a.oend)[b] - lo : 0;
-      const uint32_t* cnt = (in ? a.icnt : a.ocnt) + lo;
       const uint32_t* cum = (in ? a.icum : a.ocum) + lo;
-      // [first, first + len): where the entry is; base: the count before it
-      int first = 0, len = n;
-      const bool longrow = n > kTileMaxCap;
-      while (__any_sync(kFull, longrow && len > 8)) {
-        const bool go = longrow && len > 8;
+      // the entry is one of [first, first + len)
+      int first = 0, len = deg ? (in ? a.iend : a.oend)[b] - lo : 0;
+      while (__any_sync(kFull, len > 1)) {
+        const bool go = len > 1;
         const int step = (len + 7) >> 3;
         const int at = first + min((gl + 1) * step, len) - 1;
-        const unsigned m =
-            __ballot_sync(kFull, go && __ldg(cum + at) > t) >> hb & 0xffu;
+        const unsigned m = __ballot_sync(kFull, go && __ldg(cum + at) > t) >> hb & 0xffu;
         if (go) {
           const int j = __ffs(m) - 1;
           first += j * step;
           len = min(step, len - j * step);
         }
       }
-      int found = -1;
-      uint32_t run = 0u;
-      for (int i = 0; __any_sync(kFull, found < 0 && i < len); i += 8) {
-        const int k = first + i + gl;
-        const bool ok = i + gl < len;
-        uint32_t incl = 0u;
-        if (ok) incl = longrow ? __ldg(cum + k) : __ldg(cnt + k);
-        if (!longrow) {
-#pragma unroll
-          for (int o = 1; o < 8; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffu << hb, incl, o, 8);
-            if (gl >= o) incl += y;
-          }
-          incl += run;
-          run = __shfl_sync(0xffu << hb, incl, 7, 8);
-        }
-        __syncwarp();
-        const unsigned m = __ballot_sync(kFull, ok && incl > t) >> hb & 0xffu;
-        if (found < 0 && m) found = first + i + __ffs(m) - 1;
-      }
       if (gl == 0 && b0 < a.B) {
-        const int nb = found >= 0 ? (in ? a.icol : a.ocol)[lo + found] : 0;
+        const int nb = len > 0 ? (in ? a.icol : a.ocol)[lo + first] : 0;
         a.nbr_s[b] = accept_random(x.v[0], deg, (uint64_t)a.B) ? -1 : nb;
       }
     }
@@ -910,7 +889,7 @@ struct DenseCsrArgs {
   const int32_t *optr, *iptr;
   int32_t *oend, *iend;
   int32_t *ocol, *icol;
-  uint32_t *ocnt, *icnt;
+  uint32_t *ocnt, *icnt, *ocum, *icum;
   int32_t* nnz;
   int32_t B, fill;  // fill 0: count, 1: write the rows
 };
@@ -929,23 +908,38 @@ struct DenseCsrBody {
       const uint32_t* row = (in ? a.MTd : a.Md) + (size_t)b * B;
       int k = 0;
       int32_t* col = nullptr;
-      uint32_t* cnt = nullptr;
+      uint32_t *cnt = nullptr, *cum = nullptr;
       if (a.fill) {
         k = (in ? a.iptr : a.optr)[b];
         col = in ? a.icol : a.ocol;
         cnt = in ? a.icnt : a.ocnt;
+        cum = in ? a.icum : a.ocum;
       }
       int n = 0;
-      for (int c0 = 0; c0 < B; c0 += 32) {
-        const int c = c0 + lane;
-        const uint32_t m = c < B ? row[c] : 0u;
-        const unsigned nz = __ballot_sync(kFull, m != 0u);
-        if (a.fill && m) {
-          const int pos = k + n + __popc(nz & lt);
-          col[pos] = c;
-          cnt[pos] = m;
+      uint32_t run = 0u;
+      // four chunks of columns in flight at a time
+      for (int c0 = 0; c0 < B; c0 += 128) {
+        uint32_t m[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = c0 + 32 * u + lane;
+          m[u] = c < B ? row[c] : 0u;
         }
-        n += __popc(nz);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const unsigned nz = __ballot_sync(kFull, m[u] != 0u);
+          if (a.fill && nz) {
+            const uint32_t incl = warp_incl_scan_u(m[u], lane);
+            if (m[u]) {
+              const int pos = k + n + __popc(nz & lt);
+              col[pos] = c0 + 32 * u + lane;
+              cnt[pos] = m[u];
+              cum[pos] = run + incl;
+            }
+            run += __shfl_sync(kFull, incl, 31);
+          }
+          n += __popc(nz);
+        }
       }
       if (lane != 0) continue;
       if (!a.fill) {
@@ -1641,7 +1635,7 @@ std::vector<Slot*> RebuildSlots::all() {
 
 void add_csr_from_dense(RebuildSlots& s, int32_t B, DevBM& m, RebuildScratch& rs) {
   DenseCsrArgs a{m.Md, m.MTd, rs.d[0].cnt, rs.d[1].cnt, m.optr, m.iptr, m.oend, m.iend,
-                 m.ocol, m.icol, m.ocnt, m.icnt, m.nnz, B, 0};
+                 m.ocol, m.icol, m.ocnt, m.icnt, m.ocum, m.icum, m.nnz, B, 0};
   const int32_t vg = grid_for((long long)2 * B * 32, 256, 148 * 16);
   slot_push(slot_bind(s.dense_count, kmDenseCsr), a, vg);
   for (int dir = 0; dir < 2; ++dir)

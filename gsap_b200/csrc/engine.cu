@@ -323,7 +323,8 @@ void Engine::add_run_work(Run& r) {
     add_block_terms(m_bt, J.m, r.B);
     const MergeGrid grid = merge_grid(J, r.o);
     add_merge_props(m_props, J.m, r.B, J.np, r.o.seed, r.seq, J.props, grid);
-    add_merge_delta(m_delta, m_delta8, m_best, J.m, r.B, J.E, J.np, J.props, nullptr, J.best,
+    add_merge_delta(m_delta, m_delta8, m_best, J.m, r.B, J.E, J.np,
+                    !r.csr_fresh && r.dense_kept && r.dense(), J.props, nullptr, J.best,
                     J.best_dS, r.o.exact, grid);
     // carry_out_best_merges on the device, then the relabel: the host reads
     // back only the new block count

@@ -26,8 +26,7 @@ struct DevGraph {
 // block), weighted block degrees and their log2, and the per-block sums the
 // dS kernels start from.  Row b's entries are [ptr[b], end[b]); the rows
 // ascend but need not lie back to back.  Capacities: rows N+1, entries E.
-// ocum / icum: running counts along a row, written by the rebuild for rows
-// of more than 128 entries.  nnz: entries of the out CSR.
+// ocum / icum: running counts along a row.  nnz: entries of the out CSR.
 struct DevBM {
   int32_t *optr = nullptr, *oend = nullptr, *ocol = nullptr;
   int32_t *iptr = nullptr, *iend = nullptr, *icol = nullptr;
@@ -234,8 +233,10 @@ void add_merge_props(Slot& s, const DevBM& m, int32_t B, int32_t np, uint64_t se
 // blockmodel rows go to slot s8 (a warp per block, groups of 8 lanes per
 // proposal), the others to s32 (a warp per proposal, into grid.dS) and
 // sbest (each block's best).  Without grid.dS, dS is the scratch.
+// dense: the dense form holds this blockmodel too (cells are then read from
+// it instead of searched in the rows).
 void add_merge_delta(Slot& s32, Slot& s8, Slot& sbest, const DevBM& m, int32_t B, int32_t E,
-                     int32_t np,
+                     int32_t np, bool dense,
                      const int32_t* props, double* dS, int32_t* best, double* best_dS,
                      int32_t exact = 0, const MergeGrid& grid = MergeGrid());
 void add_relabel(Slot& s, int32_t* part, int32_t N, const int32_t* map);

@@ -5,11 +5,10 @@
 // whole rows per proposal thread (kernels.hpp:143-449, grid sized from nnz,
 // Q16) and reduces with find_best_warp (kernels.hpp:452-491).
 //
-// Here: one warp per block draws its proposals (Philox, exact integer picks
-// by a running prefix over the row in 32-entry chunks, one ballot per
-// proposal per chunk) and one warp per block computes their dS, walking only
-// the shorter of the
-// two rows being merged and looking the other up by binary search, with the
+// Here: one thread per proposal draws it (Philox, exact integer picks by
+// binary search of the rows' running counts) and a group of lanes or a warp
+// computes its dS, walking only the shorter of the two rows being merged and
+// looking the other up by binary search (or in the dense form), with the
 // unchanged remainder taken from the per-block sums; lanes 0..np-1 then hold
 // the proposals' dS and run the same 32-lane halving argmin as
 // find_best_warp, ties going to the lane further up.  FP64 throughout.
@@ -30,7 +29,8 @@ int32_t vg_merge_delta(int32_t B);
 struct MergeArgs {
   const double* xlx;
   const int32_t *optr, *oend, *ocol, *iptr, *iend, *icol;
-  const uint32_t *ocnt, *icnt, *d_out, *d_in;
+  const uint32_t *ocnt, *icnt, *ocum, *icum, *d_out, *d_in;
+  const uint32_t *Md, *MTd;  // the dense form, when it holds this blockmodel (else null)
   const int32_t* nnz;
   const double *ld_out, *ld_in, *dSout, *ambout, *ambin, *sinfull;
   int32_t B, np;
@@ -61,117 +61,73 @@ __device__ __forceinline__ long long merge_grid_end(const MergeArgs& a) {
   return T < n ? T : n;
 }
 
-// Count and column of entry k of out-row ++ in-row of block b (the scan
-// order of kernels.hpp:767-783).
-__device__ __forceinline__ uint32_t cnt_at(const MergeArgs& a, int b, int k, int no) {
-  return k < no ? __ldg(a.ocnt + a.optr[b] + k) : __ldg(a.icnt + a.iptr[b] + k - no);
-}
+// Column of entry k of out-row ++ in-row of block b (the scan order of
+// kernels.hpp:767-783).
 __device__ __forceinline__ int col_at(const MergeArgs& a, int b, int k) {
   int o0 = a.optr[b], no = a.oend[b] - o0;
   return k < no ? __ldg(a.ocol + o0 + k) : __ldg(a.icol + a.iptr[b] + k - no);
 }
 
-// Inclusive scan of 64-bit values over the warp's lanes.
-__device__ __forceinline__ unsigned long long warp_incl_scan_ull(unsigned long long x, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    unsigned long long y = __shfl_up_sync(kFull, x, o);
-    if (lane >= o) x += y;
+// First entry of out-row ++ in-row of block b whose running count exceeds t
+// (t below the block's degree): the same pick as a serial running sum, by
+// binary search of the row that the block's out-degree tells.
+__device__ __forceinline__ int pick_entry(const MergeArgs& a, int b, uint64_t t) {
+  const uint32_t dout = a.d_out[b];
+  const bool in = t >= dout;
+  const uint32_t x = (uint32_t)(in ? t - dout : t);
+  const int o0 = a.optr[b], no = a.oend[b] - o0;
+  const int i0 = a.iptr[b];
+  const uint32_t* cum = in ? a.icum + i0 : a.ocum + o0;
+  int lo = 0, hi = in ? a.iend[b] - i0 : no;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (__ldg(cum + mid) > x) hi = mid;
+    else lo = mid + 1;
   }
-  return x;
+  return in ? no + lo : lo;
 }
 
-// The whole warp walks out-row ++ in-row of block b (warp-uniform) in
-// chunks of 32 entries with a running prefix of the counts.  Each lane L
-// with want set looks for the first entry whose running count exceeds its
-// own threshold t; returns that entry's index in the lane that asked, -1
-// where none does.  The same picks as a serial running sum.
-__device__ int warp_pick(const MergeArgs& a, int b, uint64_t t, bool want, int lane) {
-  const int no = a.oend[b] - a.optr[b];
-  const int n = no + (a.iend[b] - a.iptr[b]);
-  int found = -1;
-  unsigned open = __ballot_sync(kFull, want);
-  unsigned long long base = 0;
-  for (int c0 = 0; c0 < n && open; c0 += 32) {
-    const int k = c0 + lane;
-    const unsigned long long incl =
-        warp_incl_scan_ull(k < n ? cnt_at(a, b, k, no) : 0u, lane) + base;
-    unsigned rest = open;
-    while (rest) {
-      const int L = __ffs(rest) - 1;
-      rest &= rest - 1;
-      const unsigned long long tL = __shfl_sync(kFull, (unsigned long long)t, L);
-      const unsigned m = __ballot_sync(kFull, k < n && incl > tL);
-      if (m) {
-        if (lane == L) found = c0 + __ffs(m) - 1;
-        open &= ~(1u << L);
-      }
-    }
-    base = __shfl_sync(kFull, incl, 31);
-  }
-  return found;
-}
-
-// choose_neighbors + propose_blocks (kernels.hpp:726-856): one warp per
-// block r draws its np proposals, lane k the k-th.  The first hop picks a
-// neighbour u of r by weight (all lanes in r's row at once); lanes that do
-// not propose a random block then pick in u's row, one walk per lane, and
-// take the first entry from there on whose column is not r (block 0 when
-// none is).
+// choose_neighbors + propose_blocks (kernels.hpp:726-856): a thread per
+// proposal.  The first hop picks a neighbour u of r by weight; a proposal that
+// is not of a random block then picks in u's row and takes the first entry
+// from there on whose column is not r (block 0 when none is).  A warp per
+// block that walked the rows along, its lanes' second hops one after the
+// other, took 111 us in the median over a 200k HH partition's merges (at most
+// 275); this takes 11 (at most 43).
 struct MergePropsBody {
   using Args = MergeArgs;
   static constexpr int kThreads = kMergeWarps * 32, kMinBlocks = 1;
   static constexpr size_t kSmem = 0;
-  static __device__ void run(const Args& a, int vb, int vg);
-};
-
-__device__ void MergePropsBody::run(const MergeArgs& a, int vb, int vg) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const long long T = merge_grid_end(a);
-  const uint32_t B = (uint32_t)a.B;
-  for (int r = vb * kMergeWarps + wid; r < a.B; r += vg * kMergeWarps) {
-    const long long t = (long long)r * a.np + lane;
-    const bool mine = lane < a.np && t < T;  // slots GSAP's grid leaves out keep theirs
-    if (!__any_sync(kFull, mine)) continue;
-    P4 x{};
-    if (mine) x = draw(a.seed, kRngMerge, a.seq, (uint32_t)t);
-    const int rnd = (int)(x.v[0] % B);
-    const uint64_t deg_r = (uint64_t)a.d_out[r] + a.d_in[r];
-    int s = rnd;
-    // first hop: a neighbour u of r in proportion to weight
-    const bool hop = mine && deg_r != 0;
-    const int k = warp_pick(a, r, hop ? scale_draw(x.v[1], deg_r) : 0, hop, lane);
-    int u = 0;
-    bool second = false;
-    uint64_t deg_u = 0;
-    if (hop) {
-      u = k >= 0 ? col_at(a, r, k) : 0;
-      deg_u = (uint64_t)a.d_out[u] + a.d_in[u];
-      second = !accept_random(x.v[2], deg_u, B);
-      if (second) s = 0;
-    }
-    // second hop: each lane that needs it walks its own u's row with the warp
-    unsigned need = __ballot_sync(kFull, second && deg_u > 0);
-    while (need) {
-      const int L = __ffs(need) - 1;
-      need &= need - 1;
-      const int uL = __shfl_sync(kFull, u, L);
-      const uint64_t tL = __shfl_sync(kFull, (unsigned long long)scale_draw(x.v[3], deg_u), L);
-      const int k2 = warp_pick(a, uL, tL, lane == L, lane);
-      if (lane == L && k2 >= 0) {
-        const int n = (a.oend[u] - a.optr[u]) + (a.iend[u] - a.iptr[u]);
-        for (int q = k2; q < n; ++q) {
-          const int c = col_at(a, u, q);
-          if (c != r) {
-            s = c;
-            break;
+  static __device__ void run(const Args& a, int vb, int vg) {
+    const long long T = merge_grid_end(a);  // slots GSAP's grid leaves out keep theirs
+    const uint32_t B = (uint32_t)a.B;
+    for (long long t = (long long)vb * kThreads + threadIdx.x; t < T;
+         t += (long long)vg * kThreads) {
+      const int r = (int)(t / a.np);
+      const P4 x = draw(a.seed, kRngMerge, a.seq, (uint32_t)t);
+      const uint64_t deg_r = (uint64_t)a.d_out[r] + a.d_in[r];
+      int s = (int)(x.v[0] % B);
+      if (deg_r != 0) {
+        const int u = col_at(a, r, pick_entry(a, r, scale_draw(x.v[1], deg_r)));
+        const uint64_t deg_u = (uint64_t)a.d_out[u] + a.d_in[u];
+        if (!accept_random(x.v[2], deg_u, B)) {
+          s = 0;
+          if (deg_u > 0) {
+            const int n = (a.oend[u] - a.optr[u]) + (a.iend[u] - a.iptr[u]);
+            for (int q = pick_entry(a, u, scale_draw(x.v[3], deg_u)); q < n; ++q) {
+              const int c = col_at(a, u, q);
+              if (c != r) {
+                s = c;
+                break;
+              }
+            }
           }
         }
       }
+      a.props[t] = s;
     }
-    if (mine) a.props[t] = s;
   }
-}
+};
 
 __device__ __forceinline__ double gterm(const double* tab, uint32_t x, double ld) {
   return x == 0u ? 0.0 : xlx(tab, x) - (double)x * ld;
@@ -188,22 +144,102 @@ __device__ __forceinline__ double group_sum(double x) {
   return x;
 }
 
+// Counts M[y][c] (out) or M[c][y] (in) of E cells, 0 where not wanted: cells of
+// the dense form when it holds the blockmodel, else searched in row y, all
+// searches advancing together.
+template <int E>
+__device__ __forceinline__ void cells(const MergeArgs& a, const int* y, const bool* in,
+                                      const int* c, const bool* want, uint32_t* m) {
+  if (a.Md) {
+#pragma unroll
+    for (int j = 0; j < E; ++j)
+      m[j] = want[j] ? __ldg((in[j] ? a.MTd : a.Md) + (size_t)y[j] * a.B + c[j]) : 0u;
+    return;
+  }
+  int lo[E], hi[E], end[E];
+#pragma unroll
+  for (int j = 0; j < E; ++j) {
+    lo[j] = want[j] ? __ldg((in[j] ? a.iptr : a.optr) + y[j]) : 0;
+    hi[j] = end[j] = want[j] ? __ldg((in[j] ? a.iend : a.oend) + y[j]) : 0;
+  }
+  bool go = true;
+  while (go) {
+    go = false;
+    int x[E];
+#pragma unroll
+    for (int j = 0; j < E; ++j)
+      x[j] = lo[j] < hi[j] ? __ldg((in[j] ? a.icol : a.ocol) + ((lo[j] + hi[j]) >> 1)) : 0;
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+      if (lo[j] >= hi[j]) continue;
+      const int mid = (lo[j] + hi[j]) >> 1;
+      if (x[j] < c[j]) lo[j] = mid + 1;
+      else hi[j] = mid;
+      go = go || lo[j] < hi[j];
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < E; ++j)
+    m[j] = lo[j] < end[j] && __ldg((in[j] ? a.icol : a.ocol) + lo[j]) == c[j]
+               ? __ldg((in[j] ? a.icnt : a.ocnt) + lo[j])
+               : 0u;
+}
+
+// The walks of a merge: the shorter out-row of r and s, and the shorter
+// in-row (x walked, y looked up).
+struct MergeRows {
+  int x[2], y[2], x0[2], x1[2];  // out, in
+  __device__ __forceinline__ MergeRows(const MergeArgs& a, int r, int s) {
+    const int32_t *ptr[2] = {a.optr, a.iptr}, *end[2] = {a.oend, a.iend};
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+      const int r0 = ptr[d][r], r1 = end[d][r], s0 = ptr[d][s], s1 = end[d][s];
+      const bool swap = s1 - s0 < r1 - r0;
+      x[d] = swap ? s : r;
+      y[d] = swap ? r : s;
+      x0[d] = swap ? s0 : r0;
+      x1[d] = swap ? s1 : r1;
+    }
+  }
+};
+
+// M[r][r], M[r][s], M[s][r], M[s][s] and M[s2][s], searched by five lanes of
+// the group at once.
+template <int G>
+__device__ __forceinline__ void merge_corners(const MergeArgs& a, int r, int s, int s2, int gl,
+                                              uint32_t* m) {
+  const int row = gl < 2 ? r : gl < 4 ? s : s2;
+  const int col = gl == 0 || gl == 2 ? r : s;
+  const bool in = false, want = gl < 5;
+  uint32_t x;
+  cells<1>(a, &row, &in, &col, &want, &x);
+#pragma unroll
+  for (int j = 0; j < 5; ++j) m[j] = __shfl_sync(kFull, x, j, G);
+}
+
 // Merge dS of block r with s (calculate_dS_overall, kernels.hpp:417-449) by
 // a group of G lanes (gl = lane in the group), s2 = the k-th proposal of
 // block s (its in-term leaves out s2, Q1).  With given_in_s, block s's
 // in-term is in_s_given (a slot GSAP's grid left out); in_r_out receives
 // block r's in-term.  An inactive group walks nothing but still takes part
 // in the group sums (every lane of the warp must).
+//
+// What bounds it is the chain of binary searches (a row of a giant block, the
+// commonest partner of the first merges, is 16 steps long), so the corner
+// cells are searched by different lanes, the two rows are walked together, and
+// the kernels hold six CTAs an SM (40 registers): 16.1 ms of merge kernels in
+// a 200k HH partition one search after the other at two or three CTAs, 7.3
+// this way (12.4 without the residency, 14 with two entries of each row in
+// flight at 64 registers, as much again in spills).
 template <int G>
 __device__ double merge_one(const MergeArgs& a, int r, int s, int s2, int gl, bool active,
                             bool given_in_s, double in_s_given, double* in_r_out) {
   // merged out-rows (calculate_dS_new_out, kernels.hpp:233-320)
   double acc_o = 0.0, acc_i = 0.0;
   const double ldo_r = a.ld_out[r], ldo_s = a.ld_out[s], ldi_r = a.ld_in[r], ldi_s = a.ld_in[s];
-  const uint32_t Mrr = row_lookup(a.ocol, a.ocnt, a.optr[r], a.oend[r], r);
-  const uint32_t Mrs = row_lookup(a.ocol, a.ocnt, a.optr[r], a.oend[r], s);
-  const uint32_t Msr = row_lookup(a.ocol, a.ocnt, a.optr[s], a.oend[s], r);
-  const uint32_t Mss = row_lookup(a.ocol, a.ocnt, a.optr[s], a.oend[s], s);
+  uint32_t corner[5];
+  merge_corners<G>(a, r, s, s2, gl, corner);
+  const uint32_t Mrr = corner[0], Mrs = corner[1], Msr = corner[2], Mss = corner[3];
   if (!active) {
   } else if (r == s) {
     for (int i = a.optr[r] + gl; i < a.oend[r]; i += G)
@@ -213,28 +249,34 @@ __device__ double merge_one(const MergeArgs& a, int r, int s, int s2, int gl, bo
       if (c != r) acc_i += gterm(a.xlx, 2u * a.icnt[i], a.ld_out[c]);
     }
   } else {
-    int x = r, y = s;
-    if (a.oend[s] - a.optr[s] < a.oend[r] - a.optr[r]) { x = s; y = r; }
-    int y0 = a.optr[y], y1 = a.oend[y];
-    for (int i = a.optr[x] + gl; i < a.oend[x]; i += G) {
-      int c = a.ocol[i];
-      double ld = a.ld_in[c];
-      uint32_t my = row_lookup(a.ocol, a.ocnt, y0, y1, c);
-      acc_o += gterm(a.xlx, a.ocnt[i] + my, ld) - gterm(a.xlx, my, ld);
-    }
-    if (gl == 0) acc_o += a.ambout[y];
-    x = r; y = s;
-    if (a.iend[s] - a.iptr[s] < a.iend[r] - a.iptr[r]) { x = s; y = r; }
-    y0 = a.iptr[y]; y1 = a.iend[y];
-    for (int i = a.iptr[x] + gl; i < a.iend[x]; i += G) {
-      int c = a.icol[i];
-      if (c == r || c == s) continue;
-      double ld = a.ld_out[c];
-      uint32_t my = row_lookup(a.icol, a.icnt, y0, y1, c);
-      acc_i += gterm(a.xlx, a.icnt[i] + my, ld) - gterm(a.xlx, my, ld);
+    const MergeRows w(a, r, s);
+    for (int o = w.x0[0] + gl, n = w.x0[1] + gl; o < w.x1[0] || n < w.x1[1]; o += G, n += G) {
+      const int i[2] = {o, n};
+      const bool in[2] = {false, true};
+      int c[2];
+      bool want[2];
+      uint32_t cnt[2], my[2];
+      double ld[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        c[j] = 0;
+        cnt[j] = 0u;
+        want[j] = i[j] < w.x1[j];
+        if (want[j]) {
+          c[j] = __ldg((in[j] ? a.icol : a.ocol) + i[j]);
+          cnt[j] = __ldg((in[j] ? a.icnt : a.ocnt) + i[j]);
+        }
+        if (in[j] && (c[j] == r || c[j] == s)) want[j] = false;
+        ld[j] = want[j] ? __ldg((in[j] ? a.ld_out : a.ld_in) + c[j]) : 0.0;
+      }
+      cells<2>(a, w.y, in, c, want, my);
+      if (want[0]) acc_o += gterm(a.xlx, cnt[0] + my[0], ld[0]) - gterm(a.xlx, my[0], ld[0]);
+      if (want[1]) acc_i += gterm(a.xlx, cnt[1] + my[1], ld[1]) - gterm(a.xlx, my[1], ld[1]);
     }
     if (gl == 0) {
+      acc_o += a.ambout[w.y[0]];
       // in-row y's own terms at columns r and s stay out
+      const int y = w.y[1];
       uint32_t yr = y == r ? Mrr : Mrs;  // M[r][y]
       uint32_t ys = y == r ? Msr : Mss;  // M[s][y]
       acc_i += a.ambin[y] - gterm(a.xlx, yr, ldo_r) - gterm(a.xlx, ys, ldo_s);
@@ -258,7 +300,7 @@ __device__ double merge_one(const MergeArgs& a, int r, int s, int s2, int gl, bo
   if (given_in_s) {
     in_s = in_s_given;
   } else {
-    uint32_t Ms2s = s2 == s ? 0u : row_lookup(a.ocol, a.ocnt, a.optr[s2], a.oend[s2], s);
+    const uint32_t Ms2s = s2 == s ? 0u : corner[4];
     in_s = a.sinfull[s] - fterm(a.xlx, Mss, ldo_s, ldi_s) - fterm(a.xlx, Ms2s, a.ld_out[s2], ldi_s);
   }
   *in_r_out = in_r;
@@ -318,7 +360,7 @@ __device__ double merge_one_exact(const MergeArgs& a, int r, int s, int gl, bool
 template <int G>
 struct MergeDeltaBody {
   using Args = MergeArgs;
-  static constexpr int kThreads = kMergeWarps * 32, kMinBlocks = 1;
+  static constexpr int kThreads = kMergeWarps * 32, kMinBlocks = 6;
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
   constexpr int NG = 32 / G;  // groups per warp
@@ -383,7 +425,7 @@ struct MergeDeltaBody {
 // MergeBestBody reduces each block's proposals.
 struct MergePropDeltaBody {
   using Args = MergeArgs;
-  static constexpr int kThreads = kMergeWarps * 32, kMinBlocks = 1;
+  static constexpr int kThreads = kMergeWarps * 32, kMinBlocks = 6;
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -453,6 +495,9 @@ struct RelabelBody {
 };
 
 
+int32_t vg_merge_props(int32_t B, int32_t np) {
+  return ceil_div((long long)B * np, MergePropsBody::kThreads);
+}
 int32_t vg_merge_delta(int32_t B) { return std::min(ceil_div(B, kMergeWarps), 148 * 32); }
 
 const MultiKernel kmMergeProps = multi_kernel_desc<MergePropsBody>("merge_props");
@@ -474,6 +519,7 @@ MergeArgs make_args(const DevBM& m, int32_t B, int32_t np, const MergeGrid& grid
   a.optr = m.optr; a.oend = m.oend; a.ocol = m.ocol;
   a.iptr = m.iptr; a.iend = m.iend; a.icol = m.icol;
   a.nnz = m.nnz;
+  a.ocum = m.ocum; a.icum = m.icum;
   a.ocnt = m.ocnt; a.icnt = m.icnt; a.d_out = m.d_out; a.d_in = m.d_in;
   a.ld_out = m.ld_out; a.ld_in = m.ld_in; a.dSout = m.dSout; a.ambout = m.ambout;
   a.ambin = m.ambin; a.sinfull = m.sinfull;
@@ -529,14 +575,18 @@ void add_merge_props(Slot& s, const DevBM& m, int32_t B, int32_t np, uint64_t se
   a.seed = seed;
   a.seq = seq;
   a.props = props;
-  slot_push(slot_bind(s, kmMergeProps), a, B > 0 && np > 0 ? vg_merge_delta(B) : 0);
+  slot_push(slot_bind(s, kmMergeProps), a, B > 0 && np > 0 ? vg_merge_props(B, np) : 0);
 }
 
 void add_merge_delta(Slot& s32, Slot& s8, Slot& sbest, const DevBM& m, int32_t B, int32_t E,
-                     int32_t np,
+                     int32_t np, bool dense,
                      const int32_t* props, double* dS, int32_t* best, double* best_dS,
                      int32_t exact, const MergeGrid& grid) {
   MergeArgs a = make_args(m, B, np, grid);
+  if (dense) {
+    a.Md = m.Md;
+    a.MTd = m.MTd;
+  }
   a.exact = exact;
   a.props_in = props;
   a.dS = dS;
