@@ -194,6 +194,9 @@ Engine::~Engine() {
   if (join2) cudaEventDestroy(join2);
   if (side) cudaStreamDestroy(side);
   if (side2) cudaStreamDestroy(side2);
+  if (side3) cudaStreamDestroy(side3);
+  if (fork3) cudaEventDestroy(fork3);
+  if (join3) cudaEventDestroy(join3);
   cudaStreamDestroy(st);
 }
 
@@ -204,6 +207,9 @@ sbp_status Engine::init(int dev) {
   SBP_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
   SBP_CUDA(cudaStreamCreateWithFlags(&side2, cudaStreamNonBlocking));
   SBP_CUDA(cudaEventCreateWithFlags(&join2, cudaEventDisableTiming));
+  SBP_CUDA(cudaStreamCreateWithFlags(&side3, cudaStreamNonBlocking));
+  SBP_CUDA(cudaEventCreateWithFlags(&fork3, cudaEventDisableTiming));
+  SBP_CUDA(cudaEventCreateWithFlags(&join3, cudaEventDisableTiming));
   SBP_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
   SBP_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
   return SBP_OK;
@@ -308,7 +314,7 @@ void Engine::add_run_work(Run& r) {
                                    : (size_t)r.o.max_nodal_itr;
     add_zero(s_zero, J.dsum, 2 * n);
     add_zero(s_zero, J.acc, 2 * n);
-    add_zero(s_zero, J.ctl, 2);
+    add_zero(s_zero, J.ctl, 4);
   }
   const bool dense = r.dense();
   if (r.stage == Run::kMerge) {
@@ -351,7 +357,7 @@ void Engine::add_run_work(Run& r) {
     }
     const int nb = r.o.num_batches;
     const RebuildTune tune = tune_for(J, r.B);
-    const int32_t* ctl = J.ctl;
+    int32_t* const ctl = J.ctl;
     const bool isf = std::isfinite(r.large.S) && std::isfinite(r.med.S) && std::isfinite(r.small.S);
     const double thr = isf ? (double)r.o.threshold2 : (double)r.o.threshold1;
     const double mS = model_S(r.B, J.N, J.E, r.o.exact);
@@ -364,30 +370,33 @@ void Engine::add_run_work(Run& r) {
         long long* slot_acc = r.sweeps_only ? J.acc + b : J.acc;
         const int32_t slot_mul = r.sweeps_only ? nb : 1;
         const int32_t lo = b * r.BS;
+        // a sweep's first nodal kernels run beside the end of the one before
+        const int32_t* const nctl = k > 0 && b == 0 ? ctl + 2 : ctl;
+        const bool sweep_last = b == nb - 1;
         // dense form: the tick's first batch draws here, every later one in
         // the commit of the batch before it (its seq is always one more)
         if (dense) {
           if (k == 0 && b == 0)
             add_block_terms_dense(s.bt_dense, J.m, r.B, 1, r.o.seed, seq, ctl, nb);
         } else {
-          add_block_draw(s.bt_csr, J.m, r.B, r.o.seed, seq, ctl, nb);
+          add_block_draw(s.bt_csr, J.m, r.B, r.o.seed, seq, nctl, nb);
         }
         const int ms = md.slot(dense);
         const NodalAux lists =
             nodal_lists(J, J.lists + r.list_off[b], &r.list_n[kListCounts * (size_t)b]);
         add_nodal(s.nodal[ms], s.heavy[ms], s.hub[dense ? 1 : 0], dense, md, J.g, J.part, J.m, r.B, r.o.seed, seq, lo,
                   r.BS, J.newlab, J.rec, nullptr,
-                  lists, ctl, nb);
+                  lists, nctl, nb);
         if (dense) {
           // the moved vertices' edges, applied to the dense form before the
           // labels change (it reads old and new labels)
           add_dense_update(s.dupd, J.g, J.part, lo, r.BS, J.newlab, r.B, J.m, lists, ctl);
           const bool last = k == r.sweep_k - 1 && b == nb - 1;
           add_commit(s.commit, J.part, lo, r.BS, J.newlab, J.rec, slot_sum, slot_acc, &J.m,
-                     r.B, J.cs, ctl, slot_mul, !last, r.o.seed, seq + 1, nb);
+                     r.B, J.cs, ctl, slot_mul, sweep_last, !last, r.o.seed, seq + 1, nb);
         } else {
           add_commit(s.commit, J.part, lo, r.BS, J.newlab, J.rec, slot_sum, slot_acc, nullptr,
-                     0, J.cs, ctl, slot_mul);
+                     0, J.cs, ctl, slot_mul, sweep_last);
           add_rebuild(s.rebuild, J.g, J.part, r.B, J.m, J.rs, ctl, tune);
         }
       }
@@ -588,9 +597,9 @@ sbp_status Engine::tick() {
   if (up) SBP_CUDA(cudaMemcpyAsync(up_dev, up_host, up, cudaMemcpyHostToDevice, st));
   if (desc) SBP_CUDA(cudaMemcpyAsync(desc_dev, desc_host, desc, cudaMemcpyHostToDevice, st));
   size_t i = 0;
-  auto emit_until = [&](Slot* last) -> sbp_status {
+  auto emit_until = [&](Slot* last, cudaStream_t on = nullptr) -> sbp_status {
     for (; i < order.size(); ++i) {
-      sbp_status q = launch_slot(*order[i], off[i], st);
+      sbp_status q = launch_slot(*order[i], off[i], on ? on : st);
       if (q != SBP_OK) return q;
       if (order[i] == last) {
         ++i;
@@ -651,6 +660,7 @@ sbp_status Engine::tick() {
         if (q != SBP_OK) return q;
         if (heavy) SBP_CUDA(cudaStreamWaitEvent(st, join, 0));
         if (hub) SBP_CUDA(cudaStreamWaitEvent(st, join2, 0));
+        if (k > 0 && b == 0) SBP_CUDA(cudaStreamWaitEvent(st, join3, 0));
         if (timing) SBP_CUDA(record(be[2]));
         q = emit_until(&w.commit);
         if (q != SBP_OK) return q;
@@ -659,8 +669,15 @@ sbp_status Engine::tick() {
         if (q != SBP_OK) return q;
         if (timing) SBP_CUDA(record(be[4]));
       }
-      sbp_status q = emit_until(&ends[k].ctl);
+      // the sweep's end, beside the next sweep's first nodal kernels
+      const bool beside = k + 1 < k_max;
+      if (beside) {
+        SBP_CUDA(cudaEventRecord(fork3, st));
+        SBP_CUDA(cudaStreamWaitEvent(side3, fork3, 0));
+      }
+      sbp_status q = emit_until(&ends[k].ctl, beside ? side3 : st);
       if (q != SBP_OK) return q;
+      if (beside) SBP_CUDA(cudaEventRecord(join3, side3));
     }
     return SBP_OK;
   };

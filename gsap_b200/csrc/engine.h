@@ -110,8 +110,9 @@ struct SweepEndSlots {
 class Engine {
  public:
   int device = 0;
-  cudaStream_t st = nullptr, side = nullptr, side2 = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr;
+  // side, side2: heavy vertices and hubs; side3: a sweep's end
+  cudaStream_t st = nullptr, side = nullptr, side2 = nullptr, side3 = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr, fork3 = nullptr, join3 = nullptr;
   std::vector<Run*> runs;
   long long ticks = 0;
   cudaEvent_t ev_first = nullptr;  // recorded at the first tick

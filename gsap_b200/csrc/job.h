@@ -58,7 +58,9 @@ struct Job {
   int32_t* ma_out = nullptr;    // new block count, target-out-of-range flag
   int32_t* lists = nullptr;     // batch indices by nodal kernel path (classify_batch)
   int32_t* err = nullptr;       // nodal error counter (hash-table overflow)
-  int32_t* ctl = nullptr;       // sweep control: sweeps done in the outer step, stop flag
+  // sweep control: sweeps done in the outer step, stop flag, and the pair for
+  // kernels beside a sweep's end (add_commit)
+  int32_t* ctl = nullptr;
   CommitScratch cs;
   int32_t dense_cap = 0;        // largest B the dense arrays can hold
   int32_t dense_eff = 0;        // largest B kept in dense form in this run

@@ -208,13 +208,20 @@ void add_nodal(Slot& warp, Slot& heavy, Slot& hub, bool dense, const ScoreMode& 
                const DevBM& m, int32_t B, uint64_t seed, uint32_t seq, int32_t lo, int32_t count,
                int32_t* newlab, double* rec, int32_t* props, const NodalAux& lists,
                const int32_t* ctl = nullptr, uint32_t seq_mul = 0);
+// mark: the commit of a sweep's last batch also writes ctl[2] = ctl[0] + 1 and
+// ctl[3] = ctl[1].  The next sweep's first nodal kernels run beside the
+// sweep's end (MDL terms, stop test), which writes ctl[0] and ctl[1]; with
+// ctl + 2 as their sweep control they read the sweep they belong to and the
+// stop flag as it was before, the same in every thread.  Should the end stop
+// the sweeps, what they did is not applied.
 // With draw_next (dense mode), the commit's extra CTAs also make the next
 // batch's per-block draws (the block-terms kernel's draws == 1 work) with RNG
 // sequence draw_seq + ctl[0] * draw_seq_mul, from M after the batch's moves.
 void add_commit(Slot& s, int32_t* part, int32_t lo, int32_t count, const int32_t* newlab,
                 const double* rec, double* slot_sum, long long* slot_acc, const DevBM* dense_m,
-                int32_t B, const CommitScratch& cs, const int32_t* ctl = nullptr,
-                int32_t slot_mul = 0, bool draw_next = false, uint64_t seed = 0,
+                int32_t B, const CommitScratch& cs, int32_t* ctl = nullptr,
+                int32_t slot_mul = 0, bool mark = false, bool draw_next = false,
+                uint64_t seed = 0,
                 uint32_t draw_seq = 0, uint32_t draw_seq_mul = 0);
 // GSAP's merge grid (Q16, partition.hpp:335-336): when `on`, only the
 // proposal slots below the nnz of the out CSR, rounded up to 256, are drawn

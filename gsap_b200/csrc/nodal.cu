@@ -1754,6 +1754,7 @@ struct CommitArgs {
   uint32_t draw_seq, draw_seq_mul;
   int32_t lo, count, B, slot_mul;
   int32_t ncommit, pad;
+  int32_t* mark;  // the sweep's last batch: the job's sweep control, handed on (add_commit)
 };
 
 struct CommitBody {
@@ -1761,8 +1762,12 @@ struct CommitBody {
   static constexpr int kThreads = kCommitThreads, kMinBlocks = 1;
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
-    if (ctl_stopped(a.ctl)) return;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (a.mark && vb == 0 && tid == 0) {
+      a.mark[2] = a.mark[0] + 1;
+      a.mark[3] = a.mark[1];
+    }
+    if (ctl_stopped(a.ctl)) return;
     if (vb >= a.ncommit) {
       const uint32_t seq = a.draw_seq + ctl_itr(a.ctl) * a.draw_seq_mul;
       const int nw = ((vg - a.ncommit) * kCommitThreads) >> 5;
@@ -2028,11 +2033,12 @@ void add_nodal(Slot& warp, Slot& heavy, Slot& hub, bool dense, const ScoreMode& 
 
 void add_commit(Slot& s, int32_t* part, int32_t lo, int32_t count, const int32_t* newlab,
                 const double* rec, double* slot_sum, long long* slot_acc, const DevBM* dense_m,
-                int32_t B, const CommitScratch& cs, const int32_t* ctl, int32_t slot_mul,
+                int32_t B, const CommitScratch& cs, int32_t* ctl, int32_t slot_mul, bool mark,
                 bool draw_next, uint64_t seed, uint32_t draw_seq, uint32_t draw_seq_mul) {
   CommitArgs a = commit_args(part, lo, count, newlab, rec, slot_sum, slot_acc, dense_m, B, cs);
   a.ctl = ctl;
   a.slot_mul = slot_mul;
+  if (mark) a.mark = ctl;
   int32_t vg = a.ncommit;
   if (draw_next && dense_m) {
     a.Md = dense_m->Md;
