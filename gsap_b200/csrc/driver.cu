@@ -701,11 +701,14 @@ int32_t env_dense_max() {
   return e ? std::atoi(e) : 4096;
 }
 
-// The entries are checked on a helper thread while the host thread creates
-// the arena and uploads (the upload only needs valid row pointers); no
-// kernel reads an entry before the check has passed.
+// The entries are checked on a helper thread while the host thread checks the
+// labels (part, when given, in [0, B)), creates the arena and uploads (the
+// upload only needs valid row pointers); no kernel reads an entry before the
+// check has passed.  A bad graph is reported before bad labels, and both
+// before a failed upload.
 static sbp_status job_for(Job& J, const sbp_graph_csr* g, int device, int32_t np, int32_t max_itr,
-                          int32_t dense_max) {
+                          int32_t dense_max, const int32_t* part = nullptr, int32_t B = 0,
+                          bool labels = false) {
   sbp_status s = validate_rows(g);
   if (s != SBP_OK) return s;
   std::future<const char*> entries;
@@ -715,10 +718,13 @@ static sbp_status job_for(Job& J, const sbp_graph_csr* g, int device, int32_t np
     const char* bad = graph_entry_error(g);  // no thread to spare: check first
     if (bad) return fail(SBP_ERR_INVALID, bad);
   }
-  s = job_create(J, resolve_device(device), g->N, g->E, np, max_itr, dense_max);
+  if (labels) s = validate_part(part, g->N, B);
+  if (s == SBP_OK) s = job_create(J, resolve_device(device), g->N, g->E, np, max_itr, dense_max);
   if (s == SBP_OK) s = job_upload(J, g);
   const char* bad = entries.valid() ? entries.get() : nullptr;
   if (bad) return fail(SBP_ERR_INVALID, bad);
+  if (s == SBP_OK && labels)
+    SBP_CUDA(cudaMemcpyAsync(J.part, part, 4 * (size_t)J.N, cudaMemcpyHostToDevice, J.st));
   return s;
 }
 
@@ -736,15 +742,8 @@ static RebuildTune env_rebuild_shape() {
 
 static sbp_status prepare(Job& J, const sbp_graph_csr* g, const int32_t* part, int32_t B,
                           int32_t np, int32_t max_itr) {
-  sbp_status s = validate_graph(g);
+  const sbp_status s = job_for(J, g, -1, np, max_itr, env_dense_max(), part, B, true);
   if (s != SBP_OK) return s;
-  s = validate_part(part, g->N, B);
-  if (s != SBP_OK) return s;
-  s = job_create(J, resolve_device(-1), g->N, g->E, np, max_itr, env_dense_max());
-  if (s != SBP_OK) return s;
-  s = job_upload(J, g);
-  if (s != SBP_OK) return s;
-  SBP_CUDA(cudaMemcpyAsync(J.part, part, 4 * (size_t)J.N, cudaMemcpyHostToDevice, J.st));
   rebuild_blockmodel(J.g, J.part, B, J.m, J.rs, J.st, env_rebuild_shape());
   if (is_dense(J, B)) dense_build(J.g, J.part, B, J.m, J.st);
   return SBP_OK;
@@ -1232,17 +1231,10 @@ sbp_status sbp_nodal_sweeps(const sbp_graph_csr* g, int32_t* part, int32_t B, ui
                             uint32_t seq0, int32_t num_batches, int32_t sweeps, int32_t dense_max,
                             double* sums) {
   if (!g || num_batches < 1 || sweeps < 1 || !sums) return fail(SBP_ERR_INVALID, "bad arguments");
-  sbp_status s = validate_graph(g);
-  if (s != SBP_OK) return s;
-  s = validate_part(part, g->N, B);
-  if (s != SBP_OK) return s;
   const int32_t nb = num_batches * sweeps;
   Job J;
-  s = job_create(J, resolve_device(-1), g->N, g->E, 1, nb, dense_max);
+  sbp_status s = job_for(J, g, -1, 1, nb, dense_max, part, B, true);
   if (s != SBP_OK) return s;
-  s = job_upload(J, g);
-  if (s != SBP_OK) return s;
-  SBP_CUDA(cudaMemcpyAsync(J.part, part, 4 * (size_t)J.N, cudaMemcpyHostToDevice, J.st));
   SBP_CUDA(cudaStreamSynchronize(J.st));
   s = run_sweeps(J, B, seed, seq0, num_batches, sweeps, sums);
   if (s != SBP_OK) return s;

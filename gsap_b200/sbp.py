@@ -467,14 +467,13 @@ class DeviceGraph(ResidentGraph):
     def download(self) -> Graph:
         """A host copy of the CSR pair."""
         N, E = self.N, self.E
-        arrs = dict(out_ptr=np.zeros(N + 1, np.int32), out_idx=np.zeros(max(E, 1), np.int32),
-                    out_w=np.zeros(max(E, 1), np.uint32), in_ptr=np.zeros(N + 1, np.int32),
-                    in_idx=np.zeros(max(E, 1), np.int32), in_w=np.zeros(max(E, 1), np.uint32),
-                    deg_out=np.zeros(N, np.uint32), deg_in=np.zeros(N, np.uint32))
+        # every array is written whole
+        arrs = dict(out_ptr=np.empty(N + 1, np.int32), out_idx=np.empty(E, np.int32),
+                    out_w=np.empty(E, np.uint32), in_ptr=np.empty(N + 1, np.int32),
+                    in_idx=np.empty(E, np.int32), in_w=np.empty(E, np.uint32),
+                    deg_out=np.empty(N, np.uint32), deg_in=np.empty(N, np.uint32))
         _check(_lib.sbp_graph_download(self.h, *[_p(arrs[k]) for k in (
             "out_ptr", "out_idx", "out_w", "in_ptr", "in_idx", "in_w", "deg_out", "deg_in")]))
-        for k in ("out_idx", "out_w", "in_idx", "in_w"):
-            arrs[k] = arrs[k][:E].copy()
         return Graph(N=N, E=E, true_partitions=self.true_partitions, **arrs)
 
 
