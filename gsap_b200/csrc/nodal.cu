@@ -880,7 +880,7 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
 // A vertex of more than kGroupEntries entries (at most kWarpList a
 // direction) on the CTA, an entry (of up to 256) a thread and slot: on one
 // warp such a vertex, the longest chain of a batch, set the launch time of
-// graphs whose batches fit the GPU at once (20k HH: 34 us a launch, 19 with
+// graphs whose batches fit the GPU at once (20k HH: 34 us a launch, 14 with
 // this path and group_vertex).  The terms are computed by entry and
 // subtracted by warp 0 in the order the warp's lanes would: by entry index up
 // to kWarpList entries, else by rank in the direction's (block, weight)
@@ -891,8 +891,20 @@ struct LargeBuf {
   uint32_t key[2 * T], w[2 * T];
   double t1[2 * T], t2[2 * T];
   double f[GEN ? 2 * T : 1], b[GEN ? 2 * T : 1];  // proposal weights
+  uint32_t ord[2 * T];  // (direction, block, entry), in one word
   uint32_t cnt[7];  // koR, koS, niR, niS, out-entries in r, in s, self loops
 };
+constexpr int kOrdBlocks = 1 << 22;  // blocks whose entries' order fits a word
+
+// First index in the ascending key[lo, hi) whose key exceeds x.
+__device__ __forceinline__ int upper_bound(const uint32_t* key, int lo, int hi, uint32_t x) {
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (key[mid] > x) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo;
+}
 
 template <bool GIVEN, bool DENSE, bool GEN, int T>
 __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
@@ -907,7 +919,7 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
   const int32_t i0 = a.iptr[v], ni = a.iptr[v + 1] - i0;
   const int n = no + ni;
   int32_t c[2];
-  uint32_t w[2], key[2];
+  uint32_t w[2], key[2], ord[2];
   bool in[2], ok[2];
   uint32_t selfp = 0u;
 #pragma unroll
@@ -925,8 +937,10 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
       if (GEN && !in[j] && u == v) selfp += w[j];
     }
     key[j] = ok[j] ? (uint32_t)c[j] | (in[j] ? 0x80000000u : 0u) : 0xffffffffu;
+    ord[j] = ok[j] ? (in[j] ? 1u << 30 : 0u) | (uint32_t)c[j] << 8 | (uint32_t)k : 0xffffffffu;
     sm.key[k] = key[j];
     sm.w[k] = w[j];
+    sm.ord[k] = ord[j];
   }
   const int r = a.part[v];
   if (tid < 7) sm.cnt[tid] = 0u;
@@ -1016,6 +1030,41 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
     lead[1] = false;
     pos[0] = tid;
     pos[1] = tid + T;
+  } else if (unit && a.B <= kOrdBlocks) {
+    // equal weights: the order is (direction, block, entry), a word per entry,
+    // and a block's total the length of its run in that order (the loop over
+    // pairs with weights, below, set the launch time: 20k HH partitions 43.4 ms
+    // with it, 37.8 this way)
+    int rank[2] = {0, 0};
+#pragma unroll 4
+    for (int b = 0; b < n; b += 4) {  // idle slots come last
+      const uint4 g = *reinterpret_cast<const uint4*>(sm.ord + b);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        rank[j] += (g.x < ord[j] ? 1 : 0) + (g.y < ord[j] ? 1 : 0) + (g.z < ord[j] ? 1 : 0) +
+                   (g.w < ord[j] ? 1 : 0);
+    }
+    uint32_t* const run = sm.w;  // the keys in order (the weights are all 1)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (ok[j]) run[rank[j]] = key[j];
+    sync();
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      pos[j] = rank[j];
+      lead[j] = ok[j] && (rank[j] == 0 || run[rank[j] - 1] != key[j]);
+      if (lead[j]) kc[j] = (uint32_t)(upper_bound(run, rank[j], n, key[j]) - rank[j]);
+      if constexpr (GEN) {
+        if (a.mh && lead[j]) {
+          const uint32_t other = key[j] ^ 0x80000000u;
+          const int lo = in[j] ? 0 : no, hi = in[j] ? no : n;
+          const int k1 = upper_bound(run, lo, hi, other);
+          const int k0 = other == 0u ? lo : upper_bound(run, lo, hi, other - 1u);
+          kany[j] = kc[j] + (uint32_t)(k1 - k0);
+          outside[j] = in[j] && k1 > k0;
+        }
+      }
+    }
   } else {
     int rank[2] = {0, 0}, same[2] = {0, 0};
     for (int b = 0; b < n; ++b) {
