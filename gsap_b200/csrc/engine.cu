@@ -199,10 +199,8 @@ Engine::~Engine() {
   cudaSetDevice(device);
   cudaStreamSynchronize(st);
   runs.clear();  // runs belong to the caller
-  cudaFree(up_dev);
   cudaFree(desc_dev);
   cudaFree(rd_dev);
-  cudaFreeHost(up_host);
   cudaFreeHost(desc_host);
   cudaFreeHost(rd_host);
   for (SweepGraph& g : graphs)
@@ -260,7 +258,7 @@ void Engine::ensure_slots(int K, int nb) {
 }
 
 void Engine::clear_slots() {
-  for (Slot* s : {&s_iota, &s_lists, &s_snap, &s_restore, &s_zero, &m_bt, &m_props, &m_delta,
+  for (Slot* s : {&s_iota, &s_snap, &s_restore, &s_zero, &m_bt, &m_props, &m_delta,
                   &m_delta8, &m_best, &m_relabel, &s_gather})
     s->clear();
   m_apply.clear();
@@ -325,8 +323,6 @@ void Engine::add_run_work(Run& r) {
     add_zero(s_zero, J.mdS, 2 * slots);
     add_zero(s_zero, J.mdsin, 2 * slots);
   }
-  if (r.upload_lists)
-    add_copy(s_lists, J.lists, up_dev_ptr(r.up_lists), r.lists_all.size());
   if (r.snap_slot >= 0) add_copy(s_snap, J.snap[r.snap_slot], J.part, (size_t)N);
   if (r.restore_slot >= 0) add_copy(s_restore, J.part, J.snap[r.restore_slot], (size_t)N);
   if (r.zero_itr) {
@@ -515,7 +511,7 @@ sbp_status Engine::tick() {
   for (Run* r : runs)
     if (r->stage != Run::kDone && r->o.phase_timing) timing = true;
   // pass 1: sweeps to queue, uploads (maps, batch lists) and readbacks
-  size_t up = 0, rd = 0;
+  size_t rd = 0;
   int nb_max = 0, k_max = 0;
   for (Run* r : runs) {
     if (r->stage == Run::kDone) continue;
@@ -526,16 +522,10 @@ sbp_status Engine::tick() {
       nb_max = std::max(nb_max, r->o.num_batches);
       k_max = std::max(k_max, r->sweep_k);
     }
-    if (r->upload_lists) {
-      r->up_lists = up;
-      up += align256(4 * r->lists_all.size());
-    }
     r->rd_off = rd;
     rd += rd_bytes(*r);
   }
-  sbp_status s = grow(up, up_cap, up_host, up_dev);
-  if (s != SBP_OK) return s;
-  s = grow(rd, rd_cap, rd_host, rd_dev);
+  sbp_status s = grow(rd, rd_cap, rd_host, rd_dev);
   if (s != SBP_OK) return s;
   // pass 2: records
   ensure_slots(k_max, nb_max);
@@ -543,12 +533,10 @@ sbp_status Engine::tick() {
   clear_slots();
   for (Run* r : runs) {
     if (r->stage == Run::kDone) continue;
-    if (r->upload_lists)
-      std::memcpy((char*)up_host + r->up_lists, r->lists_all.data(), 4 * r->lists_all.size());
     add_run_work(*r);
   }
   // pass 3: pack the slots' records and offsets
-  std::vector<Slot*> order = {&s_iota, &s_lists, &s_snap, &s_restore, &s_zero};
+  std::vector<Slot*> order = {&s_iota, &s_snap, &s_restore, &s_zero};
   for (Slot* x : pre_dense.all()) order.push_back(x);
   for (Slot* x : pre_rebuild.all()) order.push_back(x);
   for (Slot* x : {&m_bt, &m_props, &m_delta, &m_delta8, &m_best}) order.push_back(x);
@@ -614,7 +602,12 @@ sbp_status Engine::tick() {
       SBP_CUDA(cudaEventRecord(r->ev_begin, st));
     }
   SBP_CUDA(cudaEventRecord(ev[0], st));
-  if (up) SBP_CUDA(cudaMemcpyAsync(up_dev, up_host, up, cudaMemcpyHostToDevice, st));
+  // the batch lists by copies, not kernels: nodal kernels read them before
+  // they wait for the kernels ahead of them
+  for (Run* r : runs)
+    if (r->stage != Run::kDone && r->upload_lists)
+      SBP_CUDA(cudaMemcpyAsync(r->J->lists, r->lists_all.data(), 4 * r->lists_all.size(),
+                               cudaMemcpyHostToDevice, st));
   if (desc) SBP_CUDA(cudaMemcpyAsync(desc_dev, desc_host, desc, cudaMemcpyHostToDevice, st));
   size_t i = 0;
   auto emit_until = [&](Slot* last, cudaStream_t on = nullptr) -> sbp_status {

@@ -70,8 +70,8 @@ struct Run {
   // their blockmodel (the next merge step reads its CSR form from it)
   bool dense_kept = false;
   int snap_slot = -1, restore_slot = -1;
-  // this tick's offsets in the upload and readback buffers
-  size_t up_lists = 0, rd_off = 0;
+  // this tick's offset in the readback buffer
+  size_t rd_off = 0;
   cudaEvent_t ev_begin = nullptr;
   // scheduler / server bookkeeping
   double admit_bytes = 0.0;
@@ -132,7 +132,7 @@ class Engine {
   void reset();
 
  private:
-  Slot s_iota, s_lists, s_snap, s_restore, s_zero;
+  Slot s_iota, s_snap, s_restore, s_zero;
   DenseBuildSlots pre_dense;
   RebuildSlots pre_rebuild;
   Slot m_bt, m_props, m_delta, m_delta8, m_best;
@@ -142,9 +142,9 @@ class Engine {
   std::vector<SweepEndSlots> ends;  // [queued sweep]
   Slot s_gather;
   std::vector<cudaEvent_t> ev;
-  void *up_host = nullptr, *up_dev = nullptr, *desc_host = nullptr, *desc_dev = nullptr;
+  void *desc_host = nullptr, *desc_dev = nullptr;
   void *rd_host = nullptr, *rd_dev = nullptr;
-  size_t up_cap = 0, desc_cap = 0, rd_cap = 0;
+  size_t desc_cap = 0, rd_cap = 0;
   // The queued sweeps of a tick as an executable graph.  One per sequence of
   // kernels (`shape`), at most kMaxGraphs, the least recently used replaced:
   // a graph of the same shape takes new arguments in place (some 60 us),
@@ -163,7 +163,6 @@ class Engine {
   std::vector<unsigned char> last_key, last_shape;  // of the tick before
   int nb_slots_ = 0;  // batch positions per queued sweep in this tick's slots
 
-  void* up_dev_ptr(size_t off) { return (char*)up_dev + off; }
   void* rd_dev_ptr(size_t off) { return (char*)rd_dev + off; }
   void ensure_slots(int K, int nb);
   void clear_slots();

@@ -53,17 +53,36 @@ __device__ __forceinline__ void begin_kernel() {
   cudaGridDependencySynchronize();
 }
 
+// A body that sets kEarly makes the wait itself (wait_kernel), after loading
+// what no kernel writes: the graph, the batch lists, its launch records.
+// These come by copies that are complete before the first kernel behind them
+// starts, so they may be read before the wait.
+template <class Body, class = void>
+struct IsEarly {
+  static constexpr bool value = false;
+};
+template <class Body>
+struct IsEarly<Body, std::void_t<decltype(Body::kEarly)>> {
+  static constexpr bool value = Body::kEarly;
+};
+__device__ __forceinline__ void wait_kernel() { cudaGridDependencySynchronize(); }
+template <class Body>
+__device__ __forceinline__ void begin_body() {
+  if constexpr (IsEarly<Body>::value) cudaTriggerProgrammaticLaunchCompletion();
+  else begin_kernel();
+}
+
 template <class Body>
 __global__ void __launch_bounds__(Body::kThreads, Body::kMinBlocks)
     single_kernel(typename Body::Args a) {
-  begin_kernel();
+  begin_body<Body>();
   Body::run(a, (int)blockIdx.x, (int)gridDim.x);
 }
 
 template <class Body>
 __global__ void __launch_bounds__(Body::kThreads, Body::kMinBlocks)
     __cluster_dims__(ClusterOf<Body>::value, 1, 1) single_cluster_kernel(typename Body::Args a) {
-  begin_kernel();
+  begin_body<Body>();
   Body::run(a, (int)blockIdx.x, (int)gridDim.x);
 }
 
@@ -74,7 +93,7 @@ __device__ __forceinline__ void run_multi(const MultiSpan& sp) {
   constexpr int kWords = (int)(sizeof(Args) / 8);
   __shared__ unsigned long long raw[kWords];
   __shared__ int s_j, s_vb, s_vg;
-  begin_kernel();
+  begin_body<Body>();
   const Args& a = *reinterpret_cast<const Args*>(raw);
   int loaded = -1;
   for (int blk = blockIdx.x; blk < sp.total; blk += gridDim.x) {

@@ -690,16 +690,20 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
     in[j] = split ? j == 1 : k >= no;
     const int e = split ? hl : in[j] ? k - no : k;
     ok[j] = e < (in[j] ? ni : no);
-    c[j] = -1;
+    c[j] = -1;  // the neighbour, then its block
     w[j] = 0u;
-    loop[j] = false;
     if (ok[j]) {
-      const int32_t u = __ldg((in[j] ? a.iidx + i0 : a.oidx + o0) + e);
+      c[j] = __ldg((in[j] ? a.iidx + i0 : a.oidx + o0) + e);
       w[j] = __ldg((in[j] ? a.iw + i0 : a.ow + o0) + e);
-      c[j] = __ldg(a.part + u);
-      loop[j] = GEN && !in[j] && u == v;
     }
+    loop[j] = GEN && !in[j] && c[j] == v;
   }
+  const uint64_t deg = (uint64_t)a.kdo[v] + a.kdi[v];
+  wait_kernel();
+  if (ctl_stopped(a.ctl)) return;
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    if (ok[j]) c[j] = __ldg(a.part + c[j]);
   const int r = a.part[v];
   P4 x{};
   if (!GIVEN) x = draw(a.seed, kRngNodalVertex, a.seq + ctl_itr(a.ctl) * a.seq_mul, (uint32_t)v);
@@ -722,7 +726,6 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
     s = a.props_in[i];
   } else {
     const int rnd = (int)(x.v[0] % (uint32_t)a.B);
-    const uint64_t deg = (uint64_t)a.kdo[v] + a.kdi[v];
     const uint64_t t = scale_draw(x.v[1], deg);
     int at = -1;
     if (unit) {
@@ -928,14 +931,20 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
     ok[j] = k < n;
     in[j] = k >= no;
     const int e = in[j] ? k - no : k;
-    c[j] = -1;
+    c[j] = -1;  // the neighbour, then its block
     w[j] = 0u;
     if (ok[j]) {
-      const int32_t u = __ldg((in[j] ? a.iidx + i0 : a.oidx + o0) + e);
+      c[j] = __ldg((in[j] ? a.iidx + i0 : a.oidx + o0) + e);
       w[j] = __ldg((in[j] ? a.iw + i0 : a.ow + o0) + e);
-      c[j] = __ldg(a.part + u);
-      if (GEN && !in[j] && u == v) selfp += w[j];
+      if (GEN && !in[j] && c[j] == v) selfp += w[j];
     }
+  }
+  wait_kernel();
+  if (ctl_stopped(a.ctl)) return;  // the same in every thread
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int k = tid + T * j;
+    if (ok[j]) c[j] = __ldg(a.part + c[j]);
     key[j] = ok[j] ? (uint32_t)c[j] | (in[j] ? 0x80000000u : 0u) : 0xffffffffu;
     ord[j] = ok[j] ? (in[j] ? 1u << 30 : 0u) | (uint32_t)c[j] << 8 | (uint32_t)k : 0xffffffffu;
     sm.key[k] = key[j];
@@ -1298,9 +1307,9 @@ struct NodalBody {
   using Args = NodalArgs;
   static constexpr int kThreads = kNodalWarps * 32;
   static constexpr int kMinBlocks = GEN ? 5 : 8;
+  static constexpr bool kEarly = true;
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
-    if (ctl_stopped(a.ctl)) return;
     using Large = LargeBuf<kThreads, GEN>;
     // per warp: the keys and weights of group_vertex, or (general mode) a
     // 33-64-entry vertex's LargeBuf
