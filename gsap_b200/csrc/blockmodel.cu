@@ -194,6 +194,8 @@ struct RbArgs {
   int32_t tile_cap;   // longest segment ranked by comparison (RbTileBody)
   int32_t warp_max;   // longest segment ranked by a warp (RbRankBody)
   int32_t tile_rows;  // rows of a tile
+  int32_t unit;       // every weight is 1: tw is neither written nor read
+  int32_t pad;
 };
 
 // The rebuild bodies work on both directions: virtual block vb serves
@@ -245,7 +247,7 @@ struct RbScatterBody {
     int b = __ldg(a.part + v);
     int pos = __ldg(d.bptr + b) + __ldg(d.vofs + v) + (j - __ldg(d.gptr + v));
     d.tcol[pos] = __ldg(a.part + __ldg(d.gidx + j));
-    d.tw[pos] = __ldg(d.gw + j);
+    if (!a.unit) d.tw[pos] = __ldg(d.gw + j);
   }
 };
 
@@ -311,14 +313,14 @@ struct RbTileBody {
         if (n == 0 || o < 0 || o >= win) continue;
         for (int i = gl; i < n; i += 8) {
           key[o + i] = (uint32_t)d.tcol[src[r] + i];
-          w[o + i] = d.tw[src[r] + i];
+          w[o + i] = a.unit ? 1u : d.tw[src[r] + i];
           owner[o + i] = (uint8_t)r;
         }
       }
       __syncthreads();
       // the round's entries end where the next round's first row starts
-      int end = 0;
-      {
+      int end = total - q0;
+      if (end > win) {
         const bool mine = tid < nr && len > 0 && at - q0 >= 0 && at - q0 < win;
         end = mine ? at - q0 + len : 0;
 #pragma unroll
@@ -401,7 +403,7 @@ struct RbRankBody {
   static constexpr size_t kSmem = kRankWarps * kRankWarpBytes;
   static __device__ void run(const Args& a, int vb, int vg) {
     if (ctl_stopped(a.ctl)) return;
-    extern __shared__ unsigned char rank_sm[];
+    extern __shared__ __align__(16) unsigned char rank_sm[];
     const RbSide& d = a.s[vb & 1];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t* cnt = (uint32_t*)(rank_sm + wid * kRankWarpBytes);
@@ -414,8 +416,9 @@ struct RbRankBody {
       for (int i = lane; i < n; i += 32) cnt[i] = 0u;
       int u = 0;
       for (int w0 = 0; w0 < a.B; w0 += 32 * kRankWords) {
-        const int cols = min(32 * kRankWords, a.B - w0), nw = (cols + 31) >> 5;
-        for (int x = lane; x < nw; x += 32) bm[x] = 0u;
+        const int cols = min(32 * kRankWords, a.B - w0);
+        for (int x = 4 * lane; x < kRankWords; x += 128)
+          *reinterpret_cast<uint4*>(bm + x) = make_uint4(0u, 0u, 0u, 0u);
         __syncwarp();
 #pragma unroll 4
         for (int i = lane; i < n; i += 32) {
@@ -423,13 +426,45 @@ struct RbRankBody {
           if ((unsigned)c < (unsigned)cols) atomicOr(bm + (c >> 5), 1u << (c & 31));
         }
         __syncwarp();
-        int run = 0;
-        for (int x0 = 0; x0 < nw; x0 += 32) {
-          const int x = x0 + lane;
-          const int p = x < nw ? __popc(bm[x]) : 0;
-          const int incl = (int)warp_incl_scan_u((unsigned)p, lane);
-          if (x < nw) pre[x] = (uint16_t)(run + incl - p);
-          run += __shfl_sync(kFull, incl, 31);
+        // each lane counts sixteen consecutive words (in an order of four
+        // that spreads the lanes over the banks)
+        constexpr int kPer = kRankWords / 32;
+        int own[kPer / 4], local = 0;
+#pragma unroll
+        for (int k = 0; k < kPer / 4; ++k) {
+          const int x = lane * kPer + 4 * ((k + (lane >> 1)) & (kPer / 4 - 1));
+          const uint4 g = *reinterpret_cast<const uint4*>(bm + x);
+          const int p0 = __popc(g.x), p1 = p0 + __popc(g.y), p2 = p1 + __popc(g.z);
+          own[k] = p2 + __popc(g.w);
+          // within the four, to be offset below
+          *reinterpret_cast<ushort4*>(pre + x) = make_ushort4(0, p0, p1, p2);
+          local += own[k];
+        }
+        const int incl = (int)warp_incl_scan_u((unsigned)local, lane);
+        const int run = __shfl_sync(kFull, incl, 31);
+        {
+          // the four's places in ascending order of words
+          int at[kPer / 4];
+          int before = incl - local;
+#pragma unroll
+          for (int z = 0; z < kPer / 4; ++z) {
+            const int k = (z - (lane >> 1)) & (kPer / 4 - 1);  // the one that holds words 4z
+            int c = 0;
+#pragma unroll
+            for (int y = 0; y < kPer / 4; ++y) c = k == y ? own[y] : c;
+            at[z] = before;
+            before += c;
+          }
+#pragma unroll
+          for (int z = 0; z < kPer / 4; ++z) {
+            ushort4* q = reinterpret_cast<ushort4*>(pre + lane * kPer + 4 * z);
+            ushort4 v = *q;
+            v.x += at[z];
+            v.y += at[z];
+            v.z += at[z];
+            v.w += at[z];
+            *q = v;
+          }
         }
         __syncwarp();
 #pragma unroll 4
@@ -437,7 +472,7 @@ struct RbRankBody {
           const int c = d.tcol[base + i] - w0;
           if ((unsigned)c >= (unsigned)cols) continue;
           const int at = u + pre[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u));
-          atomicAdd(cnt + at, d.tw[base + i]);
+          atomicAdd(cnt + at, a.unit ? 1u : d.tw[base + i]);
           d.bcol[base + at] = c + w0;
         }
         u += run;
@@ -516,7 +551,7 @@ struct RbBigBody {
         const int c = d.tcol[base + i] - w0;
         if ((unsigned)c >= (unsigned)cols) continue;
         const int at = u + (int)pre[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u));
-        atomicAdd(cnt + at, d.tw[base + i]);
+        atomicAdd(cnt + at, a.unit ? 1u : d.tw[base + i]);
         d.bcol[base + at] = c + w0;
       }
       u += tot;
@@ -590,7 +625,7 @@ struct RbBigBody {
 #pragma unroll
         for (int p = 1; p < C; ++p) f = sg == p ? first[p] : f;
         const int at = (int)(f + pre[word]) + __popc(merged[word] & ((1u << (c & 31)) - 1u));
-        atomicAdd(d.bcnt + base + at, d.tw[base + i]);
+        atomicAdd(d.bcnt + base + at, a.unit ? 1u : d.tw[base + i]);
         d.bcol[base + at] = c + w0;
       }
       u = (int)run;
@@ -800,6 +835,7 @@ struct DenseArgs {
   // direction), and the vertices a warp covers
   const int32_t* heavy;
   int32_t N, E, B, lo, count, nheavy, heavy_min, per_warp;
+  int32_t unit, pad;
 };
 
 // Chunk sums of a dense cell (r, c): out-row r's chunk of column c and
@@ -820,7 +856,7 @@ struct DenseEdgesBody {
     int j = vb * blockDim.x + threadIdx.x;
     if (j >= a.E) return;
     int r = __ldg(a.part + __ldg(a.osrc + j)), c = __ldg(a.part + __ldg(a.oidx + j));
-    uint32_t w = __ldg(a.ow + j);
+    uint32_t w = a.unit ? 1u : __ldg(a.ow + j);
     const int K = (a.B + 31) >> 5;
     atomicAdd(a.Md + (size_t)r * a.B + c, w);
     atomicAdd(a.MTd + (size_t)c * a.B + r, w);
@@ -990,7 +1026,7 @@ __device__ __forceinline__ void dense_move_entry(const DenseArgs& a, const Dense
   const bool in = e >= v.no;
   const int j = in ? v.i0 + e - v.no : v.o0 + e;
   const int x = __ldg((in ? a.iidx : a.oidx) + j);
-  const uint32_t wt = __ldg((in ? a.iw : a.ow) + j);
+  const uint32_t wt = a.unit ? 1u : __ldg((in ? a.iw : a.ow) + j);
   const int bo = __ldg(a.part + x);
   const int bn = x >= lo && x < lo + count ? __ldg(a.newlab + x - lo) : bo;
   if (in && bn != bo) return;  // moved source
@@ -1294,6 +1330,7 @@ RbArgs rb_args(const DevGraph& g, const int32_t* part, int32_t B, DevBM& m, Rebu
   a.tile_rows = (int32_t)std::max<long long>(
       8, std::min<long long>(RbTileBody::kThreads,
                              (long long)kTileEntries / 2 * B / std::max(g.E, 1)));
+  a.unit = g.unit;
   a.part = part;
   a.xlx = m.xlx;
   a.nnz = m.nnz;
@@ -1374,6 +1411,7 @@ DenseArgs dense_args(const DevGraph& g, const int32_t* part, int32_t B, DevBM& m
   a.Md = m.Md; a.MTd = m.MTd; a.Sd = m.Sd; a.d_out = m.d_out; a.d_in = m.d_in;
   a.ld_out = m.ld_out; a.ld_in = m.ld_in;
   a.N = g.N; a.E = g.E; a.B = B;
+  a.unit = g.unit;
   return a;
 }
 

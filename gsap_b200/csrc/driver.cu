@@ -380,6 +380,10 @@ sbp_status job_upload(Job& J, const sbp_graph_csr* h) {
   SBP_CUDA(cudaMemcpyAsync(g.kdi, h->deg_in, 4 * (size_t)J.N, cudaMemcpyHostToDevice, st));
   ++g_launches;
   fill_src_kernel<<<(J.N + 255) / 256, 256, 0, st>>>(g.optr, J.N, g.osrc);
+  // weights are at least 1, so they all are 1 when they sum to E
+  uint64_t weight = 0;
+  for (int32_t v = 0; v < J.N; ++v) weight += h->deg_out[v];
+  g.unit = weight == (uint64_t)J.E ? 1 : 0;
   J.h_optr.assign(h->out_ptr, h->out_ptr + J.N + 1);
   J.h_iptr.assign(h->in_ptr, h->in_ptr + J.N + 1);
   ++g_launches;
@@ -806,6 +810,7 @@ static sbp_status job_from_device_edges(Job& J, int device, int32_t N, int32_t E
   SBP_CUDA(cudaMallocAsync((void**)&scratch, sb, J.st));
   int32_t* err = (int32_t*)(scratch + sb - 256);
   cudaError_t e = csr_from_device_edges(N, E, src, dst, w, J.g, err, scratch, J.st);
+  J.g.unit = w ? 0 : 1;
   int32_t herr = 0;
   J.h_optr.resize((size_t)N + 1);
   J.h_iptr.resize((size_t)N + 1);

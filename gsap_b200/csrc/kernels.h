@@ -17,6 +17,7 @@ extern thread_local long long g_launches;
 // The graph in HBM (uploaded once per job).
 struct DevGraph {
   int32_t N = 0, E = 0;
+  int32_t unit = 0;  // every weight is 1: kernels on the loop's path do not read ow and iw
   int32_t *optr = nullptr, *oidx = nullptr, *iptr = nullptr, *iidx = nullptr;
   uint32_t *ow = nullptr, *iw = nullptr, *kdo = nullptr, *kdi = nullptr;
   int32_t *osrc = nullptr, *isrc = nullptr;  // owning vertex of each CSR entry

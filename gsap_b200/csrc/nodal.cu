@@ -75,6 +75,7 @@ struct NodalArgs {
   int32_t nheavy, nhub;
   const int32_t *small, *mid;  // batch indices of the warp kernel (NodalItems)
   int32_t nsmall, nmid;
+  int32_t unit;                // every weight is 1
   int32_t nlarge, nmid64;      // mid vertices by size: large, up to kGroupEntries, the others
   int32_t* err;             // error counter (hash table overflow)
   const int32_t* ctl;       // sweep control: gate, and seq += ctl[0] * seq_mul
@@ -694,7 +695,7 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
     w[j] = 0u;
     if (ok[j]) {
       c[j] = __ldg((in[j] ? a.iidx + i0 : a.oidx + o0) + e);
-      w[j] = __ldg((in[j] ? a.iw + i0 : a.ow + o0) + e);
+      w[j] = a.unit ? 1u : __ldg((in[j] ? a.iw + i0 : a.ow + o0) + e);
     }
     loop[j] = GEN && !in[j] && c[j] == v;
   }
@@ -935,7 +936,7 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
     w[j] = 0u;
     if (ok[j]) {
       c[j] = __ldg((in[j] ? a.iidx + i0 : a.oidx + o0) + e);
-      w[j] = __ldg((in[j] ? a.iw + i0 : a.ow + o0) + e);
+      w[j] = a.unit ? 1u : __ldg((in[j] ? a.iw + i0 : a.ow + o0) + e);
       if (GEN && !in[j] && c[j] == v) selfp += w[j];
     }
   }
@@ -1939,6 +1940,7 @@ NodalArgs make_args(const DevGraph& g, const int32_t* part, const DevBM& m, int3
   a.ld_out = m.ld_out; a.ld_in = m.ld_in;
   a.nbr_s = m.nbr_s;
   a.B = B;
+  a.unit = g.unit;
   a.heavy = aux.heavy;
   a.nheavy = aux.nheavy;
   a.nhub = aux.nhub;
