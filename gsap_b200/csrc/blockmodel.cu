@@ -262,28 +262,34 @@ __device__ __forceinline__ void row_done(const RbArgs& a, const RbSide& d, int b
 constexpr int kBigCap = 12288;  // longest segment a CTA takes; longer ones go to a cluster
 
 // Short segments: a CTA takes tile_rows consecutive rows and gives every
-// entry a thread, which compares it with its segment's entries in shared
-// memory: the number before it in (column, index) order is its place in the
-// sorted segment, the equal ones give the column's total, and the first of
-// them the entry that carries it.  Eight lanes a row then close up the
-// carried entries.  Longer segments are listed for the kernels below.  A
-// warp per segment (a match over its lanes, or a bitonic sort) took 141 us a
-// rebuild of the 200k HH graph at B = 55k-85k, issuing for idle lanes.
+// entry a thread, which counts its segment's entries before it in (column,
+// index) order, its place in the sorted segment; eight lanes a row then walk
+// the sorted entries and write each run of a column once.  What bounds it is
+// the comparisons, so column and index share a word (up to kTileBlocks
+// blocks) and are compared four at a time: 86 us a rebuild of the 200k HH
+// graph comparing columns and weights one by one, 72 this way, 141 for a warp
+// per segment (a match over its lanes, or a bitonic sort).  Longer segments
+// are listed for the kernels below.
 constexpr int kTileEntries = 2048, kTileMaxCap = 128;
+constexpr int kTileBlocks = 1 << 25;  // (column, index) in a word: 7 bits of index
 struct RbTileBody {
   using Args = RbArgs;
-  static constexpr int kThreads = 256, kMinBlocks = 1;
+  static constexpr int kThreads = 256, kMinBlocks = 6;
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int) {
     if (ctl_stopped(a.ctl)) return;
-    __shared__ uint32_t key[kTileEntries], w[kTileEntries], skey[kTileEntries], sw[kTileEntries];
-    __shared__ uint8_t owner[kTileEntries];
+    // a segment starts at a multiple of four entries, padded with ~0
+    __shared__ __align__(16) uint32_t key[kTileEntries];
+    __shared__ uint32_t w[kTileEntries];
+    __shared__ uint8_t owner[kTileEntries], sorted[kTileEntries];  // row; index by place
     __shared__ int off[kThreads + 1], src[kThreads];
+    __shared__ uint8_t slen[kThreads];
     __shared__ int sh[33];
     __shared__ int s_nnz;
     const RbSide& d = a.s[vb & 1];
     const int tid = threadIdx.x, lane = tid & 31;
     const int b0 = (vb >> 1) * a.tile_rows, nr = min(a.tile_rows, a.B - b0);
+    const bool packed = a.B <= kTileBlocks;
     int len = 0;
     if (tid < nr) {
       const int b = b0 + tid, base = d.bptr[b];
@@ -297,23 +303,30 @@ struct RbTileBody {
         row_done(a, d, b, base, 0, 0u);
       }
     }
+    slen[tid] = (uint8_t)len;
     if (tid == 0) s_nnz = 0;
+    const int plen = (len + 3) & ~3;
     int total;
-    const int at = cta_excl_scan(len, sh, &total);
+    const int at = cta_excl_scan(plen, sh, &total);
     off[tid] = at;
     if (tid == 0) off[kThreads] = total;
     __syncthreads();
     // rounds of rows whose offsets lie in a window, so that their entries fit
-    const int win = kTileEntries - a.tile_cap;
+    const int win = kTileEntries - kTileMaxCap;
     const int g = tid >> 3, gl = tid & 7;
     int nnz = 0;
     for (int q0 = 0; q0 < total; q0 += win) {
       for (int r = g; r < nr; r += kThreads / 8) {
-        const int o = off[r] - q0, n = off[r + 1] - off[r];
+        const int o = off[r] - q0, n = slen[r];
         if (n == 0 || o < 0 || o >= win) continue;
-        for (int i = gl; i < n; i += 8) {
-          key[o + i] = (uint32_t)d.tcol[src[r] + i];
-          w[o + i] = a.unit ? 1u : d.tw[src[r] + i];
+        for (int i = gl; i < ((n + 3) & ~3); i += 8) {
+          uint32_t x = 0xffffffffu;
+          if (i < n) {
+            x = (uint32_t)d.tcol[src[r] + i];
+            if (packed) x = x << 7 | (uint32_t)i;
+            if (!a.unit) w[o + i] = d.tw[src[r] + i];
+          }
+          key[o + i] = x;
           owner[o + i] = (uint8_t)r;
         }
       }
@@ -322,7 +335,7 @@ struct RbTileBody {
       int end = total - q0;
       if (end > win) {
         const bool mine = tid < nr && len > 0 && at - q0 >= 0 && at - q0 < win;
-        end = mine ? at - q0 + len : 0;
+        end = mine ? at - q0 + plen : 0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) end = max(end, __shfl_xor_sync(kFull, end, o));
         if (lane == 0) sh[tid >> 5] = end;
@@ -331,43 +344,54 @@ struct RbTileBody {
         for (int i = 0; i < kThreads / 32; ++i) end = max(end, sh[i]);
       }
       for (int e = tid; e < end; e += kThreads) {
-        const int r = owner[e], s0 = off[r] - q0, s1 = s0 + off[r + 1] - off[r];
         const uint32_t k = key[e];
-        int lt = 0, before = 0;
-        uint32_t sum = 0u;
-        for (int j = s0; j < s1; ++j) {
-          const uint32_t x = key[j];
-          lt += x < k ? 1 : 0;
-          if (x == k) {
-            sum += w[j];
-            before += j < e ? 1 : 0;
+        if (k == 0xffffffffu) continue;
+        const int r = owner[e], s0 = off[r] - q0, s1 = s0 + ((slen[r] + 3) & ~3);
+        int lt = 0;
+        if (packed) {
+          for (int j = s0; j < s1; j += 4) {
+            const uint4 x = *reinterpret_cast<const uint4*>(key + j);
+            lt += (x.x < k ? 1 : 0) + (x.y < k ? 1 : 0) + (x.z < k ? 1 : 0) + (x.w < k ? 1 : 0);
           }
+        } else {
+          for (int j = s0; j < s1; ++j) lt += key[j] < k || (key[j] == k && j < e) ? 1 : 0;
         }
-        skey[s0 + lt + before] = k;
-        sw[s0 + lt + before] = before ? 0u : sum;  // weights are >= 1: 0 marks a repeat
+        sorted[s0 + lt] = (uint8_t)(e - s0);
       }
       __syncthreads();
       for (int r0 = 0; r0 < nr; r0 += kThreads / 8) {
         const int r = r0 + g;
-        const int o = r < nr ? off[r] - q0 : -1, n = r < nr ? off[r + 1] - off[r] : 0;
+        const int o = r < nr ? off[r] - q0 : -1, n = r < nr ? slen[r] : 0;
         const bool live = n > 0 && o >= 0 && o < win;
         const int steps = live ? (n + 7) >> 3 : 0;
+        auto column = [&](int p) {
+          const uint32_t x = key[o + sorted[o + p]];
+          return packed ? x >> 7 : x;
+        };
         int u = 0;
         uint32_t deg = 0u;  // the count so far
         const int most = __reduce_max_sync(kFull, steps);
         for (int i = 0; i < most; ++i) {
           const int p = 8 * i + gl;
-          const uint32_t c = live && p < n ? sw[o + p] : 0u;
+          uint32_t c = 0u, x = 0u;
+          if (live && p < n) {
+            x = column(p);
+            if (p == 0 || column(p - 1) != x) {  // the first of its column's run
+              int q = p;
+              do c += a.unit ? 1u : w[o + sorted[o + q]];
+              while (++q < n && column(q) == x);
+            }
+          }
           const unsigned m = __ballot_sync(kFull, c != 0u) >> (lane & 24) & 0xffu;
           uint32_t incl = c;
 #pragma unroll
-          for (int x = 1; x < 8; x <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, incl, x, 8);
-            if (gl >= x) incl += y;
+          for (int z = 1; z < 8; z <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, incl, z, 8);
+            if (gl >= z) incl += y;
           }
           if (c) {
             const int z = src[r] + u + __popc(m & ((1u << gl) - 1u));
-            d.bcol[z] = (int32_t)skey[o + p];
+            d.bcol[z] = (int32_t)x;
             d.bcnt[z] = c;
             d.bcum[z] = deg + incl;
           }
