@@ -229,8 +229,8 @@ __device__ __forceinline__ void merge_corners(const MergeArgs& a, int r, int s, 
 // cells are searched by different lanes, the two rows are walked together, and
 // the kernels hold six CTAs an SM (40 registers): 16.1 ms of merge kernels in
 // a 200k HH partition one search after the other at two or three CTAs, 7.3
-// this way (12.4 without the residency, 14 with two entries of each row in
-// flight at 64 registers, as much again in spills).
+// this way (7.9 at four CTAs, 7.5 at five; with two entries of each row in
+// flight 12.4 at two CTAs and 8.3 at four).
 template <int G>
 __device__ double merge_one(const MergeArgs& a, int r, int s, int s2, int gl, bool active,
                             bool given_in_s, double in_s_given, double* in_r_out) {
