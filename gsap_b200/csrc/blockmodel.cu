@@ -311,11 +311,13 @@ struct RbTileBody {
     off[tid] = at;
     if (tid == 0) off[kThreads] = total;
     __syncthreads();
-    // rounds of rows whose offsets lie in a window, so that their entries fit
+    // rounds of rows whose offsets lie in a window, so that their entries fit;
+    // the next round's window starts at its first row, so that a round writes
+    // all the entries it ranks
     const int win = kTileEntries - kTileMaxCap;
     const int g = tid >> 3, gl = tid & 7;
     int nnz = 0;
-    for (int q0 = 0; q0 < total; q0 += win) {
+    for (int q0 = 0, end; q0 < total; q0 += end) {
       for (int r = g; r < nr; r += kThreads / 8) {
         const int o = off[r] - q0, n = slen[r];
         if (n == 0 || o < 0 || o >= win) continue;
@@ -332,7 +334,7 @@ struct RbTileBody {
       }
       __syncthreads();
       // the round's entries end where the next round's first row starts
-      int end = total - q0;
+      end = total - q0;
       if (end > win) {
         const bool mine = tid < nr && len > 0 && at - q0 >= 0 && at - q0 < win;
         end = mine ? at - q0 + plen : 0;

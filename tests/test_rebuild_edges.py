@@ -47,3 +47,88 @@ def test_rebuild_edges(sbp, orc, monkeypatch, N, weighted, cap, entries):
         _, _, xa, _ = sbp.nodal_batch(g, p, B, 5, 3, 100, 1500)
         _, _, xb, _ = orc.nodal_batch(g, p, B, 5, 3, 100, 1500)
         assert np.array_equal(xa, xb), B
+
+
+# short segments side by side, so that a tile of consecutive rows takes several
+# rounds of its 1920-entry window (segments padded to fours)
+GROUP, WINDOW = 400, 1920
+
+
+def crowded_tiles(sbp, weighted):
+    """Vertices 0, 1, ... have runs of segments of 20 to 128 out-entries,
+    vertices N-1, N-2, ... as many in-entries; the others a few."""
+    N = 60000
+    rng = np.random.default_rng(11)
+    lens = np.concatenate([
+        rng.integers(20, 33, GROUP), np.full(GROUP, 32), rng.integers(20, 65, GROUP),
+        np.full(GROUP, 64), rng.integers(20, 129, GROUP), np.full(GROUP, 128),
+        np.sort(rng.integers(20, 51, GROUP))[::-1], rng.integers(0, 41, GROUP)])
+    K = lens.size
+    mid = np.arange(K, N - K)
+    own = np.repeat(np.arange(K), lens)
+    base = rng.integers(K, N - K - 30, K)
+    # neighbours near a base of the vertex's own, so that columns repeat
+    other = base[own] + rng.integers(0, 30, own.size)
+    src = np.concatenate([own, rng.permutation(mid), rng.permutation(other)])
+    dst = np.concatenate([other, mid, N - 1 - own])
+    w = rng.integers(1, 6, src.size).astype(np.uint32) if weighted else None
+    return sbp.Graph.from_edges(N, src.astype(np.int32), dst.astype(np.int32), w)
+
+
+@pytest.mark.parametrize("weighted", [False, True], ids=["unit", "weighted"])
+@pytest.mark.parametrize("cap", [32, 64, 128])
+def test_rebuild_tiles_of_several_rounds(sbp, orc, monkeypatch, weighted, cap):
+    monkeypatch.setenv("SBP_DENSE_MAX", "0")
+    monkeypatch.setenv("SBP_REBUILD_WARP_CAP", str(cap))
+    g = crowded_tiles(sbp, weighted)
+    N, p = g.N, np.arange(g.N, dtype=np.int32)
+    rows = max(8, min(256, 1024 * N // g.E))
+    for ptr in (g.out_ptr, g.in_ptr):
+        n = np.diff(ptr)
+        padded = np.where(n <= cap, (n + 3) & ~3, 0)
+        tiles = np.pad(padded, (0, -N % rows)).reshape(-1, rows)
+        at = np.cumsum(tiles, axis=1) - tiles
+        assert (tiles.sum(1) > 2 * WINDOW).any()
+        assert ((at < WINDOW) & (at + tiles > WINDOW)).any() and (at == WINDOW).any()
+    a = sbp.build_blockmodel(g, p, N)
+    b = orc.build_blockmodel(g, p, N)
+    for k in ("optr", "ocol", "ocnt", "iptr", "icol", "icnt", "d_out", "d_in"):
+        assert np.array_equal(a[k], b[k]), k
+
+
+def by_degree(sbp, variant, N, B, seed):
+    """A DCSBM graph with its vertices numbered by falling degree."""
+    g = sbp.dcsbm_variant(variant, N, B, seed=seed)
+    new = np.empty(N, np.int32)
+    new[np.argsort(-(g.deg_out.astype(np.int64) + g.deg_in), kind="stable")] = np.arange(N)
+    src, dst, w = g.edges()
+    truth = np.empty(N, np.int32)
+    truth[new] = g.true_partitions
+    return sbp.Graph.from_edges(N, new[src], new[dst], w, truth)
+
+
+@pytest.mark.parametrize("per_block", [1, 3])
+def test_batches_of_a_graph_numbered_by_degree(sbp, orc, monkeypatch, per_block):
+    monkeypatch.setenv("SBP_DENSE_MAX", "0")
+    g = by_degree(sbp, "HH", 20000, 32, 4)
+    q = np.arange(g.N, dtype=np.int32) // per_block
+    B = int(q[-1]) + 1
+    for b in range(4):
+        lo, hi = b * 5000, (b + 1) * 5000
+        pa, da, xa, _ = sbp.nodal_batch(g, q, B, 13, 40 + b, lo, hi)
+        pb, db, xb, _ = orc.nodal_batch(g, q, B, 13, 40 + b, lo, hi)
+        assert np.array_equal(xa, xb), "proposals differ"
+        with np.errstate(invalid="ignore"):  # -inf on both sides (a block of degree 0)
+            assert ((da == db) | (np.abs(da - db) <= 1e-9 * np.maximum(np.abs(db), 1.0))).all()
+        # a dS within its tolerance of 0 may round to either sign
+        moves = (np.abs(da) > 1e-9) | (np.abs(db) > 1e-9)
+        assert np.array_equal(pa[lo:hi][moves], pb[lo:hi][moves]), "accepted moves differ"
+        q = pb
+
+
+def test_partition_of_a_graph_numbered_by_degree(sbp, orc):
+    g = by_degree(sbp, "LL", 1000, 11, 0)
+    rep = sbp.partition(g, seed=0, dense_max=0)
+    lab, rep_o, _ = orc.partition(g, seed=0)
+    assert rep["B"] == rep_o["B"] and abs(rep["S"] - rep_o["S"]) <= 1e-9 * abs(rep_o["S"])
+    assert sbp.evaluate(lab, g.partitions)[2] > 0.999
