@@ -374,9 +374,12 @@ struct MergeDeltaBody {
       const int k = k0 + g;
       const bool act = k < a.np;
       const long long t = (long long)r * a.np + (act ? k : 0);
-      const int s = act ? a.props_in[t] : r;
+      const int target = act ? a.props_in[t] : r;
       const bool stale = act && t >= T;  // a slot GSAP's grid leaves out keeps its values
       const bool comp = act && !stale;
+      // a kept target may be a block of an earlier, larger B: it is handed on
+      // but never an index
+      const int s = comp ? target : r;
       double d, in_r = 0.0;
       if (a.exact) {
         d = merge_one_exact<G>(a, r, s, gl, comp);
@@ -397,7 +400,7 @@ struct MergeDeltaBody {
       // proposal k0 + j's dS and target from group j's first lane
       const int j = (lane - k0) & (NG - 1);
       const double dj = __shfl_sync(kFull, d, j * G);
-      const int sj = __shfl_sync(kFull, s, j * G);
+      const int sj = __shfl_sync(kFull, target, j * G);
       if (lane >= k0 && lane < k0 + NG && lane < a.np) {
         mine = dj;
         who = sj;
