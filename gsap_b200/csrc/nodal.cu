@@ -1735,7 +1735,10 @@ struct NodalHubBody {
   static constexpr int kThreads = kHeavyThreads, kMinBlocks = 1, kCluster = kHubCluster;
   static constexpr size_t kSmem = kHubSmem;
   static __device__ void run(const Args& a, int vb, int vg) {
-    if (ctl_stopped(a.ctl)) return;
+    if (ctl_stopped(a.ctl)) return;  // the same in every thread of the cluster
+    // every CTA of the cluster has started before one stores into another's
+    // shared memory
+    cooperative_groups::this_cluster().sync();
     int parity = 0;
     for (int h = vb / kHubCluster; h < a.nhub; h += vg / kHubCluster)
       hub_vertex<GIVEN, DENSE>(a, a.heavy[h], parity);
