@@ -244,9 +244,9 @@ struct RbScatterBody {
     int j = (vb >> 1) * blockDim.x + threadIdx.x;
     if (j >= a.E) return;
     int v = __ldg(d.gsrc + j);
-    int b = __ldg(a.part + v);
-    int pos = __ldg(d.bptr + b) + __ldg(d.vofs + v) + (j - __ldg(d.gptr + v));
-    d.tcol[pos] = __ldg(a.part + __ldg(d.gidx + j));
+    int b = a.part[v];
+    int pos = d.bptr[b] + d.vofs[v] + (j - __ldg(d.gptr + v));
+    d.tcol[pos] = a.part[__ldg(d.gidx + j)];
     if (!a.unit) d.tw[pos] = __ldg(d.gw + j);
   }
 };
@@ -795,7 +795,7 @@ struct BlockDrawBody {
         const bool go = len > 1;
         const int step = (len + 7) >> 3;
         const int at = first + min((gl + 1) * step, len) - 1;
-        const unsigned m = __ballot_sync(kFull, go && __ldg(cum + at) > t) >> hb & 0xffu;
+        const unsigned m = __ballot_sync(kFull, go && cum[at] > t) >> hb & 0xffu;
         if (go) {
           const int j = __ffs(m) - 1;
           first += j * step;
@@ -881,7 +881,7 @@ struct DenseEdgesBody {
   static __device__ void run(const Args& a, int vb, int) {
     int j = vb * blockDim.x + threadIdx.x;
     if (j >= a.E) return;
-    int r = __ldg(a.part + __ldg(a.osrc + j)), c = __ldg(a.part + __ldg(a.oidx + j));
+    int r = a.part[__ldg(a.osrc + j)], c = a.part[__ldg(a.oidx + j)];
     uint32_t w = a.unit ? 1u : __ldg(a.ow + j);
     const int K = (a.B + 31) >> 5;
     atomicAdd(a.Md + (size_t)r * a.B + c, w);
@@ -1045,28 +1045,40 @@ struct DenseMove {
   int32_t r, s, o0, no, i0, ni;
 };
 
-// Applies entry e (out-entries, then in-entries) of a moved vertex.
-__device__ __forceinline__ void dense_move_entry(const DenseArgs& a, const DenseMove& v, int e) {
-  const int32_t lo = a.lo, count = a.count, B = a.B;
-  const int K = (B + 31) >> 5;
+// What entry e (out-entries, then in-entries) of a moved vertex does: its
+// weight moves from cell (r0, c0) to (r1, c1).  Loaded apart from being
+// applied, so that the loads of several entries are in flight together (none
+// may pass an atomic).
+struct DenseCells {
+  int32_t r0, c0, r1, c1;
+  uint32_t w;  // 0: nothing to do
+};
+__device__ __forceinline__ DenseCells dense_move_load(const DenseArgs& a, const DenseMove& v,
+                                                      int e) {
+  const int32_t lo = a.lo, count = a.count;
   const bool in = e >= v.no;
   const int j = in ? v.i0 + e - v.no : v.o0 + e;
   const int x = __ldg((in ? a.iidx : a.oidx) + j);
   const uint32_t wt = a.unit ? 1u : __ldg((in ? a.iw : a.ow) + j);
-  const int bo = __ldg(a.part + x);
-  const int bn = x >= lo && x < lo + count ? __ldg(a.newlab + x - lo) : bo;
-  if (in && bn != bo) return;  // moved source
-  // the cell the edge leaves and the one it joins
-  const int r0 = in ? bo : v.r, c0 = in ? v.r : bo;
-  const int r1 = in ? bo : v.s, c1 = in ? v.s : bn;
-  atomicSub(a.Md + (size_t)r0 * B + c0, wt);
-  atomicSub(a.MTd + (size_t)c0 * B + r0, wt);
-  atomicAdd(a.Md + (size_t)r1 * B + c1, wt);
-  atomicAdd(a.MTd + (size_t)c1 * B + r1, wt);
-  atomicSub(sd_out(a.Sd, K, r0, c0), wt);
-  atomicSub(sd_in(a.Sd, K, r0, c0), wt);
-  atomicAdd(sd_out(a.Sd, K, r1, c1), wt);
-  atomicAdd(sd_in(a.Sd, K, r1, c1), wt);
+  const int bo = a.part[x];
+  const int bn = x >= lo && x < lo + count ? a.newlab[x - lo] : bo;
+  // an in-edge of a moved source is the source's
+  return DenseCells{in ? bo : v.r, in ? v.r : bo, in ? bo : v.s, in ? v.s : bn,
+                    in && bn != bo ? 0u : wt};
+}
+
+__device__ __forceinline__ void dense_move_apply(const DenseArgs& a, const DenseCells& m) {
+  if (m.w == 0u) return;
+  const int32_t B = a.B;
+  const int K = (B + 31) >> 5;
+  atomicSub(a.Md + (size_t)m.r0 * B + m.c0, m.w);
+  atomicSub(a.MTd + (size_t)m.c0 * B + m.r0, m.w);
+  atomicAdd(a.Md + (size_t)m.r1 * B + m.c1, m.w);
+  atomicAdd(a.MTd + (size_t)m.c1 * B + m.r1, m.w);
+  atomicSub(sd_out(a.Sd, K, m.r0, m.c0), m.w);
+  atomicSub(sd_in(a.Sd, K, m.r0, m.c0), m.w);
+  atomicAdd(sd_out(a.Sd, K, m.r1, m.c1), m.w);
+  atomicAdd(sd_in(a.Sd, K, m.r1, m.c1), m.w);
 }
 
 __device__ __forceinline__ void dense_move_degrees(const DenseArgs& a, int v, int r, int s) {
@@ -1091,8 +1103,18 @@ struct DenseUpdateBody {
       m.ni = a.iptr[v + 1] - m.i0;
       if (m.r == m.s) return;
       if (threadIdx.x == 0) dense_move_degrees(a, v, m.r, m.s);
-#pragma unroll 4
-      for (int e = threadIdx.x; e < m.no + m.ni; e += kThreads) dense_move_entry(a, m, e);
+      constexpr int U = 4;
+      const int n = m.no + m.ni;
+      for (int e = threadIdx.x; e < n; e += U * kThreads) {
+        DenseCells c[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          c[u].w = 0u;
+          if (e + u * kThreads < n) c[u] = dense_move_load(a, m, e + u * kThreads);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) dense_move_apply(a, c[u]);
+      }
       return;
     }
     const int per = a.per_warp;
@@ -1119,23 +1141,29 @@ struct DenseUpdateBody {
       if (lane >= o) incl += y;
     }
     const int total = __shfl_sync(kFull, incl, kDuVerts - 1);
-#pragma unroll 2
-    for (int e0 = 0; e0 < total; e0 += 32) {
-      const int e = e0 + lane;
-      // the vertex of entry e: the first whose running count exceeds it
-      int j = 0;
+    for (int e0 = 0; e0 < total; e0 += 64) {
+      DenseCells c[2];
 #pragma unroll
-      for (int q = 0; q < kDuVerts; ++q) j += __shfl_sync(kFull, incl, q) <= e ? 1 : 0;
-      j = min(j, kDuVerts - 1);
-      DenseMove u;
-      u.r = __shfl_sync(kFull, m.r, j);
-      u.s = __shfl_sync(kFull, m.s, j);
-      u.o0 = __shfl_sync(kFull, m.o0, j);
-      u.no = __shfl_sync(kFull, m.no, j);
-      u.i0 = __shfl_sync(kFull, m.i0, j);
-      u.ni = __shfl_sync(kFull, m.ni, j);
-      const int first = __shfl_sync(kFull, incl, j) - u.no - u.ni;
-      if (e < total) dense_move_entry(a, u, e - first);
+      for (int h = 0; h < 2; ++h) {
+        const int e = e0 + 32 * h + lane;
+        // the vertex of entry e: the first whose running count exceeds it
+        int j = 0;
+#pragma unroll
+        for (int q = 0; q < kDuVerts; ++q) j += __shfl_sync(kFull, incl, q) <= e ? 1 : 0;
+        j = min(j, kDuVerts - 1);
+        DenseMove u;
+        u.r = __shfl_sync(kFull, m.r, j);
+        u.s = __shfl_sync(kFull, m.s, j);
+        u.o0 = __shfl_sync(kFull, m.o0, j);
+        u.no = __shfl_sync(kFull, m.no, j);
+        u.i0 = __shfl_sync(kFull, m.i0, j);
+        u.ni = __shfl_sync(kFull, m.ni, j);
+        const int first = __shfl_sync(kFull, incl, j) - u.no - u.ni;
+        c[h].w = 0u;
+        if (e < total) c[h] = dense_move_load(a, u, e - first);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) dense_move_apply(a, c[h]);
     }
   }
 };

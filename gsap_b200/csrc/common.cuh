@@ -141,16 +141,15 @@ __device__ __forceinline__ uint32_t ctl_itr(const int32_t* ctl) {
 }
 
 // Binary search of column c in the CSR row [lo, hi); its count, or 0.
-__device__ __forceinline__ uint32_t row_lookup(const int32_t* __restrict__ col,
-                                               const uint32_t* __restrict__ cnt, int32_t lo,
-                                               int32_t hi, int32_t c) {
+__device__ __forceinline__ uint32_t row_lookup(const int32_t* col, const uint32_t* cnt,
+                                               int32_t lo, int32_t hi, int32_t c) {
   int32_t end = hi;
   while (lo < hi) {
     int32_t mid = (lo + hi) >> 1;
-    if (__ldg(col + mid) < c) lo = mid + 1;
+    if (col[mid] < c) lo = mid + 1;
     else hi = mid;
   }
-  return (lo < end && __ldg(col + lo) == c) ? __ldg(cnt + lo) : 0u;
+  return (lo < end && col[lo] == c) ? cnt[lo] : 0u;
 }
 
 }  // namespace sbp

@@ -18,7 +18,7 @@ __device__ __forceinline__ int warp_pick_chunked(const uint32_t* orow, const uin
   uint64_t acc = 0;
   for (int k0 = 0; k0 < 2 * K; k0 += 32) {
     const int k = k0 + lane;
-    const uint64_t w = k < 2 * K ? __ldg(srow + k) : 0u;
+    const uint64_t w = k < 2 * K ? srow[k] : 0u;
     uint64_t incl = w;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -33,7 +33,7 @@ __device__ __forceinline__ int warp_pick_chunked(const uint32_t* orow, const uin
       const int c0 = (kc < K ? kc : kc - K) * 32;
       const uint32_t* row = kc < K ? orow : irow;
       const int c = c0 + lane;
-      uint64_t in2 = c < B ? __ldg(row + c) : 0u;
+      uint64_t in2 = c < B ? row[c] : 0u;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const uint64_t y = __shfl_up_sync(kFull, in2, o);

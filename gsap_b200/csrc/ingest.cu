@@ -129,7 +129,7 @@ struct RowPtrBody {
     int lo = 0, hi = a.n;
     while (lo < hi) {
       const int mid = (int)(((unsigned)lo + (unsigned)hi) >> 1);
-      if (__ldg(a.keys + mid) < v) lo = mid + 1;
+      if (a.keys[mid] < v) lo = mid + 1;
       else hi = mid;
     }
     a.ptr[v] = lo;
@@ -153,7 +153,7 @@ struct GatherBody {
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
     for (int p = vb * kThreads + threadIdx.x; p < a.n; p += vg * kThreads) {
-      const int j = __ldg(a.perm + p);
+      const int j = a.perm[p];
       a.idx[p] = __ldg(a.other + j);
       a.wout[p] = a.w ? __ldg(a.w + j) : 1u;
     }
@@ -202,7 +202,7 @@ struct DegreeBody {
     const int lane = threadIdx.x & 31;
     for (int v = (vb * kThreads + threadIdx.x) >> 5; v < a.N; v += (vg * kThreads) >> 5) {
       unsigned long long s = 0;
-      for (int p = a.ptr[v] + lane; p < a.ptr[v + 1]; p += 32) s += __ldg(a.w + p);
+      for (int p = a.ptr[v] + lane; p < a.ptr[v + 1]; p += 32) s += a.w[p];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
       if (lane == 0) {

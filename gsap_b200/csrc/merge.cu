@@ -65,7 +65,7 @@ __device__ __forceinline__ long long merge_grid_end(const MergeArgs& a) {
 // kernels.hpp:767-783).
 __device__ __forceinline__ int col_at(const MergeArgs& a, int b, int k) {
   int o0 = a.optr[b], no = a.oend[b] - o0;
-  return k < no ? __ldg(a.ocol + o0 + k) : __ldg(a.icol + a.iptr[b] + k - no);
+  return k < no ? a.ocol[o0 + k] : a.icol[a.iptr[b] + k - no];
 }
 
 // First entry of out-row ++ in-row of block b whose running count exceeds t
@@ -81,7 +81,7 @@ __device__ __forceinline__ int pick_entry(const MergeArgs& a, int b, uint64_t t)
   int lo = 0, hi = in ? a.iend[b] - i0 : no;
   while (lo < hi) {
     const int mid = (lo + hi) >> 1;
-    if (__ldg(cum + mid) > x) hi = mid;
+    if (cum[mid] > x) hi = mid;
     else lo = mid + 1;
   }
   return in ? no + lo : lo;
@@ -153,14 +153,14 @@ __device__ __forceinline__ void cells(const MergeArgs& a, const int* y, const bo
   if (a.Md) {
 #pragma unroll
     for (int j = 0; j < E; ++j)
-      m[j] = want[j] ? __ldg((in[j] ? a.MTd : a.Md) + (size_t)y[j] * a.B + c[j]) : 0u;
+      m[j] = want[j] ? (in[j] ? a.MTd : a.Md)[(size_t)y[j] * a.B + c[j]] : 0u;
     return;
   }
   int lo[E], hi[E], end[E];
 #pragma unroll
   for (int j = 0; j < E; ++j) {
-    lo[j] = want[j] ? __ldg((in[j] ? a.iptr : a.optr) + y[j]) : 0;
-    hi[j] = end[j] = want[j] ? __ldg((in[j] ? a.iend : a.oend) + y[j]) : 0;
+    lo[j] = want[j] ? (in[j] ? a.iptr : a.optr)[y[j]] : 0;
+    hi[j] = end[j] = want[j] ? (in[j] ? a.iend : a.oend)[y[j]] : 0;
   }
   bool go = true;
   while (go) {
@@ -168,7 +168,7 @@ __device__ __forceinline__ void cells(const MergeArgs& a, const int* y, const bo
     int x[E];
 #pragma unroll
     for (int j = 0; j < E; ++j)
-      x[j] = lo[j] < hi[j] ? __ldg((in[j] ? a.icol : a.ocol) + ((lo[j] + hi[j]) >> 1)) : 0;
+      x[j] = lo[j] < hi[j] ? (in[j] ? a.icol : a.ocol)[(lo[j] + hi[j]) >> 1] : 0;
 #pragma unroll
     for (int j = 0; j < E; ++j) {
       if (lo[j] >= hi[j]) continue;
@@ -180,8 +180,8 @@ __device__ __forceinline__ void cells(const MergeArgs& a, const int* y, const bo
   }
 #pragma unroll
   for (int j = 0; j < E; ++j)
-    m[j] = lo[j] < end[j] && __ldg((in[j] ? a.icol : a.ocol) + lo[j]) == c[j]
-               ? __ldg((in[j] ? a.icnt : a.ocnt) + lo[j])
+    m[j] = lo[j] < end[j] && (in[j] ? a.icol : a.ocol)[lo[j]] == c[j]
+               ? (in[j] ? a.icnt : a.ocnt)[lo[j]]
                : 0u;
 }
 
@@ -263,11 +263,11 @@ __device__ double merge_one(const MergeArgs& a, int r, int s, int s2, int gl, bo
         cnt[j] = 0u;
         want[j] = i[j] < w.x1[j];
         if (want[j]) {
-          c[j] = __ldg((in[j] ? a.icol : a.ocol) + i[j]);
-          cnt[j] = __ldg((in[j] ? a.icnt : a.ocnt) + i[j]);
+          c[j] = (in[j] ? a.icol : a.ocol)[i[j]];
+          cnt[j] = (in[j] ? a.icnt : a.ocnt)[i[j]];
         }
         if (in[j] && (c[j] == r || c[j] == s)) want[j] = false;
-        ld[j] = want[j] ? __ldg((in[j] ? a.ld_out : a.ld_in) + c[j]) : 0.0;
+        ld[j] = want[j] ? (in[j] ? a.ld_out : a.ld_in)[c[j]] : 0.0;
       }
       cells<2>(a, w.y, in, c, want, my);
       if (want[0]) acc_o += gterm(a.xlx, cnt[0] + my[0], ld[0]) - gterm(a.xlx, my[0], ld[0]);
@@ -493,7 +493,7 @@ struct RelabelBody {
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int) {
     int v = vb * kThreads + threadIdx.x;
-    if (v < a.N) a.part[v] = __ldg(a.map + a.part[v]);
+    if (v < a.N) a.part[v] = a.map[a.part[v]];
   }
 };
 

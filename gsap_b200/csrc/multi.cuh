@@ -48,6 +48,10 @@ struct ClusterOf<Body, std::void_t<decltype(Body::kCluster)>> {
 // before it, since it has waited for them.  A batch of a small graph is a
 // chain of launches of a few microseconds each: 1k LL partitions 16.8 -> 15.3
 // ms, 20k HH 55.1 -> 53.2 ms, 200k HH unchanged.
+// Read-only loads (__ldg) are for data that stays the same while a kernel is
+// resident, which now includes the time its predecessors still write: the
+// graph, the x log2 x table and the launch records, nothing that a kernel of
+// the loop writes.
 __device__ __forceinline__ void begin_kernel() {
   cudaTriggerProgrammaticLaunchCompletion();
   cudaGridDependencySynchronize();

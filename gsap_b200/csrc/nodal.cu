@@ -119,12 +119,12 @@ struct Rows<true> {
   __device__ Rows(const NodalArgs& a, int r, int s)
       : orr(a.Md + (size_t)r * a.B), ors(a.Md + (size_t)s * a.B), irr(a.MTd + (size_t)r * a.B),
         irs(a.MTd + (size_t)s * a.B) {}
-  __device__ __forceinline__ uint32_t out_r(int c) const { return __ldg(orr + c); }
-  __device__ __forceinline__ uint32_t out_s(int c) const { return __ldg(ors + c); }
-  __device__ __forceinline__ uint32_t in_r(int c) const { return __ldg(irr + c); }
-  __device__ __forceinline__ uint32_t in_s(int c) const { return __ldg(irs + c); }
+  __device__ __forceinline__ uint32_t out_r(int c) const { return orr[c]; }
+  __device__ __forceinline__ uint32_t out_s(int c) const { return ors[c]; }
+  __device__ __forceinline__ uint32_t in_r(int c) const { return irr[c]; }
+  __device__ __forceinline__ uint32_t in_s(int c) const { return irs[c]; }
   __device__ __forceinline__ uint32_t out_at(bool row_s, int c) const {
-    return __ldg((row_s ? ors : orr) + c);
+    return (row_s ? ors : orr)[c];
   }
 };
 
@@ -580,13 +580,13 @@ __device__ __forceinline__ void row_counts(const NodalArgs& a, int row, const bo
   if constexpr (DENSE) {
 #pragma unroll
     for (int j = 0; j < E; ++j)
-      m[j] = want[j] ? __ldg((in[j] ? a.MTd : a.Md) + (size_t)row * a.B + c[j]) : 0u;
+      m[j] = want[j] ? (in[j] ? a.MTd : a.Md)[(size_t)row * a.B + c[j]] : 0u;
   } else {
     int32_t lo[E], hi[E], end[E];
 #pragma unroll
     for (int j = 0; j < E; ++j) {
-      lo[j] = want[j] ? __ldg((in[j] ? a.bip : a.bop) + row) : 0;
-      hi[j] = end[j] = want[j] ? __ldg((in[j] ? a.bie : a.boe) + row) : 0;
+      lo[j] = want[j] ? (in[j] ? a.bip : a.bop)[row] : 0;
+      hi[j] = end[j] = want[j] ? (in[j] ? a.bie : a.boe)[row] : 0;
     }
     bool go = true;
     while (go) {
@@ -594,7 +594,7 @@ __device__ __forceinline__ void row_counts(const NodalArgs& a, int row, const bo
       int32_t x[E];
 #pragma unroll
       for (int j = 0; j < E; ++j)
-        x[j] = lo[j] < hi[j] ? __ldg((in[j] ? a.bic : a.boc) + ((lo[j] + hi[j]) >> 1)) : 0;
+        x[j] = lo[j] < hi[j] ? (in[j] ? a.bic : a.boc)[(lo[j] + hi[j]) >> 1] : 0;
 #pragma unroll
       for (int j = 0; j < E; ++j) {
         if (lo[j] >= hi[j]) continue;
@@ -606,8 +606,8 @@ __device__ __forceinline__ void row_counts(const NodalArgs& a, int row, const bo
     }
 #pragma unroll
     for (int j = 0; j < E; ++j)
-      m[j] = lo[j] < end[j] && __ldg((in[j] ? a.bic : a.boc) + lo[j]) == c[j]
-                 ? __ldg((in[j] ? a.bin : a.bon) + lo[j])
+      m[j] = lo[j] < end[j] && (in[j] ? a.bic : a.boc)[lo[j]] == c[j]
+                 ? (in[j] ? a.bin : a.bon)[lo[j]]
                  : 0u;
   }
 }
@@ -704,7 +704,7 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
   if (ctl_stopped(a.ctl)) return;
 #pragma unroll
   for (int j = 0; j < 2; ++j)
-    if (ok[j]) c[j] = __ldg(a.part + c[j]);
+    if (ok[j]) c[j] = a.part[c[j]];
   const int r = a.part[v];
   P4 x{};
   if (!GIVEN) x = draw(a.seed, kRngNodalVertex, a.seq + ctl_itr(a.ctl) * a.seq_mul, (uint32_t)v);
@@ -760,7 +760,7 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, int i, bool act
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       want[j] = ok[j] && c[j] != r;
-      ld[j] = ok[j] ? __ldg((in[j] ? a.ld_out : a.ld_in) + c[j]) : 0.0;
+      ld[j] = ok[j] ? (in[j] ? a.ld_out : a.ld_in)[c[j]] : 0.0;
     }
     row_counts<DENSE, 2>(a, r, in, c, want, Mo);
     row_counts<DENSE, 2>(a, s, in, c, ok, Mt);
@@ -945,7 +945,7 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int k = tid + T * j;
-    if (ok[j]) c[j] = __ldg(a.part + c[j]);
+    if (ok[j]) c[j] = a.part[c[j]];
     key[j] = ok[j] ? (uint32_t)c[j] | (in[j] ? 0x80000000u : 0u) : 0xffffffffu;
     ord[j] = ok[j] ? (in[j] ? 1u << 30 : 0u) | (uint32_t)c[j] << 8 | (uint32_t)k : 0xffffffffu;
     sm.key[k] = key[j];
@@ -1003,7 +1003,7 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     want[j] = ok[j] && c[j] != r;
-    ld[j] = ok[j] ? __ldg((in[j] ? a.ld_out : a.ld_in) + c[j]) : 0.0;
+    ld[j] = ok[j] ? (in[j] ? a.ld_out : a.ld_in)[c[j]] : 0.0;
     if (c[j] == r) {
       atomicAdd(sm.cnt + (in[j] ? 2 : 0), w[j]);
       if (!in[j]) atomicAdd(sm.cnt + 4, 1u);
@@ -1213,13 +1213,13 @@ __device__ double delta_hashed_gen(const NodalArgs& a, int v, int r, int s, Hash
   logH = 0.0;
   uint32_t koR = 0, koS = 0, niR = 0, niS = 0;
   for (int k = t; k < no; k += G) {
-    int32_t c = __ldg(a.part + __ldg(a.oidx + o0 + k));
+    int32_t c = a.part[__ldg(a.oidx + o0 + k)];
     uint32_t w = __ldg(a.ow + o0 + k);
     koR += c == r ? w : 0u;
     koS += c == s ? w : 0u;
   }
   for (int k = t; k < ni; k += G) {
-    int32_t c = __ldg(a.part + __ldg(a.iidx + i0 + k));
+    int32_t c = a.part[__ldg(a.iidx + i0 + k)];
     uint32_t w = __ldg(a.iw + i0 + k);
     niR += c == r ? w : 0u;
     niS += c == s ? w : 0u;
@@ -1244,13 +1244,13 @@ __device__ double delta_hashed_gen(const NodalArgs& a, int v, int r, int s, Hash
       if (t == 0) *flag = 0;
       grp.sync();
       for (int k = t; k < n; k += G) {
-        int32_t c = __ldg(a.part + __ldg(idx + base + k));
+        int32_t c = a.part[__ldg(idx + base + k)];
         if (hclass(c, P) == pass && !hash_add(h, c, __ldg(wt + base + k), k)) *flag = 1;
       }
       grp.sync();
       if (*flag) return __longlong_as_double(0x7ff8000000000000ll);  // table overflow
       for (int k = t; k < n; k += G) {
-        int32_t c = __ldg(a.part + __ldg(idx + base + k));
+        int32_t c = a.part[__ldg(idx + base + k)];
         if (hclass(c, P) != pass) continue;
         const int slot = hash_find(h, c);
         const bool leader = h.first[slot] == k;
@@ -1276,7 +1276,7 @@ __device__ double delta_hashed_gen(const NodalArgs& a, int v, int r, int s, Hash
       for (int k = t; k < n; k += G) {
         const bool in = k >= no;
         const int j = in ? k - no : k;
-        const int32_t c = __ldg(a.part + __ldg((in ? a.iidx + i0 : a.oidx + o0) + j));
+        const int32_t c = a.part[__ldg((in ? a.iidx + i0 : a.oidx + o0) + j)];
         if (c == r || c == s || hclass(c, P) != pass) continue;
         if (!hash_add(h, c, __ldg((in ? a.iw + i0 : a.ow + o0) + j), k)) *flag = 1;
       }
@@ -1369,8 +1369,8 @@ struct HeavyEntries {
     unit = (uint64_t)args.kdo[v] + args.kdi[v] == (uint64_t)n;
   }
   __device__ __forceinline__ uint32_t key(int k) const {
-    return k < no ? (uint32_t)__ldg(a.part + __ldg(a.oidx + o0 + k))
-                  : (uint32_t)__ldg(a.part + __ldg(a.iidx + i0 + k - no)) | 0x80000000u;
+    return k < no ? (uint32_t)a.part[__ldg(a.oidx + o0 + k)]
+                  : (uint32_t)a.part[__ldg(a.iidx + i0 + k - no)] | 0x80000000u;
   }
   __device__ __forceinline__ uint32_t w(int k) const {
     return unit ? 1u : k < no ? __ldg(a.ow + o0 + k) : __ldg(a.iw + i0 + k - no);
@@ -1538,7 +1538,7 @@ __device__ void heavy_vertex(const NodalArgs& a, int i, const Group<kHeavyThread
         lead[u] = tab.first[sl] == at;
         kc[u] = tab.sum[sl];
         want[u] = ok[u] && c[u] != r;
-        ld[u] = ok[u] ? __ldg((dir ? a.ld_out : a.ld_in) + c[u]) : 0.0;
+        ld[u] = ok[u] ? (dir ? a.ld_out : a.ld_in)[c[u]] : 0.0;
       }
       row_counts<DENSE, U>(a, r, in, c, want, Mo);
       row_counts<DENSE, U>(a, s, in, c, ok, Mt);
@@ -1670,7 +1670,7 @@ __device__ void hub_vertex(const NodalArgs& a, int i, int& parity) {
         const uint32_t w = ok ? e.w(k) : 0u;
         const uint32_t sl = ok ? tab.find(key) : 0u;
         const bool want = ok && c != r;
-        const double ld = ok ? __ldg((in ? a.ld_out : a.ld_in) + c) : 0.0;
+        const double ld = ok ? (in ? a.ld_out : a.ld_in)[c] : 0.0;
         uint32_t Mo, Mt;
         row_counts<DENSE, 1>(a, r, &in, &c, &want, &Mo);
         row_counts<DENSE, 1>(a, s, &in, &c, &ok, &Mt);
