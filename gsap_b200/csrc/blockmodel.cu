@@ -271,7 +271,8 @@ constexpr int kBigCap = 12288;  // longest segment a CTA takes; longer ones go t
 // per segment (a match over its lanes, or a bitonic sort).  Longer segments
 // are listed for the kernels below.
 constexpr int kTileEntries = 2048, kTileMaxCap = 128;
-constexpr int kTileBlocks = 1 << 25;  // (column, index) in a word: 7 bits of index
+// (column, index) in a word: 7 bits of index, and no such word is the padding
+constexpr int kTileBlocks = (1 << 25) - 1;
 struct RbTileBody {
   using Args = RbArgs;
   static constexpr int kThreads = 256, kMinBlocks = 6;

@@ -132,3 +132,19 @@ def test_partition_of_a_graph_numbered_by_degree(sbp, orc):
     lab, rep_o, _ = orc.partition(g, seed=0)
     assert rep["B"] == rep_o["B"] and abs(rep["S"] - rep_o["S"]) <= 1e-9 * abs(rep_o["S"])
     assert sbp.evaluate(lab, g.partitions)[2] > 0.999
+
+
+def test_tile_word_of_the_last_block(sbp, monkeypatch):
+    # at 2^25 blocks the last column at the last place of the longest segment a
+    # tile takes would be the word of ones that pads a tile
+    monkeypatch.setenv("SBP_DENSE_MAX", "0")
+    monkeypatch.setenv("SBP_REBUILD_WARP_CAP", "128")
+    N = 1 << 25
+    dst = np.concatenate([np.arange(1, 128), [N - 1]]).astype(np.int32)
+    g = sbp.Graph.from_edges(N, np.zeros(128, np.int32), dst, None)
+    a = sbp.build_blockmodel(g, np.arange(N, dtype=np.int32), N)
+    assert np.array_equal(a["ocol"], dst) and (a["ocnt"] == 1).all()
+    assert a["optr"][0] == 0 and (a["optr"][1:] == 128).all()
+    assert np.array_equal(a["icol"], np.zeros(128)) and (a["icnt"] == 1).all()
+    assert np.array_equal(np.flatnonzero(np.diff(a["iptr"])), dst)
+    assert a["d_out"][0] == 128 and a["d_out"].sum() == 128 and (a["d_in"][dst] == 1).all()
