@@ -19,8 +19,9 @@
 //     the entry point must not be called on that device afterwards;
 //   * every call on a device shares the one array, and the array keeps the
 //     last call's contents: calls that overlap on the GPU (different
-//     streams, or work still running) race on it.  Each call leaves what must
-//     start at zero (the CTA ticket of the reduction) at zero.
+//     streams, or work still running) race on it and may give wrong values.
+//     The CTA ticket of the reduction wraps to zero by itself, so that calls
+//     that overlapped spoil no later call.
 #include "../../include/sbp.h"
 #include "common.cuh"
 
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(kStaticThreads) static_mdl_kernel(
     sc->sum[blockIdx.x] = acc.s;
     sc->err[blockIdx.x] = acc.e;
     __threadfence();
-    last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
+    last = atomicInc(&sc->ticket, gridDim.x - 1) == gridDim.x - 1;
   }
   __syncthreads();
   if (last && wid == 0) {
@@ -131,7 +132,6 @@ __global__ void __launch_bounds__(kStaticThreads) static_mdl_kernel(
     if (lane == 0) {
       *data_S = t.value();
       *S = model - t.value();
-      sc->ticket = 0u;
     }
   }
 }

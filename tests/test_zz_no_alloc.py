@@ -61,3 +61,36 @@ def test_mdl_device_static_rejects_too_many_blocks(sbp):
     with pytest.raises(sbp.SbpError, match="bad arguments"):
         sbp.mdl_device_static(10, 10, 4, z.data_ptr(), 0, z.data_ptr(), z.data_ptr(),
                               z.data_ptr(), d[0:1].data_ptr(), d[1:2].data_ptr(), 0)
+
+
+@pytest.mark.gpu
+def test_mdl_device_static_after_overlapping_calls(sbp):
+    # calls that overlap share the scratch and may give wrong values; a later
+    # call by itself must not
+    import torch
+    g = dcsbm("HH", 4000, seed=7)
+    B = 64
+    part = np.random.default_rng(5).integers(0, B, g.N).astype(np.int32)
+    part[:B] = np.arange(B)
+    S_ref, data_ref = sbp.mdl(g, part, B)
+    dev = _device_blockmodel(sbp, g, part, B)
+    out = torch.zeros(3, 2, dtype=torch.float64, device="cuda")
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+
+    def call(k, stream):
+        sbp.mdl_device_static(g.N, g.E, B, *[dev[x].data_ptr() for x in (
+            "optr", "ocol", "ocnt", "d_out", "d_in")], out[k, 0:1].data_ptr(),
+            out[k, 1:2].data_ptr(), stream.cuda_stream)
+
+    torch.cuda.synchronize()
+    for _ in range(500):
+        for k in range(2):
+            call(k, streams[k])
+    torch.cuda.synchronize()
+    for _ in range(3):
+        out[2].fill_(float("nan"))
+        call(2, torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        S, data_S = out[2].cpu().tolist()
+        assert abs(S - S_ref) <= REL * abs(S_ref), (S, S_ref)
+        assert abs(data_S - data_ref) <= REL * abs(data_ref), (data_S, data_ref)
