@@ -380,10 +380,14 @@ sbp_status job_upload(Job& J, const sbp_graph_csr* h) {
   SBP_CUDA(cudaMemcpyAsync(g.kdi, h->deg_in, 4 * (size_t)J.N, cudaMemcpyHostToDevice, st));
   ++g_launches;
   fill_src_kernel<<<(J.N + 255) / 256, 256, 0, st>>>(g.optr, J.N, g.osrc);
-  // weights are at least 1, so they all are 1 when they sum to E
-  uint64_t weight = 0;
-  for (int32_t v = 0; v < J.N; ++v) weight += h->deg_out[v];
-  g.unit = weight == (uint64_t)J.E ? 1 : 0;
+  // weights are at least 1, so a direction's all are 1 when its degrees sum to
+  // E; each direction is asked, since nothing requires the two to agree
+  uint64_t out = 0, in = 0;
+  for (int32_t v = 0; v < J.N; ++v) {
+    out += h->deg_out[v];
+    in += h->deg_in[v];
+  }
+  g.unit = out == (uint64_t)J.E && in == (uint64_t)J.E ? 1 : 0;
   J.h_optr.assign(h->out_ptr, h->out_ptr + J.N + 1);
   J.h_iptr.assign(h->in_ptr, h->in_ptr + J.N + 1);
   ++g_launches;
