@@ -31,11 +31,11 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <future>
 #include <map>
 #include <memory>
 #include <mutex>
 #include <system_error>
-#include <thread>
 
 namespace sbp {
 
@@ -58,16 +58,19 @@ void Run::setup_batches() {
     }
   };
   const int32_t T = (int32_t)std::max<int64_t>(1, std::min<int64_t>({8, nb, J->N / 16384}));
-  std::vector<std::thread> helpers;
+  // an exception of a share (memory) is the caller's: a future hands it on,
+  // and its destructor waits for the share
+  std::vector<std::future<void>> helpers;
   int32_t spawned = 1;
   try {
-    for (; spawned < T; ++spawned) helpers.emplace_back(classify, spawned, T);
+    for (; spawned < T; ++spawned)
+      helpers.push_back(std::async(std::launch::async, classify, spawned, T));
   } catch (const std::system_error&) {
     // no more threads: the remaining shares run here
   }
   for (int32_t t = spawned; t < T; ++t) classify(t, T);
   classify(0, T);
-  for (std::thread& x : helpers) x.join();
+  for (std::future<void>& x : helpers) x.get();
   for (int32_t b = 0; b < nb; ++b) list_off[b + 1] = list_off[b] + (int32_t)lists[b].size();
   lists_all.resize((size_t)list_off[nb]);
   for (int32_t b = 0; b < nb; ++b)
