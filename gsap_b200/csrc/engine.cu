@@ -545,6 +545,7 @@ sbp_status Engine::tick() {
   for (Slot* x : {&m_bt, &m_props, &m_delta, &m_delta8, &m_best}) order.push_back(x);
   for (Slot* x : m_apply.all()) order.push_back(x);
   order.push_back(&m_relabel);
+  const size_t sweep_first = order.size();
   for (int k = 0; k < k_max; ++k) {
     for (int b = 0; b < nb_max; ++b) {
       SweepSlots& w = sw[k * nb_max + b];
@@ -566,13 +567,21 @@ sbp_status Engine::tick() {
   // one-job slots packs and uploads nothing.
   bool multi = false;
   for (const Slot* x : order) multi = multi || x->njobs() > 1;
+  // The sweeps' records lie first, so that their offsets, and with them a
+  // captured graph's launches, are the same in a step's first tick, which has
+  // builds and copies before its sweeps, and in the ticks after it.
   size_t desc = 0;
   std::vector<size_t> off(order.size(), 0);
-  for (size_t i = 0; i < order.size() && multi; ++i) {
-    if (order[i]->empty()) continue;
-    off[i] = desc;
-    desc += align256(order[i]->recs.size()) + align256(4 * order[i]->cta0.size());
-  }
+  auto place = [&](size_t first, size_t last) {
+    for (size_t i = first; i < last && multi; ++i) {
+      if (order[i]->empty()) continue;
+      off[i] = desc;
+      desc += align256(order[i]->recs.size()) + align256(4 * order[i]->cta0.size());
+    }
+  };
+  place(sweep_first, order.size() - 1);
+  place(0, sweep_first);
+  place(order.size() - 1, order.size());  // the readback
   s = grow(desc, desc_cap, desc_host, desc_dev);
   if (s != SBP_OK) return s;
   for (size_t i = 0; i < order.size() && multi; ++i) {
@@ -632,7 +641,6 @@ sbp_status Engine::tick() {
   SBP_CUDA(cudaEventRecord(ev[2], st));
   // the queued sweeps; timing events are external records so that they
   // also time a replayed graph
-  const size_t sweep_first = i;
   bool capturing = false;
   auto record = [&](cudaEvent_t e) {
     return capturing ? cudaEventRecordWithFlags(e, st, cudaEventRecordExternal)
