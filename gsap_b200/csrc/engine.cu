@@ -744,10 +744,20 @@ sbp_status Engine::tick() {
     // A tick of several runs repeats only while none of them changes its
     // step, so it is captured when it comes a second time; captured at once,
     // every new mix of steps was a shape to instantiate (24 served requests
-    // seen for the first time: 490 ms, this way 237).
+    // seen for the first time: 490 ms, this way 237).  A run of sweeps only
+    // knows its ticks: it is captured when one comes a second time and a third
+    // will follow (captured at once, five sweeps of a 200k graph took 13.3 ms on
+    // a graph not seen before and 9.8 on one that was; issued, 8.6 and 8.2).
     int active = 0;
-    for (Run* r : runs) active += r->stage != Run::kDone ? 1 : 0;
-    const bool again = active == 1 || (shape == last_shape && key == last_key);
+    bool steps = true, more = true;
+    for (Run* r : runs) {
+      active += r->stage != Run::kDone ? 1 : 0;
+      if (!r->sweeps_only) continue;
+      steps = false;
+      more = r->sweeps_total - r->itr >= 2 * r->sweep_k;
+    }
+    const bool again =
+        (active == 1 && steps) || (more && shape == last_shape && key == last_key);
     last_shape = shape;
     last_key = key;
     const bool replay = sg && sg->exec && sg->key == key;
@@ -984,6 +994,8 @@ sbp_status Engine::tick() {
 void Engine::reset() {
   runs.clear();
   ticks = 0;
+  last_key.clear();  // the next call's first tick repeats none
+  last_shape.clear();
   if (ev_first) cudaEventDestroy(ev_first);
   ev_first = nullptr;
 }
