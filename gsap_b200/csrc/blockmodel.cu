@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 namespace sbp {
@@ -529,24 +530,40 @@ struct RbRankBody {
 // by a cluster of eight CTAs, each with an eighth of the entries.  Each CTA
 // marks its entries' columns, merges an eighth of the eight bitmaps through
 // distributed shared memory and hands the merged words and their running
-// counts to all; the totals are then added in place.  One CTA for such a
-// segment took 157 us of every rebuild of the 200k HH graph, and up to 1.1 ms;
-// the cluster 17 us (at most 48).
+// counts to all; the totals are then added in place, or (few columns) in
+// shared memory first.  One CTA for such a segment took 157 us of every
+// rebuild of the 200k HH graph, and up to 1.1 ms; the cluster 17 us (at most
+// 48).
+// Where many segments are that long the clusters take their turns, and a CTA
+// each is faster as long as none of them takes much more than its share of the
+// whole; a CTA can where the columns' totals fit its shared memory (at most
+// kBigCap blocks).  A rebuild of 200k vertices of degree 10 in B even blocks,
+// clusters only with all totals in place / now: B = 150 212 / 115 us, B = 71
+// 174 / 106, B = 32 146 / 106, B = 2 550 / 196.
 constexpr int kBigThreads = 512, kBigCluster = 8;
 constexpr int kBigWords = 4096;  // bitmap words of a window (131072 columns)
 constexpr size_t kBigSmem = (size_t)(2 * kBigWords + kBigCap) * 4;
 static_assert(kBigCap >= kBigWords, "the giant path's third array of words");
+constexpr int kCtaShare = 768;
 struct RbBigBody {
   using Args = RbArgs;
   static constexpr int kThreads = kBigThreads, kMinBlocks = 2, kCluster = kBigCluster;
   static constexpr size_t kSmem = kBigSmem;
+
+  // The columns of a bitmap word from place `at` on.
+  // Where a window's entries are many to a column, its columns are written
+  // this way, once each; else by the entries, which is faster then.
+  static __device__ __forceinline__ void write_columns(uint32_t m, int col0, int32_t* bcol,
+                                                       int at) {
+    for (; m; m &= m - 1) bcol[at++] = col0 + __ffs((int)m) - 1;
+  }
 
   static __device__ void big_row(const RbArgs& a, const RbSide& d, int b, uint32_t* bm,
                                  uint32_t* pre, uint32_t* cnt, int* sh, int& nnz) {
     constexpr int T = kBigThreads, kPer = kBigWords / T;
     const int tid = threadIdx.x;
     const int base = d.bptr[b], n = d.bptr[b + 1] - base;
-    for (int i = tid; i < n; i += T) cnt[i] = 0u;
+    for (int i = tid; i < min(n, a.B); i += T) cnt[i] = 0u;
     int u = 0;
     for (int w0 = 0; w0 < a.B; w0 += 32 * kBigWords) {
       const int cols = min(32 * kBigWords, a.B - w0), nw = (cols + 31) >> 5;
@@ -566,21 +583,27 @@ struct RbBigBody {
       }
       int tot;
       int run = cta_excl_scan(nz, sh, &tot);
+      const bool many = n > 4LL * tot;
       for (int j = 0; j < per && j < kPer; ++j) {
         const int x = tid * per + j;
         if (x >= nw) break;
         pre[x] = (uint32_t)run;
+        if (many) write_columns(bm[x], w0 + 32 * x, d.bcol + base + u, run);
         run += __popc(bm[x]);
       }
       __syncthreads();
+      auto add = [&](auto by_entry) {
 #pragma unroll 4
-      for (int i = tid; i < n; i += T) {
-        const int c = d.tcol[base + i] - w0;
-        if ((unsigned)c >= (unsigned)cols) continue;
-        const int at = u + (int)pre[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u));
-        atomicAdd(cnt + at, a.unit ? 1u : d.tw[base + i]);
-        d.bcol[base + at] = c + w0;
-      }
+        for (int i = tid; i < n; i += T) {
+          const int c = d.tcol[base + i] - w0;
+          if ((unsigned)c >= (unsigned)cols) continue;
+          const int at = u + (int)pre[c >> 5] + __popc(bm[c >> 5] & ((1u << (c & 31)) - 1u));
+          atomicAdd(cnt + at, a.unit ? 1u : d.tw[base + i]);
+          if (by_entry) d.bcol[base + at] = c + w0;
+        }
+      };
+      if (many) add(std::false_type{});
+      else add(std::true_type{});
       u += tot;
       __syncthreads();
     }
@@ -638,22 +661,49 @@ struct RbBigBody {
       if (tid < C) cl.map_shared_rank(tots, tid)[q] = (uint32_t)tot;
       cl.sync();
       uint32_t first[C];  // distinct columns before each segment of words
-      uint32_t run = (uint32_t)u;
+      uint32_t run = (uint32_t)u, own = 0u;
 #pragma unroll
       for (int p = 0; p < C; ++p) {
         first[p] = run;
+        if (p == q) own = run;
         run += tots[p];
       }
-      for (int i = e0 + tid; i < e1; i += T) {
-        const int c = d.tcol[base + i] - w0;
-        if ((unsigned)c >= (unsigned)cols) continue;
-        const int word = c >> 5, sg = word / seg;
-        uint32_t f = first[0];
+      // the totals of a window's few distinct columns are added up in shared
+      // memory first: the entries of a row of few columns, all added in place,
+      // queue at the same few words
+      const int distinct = (int)run - u;
+      const bool many = n > 4LL * distinct;
+      if (many && mine) write_columns(m, w0 + 32 * x, d.bcol + base, (int)own + ex);
+      const bool local = distinct <= kBigCap - kBigWords;
+      uint32_t* const sum = pre + kBigWords;
+      auto add = [&](auto by_entry, auto in_shared) {
+#pragma unroll 4
+        for (int i = e0 + tid; i < e1; i += T) {
+          const int c = d.tcol[base + i] - w0;
+          if ((unsigned)c >= (unsigned)cols) continue;
+          const int word = c >> 5, sg = word / seg;
+          uint32_t f = first[0];
 #pragma unroll
-        for (int p = 1; p < C; ++p) f = sg == p ? first[p] : f;
-        const int at = (int)(f + pre[word]) + __popc(merged[word] & ((1u << (c & 31)) - 1u));
-        atomicAdd(d.bcnt + base + at, a.unit ? 1u : d.tw[base + i]);
-        d.bcol[base + at] = c + w0;
+          for (int p = 1; p < C; ++p) f = sg == p ? first[p] : f;
+          const int at = (int)(f + pre[word]) + __popc(merged[word] & ((1u << (c & 31)) - 1u));
+          const uint32_t w = a.unit ? 1u : d.tw[base + i];
+          if (in_shared) atomicAdd(sum + at - u, w);
+          else atomicAdd(d.bcnt + base + at, w);
+          if (by_entry) d.bcol[base + at] = c + w0;
+        }
+      };
+      if (local) {
+        for (int i = tid; i < distinct; i += T) sum[i] = 0u;
+        __syncthreads();
+        if (many) add(std::false_type{}, std::true_type{});
+        else add(std::true_type{}, std::true_type{});
+        __syncthreads();
+        for (int i = tid; i < distinct; i += T)
+          if (sum[i]) atomicAdd(d.bcnt + base + u + i, sum[i]);
+      } else if (many) {
+        add(std::false_type{}, std::false_type{});
+      } else {
+        add(std::true_type{}, std::false_type{});
       }
       u = (int)run;
     }
@@ -699,8 +749,14 @@ struct RbBigBody {
     const int dir = cluster & 1, ci = cluster >> 1;
     const RbSide& d = a.s[dir];
     const int nbig = d.nlist[1], ngiant = d.nlist[2];
+    // giants a CTA takes: of up to kCtaShare entries a giant there is
+    const int cta_max = a.B <= kBigCap ? kCtaShare * ngiant : 0;
+    const auto len = [&](int b) { return d.bptr[b + 1] - d.bptr[b]; };
     int nnz = 0;
-    for (int k = ci; k < ngiant; k += nc) giant_row(a, d, d.giant[k], w1, w2, w3, tots, sh, nnz);
+    for (int k = ci; k < ngiant; k += nc)
+      if (len(d.giant[k]) > cta_max) giant_row(a, d, d.giant[k], w1, w2, w3, tots, sh, nnz);
+    for (int k = ci * kBigCluster + rank; k < ngiant; k += nc * kBigCluster)
+      if (len(d.giant[k]) <= cta_max) big_row(a, d, d.giant[k], w1, w2, w3, sh, nnz);
     for (int k = ci * kBigCluster + rank; k < nbig; k += nc * kBigCluster)
       big_row(a, d, d.big[k], w1, w2, w3, sh, nnz);
     if (dir == 0 && threadIdx.x == 0 && nnz) atomicAdd(a.nnz, nnz);

@@ -148,3 +148,32 @@ def test_tile_word_of_the_last_block(sbp, monkeypatch):
     assert np.array_equal(a["icol"], np.zeros(128)) and (a["icnt"] == 1).all()
     assert np.array_equal(np.flatnonzero(np.diff(a["iptr"])), dst)
     assert a["d_out"][0] == 128 and a["d_out"].sum() == 128 and (a["d_in"][dst] == 1).all()
+
+
+@pytest.mark.parametrize("weighted", [False, True], ids=["unit", "weighted"])
+@pytest.mark.parametrize("B", [300, 9000, 12288, 12289])
+def test_many_long_segments(sbp, orc, monkeypatch, B, weighted):
+    # twenty blocks of some 15k entries (a CTA each up to 12288 blocks, else a
+    # cluster), one of 30k (a cluster); their columns few, and about and above
+    # the 8192 whose totals a cluster adds up in shared memory
+    monkeypatch.setenv("SBP_DENSE_MAX", "0")
+    rng = np.random.default_rng(B)
+    size = np.concatenate([np.full(20, 2000), [4300], np.ones(B - 21, np.int64)])
+    size[21:] += np.bincount(rng.integers(0, B - 21, 13000 - (B - 21)), minlength=B - 21)
+    N = int(size.sum())
+    p = np.repeat(np.arange(B, dtype=np.int32), size)
+    first = np.cumsum(size) - size
+    b = rng.integers(0, B, 7 * N)
+    u, v = np.repeat(np.arange(N), 7), first[b] + rng.integers(0, size[b])
+    src, dst = np.concatenate([u, v]).astype(np.int32), np.concatenate([v, u]).astype(np.int32)
+    order = rng.permutation(N).astype(np.int32)  # a block's vertices lie apart
+    w = rng.integers(1, 6, src.size).astype(np.uint32) if weighted else None
+    g = sbp.Graph.from_edges(N, order[src], order[dst], w)
+    lab = np.empty(N, np.int32)
+    lab[order] = p
+    n = np.bincount(lab, weights=np.diff(g.out_ptr), minlength=B)
+    giants = int((n > 12288).sum())
+    assert giants >= 21 and n.max() > 768 * giants > np.sort(n)[-2]
+    a, o = sbp.build_blockmodel(g, lab, B), orc.build_blockmodel(g, lab, B)
+    for k in ("optr", "ocol", "ocnt", "iptr", "icol", "icnt", "d_out", "d_in"):
+        assert np.array_equal(a[k], o[k]), k
