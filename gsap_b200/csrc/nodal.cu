@@ -1040,11 +1040,14 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
     lead[1] = false;
     pos[0] = tid;
     pos[1] = tid + T;
-  } else if (unit && a.B <= kOrdBlocks) {
-    // equal weights: the order is (direction, block, entry), a word per entry,
-    // and a block's total the length of its run in that order (the loop over
+  } else if (a.B <= kOrdBlocks) {
+    // the order by (direction, block, entry) is that of one word per entry; in
+    // it a block's entries are a run.  With equal weights it is the order
+    // wanted, and a block's total the length of its run; otherwise its run is
+    // walked for the total and for the entries of less weight.  (The loop over
     // pairs with weights, below, set the launch time: 20k HH partitions 43.4 ms
-    // with it, 37.8 this way)
+    // with it, 37.8 this way; a weighted sweep of 30k vertices of 150 entries
+    // 0.93 and 0.58 ms.)
     int rank[2] = {0, 0};
 #pragma unroll 4
     for (int b = 0; b < n; b += 4) {  // idle slots come last
@@ -1054,16 +1057,34 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
         rank[j] += (g.x < ord[j] ? 1 : 0) + (g.y < ord[j] ? 1 : 0) + (g.z < ord[j] ? 1 : 0) +
                    (g.w < ord[j] ? 1 : 0);
     }
-    uint32_t* const run = sm.w;  // the keys in order (the weights are all 1)
+    // the keys in order, then the weights (unless all are 1), where the terms
+    // will go
+    uint32_t* const run = reinterpret_cast<uint32_t*>(sm.t1);
+    uint32_t* const runw = run + 2 * T;
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
-      if (ok[j]) run[rank[j]] = key[j];
+    for (int j = 0; j < 2; ++j) {
+      if (!ok[j]) continue;
+      run[rank[j]] = key[j];
+      if (!unit) runw[rank[j]] = w[j];
+    }
     sync();
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      pos[j] = rank[j];
       lead[j] = ok[j] && (rank[j] == 0 || run[rank[j] - 1] != key[j]);
-      if (lead[j]) kc[j] = (uint32_t)(upper_bound(run, rank[j], n, key[j]) - rank[j]);
+      pos[j] = rank[j];
+      if (unit) {
+        if (lead[j]) kc[j] = (uint32_t)(upper_bound(run, rank[j], n, key[j]) - rank[j]);
+      } else if (ok[j]) {
+        int lo = rank[j], less = 0;
+        while (lo > 0 && run[lo - 1] == key[j]) --lo;
+        for (int q = lo; q < n && run[q] == key[j]; ++q) {
+          const uint32_t u = runw[q];
+          kc[j] += u;
+          less += u < w[j] || (u == w[j] && q < rank[j]) ? 1 : 0;
+        }
+        lead[j] = less == 0;
+        pos[j] = lo + less;
+      }
       if constexpr (GEN) {
         if (a.mh && lead[j]) {
           const uint32_t other = key[j] ^ 0x80000000u;
@@ -1071,6 +1092,10 @@ __device__ void large_vertex(const NodalArgs& a, int i, LargeBuf<T, GEN>& sm) {
           const int k1 = upper_bound(run, lo, hi, other);
           const int k0 = other == 0u ? lo : upper_bound(run, lo, hi, other - 1u);
           kany[j] = kc[j] + (uint32_t)(k1 - k0);
+          if (!unit) {
+            kany[j] = kc[j];
+            for (int q = k0; q < k1; ++q) kany[j] += runw[q];
+          }
           outside[j] = in[j] && k1 > k0;
         }
       }

@@ -113,3 +113,30 @@ def test_dense_update_edges(sbp, weighted, B, batches):
             for d in (0, N))
     assert (a[0] != p).any()
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+# log of a ratio of two FP64 sums of positive terms
+LOGH_TOL = 1e-9
+
+
+@pytest.mark.parametrize("B", [2, 40, 3000])
+@pytest.mark.parametrize("dmax", ["0", "4096"], ids=["csr", "dense"])
+def test_path_edges_general_mode(sbp, orc, monkeypatch, dmax, B):
+    # every path's edges with mixed weights, exact dS and Hastings ratio: long
+    # runs of one block (B = 2) and blocks met once
+    monkeypatch.setenv("SBP_DENSE_MAX", dmax)
+    g = shaped_graph(sbp, True)
+    rng = np.random.default_rng(B)
+    p = rng.integers(0, B, N).astype(np.int32)
+    p[-B:] = np.arange(B, dtype=np.int32)
+    K = len(SHAPES)
+    verts = np.tile(np.arange(K, dtype=np.int32), 8)
+    props = rng.integers(0, B, verts.size).astype(np.int32)
+    src, dst, _ = g.edges()
+    for i, v in enumerate(verts):
+        near = dst[src == v] if i % 3 == 0 else src[dst == v]
+        if i % 3 < 2 and near.size:
+            props[i] = p[near[rng.integers(near.size)]]
+    got, lh = sbp.delta_mdl_nodal_mode(g, p, B, verts, props, exact=1)
+    want, lh_o = orc.nodal_delta_exact(g, p, B, verts, props)
+    assert close(got, want).all() and (np.abs(lh - lh_o) <= LOGH_TOL).all()
