@@ -551,8 +551,6 @@ struct RbBigBody {
   static constexpr size_t kSmem = kBigSmem;
 
   // The columns of a bitmap word from place `at` on.
-  // Where a window's entries are many to a column, its columns are written
-  // this way, once each; else by the entries, which is faster then.
   static __device__ __forceinline__ void write_columns(uint32_t m, int col0, int32_t* bcol,
                                                        int at) {
     for (; m; m &= m - 1) bcol[at++] = col0 + __ffs((int)m) - 1;
@@ -583,6 +581,7 @@ struct RbBigBody {
       }
       int tot;
       int run = cta_excl_scan(nz, sh, &tot);
+      // columns from the bitmap where the entries are many to a column
       const bool many = n > 4LL * tot;
       for (int j = 0; j < per && j < kPer; ++j) {
         const int x = tid * per + j;
@@ -669,14 +668,13 @@ struct RbBigBody {
         run += tots[p];
       }
       // the totals of a window's few distinct columns are added up in shared
-      // memory first: the entries of a row of few columns, all added in place,
-      // queue at the same few words
+      // memory first, and the columns written from the bitmap: the entries of
+      // a row of few columns, all of them done in place, queue at the same few
+      // words
       const int distinct = (int)run - u;
-      const bool many = n > 4LL * distinct;
-      if (many && mine) write_columns(m, w0 + 32 * x, d.bcol + base, (int)own + ex);
       const bool local = distinct <= kBigCap - kBigWords;
       uint32_t* const sum = pre + kBigWords;
-      auto add = [&](auto by_entry, auto in_shared) {
+      auto add = [&](auto in_shared) {
 #pragma unroll 4
         for (int i = e0 + tid; i < e1; i += T) {
           const int c = d.tcol[base + i] - w0;
@@ -687,23 +685,24 @@ struct RbBigBody {
           for (int p = 1; p < C; ++p) f = sg == p ? first[p] : f;
           const int at = (int)(f + pre[word]) + __popc(merged[word] & ((1u << (c & 31)) - 1u));
           const uint32_t w = a.unit ? 1u : d.tw[base + i];
-          if (in_shared) atomicAdd(sum + at - u, w);
-          else atomicAdd(d.bcnt + base + at, w);
-          if (by_entry) d.bcol[base + at] = c + w0;
+          if (in_shared) {
+            atomicAdd(sum + at - u, w);
+          } else {
+            atomicAdd(d.bcnt + base + at, w);
+            d.bcol[base + at] = c + w0;
+          }
         }
       };
       if (local) {
+        if (mine) write_columns(m, w0 + 32 * x, d.bcol + base, (int)own + ex);
         for (int i = tid; i < distinct; i += T) sum[i] = 0u;
         __syncthreads();
-        if (many) add(std::false_type{}, std::true_type{});
-        else add(std::true_type{}, std::true_type{});
+        add(std::true_type{});
         __syncthreads();
         for (int i = tid; i < distinct; i += T)
           if (sum[i]) atomicAdd(d.bcnt + base + u + i, sum[i]);
-      } else if (many) {
-        add(std::false_type{}, std::false_type{});
       } else {
-        add(std::true_type{}, std::false_type{});
+        add(std::false_type{});
       }
       u = (int)run;
     }
@@ -749,6 +748,7 @@ struct RbBigBody {
     const int dir = cluster & 1, ci = cluster >> 1;
     const RbSide& d = a.s[dir];
     const int nbig = d.nlist[1], ngiant = d.nlist[2];
+    if (nbig + ngiant == 0) return;  // the same in every thread of the cluster
     // giants a CTA takes: of up to kCtaShare entries a giant there is
     const int cta_max = a.B <= kBigCap ? kCtaShare * ngiant : 0;
     const auto len = [&](int b) { return d.bptr[b + 1] - d.bptr[b]; };
