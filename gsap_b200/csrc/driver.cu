@@ -627,6 +627,7 @@ void classify_batch(const Job& J, const int32_t* verts, int32_t lo, int32_t coun
     cls[i] = heavy_vertex(J, v) ? 2 : e <= kSmallEntries ? 0 : 1;
     ++n[cls[i]];
     if (cls[i] == 1 && e > kGroupEntries / 2) ++n[e > kGroupEntries ? 3 : 4];
+    if (cls[i] == 1 && e > kWideEntries) ++n[6];
     if (cls[i] == 2 && e > kHubEntries) ++n[5];
     if (cls[i] < 2) emax = std::max(emax, e);
   }
@@ -656,6 +657,7 @@ NodalAux nodal_lists(Job& J, const int32_t* dev, const int32_t n[kListCounts]) {
   a.mid = dev + n[0];
   a.nmid = n[1];
   a.nlarge = n[3];
+  a.nlong = n[6];
   a.nmid64 = n[4];
   a.heavy = dev + n[0] + n[1];
   a.nheavy = n[2];

@@ -135,8 +135,9 @@ bool heavy_vertex(const Job& J, int32_t v);
 // Appends the batch indices i in [0, count) of vertices lo + i (verts[i]
 // when verts is given) to `out`, grouped by nodal kernel path: small, mid,
 // heavy (NodalAux); n receives the three group sizes, the mid list's counts of
-// large vertices and of those of up to kGroupEntries entries, and the hubs.
-constexpr int kListCounts = 6;
+// large vertices and of those of up to kGroupEntries entries, the hubs, and the
+// large vertices of more than kWideEntries entries.
+constexpr int kListCounts = 7;
 void classify_batch(const Job& J, const int32_t* verts, int32_t lo, int32_t count,
                     std::vector<int32_t>& out, int32_t n[kListCounts]);
 // The NodalAux of groups of such sizes stored back to back at `dev`.

@@ -357,15 +357,16 @@ int nodal_heavy_threshold();
 // A batch's vertices (indices into the batch) by kernel path: small ones (at
 // most kSmallEntries neighbour entries), mid ones, and heavy ones (more than
 // nodal_heavy_threshold() entries in a direction), on a side stream; the first
-// nhub of these have more than kHubEntries entries in all.  The mid list runs from the most entries down: the first nlarge
-// have more than kGroupEntries, the next nmid64 more than kGroupEntries / 2.
-// err counts hash-table overflows (should stay 0).
-constexpr int32_t kSmallEntries = 16, kGroupEntries = 64, kHubEntries = 1024;
+// nhub of these have more than kHubEntries entries in all.  The mid list runs
+// from the most entries down: the first nlarge have more than kGroupEntries
+// (nlong of them more than kWideEntries), the next nmid64 more than
+// kGroupEntries / 2.  err counts hash-table overflows (should stay 0).
+constexpr int32_t kSmallEntries = 16, kGroupEntries = 64, kWideEntries = 128, kHubEntries = 1024;
 struct NodalAux {
   const int32_t* small = nullptr;
   int32_t nsmall = 0;
   const int32_t* mid = nullptr;
-  int32_t nmid = 0, nlarge = 0, nmid64 = 0;
+  int32_t nmid = 0, nlarge = 0, nlong = 0, nmid64 = 0;
   const int32_t* heavy = nullptr;
   int32_t nheavy = 0, nhub = 0;
   int32_t* err = nullptr;

@@ -76,7 +76,7 @@ struct NodalArgs {
   const int32_t *small, *mid;  // batch indices of the warp kernel (NodalItems)
   int32_t nsmall, nmid;
   int32_t unit;                // every weight is 1
-  int32_t nlarge, nmid64;      // mid vertices by size: large, up to kGroupEntries, the others
+  int32_t nlarge, nwide, nmid64;  // mid vertices by path: a CTA, wide_vertex, 32 lanes, the others
   int32_t* err;             // error counter (hash table overflow)
   const int32_t* ctl;       // sweep control: gate, and seq += ctl[0] * seq_mul
   uint32_t seq_mul;
@@ -1316,15 +1316,177 @@ __device__ double delta_hashed_gen(const NodalArgs& a, int v, int r, int s, Hash
   return finish_gen<DENSE, G>(a, R, v, r, s, rw, self, q, hs, grp, logH);
 }
 
+// A vertex of kGroupEntries to kWideEntries entries on a warp, four entries a
+// lane: the terms and sums of large_vertex (by index), with fewer instructions
+// and a longer chain.  A batch of more such vertices than the GPU holds CTAs is
+// bound by instructions, one of fewer by the chain.  buf: 512 words of the
+// warp's shared memory.
+template <bool GIVEN, bool DENSE>
+__device__ void wide_vertex(const NodalArgs& a, int i, int lane, uint32_t* buf) {
+  constexpr int S = kWideEntries / 32;
+  const int v = GIVEN ? a.verts[i] : a.lo + i;
+  const int32_t o0 = a.optr[v], no = a.optr[v + 1] - o0;
+  const int32_t i0 = a.iptr[v], ni = a.iptr[v + 1] - i0;
+  const int n = no + ni;
+  int32_t c[S];
+  uint32_t w[S];
+#pragma unroll
+  for (int j = 0; j < S; ++j) {
+    const int k = lane + 32 * j;
+    const bool in = k >= no;
+    const int e = in ? k - no : k;
+    c[j] = -1;  // the neighbour, then its block
+    w[j] = 0u;
+    if (k < n) {
+      c[j] = __ldg((in ? a.iidx + i0 : a.oidx + o0) + e);
+      w[j] = a.unit ? 1u : __ldg((in ? a.iw + i0 : a.ow + o0) + e);
+    }
+  }
+  const uint64_t deg = (uint64_t)a.kdo[v] + a.kdi[v];
+  wait_kernel();
+  if (ctl_stopped(a.ctl)) return;
+  uint32_t* const skey = buf;
+  uint32_t* const sw = buf + kWideEntries;
+  bool light = true;
+#pragma unroll
+  for (int j = 0; j < S; ++j) {
+    const int k = lane + 32 * j;
+    if (k < n) c[j] = a.part[c[j]];
+    // direction in the top bit; idle slots match no entry
+    skey[k] = k < n ? (uint32_t)c[j] | (k >= no ? 0x80000000u : 0u) : 0xffffffffu;
+    sw[k] = w[j];
+    light = light && w[j] <= 1u;
+  }
+  const int r = a.part[v];
+  const bool unit = __all_sync(kFull, light);
+  __syncwarp();
+  int s;
+  if (GIVEN) {
+    s = a.props_in[i];
+  } else {
+    const P4 x = draw(a.seed, kRngNodalVertex, a.seq + ctl_itr(a.ctl) * a.seq_mul, (uint32_t)v);
+    const int rnd = (int)(x.v[0] % (uint32_t)a.B);
+    const uint64_t t = scale_draw(x.v[1], deg);
+    int at = (int)t;
+    if (!unit) {  // the first entry whose running weight exceeds t
+      at = -1;
+      uint64_t acc = 0;
+      for (int k0 = 0; k0 < n && at < 0; k0 += 32) {
+        uint64_t incl = sw[k0 + lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint64_t y = __shfl_up_sync(kFull, incl, o);
+          if (lane >= o) incl += y;
+        }
+        const unsigned hit = __ballot_sync(kFull, k0 + lane < n && acc + incl > t);
+        if (hit) at = k0 + __ffs(hit) - 1;
+        acc += __shfl_sync(kFull, incl, 31);
+      }
+    }
+    s = proposed(a, at >= 0 ? (int)(skey[at] & 0x7fffffffu) : a.part[0], rnd);
+  }
+  double d = 0.0;
+  if (r != s) {  // the same in every lane
+    // the counts first: the table below is built while they are on their way
+    uint32_t Mo[S], Mt[S];
+    bool in[S], ok[S], want[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const int k = lane + 32 * j;
+      in[j] = k >= no;
+      ok[j] = k < n;
+      want[j] = ok[j] && c[j] != r;
+    }
+    row_counts<DENSE, S>(a, r, in, c, want, Mo);
+    row_counts<DENSE, S>(a, s, in, c, ok, Mt);
+    const uint32_t mm =
+        lane < 4 ? Rows<DENSE>(a, r, s).out_at((lane & 2) != 0, (lane & 1) ? s : r) : 0u;
+    // v's weights to and from r and s, and its out-entries there
+    uint32_t oR = 0u, oS = 0u, iR = 0u, iS = 0u, nR = 0u, nS = 0u;
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const bool in = lane + 32 * j >= no, hr = c[j] == r, hs = c[j] == s;
+      oR += hr && !in ? w[j] : 0u;
+      oS += hs && !in ? w[j] : 0u;
+      iR += hr && in ? w[j] : 0u;
+      iS += hs && in ? w[j] : 0u;
+      nR += hr && !in ? 1u : 0u;
+      nS += hs && !in ? 1u : 0u;
+    }
+    const RsWeights rw{__reduce_add_sync(kFull, oR), __reduce_add_sync(kFull, oS),
+                       __reduce_add_sync(kFull, iR), __reduce_add_sync(kFull, iS)};
+    nR = __reduce_add_sync(kFull, nR);
+    nS = __reduce_add_sync(kFull, nS);
+    // each entry's block by a table from key to one of its entries, and there
+    // the block's total and first entry
+    uint32_t* const tab = buf + 2 * kWideEntries;
+    auto fill = [&](uint32_t x, uint32_t y) {
+      *reinterpret_cast<uint4*>(tab + 4 * lane) = make_uint4(x, x, x, x);
+      *reinterpret_cast<uint4*>(tab + kWideEntries + 4 * lane) = make_uint4(y, y, y, y);
+      __syncwarp();
+    };
+    fill(~0u, ~0u);
+    int own[S];
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const int k = lane + 32 * j;
+      own[j] = k;
+      if (k >= n) continue;
+      const uint32_t key = skey[k];
+      for (uint32_t q = key * 2654435761u >> 24;; q = (q + 1) & (2 * kWideEntries - 1)) {
+        const uint32_t cur = atomicCAS(tab + q, ~0u, (uint32_t)k);
+        if (cur != ~0u) own[j] = (int)cur;
+        if (cur == ~0u || skey[cur] == key) break;  // at most half the slots fill
+        own[j] = k;
+      }
+    }
+    __syncwarp();
+    fill(0u, ~0u);
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const int k = lane + 32 * j;
+      if (k >= n) continue;
+      atomicAdd(tab + own[j], w[j]);
+      atomicMin(tab + kWideEntries + own[j], (uint32_t)k);
+    }
+    __syncwarp();
+    double acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      if (32 * j >= n) break;
+      const bool lead = tab[kWideEntries + own[j]] == (uint32_t)(lane + 32 * j);
+      const double ld = ok[j] ? (in[j] ? a.ld_out : a.ld_in)[c[j]] : 0.0;
+      double t1, t2;
+      entry_terms(a.xlx, ok[j], in[j], c[j], w[j], lead, tab[own[j]], Mo[j], Mt[j], ld, r, s,
+                  rw.niS, t1, t2);
+      acc -= t1;
+      acc -= t2;
+    }
+    Corner q;
+    load_degrees(a, v, r, s, q);
+    q.Mrr = __shfl_sync(kFull, mm, 0);
+    q.Mrs = __shfl_sync(kFull, mm, 1);
+    q.Msr = __shfl_sync(kFull, mm, 2);
+    q.Mss = __shfl_sync(kFull, mm, 3);
+    const RowChange m = row_change(q, rw, nR, nS);
+    acc += corner_term<true, true>(a.xlx, q, rw, m.m4, m.m5, m.m6, m.m7, lane);
+    d = warp_sum(acc);
+  }
+  if (lane == 0) write_result(a, GIVEN, i, r, s, d);
+  __syncwarp();
+}
+
 // Work items of the warp kernel, larger vertices first (as the host lists
 // them: a longest-first schedule): a CTA per large vertex, then a warp per
-// vertex of up to 64 entries, per two of up to 32 and per four small ones.
+// vertex that wide_vertex takes and per vertex of up to 64 entries, per two of
+// up to 32 and per four small ones.
 struct NodalItems {
-  int large, mid64, mid32, small;  // large in CTAs, the others in warps
-  __host__ __device__ NodalItems(int nlarge, int nmid64, int nmid32, int nsmall)
-      : large(nlarge), mid64(nmid64), mid32((nmid32 + 1) / 2), small((nsmall + 3) / 4) {}
+  int large, wide, mid64, mid32, small;  // large in CTAs, the others in warps
+  __host__ __device__ NodalItems(const NodalArgs& a)
+      : large(a.nlarge), wide(a.nwide), mid64(a.nmid64),
+        mid32((a.nmid - a.nlarge - a.nwide - a.nmid64 + 1) / 2), small((a.nsmall + 3) / 4) {}
   __host__ __device__ int ctas() const {
-    return large + (mid64 + mid32 + small + kNodalWarps - 1) / kNodalWarps;
+    return large + (wide + mid64 + mid32 + small + kNodalWarps - 1) / kNodalWarps;
   }
 };
 
@@ -1337,25 +1499,33 @@ struct NodalBody {
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
     using Large = LargeBuf<kThreads, GEN>;
-    // per warp: the keys and weights of group_vertex, or (general mode) a
-    // 33-64-entry vertex's LargeBuf
+    // per warp: the keys and weights of wide_vertex and group_vertex, or
+    // (general mode) a 33-64-entry vertex's LargeBuf
     using Mid = LargeBuf<32, GEN>;
-    constexpr size_t kWarpBytes = GEN ? (sizeof(Mid) + 15) / 16 * 16 : 128 * sizeof(uint32_t);
+    constexpr size_t kWarpBytes =
+        GEN ? (sizeof(Mid) + 15) / 16 * 16 : 4 * kWideEntries * sizeof(uint32_t);
     constexpr size_t kBytes =
         sizeof(Large) > kNodalWarps * kWarpBytes ? sizeof(Large) : kNodalWarps * kWarpBytes;
     __shared__ __align__(16) unsigned char raw[kBytes];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     unsigned char* const own = raw + kWarpBytes * wid;
     uint32_t* const buf = reinterpret_cast<uint32_t*>(own);
-    const int nmid32 = a.nmid - a.nlarge - a.nmid64;
-    const NodalItems n(a.nlarge, a.nmid64, nmid32, a.nsmall);
-    const int32_t *mid64 = a.mid + a.nlarge, *mid32 = mid64 + a.nmid64;
+    const NodalItems n(a);
+    const int nmid32 = a.nmid - a.nlarge - a.nwide - a.nmid64;
+    const int32_t *wide = a.mid + a.nlarge, *mid64 = wide + a.nwide, *mid32 = mid64 + a.nmid64;
     for (int blk = vb; blk < n.ctas(); blk += vg) {
       if (blk < n.large) {
         large_vertex<GIVEN, DENSE, GEN, kThreads>(a, a.mid[blk], *reinterpret_cast<Large*>(raw));
         continue;
       }
       int it = (blk - n.large) * kNodalWarps + wid;
+      if constexpr (!GEN) {  // general mode has none
+        if (it < n.wide) {
+          wide_vertex<GIVEN, DENSE>(a, wide[it], lane, buf);
+          continue;
+        }
+        it -= n.wide;
+      }
       if (it < n.mid64) {
         if constexpr (GEN)
           large_vertex<GIVEN, DENSE, GEN, 32>(a, mid64[it], *reinterpret_cast<Mid*>(own));
@@ -1954,9 +2124,19 @@ CommitArgs commit_args(int32_t* part, int32_t lo, int32_t count, const int32_t* 
   return a;
 }
 
+// Vertices of kGroupEntries to kWideEntries entries go to wide_vertex where a
+// batch has more than kWideMin of them, the CTAs that the GPU holds at once.
+// Dense sweeps of four batches of vertices of 80 entries, B = 1000, a CTA each /
+// this way: 1000 a batch 0.096 / 0.117 ms, 2000 0.123 / 0.120, 4000 0.170 /
+// 0.125, 16000 0.452 / 0.267.
+constexpr int32_t kWideMin = 8 * 148;
+
 NodalArgs make_args(const DevGraph& g, const int32_t* part, const DevBM& m, int32_t B,
-                    const NodalAux& aux) {
+                    const NodalAux& aux, const ScoreMode& md) {
   NodalArgs a{};
+  a.exact = md.exact;
+  a.mh = md.mh;
+  a.beta = md.beta;
   a.xlx = m.xlx;
   a.optr = g.optr; a.oidx = g.oidx; a.iptr = g.iptr; a.iidx = g.iidx;
   a.ow = g.ow; a.iw = g.iw; a.kdo = g.kdo; a.kdi = g.kdi;
@@ -1976,7 +2156,8 @@ NodalArgs make_args(const DevGraph& g, const int32_t* part, const DevBM& m, int3
   a.nsmall = aux.nsmall;
   a.mid = aux.mid;
   a.nmid = aux.nmid;
-  a.nlarge = aux.nlarge;
+  a.nwide = !md.general() && aux.nlarge - aux.nlong > kWideMin ? aux.nlarge - aux.nlong : 0;
+  a.nlarge = aux.nlarge - a.nwide;
   a.nmid64 = aux.nmid64;
   a.err = aux.err;
   return a;
@@ -1984,7 +2165,7 @@ NodalArgs make_args(const DevGraph& g, const int32_t* part, const DevBM& m, int3
 
 // CTAs of the warp kernel.
 int32_t nodal_ctas(const NodalArgs& a) {
-  return NodalItems(a.nlarge, a.nmid64, a.nmid - a.nlarge - a.nmid64, a.nsmall).ctas();
+  return NodalItems(a).ctas();
 }
 
 template <bool GIVEN, bool DENSE, bool GEN>
@@ -2025,11 +2206,6 @@ const MultiKernel kmNodalHeavy[4] = {
 const MultiKernel kmNodalHub[2] = {multi_kernel_desc<NodalHubBody<false, false>>("nodal_hub_csr"),
                                    multi_kernel_desc<NodalHubBody<false, true>>("nodal_hub_dense")};
 
-void set_mode(NodalArgs& a, const ScoreMode& md) {
-  a.exact = md.exact;
-  a.mh = md.mh;
-  a.beta = md.beta;
-}
 const MultiKernel kmCommit = multi_kernel_desc<CommitBody>("commit");
 
 }  // namespace
@@ -2058,8 +2234,7 @@ void nodal_batch_sample(const DevGraph& g, const int32_t* part, const DevBM& m, 
                         bool dense, uint64_t seed, uint32_t seq, int32_t lo, int32_t count,
                         int32_t* newlab, double* rec, int32_t* props, const NodalAux& aux,
                         cudaStream_t st, const ScoreMode& md) {
-  NodalArgs a = make_args(g, part, m, B, aux);
-  set_mode(a, md);
+  NodalArgs a = make_args(g, part, m, B, aux, md);
   a.seed = seed;
   a.seq = seq;
   a.lo = lo;
@@ -2076,8 +2251,7 @@ void nodal_delta_given(const DevGraph& g, const int32_t* part, const DevBM& m, i
                        bool dense, int32_t nv, const int32_t* verts, const int32_t* props,
                        double* dS, const NodalAux& aux, cudaStream_t st, const ScoreMode& md,
                        double* logH) {
-  NodalArgs a = make_args(g, part, m, B, aux);
-  set_mode(a, md);
+  NodalArgs a = make_args(g, part, m, B, aux, md);
   a.count = nv;
   a.verts = verts;
   a.props_in = props;
@@ -2102,7 +2276,7 @@ void add_nodal(Slot& warp, Slot& heavy, Slot& hub, bool dense, const ScoreMode& 
                int32_t* newlab, double* rec, int32_t* props, const NodalAux& aux,
                const int32_t* ctl, uint32_t seq_mul) {
   if (count <= 0) return;
-  NodalArgs a = make_args(g, part, m, B, aux);
+  NodalArgs a = make_args(g, part, m, B, aux, md);
   a.seed = seed;
   a.seq = seq;
   a.lo = lo;
@@ -2112,7 +2286,6 @@ void add_nodal(Slot& warp, Slot& heavy, Slot& hub, bool dense, const ScoreMode& 
   a.props_out = props;
   a.ctl = ctl;
   a.seq_mul = seq_mul;
-  set_mode(a, md);
   slot_push(slot_bind(warp, kmNodal[md.slot(dense)]), a, nodal_ctas(a));
   const int32_t nhub = md.general() ? 0 : aux.nhub;
   slot_push(slot_bind(heavy, kmNodalHeavy[md.slot(dense)]), a, aux.nheavy - nhub);

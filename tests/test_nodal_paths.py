@@ -140,3 +140,38 @@ def test_path_edges_general_mode(sbp, orc, monkeypatch, dmax, B):
     got, lh = sbp.delta_mdl_nodal_mode(g, p, B, verts, props, exact=1)
     want, lh_o = orc.nodal_delta_exact(g, p, B, verts, props)
     assert close(got, want).all() and (np.abs(lh - lh_o) <= LOGH_TOL).all()
+
+
+@pytest.mark.parametrize("weighted", [False, True], ids=["unit", "weighted"])
+@pytest.mark.parametrize("B", [3, 200, 5000])
+@pytest.mark.parametrize("dmax", ["0", "4096"], ids=["csr", "dense"])
+def test_many_wide_vertices(sbp, orc, monkeypatch, dmax, B, weighted):
+    # more vertices of 65 to 128 entries in a batch than take a CTA each: a warp
+    # each, every count of entries, all out, all in and mixed, few blocks (many
+    # entries of one block) and many
+    monkeypatch.setenv("SBP_DENSE_MAX", dmax)
+    total = np.resize(np.arange(65, 129), 1600)
+    out = np.where(np.arange(1600) % 4 == 0, total,
+                   np.where(np.arange(1600) % 4 == 1, 0, total * (np.arange(1600) % 7) // 6))
+    monkeypatch.setattr("test_nodal_paths.SHAPES", list(zip(out, total - out)))
+    g = shaped_graph(sbp, weighted)
+    rng = np.random.default_rng(B)
+    p = rng.integers(0, B, N).astype(np.int32)
+    p[-B:] = np.arange(B, dtype=np.int32)
+    verts = np.arange(1600, dtype=np.int32)
+    props = rng.integers(0, B, 1600).astype(np.int32)
+    props[::3] = p[g.out_idx[g.out_ptr[verts[::3]] % g.E]]  # blocks of some neighbours
+    got = sbp.delta_mdl_nodal(g, p, B, verts, props)
+    want, mag = orc.nodal_delta_scale(g, p, B, verts, props)
+    # at B = 3 cells of 17,000: FP64 rounding of the row sums (mag) passes REL
+    ok = close(got, want) | (np.abs(got - want) <= 1e-12 * mag)
+    assert ok.all(), (verts[~ok], got[~ok], want[~ok], mag[~ok])
+    # the same bits as on a CTA each: the batch in parts below the limit
+    parts = [sbp.delta_mdl_nodal(g, p, B, verts[i:i + 400], props[i:i + 400])
+             for i in range(0, 1600, 400)]
+    assert np.array_equal(got.view(np.int64), np.concatenate(parts).view(np.int64))
+    pa, da, xa, _ = sbp.nodal_batch(g, p, B, 21, 4, 0, 1600)
+    pb, db, xb, _ = orc.nodal_batch(g, p, B, 21, 4, 0, 1600)
+    assert np.array_equal(xa, xb), "proposals differ"
+    _, mag = orc.nodal_delta_scale(g, p, B, verts, xb)
+    assert (close(da, db) | (np.abs(da - db) <= 1e-12 * mag)).all()
