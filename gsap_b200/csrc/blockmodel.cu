@@ -918,7 +918,7 @@ struct DenseArgs {
   // direction), and the vertices a warp covers
   const int32_t* heavy;
   int32_t N, E, B, lo, count, nheavy, heavy_min, per_warp;
-  int32_t unit, pad;
+  int32_t unit, combine;  // combine: chunk sums over a warp's lanes first (dense_move_apply)
 };
 
 // Chunk sums of a dense cell (r, c): out-row r's chunk of column c and
@@ -1109,6 +1109,7 @@ struct DenseMove {
 struct DenseCells {
   int32_t r0, c0, r1, c1;
   uint32_t w;  // 0: nothing to do
+  bool in;
 };
 __device__ __forceinline__ DenseCells dense_move_load(const DenseArgs& a, const DenseMove& v,
                                                       int e) {
@@ -1121,21 +1122,63 @@ __device__ __forceinline__ DenseCells dense_move_load(const DenseArgs& a, const 
   const int bn = x >= lo && x < lo + count ? a.newlab[x - lo] : bo;
   // an in-edge of a moved source is the source's
   return DenseCells{in ? bo : v.r, in ? v.r : bo, in ? bo : v.s, in ? v.s : bn,
-                    in && bn != bo ? 0u : wt};
+                    in && bn != bo ? 0u : wt, in};
 }
 
+// The whole warp calls it.  In few blocks the chunk sums are few words that
+// every entry of every moved vertex adds to, and that is what a launch takes:
+// there the sums at the vertex's own blocks r and s are added up over the
+// warp's lanes first, and those at the entry's block, whose change is 0 where r
+// and s lie in one chunk, left out.  A launch over 16000 vertices of 24 entries
+// that all move, entry by entry / this way: B = 20 319 / 72 us, 50 229 / 84, 130
+// 90 / 62, 300 38 / 34, 1000 26 / 26 (and 18 / 20 with fewer moves).  It lengthens
+// the chain of a small batch, where nothing queues: weighted 5k partitions 43 /
+// 46 ms, so batches of a few thousand vertices go entry by entry.
+constexpr int kDuCombine = 512;
+template <bool COMBINE>
 __device__ __forceinline__ void dense_move_apply(const DenseArgs& a, const DenseCells& m) {
-  if (m.w == 0u) return;
   const int32_t B = a.B;
   const int K = (B + 31) >> 5;
+  const bool on = m.w != 0u;
+  const unsigned act = COMBINE ? __ballot_sync(kFull, on) : 0u;
+  if (!on) return;
   atomicSub(a.Md + (size_t)m.r0 * B + m.c0, m.w);
   atomicSub(a.MTd + (size_t)m.c0 * B + m.r0, m.w);
   atomicAdd(a.Md + (size_t)m.r1 * B + m.c1, m.w);
   atomicAdd(a.MTd + (size_t)m.c1 * B + m.r1, m.w);
-  atomicSub(sd_out(a.Sd, K, m.r0, m.c0), m.w);
-  atomicSub(sd_in(a.Sd, K, m.r0, m.c0), m.w);
-  atomicAdd(sd_out(a.Sd, K, m.r1, m.c1), m.w);
-  atomicAdd(sd_in(a.Sd, K, m.r1, m.c1), m.w);
+  uint32_t *const o0 = sd_out(a.Sd, K, m.r0, m.c0), *const i0 = sd_in(a.Sd, K, m.r0, m.c0);
+  uint32_t *const o1 = sd_out(a.Sd, K, m.r1, m.c1), *const i1 = sd_in(a.Sd, K, m.r1, m.c1);
+  if constexpr (COMBINE) {
+    uint32_t *const e0 = m.in ? o0 : i0, *const e1 = m.in ? o1 : i1;
+    if (e0 != e1) {
+      atomicSub(e0, m.w);
+      atomicAdd(e1, m.w);
+    }
+    const int lane = threadIdx.x & 31;
+    auto add = [&](uint32_t* p, bool minus) {
+      const unsigned peers = __match_any_sync(act, (unsigned)(p - a.Sd));
+      const uint32_t w = a.unit ? (uint32_t)__popc(peers) : __reduce_add_sync(peers, m.w);
+      if (__ffs(peers) - 1 == lane) atomicAdd(p, minus ? 0u - w : w);
+    };
+    add(m.in ? i0 : o0, true);
+    add(m.in ? i1 : o1, false);
+  } else {
+    atomicSub(o0, m.w);
+    atomicSub(i0, m.w);
+    atomicAdd(o1, m.w);
+    atomicAdd(i1, m.w);
+  }
+}
+
+template <int U>
+__device__ __forceinline__ void dense_move_apply_all(const DenseArgs& a, const DenseCells* c) {
+  if (a.combine) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) dense_move_apply<true>(a, c[u]);
+  } else {
+#pragma unroll
+    for (int u = 0; u < U; ++u) dense_move_apply<false>(a, c[u]);
+  }
 }
 
 __device__ __forceinline__ void dense_move_degrees(const DenseArgs& a, int v, int r, int s) {
@@ -1162,15 +1205,15 @@ struct DenseUpdateBody {
       if (threadIdx.x == 0) dense_move_degrees(a, v, m.r, m.s);
       constexpr int U = 4;
       const int n = m.no + m.ni;
-      for (int e = threadIdx.x; e < n; e += U * kThreads) {
+      for (int e0 = threadIdx.x & ~31; e0 < n; e0 += U * kThreads) {
         DenseCells c[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
+          const int e = e0 + lane + u * kThreads;
           c[u].w = 0u;
-          if (e + u * kThreads < n) c[u] = dense_move_load(a, m, e + u * kThreads);
+          if (e < n) c[u] = dense_move_load(a, m, e);
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) dense_move_apply(a, c[u]);
+        dense_move_apply_all<U>(a, c);
       }
       return;
     }
@@ -1219,8 +1262,7 @@ struct DenseUpdateBody {
         c[h].w = 0u;
         if (e < total) c[h] = dense_move_load(a, u, e - first);
       }
-#pragma unroll
-      for (int h = 0; h < 2; ++h) dense_move_apply(a, c[h]);
+      dense_move_apply_all<2>(a, c);
     }
   }
 };
@@ -1539,6 +1581,7 @@ void set_update(DenseArgs& a, int32_t lo, int32_t count, const int32_t* newlab,
   a.nheavy = lists.nheavy;
   a.heavy_min = nodal_heavy_threshold();
   a.per_warp = std::max(1, std::min(kDuVerts, count / (148 * 16)));
+  a.combine = a.B <= kDuCombine && a.per_warp > 1 ? 1 : 0;
 }
 int32_t vg_dense_update(const DenseArgs& a) {
   return a.nheavy + ceil_div(a.count, DenseUpdateBody::kThreads / 32 * a.per_warp);

@@ -175,3 +175,16 @@ def test_many_wide_vertices(sbp, orc, monkeypatch, dmax, B, weighted):
     assert np.array_equal(xa, xb), "proposals differ"
     _, mag = orc.nodal_delta_scale(g, p, B, verts, xb)
     assert (close(da, db) | (np.abs(da - db) <= 1e-12 * mag)).all()
+
+
+@pytest.mark.parametrize("weighted", [False, True], ids=["unit", "weighted"])
+@pytest.mark.parametrize("B", [31, 32, 64, 65, 512, 513])
+def test_dense_update_in_few_blocks(sbp, weighted, B):
+    # the chunk sums of the dense form added up over a warp (large batches, up to
+    # 512 blocks) or entry by entry: draws read them, so the labels would differ
+    g = shaped_graph(sbp, weighted)
+    p = np.random.default_rng(B).integers(0, B, N).astype(np.int32)
+    p[-B:] = np.arange(B, dtype=np.int32)
+    a, b = (sbp.nodal_sweeps(g, p, B, 7, 2, num_batches=2, sweeps=4, dense_max=d) for d in (0, N))
+    assert (a[0] != p).sum() > 10
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
