@@ -539,12 +539,12 @@ struct RbRankBody {
 // whole; a CTA can where the columns' totals fit its shared memory (at most
 // kBigCap blocks).  A rebuild of 200k vertices of degree 10 in B even blocks,
 // clusters only with all totals in place / now: B = 150 212 / 115 us, B = 71
-// 174 / 106, B = 32 146 / 106, B = 2 550 / 196.
+// 174 / 106, B = 50 127 / 99 (share 768 / 1024), B = 32 146 / 106, B = 2 550 / 196.
 constexpr int kBigThreads = 512, kBigCluster = 8;
 constexpr int kBigWords = 4096;  // bitmap words of a window (131072 columns)
 constexpr size_t kBigSmem = (size_t)(2 * kBigWords + kBigCap) * 4;
 static_assert(kBigCap >= kBigWords, "the giant path's third array of words");
-constexpr int kCtaShare = 768;
+constexpr int kCtaShare = 1024;
 struct RbBigBody {
   using Args = RbArgs;
   static constexpr int kThreads = kBigThreads, kMinBlocks = 2, kCluster = kBigCluster;

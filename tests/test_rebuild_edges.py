@@ -173,7 +173,7 @@ def test_many_long_segments(sbp, orc, monkeypatch, B, weighted):
     lab[order] = p
     n = np.bincount(lab, weights=np.diff(g.out_ptr), minlength=B)
     giants = int((n > 12288).sum())
-    assert giants >= 21 and n.max() > 768 * giants > np.sort(n)[-2]
+    assert giants >= 21 and n.max() > 1024 * giants > np.sort(n)[-2]
     a, o = sbp.build_blockmodel(g, lab, B), orc.build_blockmodel(g, lab, B)
     for k in ("optr", "ocol", "ocnt", "iptr", "icol", "icnt", "d_out", "d_in"):
         assert np.array_equal(a[k], o[k]), k
