@@ -12,10 +12,11 @@
 // A tick gathers the device work of every active Run and issues it as
 // multi-job launches: one launch per kernel body covers all jobs that need
 // it (multi.cuh), so a tick costs about the same number of launches for one
-// job as for hundreds.  Argument records and heavy-vertex lists go up in two
-// host-to-device copies per tick, every result the host needs (new block
-// counts, sweep sums, MDL terms, final labels) comes back in one
-// device-to-host copy, and the host synchronises once per tick.
+// job as for hundreds.  The argument records of launches over several jobs go
+// up in one host-to-device copy per tick (and a new run's batch lists in one of
+// their own), every result the host needs (new block counts, sweep sums, MDL
+// terms, final labels) comes back in one device-to-host copy, and the host
+// synchronises once per tick.
 //
 // sbp_partition is a batch of one.  sbp_partition_batch and the server
 // (server.cu) admit jobs against an HBM budget as earlier jobs finish.
@@ -705,8 +706,8 @@ sbp_status Engine::tick() {
     }
     return SBP_OK;
   };
-  // A tick's queued sweeps are one CUDA graph: their launches and arguments
-  // repeat tick after tick within an outer step (RNG sequence and result
+  // A tick's queued sweeps are one CUDA graph where it will be replayed: their
+  // launches and arguments repeat tick after tick within an outer step (RNG sequence and result
   // slots come from the device-side sweep control), so they are captured
   // once, in the step's first tick behind its builds and copies, and
   // replayed; a changed step (new B) updates the graph of its shape in place.

@@ -7,9 +7,10 @@
 //
 // Here a group of threads owns one vertex: 8, 16 or 32 lanes for vertices of
 // up to 16, 32 or 64 neighbour entries (two entries a lane), a CTA of four
-// warps for up to kWarpList entries a direction, a larger CTA for the few
-// heavier ones (run on a second stream next to the warp kernel).  The host
-// sorts each batch's vertices into these lists once per job.
+// warps for up to kWarpList entries a direction (or, up to kWideEntries in all
+// and many to a batch, a warp), a larger CTA or a cluster for the few heavier
+// ones (run on streams of their own next to the warp kernel).  The host sorts
+// each batch's vertices into these lists once per job.
 //   * proposal: Philox draws, an exact integer inverse-CDF pick of a
 //     neighbour (out- then in-entries; with unit weights the drawn number is
 //     the entry's index, else a prefix scan), then the per-block draws of the
