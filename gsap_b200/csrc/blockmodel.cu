@@ -1189,9 +1189,11 @@ __device__ __forceinline__ void dense_move_degrees(const DenseArgs& a, int v, in
   atomicAdd(a.d_in + s, i);
 }
 
+// Four CTAs an SM (64 registers, no spills): at the 90 that the multi-job kernel
+// takes otherwise, two, 24 served requests took 195 ms, this way 186.
 struct DenseUpdateBody {
   using Args = DenseArgs;
-  static constexpr int kThreads = 256, kMinBlocks = 1;
+  static constexpr int kThreads = 256, kMinBlocks = 4;
   static constexpr size_t kSmem = 0;
   static __device__ void run(const Args& a, int vb, int vg) {
     if (ctl_stopped(a.ctl)) return;
